@@ -258,6 +258,10 @@ int mmoe_forward_ep(const MmoeGeometry* geo, void* workspace, const void* const*
 int mmoe_transform_weights(const void* w_in, void* w_out, const int32_t* sf_in, int32_t* sf_out, int32_t num_groups,
                            int32_t rows, int32_t k_packed_bytes, int32_t k_words, int32_t interleave, void* stream);
 
+/* Two-slice copy of `num_groups` row-major matrices (`localize`, backend/locality.py:573-587): the two row halves of
+ * matrix g, `half_bytes` each and adjacent in `src`, go to `dst + g * half_bytes` and `dst + slice_stride + g * half_bytes`. */
+int mmoe_split_halves(const void* src, void* dst, int32_t num_groups, int64_t half_bytes, int64_t slice_stride, void* stream);
+
 /* Copy the device status words to the host (synchronises the stream), clear them on the device and translate them:
  * MMOE_OK, MMOE_ERR_DEVICE_TIMEOUT (a bounded wait expired: the outputs of that call are not valid) or
  * MMOE_ERR_INVALID_ARGUMENT (expert ids >= num_experts were seen and treated as masked).  The words are sticky until

@@ -57,3 +57,13 @@ def test_native_transform_matches_reference_golden_vectors():
     assert torch.equal(t13.cpu(), torch.from_numpy(g["t13"]))
     assert torch.equal(t13sf.cpu(), torch.from_numpy(g["t13sf"]))
     assert torch.equal(t2sf.cpu(), torch.from_numpy(g["t2sf"]))
+
+
+@pytest.mark.parametrize("shape", [(1, 2, 16), (3, 256, 128), (2, 6, 16), (1, 64, 16400), (4, 2, 8)])
+def test_device_localize_equals_host_localize(shape):
+    """Halves of one vector, less than / exactly / more than a 16 KB piece, and one too short for the vector copy."""
+    from vllm_plugin_b200.backend.locality import localize
+
+    t = torch.randint(-128, 128, shape, dtype=torch.int8)
+    host, dev = localize(t), localize(t.cuda())
+    assert dev.stride() == host.stride() and torch.equal(dev.cpu(), host)

@@ -31,7 +31,7 @@ EXPORTED_SYMBOLS = (
     "mmoe_last_error", "mmoe_abi_version", "mmoe_set_tuning", "mmoe_route_order_noalloc", "mmoe_ep_dispatch", "mmoe_ep_return",
     "mmoe_experts_ep_return", "mmoe_forward_ep", "mmoe_transform_weights",
     "mmoe_plan_shared", "mmoe_experts_select", "mmoe_route_stage_inputs", "mmoe_stage_inputs_nvfp4",
-    "mmoe_combine_residual",
+    "mmoe_combine_residual", "mmoe_split_halves",
 )
 
 
@@ -109,6 +109,7 @@ def load() -> ctypes.CDLL:
     lib.mmoe_plan_shared.argtypes = [geo_p, vp, i32, i32, vp]
     lib.mmoe_experts_select.argtypes = [geo_p, vp, ctypes.POINTER(MmoeWeights), ctypes.POINTER(MmoeOptions), i32, i32, i32, vp]
     lib.mmoe_transform_weights.argtypes = [vp, vp, vp, vp, i32, i32, i32, i32, i32, vp]
+    lib.mmoe_split_halves.argtypes = [vp, vp, i32, ctypes.c_int64, ctypes.c_int64, vp]
     lib.mmoe_experts_ep_return.argtypes = [geo_p, vp, ctypes.POINTER(vp), ctypes.POINTER(MmoeWeights),
                                            ctypes.POINTER(MmoeOptions), i32, i32, vp]
     lib.mmoe_route_order_noalloc.argtypes = [vp, i32, i32, i32, vp, vp, vp, vp, vp]

@@ -63,6 +63,15 @@ def localize(t: torch.Tensor, dim: int = -2) -> torch.Tensor:
         acc *= s
     contiguous_strides.reverse()
     out = torch.as_strided(flat, [2] + half_shape, [stride_e] + contiguous_strides)
+    half_bytes = t.element_size() * half_shape[-2] * half_shape[-1] if t.dim() >= 2 else 0
+    if t.is_cuda and dim == t.dim() - 2 and numel > 0 and t.is_contiguous() and half_bytes % 16 == 0 and t.data_ptr() % 16 == 0:
+        # device tensors: one HBM-bound kernel (a strided copy of a byte tensor moves one byte per thread)
+        from . import _native
+        with torch.cuda.device(t.device):
+            _native.check(_native.load().mmoe_split_halves(
+                t.data_ptr(), out.data_ptr(), t.element_size() * numel // half_bytes, half_bytes, stride_b,
+                torch.cuda.current_stream(t.device).cuda_stream))
+        return out
     halves = t.split(n // 2, dim=dim)
     out[0].copy_(halves[0])
     out[1].copy_(halves[1])

@@ -657,6 +657,19 @@ int mmoe_transform_weights(const void* w_in, void* w_out, const int32_t* sf_in, 
   return e == cudaSuccess ? MMOE_OK : cuda_fail(e, "weight transform launch");
 }
 
+int mmoe_split_halves(const void* src, void* dst, int32_t num_groups, int64_t half_bytes, int64_t slice_stride, void* stream) {
+  if (num_groups <= 0 || half_bytes <= 0 || half_bytes % 16 != 0)
+    return fail(MMOE_ERR_INVALID_ARGUMENT, "split: num_groups=%d must be positive and a half (%lld bytes) a positive multiple of 16 bytes",
+                num_groups, (long long)half_bytes);
+  if (slice_stride < num_groups * half_bytes || slice_stride % 16 != 0)
+    return fail(MMOE_ERR_INVALID_ARGUMENT, "split: the slice stride must hold every group's half and be a multiple of 16 bytes");
+  if (src == nullptr || dst == nullptr || src == dst) return fail(MMOE_ERR_INVALID_ARGUMENT, "split: pointers must be distinct and non-NULL");
+  if ((reinterpret_cast<uintptr_t>(src) & 15u) != 0 || (reinterpret_cast<uintptr_t>(dst) & 15u) != 0)
+    return fail(MMOE_ERR_INVALID_ARGUMENT, "split: pointers must be 16-byte aligned");
+  cudaError_t e = mmoe::launch_split_halves(src, dst, num_groups, half_bytes, slice_stride, static_cast<cudaStream_t>(stream));
+  return e == cudaSuccess ? MMOE_OK : cuda_fail(e, "two-slice copy launch");
+}
+
 int mmoe_read_status(const MmoeGeometry* geo, void* workspace, int32_t* words8, void* stream) {
   mmoe::Ctx c;
   int rc = make_ctx(geo, workspace, &c);

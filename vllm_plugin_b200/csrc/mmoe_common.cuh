@@ -265,6 +265,7 @@ int route_order_static_max_experts();
 cudaError_t launch_interleave_rows(const void* src, void* dst, int groups, int rows, int row_bytes, cudaStream_t s);
 cudaError_t launch_scale_layout(const int32_t* src, int32_t* dst, int groups, int rows, int row_stride, int kwords,
                                 int interleave, cudaStream_t s);
+cudaError_t launch_split_halves(const void* src, void* dst, int groups, int64_t half_bytes, int64_t slice_stride, cudaStream_t s);
 int ep_sync_bytes();
 int ep_totals_offset();                      // byte offset of the [32][32] route-total table inside the ep_sync region
 cudaError_t launch_ep_signal_return(const Ctx& c, const void* const* peer_ws, int64_t timeout_ns, cudaStream_t s);
