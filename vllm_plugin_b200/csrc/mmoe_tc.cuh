@@ -167,6 +167,14 @@ struct Waiter {
     if ((threadIdx.x & 31) == 0) ok = wait(bar, parity);
     return __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
   }
+  // wait of a role that the whole warp walks in step (its copies and tensor-core instructions come from one elected
+  // lane): every lane suspends on the barrier -- one broadcast request -- and a vote keeps the outcome warp-uniform
+  __device__ __forceinline__ bool wait_uniform(uint32_t bar, uint32_t parity) {
+    for (uint32_t spin = 0;; ++spin) {
+      if (__any_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+      if ((spin & 63u) == 63u && __any_sync(0xffffffffu, abandoned())) return false;
+    }
+  }
   // true when the call is being abandoned: another role gave up, or this wait has used up the budget (recorded)
   __device__ __forceinline__ bool abandoned() {
     if (*abort_flag != 0) return true;

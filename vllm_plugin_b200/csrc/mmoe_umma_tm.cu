@@ -25,11 +25,12 @@
 //   warp 1     MMA issuer: per stage one barrier probe, 4 UMMAs, one commit
 //   warps 2-5  epilogue
 //
-// Every tcgen05 instruction costs its issuing thread about 50 clk, so the one thread that feeds the tensor pipe issues
-// nothing but the UMMAs and the commit (measured: with the three scale copies and a whole-warp barrier probe in the
-// same loop a stage took 510 clk of issue against 384 clk of tensor work).  The scale columns are per pipeline stage
-// (12 of the 128 TMEM columns the two accumulators leave free), so the copier runs ahead of the issuer like the
-// producers do.
+// Copies and tensor-core instructions are issued by one elected lane of a warp that walks its loop in step (all lanes wait,
+// elect.sync around the issue): operands then stay in uniform registers.  From a lane that alone runs the loop every tcgen05
+// instruction pays for moving its operands there -- 4 UMMAs, a commit and a barrier probe took 563 clk per stage in that
+// form and take 434 in this one (384 is the tensor work), GEMM1 of 48 experts x 480 rows 485 -> 430 us.  The scale columns
+// are per pipeline stage (12 of the 128 TMEM columns the two accumulators leave free), so the copier runs ahead of the
+// issuer like the producers do.
 //
 // CTA pairs (kCtas = 2, `tcgen05.mma.cta_group::2`, M = 256): two token tiles of the same expert share one task.  Each
 // CTA stages its own token tile and HALF of the task's weight rows (96), the pair's tensor cores read both halves; the
@@ -207,7 +208,7 @@ __global__ void __launch_bounds__(kTmThreads, 1) tm_kernel(const __grid_constant
   uint8_t* b_base = a_base + S::kStages * S::kABytes;
   uint8_t* sf_base = b_base + S::kStages * S::kBBytes;
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   const uint32_t cta = kCtas == 2 ? cluster_ctarank() : 0u;      // 0 = leader
   const bool leader = cta == 0;
   const int unit = blockIdx.x / kCtas, num_units = gridDim.x / kCtas;   // a unit = one CTA or one CTA pair
@@ -258,7 +259,7 @@ __global__ void __launch_bounds__(kTmThreads, 1) tm_kernel(const __grid_constant
   __syncthreads();
   if (kCtas == 2) cluster_sync_all();       // the peer's barriers are initialised before anything arrives on them
   tc_fence_after();
-  const uint32_t tmem_base = ctl->tmem_base;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, ctl->tmem_base, 0);
   PlanView pv = plan_view(const_cast<char*>(p.plan), p.e_local, p.num_ranks);
   const Tile* tiles = pv.tiles + (p.tile_select == 2 ? p.early_shared_first : 0);
   const int num_tiles = p.tile_select == 2
@@ -283,7 +284,7 @@ __global__ void __launch_bounds__(kTmThreads, 1) tm_kernel(const __grid_constant
   // of a task and consumed at the bottom: its latency hides behind the task instead of stalling the next one.
   if (warp == 0) {
     // --------------------------------------------------------------------------------------------- tile producer
-    if (lane == 0) {
+    {
       uint32_t stage = 0, phase = 0;
       const uint32_t a0 = smem_u32(a_base), b0 = smem_u32(b_base);
       bool ok = true;
@@ -308,11 +309,14 @@ __global__ void __launch_bounds__(kTmThreads, 1) tm_kernel(const __grid_constant
         const uint32_t tx = (box_sel ? kTmRows : 64) * kTileK + (shared ? S::kBoxN * kTileK : S::kBoxN * kTileK / 2);
         int k0 = 0;
         for (int kb = 0; kb < k_stages; ++kb, k0 += kTileK) {
-          if (!waiter.wait(empty0 + 8 * stage, phase ^ 1u)) { ok = false; break; }
+          if (!waiter.wait_uniform(empty0 + 8 * stage, phase ^ 1u)) { ok = false; break; }
           const uint32_t bar = tile_full0 + 8 * stage;
-          mbar_expect_tx(bar, tx);
-          tma_load_3d(b0 + stage * S::kBBytes, wmap, k0, row, slice, bar);
-          tma_load_2d(a0 + stage * S::kABytes, tmap, k0, tile.row0, bar);
+          if (elect_one()) {
+            mbar_expect_tx(bar, tx);
+            tma_load_3d(b0 + stage * S::kBBytes, wmap, k0, row, slice, bar);
+            tma_load_2d(a0 + stage * S::kABytes, tmap, k0, tile.row0, bar);
+          }
+          __syncwarp();
           if (++stage == S::kStages) { stage = 0; phase ^= 1u; }
         }
         tile = next_tile;
@@ -320,7 +324,7 @@ __global__ void __launch_bounds__(kTmThreads, 1) tm_kernel(const __grid_constant
     }
   } else if (warp == 6) {
     // --------------------------------------------------------------------------------------------- scale producer
-    if (lane == 0) {
+    {
       uint32_t stage = 0, phase = 0;
       const uint32_t sf0 = smem_u32(sf_base);
       bool ok = true;
@@ -339,19 +343,22 @@ __global__ void __launch_bounds__(kTmThreads, 1) tm_kernel(const __grid_constant
         const int32_t* tsf = (shared ? p.tsf_shared : p.tsf_routed) + (int64_t)tile.sf_chunk * kChunkRows;
         for (int kb = 0; kb < k_stages; ++kb, wsf += p.rows_per_expert, tsf += tsf_rows) {
           // the stage's previous UMMAs have retired: its shared memory AND its scale columns in TMEM are free
-          if (!waiter.wait(empty0 + 8 * stage, phase ^ 1u)) { ok = false; break; }
+          if (!waiter.wait_uniform(empty0 + 8 * stage, phase ^ 1u)) { ok = false; break; }
           const uint32_t bar = sf_full0 + 8 * stage;
           const uint32_t dst = sf0 + stage * S::kSfBytes;
-          mbar_expect_tx(bar, 512u + sfb_bytes);
-          bulk_load(dst + 512, wsf, sfb_bytes, bar);          // every CTA of a pair holds the scales of all the block's rows
-          bulk_load(dst, tsf, 512, bar);
+          if (elect_one()) {
+            mbar_expect_tx(bar, 512u + sfb_bytes);
+            bulk_load(dst + 512, wsf, sfb_bytes, bar);        // every CTA of a pair holds the scales of all the block's rows
+            bulk_load(dst, tsf, 512, bar);
+          }
+          __syncwarp();
           if (++stage == S::kStages) { stage = 0; phase ^= 1u; }
         }
         tile = next_tile;
       }
     }
   } else if (warp == 7) {
-    if (lane == 0) {
+    {
       uint32_t stage = 0, phase = 0;
       bool ok = true;
       if (leader) {
@@ -363,16 +370,19 @@ __global__ void __launch_bounds__(kTmThreads, 1) tm_kernel(const __grid_constant
           const TmBlock blk = tm_block(nb, half, blocks_per_half);
           const bool two_chunks = (blk.r0 % kChunkRows) + blk.n_cols > kChunkRows;
           for (int kb = 0; kb < k_stages; ++kb) {
-            if (!waiter.wait(sf_full0 + 8 * stage, phase)) { ok = false; break; }
-            if (!waiter.wait(tile_full0 + 8 * stage, phase)) { ok = false; break; }
-            if (kCtas == 2 && !waiter.wait(pair_ready0 + 8 * stage, phase)) { ok = false; break; }
+            if (!waiter.wait_uniform(sf_full0 + 8 * stage, phase)) { ok = false; break; }
+            if (!waiter.wait_uniform(tile_full0 + 8 * stage, phase)) { ok = false; break; }
+            if (kCtas == 2 && !waiter.wait_uniform(pair_ready0 + 8 * stage, phase)) { ok = false; break; }
             const uint32_t sf_lo = sf_lo0 + stage * (S::kSfBytes >> 4);
             const uint32_t col = tmem_base + S::kSfCol + stage * kTmSfColsPerStage;
             // cta_group::2: every CTA of the pair copies from its own shared memory into its own tensor memory
-            tm_cp_sf<kCtas>(col, sf_hi | sf_lo);                                   // token scales
-            tm_cp_sf<kCtas>(col + 4, sf_hi | (sf_lo + 32));                        // weight scales, first chunk
-            if (two_chunks) tm_cp_sf<kCtas>(col + 8, sf_hi | (sf_lo + 64));
-            tm_commit<kCtas>(mma_ready0 + 8 * stage);                              // arrives when the copies have completed
+            if (elect_one()) {
+              tm_cp_sf<kCtas>(col, sf_hi | sf_lo);                                 // token scales
+              tm_cp_sf<kCtas>(col + 4, sf_hi | (sf_lo + 32));                      // weight scales, first chunk
+              if (two_chunks) tm_cp_sf<kCtas>(col + 8, sf_hi | (sf_lo + 64));
+              tm_commit<kCtas>(mma_ready0 + 8 * stage);                            // arrives when the copies have completed
+            }
+            __syncwarp();
             if (++stage == S::kStages) { stage = 0; phase ^= 1u; }
           }
         }
@@ -382,9 +392,10 @@ __global__ void __launch_bounds__(kTmThreads, 1) tm_kernel(const __grid_constant
         const uint32_t remote0 = map_to_cta(pair_ready0, 0);
         for (int64_t task = unit; task < num_tasks && ok; task += num_units) {
           for (int kb = 0; kb < k_stages; ++kb) {
-            if (!waiter.wait(sf_full0 + 8 * stage, phase)) { ok = false; break; }
-            if (!waiter.wait(tile_full0 + 8 * stage, phase)) { ok = false; break; }
-            mbar_arrive_cluster_relaxed(remote0 + 8 * stage);
+            if (!waiter.wait_uniform(sf_full0 + 8 * stage, phase)) { ok = false; break; }
+            if (!waiter.wait_uniform(tile_full0 + 8 * stage, phase)) { ok = false; break; }
+            if (elect_one()) mbar_arrive_cluster_relaxed(remote0 + 8 * stage);
+            __syncwarp();
             if (++stage == S::kStages) { stage = 0; phase ^= 1u; }
           }
         }
@@ -392,7 +403,7 @@ __global__ void __launch_bounds__(kTmThreads, 1) tm_kernel(const __grid_constant
     }
   } else if (warp == 1) {
     // --------------------------------------------------------------------------------------------- MMA issuer
-    if (lane == 0 && leader) {
+    if (leader) {
       uint32_t stage = 0, phase = 0, it = 0;
       bool ok = true;
       const uint64_t sw128_hi = desc_hi_sw128();
@@ -408,7 +419,7 @@ __global__ void __launch_bounds__(kTmThreads, 1) tm_kernel(const __grid_constant
         const bool shared = tile.expert == kSharedExpert;
         const TmBlock blk = tm_block(nb, half, blocks_per_half);
         const uint32_t acc_stage = it & 1u, acc_phase = (it >> 1) & 1u;
-        if (!waiter.wait(smem_u32(&ctl->tmem_empty[acc_stage]), acc_phase ^ 1u)) { ok = false; break; }
+        if (!waiter.wait_uniform(smem_u32(&ctl->tmem_empty[acc_stage]), acc_phase ^ 1u)) { ok = false; break; }
         tc_fence_after();
         // M = 128 per CTA (256 over a pair); idesc field [24,29) = M >> 4
         const uint32_t idesc0 = make_idesc(0u, shared ? 0u : 5u, static_cast<uint32_t>(blk.n_cols), 0) +
@@ -419,24 +430,28 @@ __global__ void __launch_bounds__(kTmThreads, 1) tm_kernel(const __grid_constant
         // rows skipped at the start of this CTA's box (whole 8-row swizzle groups); the same in both CTAs
         const uint32_t b_skip = static_cast<uint32_t>((S::kBoxN - blk.n_cols / kCtas) * kTileK) >> 4;
         for (int kb = 0; kb < k_stages; ++kb) {
-          if (!waiter.wait(mma_ready0 + 8 * stage, phase)) { ok = false; break; }
+          if (!waiter.wait_uniform(mma_ready0 + 8 * stage, phase)) { ok = false; break; }
           const uint32_t a_lo = a_lo0 + stage * (S::kABytes >> 4);
           const uint32_t b_lo = b_lo0 + stage * (S::kBBytes >> 4) + b_skip;
           const uint32_t sfa = sfa0 + stage * kTmSfColsPerStage, sfb = sfb0 + stage * kTmSfColsPerStage;
+          if (elect_one()) {
 #pragma unroll
-          for (int k = 0; k < kTileK / 32; ++k)
-            tm_mma<kCtas>(d, sw128_hi | (a_lo + 2 * k), sw128_hi | (b_lo + 2 * k),
-                          idesc0 + k * ((1u << 4) | (1u << 29)),            // scale byte k of both operands
-                          sfa, sfb, (kb | k) != 0 ? 1u : 0u);
-          // the stage is free in every CTA of the unit once these UMMAs retire
-          tm_commit<kCtas>(empty0 + 8 * stage);
-          if (kCtas == 2) tm_commit<kCtas>(peer_empty0 + 8 * stage);
+            for (int k = 0; k < kTileK / 32; ++k)
+              tm_mma<kCtas>(d, sw128_hi | (a_lo + 2 * k), sw128_hi | (b_lo + 2 * k),
+                            idesc0 + k * ((1u << 4) | (1u << 29)),          // scale byte k of both operands
+                            sfa, sfb, (kb | k) != 0 ? 1u : 0u);
+            // the stage is free in every CTA of the unit once these UMMAs retire
+            tm_commit<kCtas>(empty0 + 8 * stage);
+            if (kCtas == 2) tm_commit<kCtas>(peer_empty0 + 8 * stage);
+          }
+          __syncwarp();
           if (++stage == S::kStages) { stage = 0; phase ^= 1u; }
         }
-        if (ok) {
+        if (ok && elect_one()) {
           tm_commit<kCtas>(smem_u32(&ctl->tmem_full[acc_stage]));
           if (kCtas == 2) tm_commit<kCtas>(peer_tmem_full0 + 8 * acc_stage);
         }
+        __syncwarp();
         tile = next_tile;
       }
     }
