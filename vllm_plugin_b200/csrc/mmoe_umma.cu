@@ -36,7 +36,7 @@ namespace mmoe {
 
 namespace {
 
-constexpr int kThreads = 224;   // producer, MMA 0, 4 epilogue warps, MMA 1
+constexpr int kThreads = 256;   // producer, MMA 0, 4 epilogue warps, MMA 1, scale arranger (layer 1)
 
 struct UmmaParams {
   CUtensorMap map_w_routed;    // FP4 weights, box 128 K x 256 rows (layer 1: the 5-D de-interleaving form)
@@ -84,8 +84,10 @@ struct UmmaParams {
 };
 
 struct Control {          // lives at the start of shared memory
-  uint64_t full[16];      // producer -> MMA warps: the stage's copies have landed
-  uint64_t empty[16];     // MMA -> producer: the stage's shared memory may be overwritten
+  uint64_t full[8];       // producer -> MMA warps: the stage's copies have landed
+  uint64_t empty[8];      // MMA -> producer: the stage's shared memory may be overwritten
+  uint64_t sf_full[8];    // layer 1, producer -> scale arranger: the stage's weight scales have landed (in stored order)
+  uint64_t sf_ready[8];   // layer 1, scale arranger -> MMA warps: ... and are in tensor-memory order
   uint64_t tmem_full[2];
   uint64_t tmem_empty[2];
   uint32_t tmem_base;
@@ -109,14 +111,11 @@ struct Shape {
   static constexpr int kBBytes = kBoxRows * kTileK;
   // scale area of a stage: [weight scales of the two tiles, 2 x 512][token scales 512][layer 1: stored-order scales
   // 1024].  Layer 2 receives the two 512-byte chunks in tensor-memory order.  Layer 1 receives them in stored (gate/up
-  // interleaved) order and the MMA warps rearrange them: into the first 1024 bytes from a separate landing area, or --
-  // for the 32-token variant, where the saved KB is a sixth pipeline stage -- in place (measured: in place costs the
-  // 4-stage 128-row variant 5 % of its GEMM1 time and buys the others nothing).
-  static constexpr bool kSfInPlace = kLayer == 1 && kBoxRows == 32;
-  static constexpr int kSfBytes = 3 * 512 + (kLayer == 1 && !kSfInPlace ? 1024 : 0);
+  // interleaved) order and the scale arranger rewrites them into the first 1024 bytes.
+  static constexpr int kSfBytes = 3 * 512 + (kLayer == 1 ? 1024 : 0);
   static constexpr int kStageBytes = kABytes + kBBytes + kSfBytes;
   static constexpr int kStagesRaw = (kSmemBudget - 1024) / kStageBytes;
-  static constexpr int kStages = kStagesRaw > 12 ? 12 : kStagesRaw;
+  static constexpr int kStages = kStagesRaw > 8 ? 8 : kStagesRaw;
   static constexpr int kSmemBytes = 1024 + kStages * kStageBytes + 1024;   // control block + stages + alignment slack
   static constexpr int kAccCols = 2 * kNCap;                        // TMEM columns of one accumulator stage
   static constexpr int kSfCol = 2 * kAccCols;                       // scale region: A0, A1, token scales (one copy per MMA warp)
@@ -157,14 +156,14 @@ __device__ __forceinline__ TaskList task_list(const UmmaParams& p) {
 }
 
 // ------------------------------------------------------------------------------------------------ producer
-// One thread.  Everything that does not change inside a task is computed once per task; the K loop only bumps 32-bit
-// coordinates and two pointers, because a one-thread loop runs at instruction latency, not throughput.
+// One warp in step, one elected lane issues.  Everything that does not change inside a task is computed once per task; the
+// K loop only bumps 32-bit coordinates and two pointers, because such a loop runs at instruction latency, not throughput.
 template <int kLayer, int kBoxRows, typename L>
 __device__ __forceinline__ void sa_producer(const UmmaParams& p, const Cta& c, const TaskList& tl, Waiter& waiter,
                                             RoleState& st) {
-  constexpr bool kInPlace = kLayer == 1 && kBoxRows == 32;
   const int k_stages = p.k_dim / kTileK;
   const uint32_t full0 = smem_u32(&c.ctl->full[0]), empty0 = smem_u32(&c.ctl->empty[0]);
+  const uint32_t sf_full0 = smem_u32(&c.ctl->sf_full[0]);
   const uint32_t a0 = smem_u32(c.a_base), b0 = smem_u32(c.b_base), sf0 = smem_u32(c.sf_base);
   for (int64_t task = blockIdx.x; task < tl.num_tasks && st.ok; task += gridDim.x) {
     const int tile_idx = static_cast<int>(task / p.n_blocks);
@@ -191,100 +190,106 @@ __device__ __forceinline__ void sa_producer(const UmmaParams& p, const Cta& c, c
     const int64_t tsf_rows = shared ? p.tsf_rows_shared : p.tsf_rows_routed;
     const int32_t* tsf = (shared ? p.tsf_shared : p.tsf_routed) + (int64_t)tile.sf_chunk * kChunkRows;
     const uint32_t a_tx = shared ? 2 * kTileRows * kTileK : kTileRows * kTileK;   // packed FP4 counts its global bytes
-    const uint32_t tx = a_tx + box_rows * kTileK + 1024 + 512;
+    const uint32_t tx = a_tx + box_rows * kTileK + 512 + (kLayer == 1 ? 0 : 1024);
     int k0 = 0;
     for (int kb = 0; kb < k_stages; ++kb, k0 += kTileK, wsf += p.rows_per_expert, tsf += tsf_rows) {
-      if (!waiter.wait(empty0 + 8 * st.stage, st.phase ^ 1u)) { st.ok = false; break; }
+      if (!waiter.wait_uniform(empty0 + 8 * st.stage, st.phase ^ 1u)) { st.ok = false; break; }
       const uint32_t bar = full0 + 8 * st.stage;
-      mbar_expect_tx(bar, tx);
       const uint32_t a_dst = a0 + st.stage * L::kABytes;
       const uint32_t sf_dst = sf0 + st.stage * L::kSfBytes;
-      if (kLayer == 1) tma_load_5d(a_dst, wmap, k0, 0, group, 0, slice, bar);
-      else tma_load_3d(a_dst, wmap, k0, row, slice, bar);
-      // layer 1: raw scales of the 256 stored rows, permuted by the MMA warps; layer 2: two chunks already in order
-      bulk_load(sf_dst + (kLayer == 1 && !kInPlace ? 3 * 512 : 0), wsf, 1024, bar);
-      tma_load_2d(b0 + st.stage * L::kBBytes, tmap, k0, tile.row0, bar);
-      bulk_load(sf_dst + 2 * 512, tsf, 512, bar);
+      if (elect_one()) {
+        if (kLayer == 1) {
+          // scales of the 256 stored rows, rearranged by the scale arranger: their own barrier, first in the queue
+          mbar_expect_tx(sf_full0 + 8 * st.stage, 1024);
+          bulk_load(sf_dst + 3 * 512, wsf, 1024, sf_full0 + 8 * st.stage);
+        }
+        mbar_expect_tx(bar, tx);
+        if (kLayer == 1) tma_load_5d(a_dst, wmap, k0, 0, group, 0, slice, bar);
+        else tma_load_3d(a_dst, wmap, k0, row, slice, bar);
+        if (kLayer == 2) bulk_load(sf_dst, wsf, 1024, bar);        // two chunks already in tensor-memory order
+        tma_load_2d(b0 + st.stage * L::kBBytes, tmap, k0, tile.row0, bar);
+        bulk_load(sf_dst + 2 * 512, tsf, 512, bar);
+      }
+      __syncwarp();
       if (++st.stage == c.num_stages) { st.stage = 0; st.phase ^= 1u; }
     }
   }
 }
 
 // ------------------------------------------------------------------------------------------------ MMA issuers
+// Layer 1: one warp rewrites each stage's weight scales from stored order into tensor-memory order while the stage's tile
+// copies are still in flight.  The stored W13 scales follow the stored row order (gate/up interleaved by 8, then the 4x32
+// transpose inside each 128-row block); the accumulators want the scales of 128 gate (h = 0) and 128 up (h = 1) channels.
+// On the MMA warps' path this work was a third of a stage's issue time (about 230 of 700 clk, and a stage is 580 clk of
+// HBM time at the clock a power-capped B200 runs this kernel at).
+template <typename L>
+__device__ __forceinline__ void sa_arrange_scales(const UmmaParams& p, const Cta& c, const TaskList& tl, Waiter& waiter,
+                                                  RoleState& st) {
+  const int lane = threadIdx.x & 31;
+  const int k_stages = p.k_dim / kTileK;
+  const uint32_t sf_full0 = smem_u32(&c.ctl->sf_full[0]), sf_ready0 = smem_u32(&c.ctl->sf_ready[0]);
+  int src[8];                                    // source word of the 8 destination words this lane writes
+#pragma unroll
+  for (int t = 0; t < 8; ++t) {
+    const int h = t >> 2;
+    const int q = lane + 32 * (t & 3);           // destination position inside the tile's 128-word block
+    const int m = 32 * (q & 3) + (q >> 2);       // channel of the tile that position serves
+    const int r = 16 * ((m & 63) >> 3) + 8 * h + (m & 7);   // stored row inside its 128-row block
+    src[t] = 128 * (m >> 6) + 4 * (r & 31) + (r >> 5);
+  }
+  for (int64_t task = blockIdx.x; task < tl.num_tasks && st.ok; task += gridDim.x) {
+    for (int kb = 0; kb < k_stages; ++kb) {
+      // the stage's scales have landed, which also says that the MMAs which read the previous ones have retired
+      if (!waiter.wait_uniform(sf_full0 + 8 * st.stage, st.phase)) { st.ok = false; break; }
+      uint32_t* area = reinterpret_cast<uint32_t*>(c.sf_base + st.stage * L::kSfBytes);
+      uint32_t v[8];
+#pragma unroll
+      for (int t = 0; t < 8; ++t) v[t] = area[3 * 128 + src[t]];
+#pragma unroll
+      for (int t = 0; t < 8; ++t) area[lane + 32 * t] = v[t];
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // generic writes -> visible to tcgen05.cp
+      __syncwarp();
+      if (elect_one()) mbar_arrive(sf_ready0 + 8 * st.stage);
+      __syncwarp();
+      if (++st.stage == c.num_stages) { st.stage = 0; st.phase ^= 1u; }
+    }
+  }
+}
+
 // Two warps, one per weight tile / accumulator (h = 0, 1).  The whole warp walks the loop so that loop state stays
 // warp-uniform; one elected lane issues.  Each warp copies the scales it needs into its own TMEM columns, so no
 // ordering between the two warps' tensor-core instructions is needed.
-// Layer 1 first rearranges its tile's weight scales: the stored W13 scales follow the stored row order (gate/up
-// interleaved by 8, then the 4x32 transpose inside each 128-row block), the accumulator wants the scales of 128 gate
-// (h = 0) or up (h = 1) channels in tensor-memory order; each lane moves 4 of the 128 words.
 template <int kLayer, int kBoxRows, typename L>
 __device__ __forceinline__ void sa_mma(const UmmaParams& p, const Cta& c, const TaskList& tl, Waiter& waiter,
                                        RoleState& st, int h) {
-  constexpr bool kInPlace = kLayer == 1 && kBoxRows == 32;
-  const int lane = threadIdx.x & 31;
   const int k_stages = p.k_dim / kTileK;
-  const uint32_t ready0 = smem_u32(&c.ctl->full[0]);
+  const uint32_t full0 = smem_u32(&c.ctl->full[0]), sf_ready0 = smem_u32(&c.ctl->sf_ready[0]);
   const uint32_t empty0 = smem_u32(&c.ctl->empty[0]);
   const uint64_t sw128_hi = desc_hi_sw128();
   const uint64_t sf_hi = desc_hi_sf(128);
-  // layer 1: the four 8-row groups of a weight tile's scales sit 256 bytes apart (see the rearrangement below)
-  const uint64_t sfa_hi = kInPlace ? desc_hi_sf(256) : sf_hi;
   const uint32_t a_lo0 = ((smem_u32(c.a_base) & 0x3FFFFu) >> 4) + h * (kTileRows * kTileK >> 4);
   const uint32_t b_lo0 = (smem_u32(c.b_base) & 0x3FFFFu) >> 4;
   const uint32_t sf_lo0 = (smem_u32(c.sf_base) & 0x3FFFFu) >> 4;
   const uint32_t sfa_col = c.tmem_base + L::kSfCol + 4 * h;
   const uint32_t sfb_col = c.tmem_base + L::kSfCol + 8 + 4 * h;
-  int src[4];                                    // layer 1: source word of the 4 destination words this lane writes
-#pragma unroll
-  for (int t = 0; t < 4; ++t) {
-    const int q = lane + 32 * t;                 // destination position inside the 128-word block
-    const int m = 32 * (q & 3) + (q >> 2);       // channel of the tile that position serves
-    const int r = 16 * ((m & 63) >> 3) + 8 * h + (m & 7);   // stored row inside its 128-row block
-    src[t] = 128 * (m >> 6) + 4 * (r & 31) + (r >> 5);
-  }
   for (int64_t task = blockIdx.x; task < tl.num_tasks && st.ok; task += gridDim.x, ++st.it) {
     const Tile tile = tl.tiles[task / p.n_blocks];
     const bool shared = tile.expert == kSharedExpert;
     const uint32_t acc_stage = st.it & 1u, acc_phase = (st.it >> 1) & 1u;
-    if (!waiter.wait_warp(smem_u32(&c.ctl->tmem_empty[acc_stage]), acc_phase ^ 1u)) { st.ok = false; break; }
+    if (!waiter.wait_uniform(smem_u32(&c.ctl->tmem_empty[acc_stage]), acc_phase ^ 1u)) { st.ok = false; break; }
     tc_fence_after();
     const uint32_t n = static_cast<uint32_t>((tile.n_valid + 15) & ~15);
     const uint32_t idesc0 = make_idesc(shared ? 0u : 5u, 0u, n, 0);
     const uint32_t d = c.tmem_base + acc_stage * L::kAccCols + h * L::kNCap;
     const uint32_t sfb = sfb_col + tile.sf_col;
     for (int kb = 0; kb < k_stages; ++kb) {
-      if (!waiter.wait_warp(ready0 + 8 * st.stage, st.phase)) { st.ok = false; break; }
+      if (kLayer == 1 && !waiter.wait_uniform(sf_ready0 + 8 * st.stage, st.phase)) { st.ok = false; break; }
+      if (!waiter.wait_uniform(full0 + 8 * st.stage, st.phase)) { st.ok = false; break; }
       const uint32_t a_lo = a_lo0 + st.stage * (L::kABytes >> 4);
       const uint32_t b_lo = b_lo0 + st.stage * (L::kBBytes >> 4);
       const uint32_t sf_lo = sf_lo0 + st.stage * (L::kSfBytes >> 4);
-      if (kLayer == 1 && !kInPlace) {
-        uint32_t* out = reinterpret_cast<uint32_t*>(c.sf_base + st.stage * L::kSfBytes) + 128 * h;
-        const uint32_t* in = reinterpret_cast<const uint32_t*>(c.sf_base + st.stage * L::kSfBytes) + 3 * 128;
-        uint32_t v[4];
-#pragma unroll
-        for (int t = 0; t < 4; ++t) v[t] = in[src[t]];
-#pragma unroll
-        for (int t = 0; t < 4; ++t) out[lane + 32 * t] = v[t];
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // generic writes -> visible to tcgen05.cp
-        __syncwarp();
-      }
-      if (kInPlace) {
-        // In stored order the scale words of the gate rows (h = 0) occupy words [64b, 64b + 32) of the 256-word
-        // area (b = 0..3) and those of the up rows (h = 1) words [64b + 32, 64b + 64): the 128 words a warp reads
-        // are exactly the 128 it may overwrite, so the two warps never touch each other's words.  The rearranged
-        // tile is four 128-byte groups of 8 rows, 256 bytes apart, which is what the copy descriptor describes.
-        uint32_t* area = reinterpret_cast<uint32_t*>(c.sf_base + st.stage * L::kSfBytes);
-        uint32_t v[4];
-#pragma unroll
-        for (int t = 0; t < 4; ++t) v[t] = area[src[t]];
-        __syncwarp();                                                  // every lane has read before any lane writes
-#pragma unroll
-        for (int t = 0; t < 4; ++t) area[64 * t + 32 * h + lane] = v[t];
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        __syncwarp();
-      }
       if (elect_one()) {
-        tc_cp_sf(sfa_col, sfa_hi | (sf_lo + (kInPlace ? 8 : 32) * h));
+        tc_cp_sf(sfa_col, sf_hi | (sf_lo + 32 * h));
         tc_cp_sf(sfb_col, sf_hi | (sf_lo + 64));
 #pragma unroll
         for (int k = 0; k < kTileK / 32; ++k)
@@ -445,6 +450,8 @@ __device__ __forceinline__ void sa_setup(Control* ctl) {
     for (int i = 0; i < L::kStages; ++i) {
       mbar_init(smem_u32(&ctl->full[i]), 1);
       mbar_init(smem_u32(&ctl->empty[i]), 2);          // both MMA warps release a stage
+      mbar_init(smem_u32(&ctl->sf_full[i]), 1);
+      mbar_init(smem_u32(&ctl->sf_ready[i]), 1);
     }
     for (int i = 0; i < 2; ++i) {
       mbar_init(smem_u32(&ctl->tmem_full[i]), 2);      // both MMA warps finish an accumulator pair
@@ -484,7 +491,7 @@ __global__ void __launch_bounds__(kThreads, 1) umma_kernel(const __grid_constant
   extern __shared__ uint8_t smem_raw[];
   Cta c = sa_carve<L>(smem_raw);
   Control* ctl = c.ctl;
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);   // warp-uniform for the compiler too
   chain_release();
   sa_setup<L>(ctl);
   // Everything above touches only this CTA's own shared and tensor memory, so it may run while the kernel before this
@@ -508,15 +515,17 @@ __global__ void __launch_bounds__(kThreads, 1) umma_kernel(const __grid_constant
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  c.tmem_base = ctl->tmem_base;
+  c.tmem_base = __shfl_sync(0xffffffffu, ctl->tmem_base, 0);
   c.num_stages = static_cast<uint32_t>(p.num_stages);
   const TaskList tl = task_list(p);
   Waiter waiter{&ctl->abort_flag, p.status, global_timer() + static_cast<uint64_t>(p.timeout_ns), kLayer, warp};
   RoleState st;
   if (warp == 0) {
-    if ((threadIdx.x & 31) == 0) sa_producer<kLayer, kBoxRows, L>(p, c, tl, waiter, st);
+    sa_producer<kLayer, kBoxRows, L>(p, c, tl, waiter, st);
   } else if (warp == 1 || warp == 6) {
     sa_mma<kLayer, kBoxRows, L>(p, c, tl, waiter, st, warp == 1 ? 0 : 1);
+  } else if (warp == 7) {
+    if (kLayer == 1) sa_arrange_scales<L>(p, c, tl, waiter, st);
   } else {
     sa_epilogue<kLayer, kBoxRows, L, kFused>(p, c, tl, waiter, st);
   }
