@@ -297,11 +297,12 @@ def run_ours(args):
     barrier()
     step_ms = reduce_ranks(ev0.elapsed_time(ev1) / args.steps)
     value = world * m / (step_ms * 1e-3)
-    # EP1: quantiser, 3 route-ordering passes, plan, place, shared-expert plan, 2 shared-expert GEMMs (running beside
-    # the ordering / placement on a second stream), 2 routed GEMMs, combine = 12 (6 at M <= 128: one fused ordering/plan
-    # launch and one launch per GEMM).  The peer exchange adds publish, push, 2 flag waits and a flag kernel (17);
-    # its unfused form has one launch per GEMM and a return copy (14); NCCL: the pack kernel, one launch per GEMM (10)
-    launches_per_step = (12 if m > 128 else (6 if m * K > 128 else 5)) if world == 1 else {"nccl": 10, "peer-unfused": 14, "peer": 17}[args.ep_transport]
+    # EP1: quantiser, route counting + plan, placement, two launches per GEMM (experts with few rows, CTA pairs), combine = 8;
+    # one launch per GEMM up to 192 tokens, one routing launch up to 128.  The peer exchange: quantiser, 3 route-ordering
+    # passes, publish, push, 2 flag waits, a flag kernel, shared-expert plan and 2 GEMMs, plan, place, 4 GEMM launches,
+    # combine = 19; its unfused form has the shared expert in the same launches and a return copy (16); NCCL: the pack
+    # kernel instead of the exchange (12)
+    launches_per_step = (8 if m > 192 else 6 if m > 128 else 5) if world == 1 else {"nccl": 12, "peer-unfused": 16, "peer": 19}[args.ep_transport]
 
     # ---- eager host cost of one call (staging + layer), microseconds of CPU time per call with nothing to wait for
     torch.cuda.synchronize(dev)
@@ -380,8 +381,7 @@ def run_ours(args):
     sp = stream.cuda_stream
     ws = buf.base_ptr
     peers = (ctypes.c_void_p * world)(*buf.peer_ptrs) if world > 1 and buf.peer_ptrs is not None else None
-    # past 128 tokens the product call runs the shared expert as launches of its own (tiles planned from the token
-    # count alone) and the routed experts as one launch per GEMM; the phases are timed in that structure
+    # past 128 tokens the shared expert is timed in launches of its own (tiles planned from the token count alone)
     split = m > 128
     opts0 = _native.MmoeOptions(10.0, 1, 0, 2000, 0)
     names = ["stage", "order", "exchange", "place", "shared", "gemm1", "gemm2", "return", "combine"]
@@ -440,11 +440,12 @@ def run_ours(args):
     distinct_mean = reduce_ranks(float(distinct_here), "sum") / world
     pairs_mean = reduce_ranks(float(routes_here + m), "sum") / world       # (token, expert) pairs incl. the shared expert
     expected_rows = m * world * K / E
-    family = {0: "tokens-as-A" if (bm >= 64 and expected_rows >= 80) else "weights-as-A", 1: "weights-as-A",
+    # experts with more than 192 rows run on CTA pairs; with the benchmark's uniform routing nearly all are on one side
+    family = {0: "tokens-as-A" if expected_rows > 192 else "weights-as-A", 1: "weights-as-A",
               2: "tokens-as-A", 3: "tokens-as-A"}[args.orientation]
-    kernel_name = ("tm_kernel<1> (grouped GEMM1 + SwiGLU/requant, tokens-as-A)" if family == "tokens-as-A"
+    kernel_name = ("tm_kernel<1> (grouped GEMM1 + SwiGLU/requant, tokens-as-A on CTA pairs)" if family == "tokens-as-A"
                    else "umma_kernel<1> (grouped GEMM1 + SwiGLU/requant, weights-as-A)")
-    kernel_name += ", the launch over the routed experts' tiles" if m > 128 else ", one launch over routed and shared tiles"
+    kernel_name += ", the launches over the routed experts' tiles" if m > 128 else ", one launch over routed and shared tiles"
     sm_mhz = float((clocks or {}).get("sm_mhz") or 0.0)
     sm_mhz = reduce_ranks(sm_mhz, "max") or 1965.0                               # rank 0 samples its GPU
     tensor_peak = 2 * TENSOR_MAC_PER_CLK_SM * NUM_SMS * sm_mhz * 1e6 / 1e12      # TFLOP/s at the sampled SM clock
@@ -484,9 +485,10 @@ def run_ours(args):
             "gemm1_tensor_frac": g1_tflops / tensor_peak, "gemm2_tensor_frac": g2_flops / (g2_ms * 1e-3) / 1e12 / tensor_peak})
     kernels.update({
         "kernel_family": family,
-        "phase_note": "phases timed back to back on one stream in the product call's launch structure (past 128 tokens: "
-                      "shared_ms = the shared expert's two GEMM launches, gemm1_ms / gemm2_ms = the routed experts' "
-                      "launches); the product call overlaps ordering / exchange with the shared expert",
+        "phase_note": "phases timed back to back on one stream through the C ABI (past 128 tokens: shared_ms = the shared "
+                      "expert's two GEMM launches, gemm1_ms / gemm2_ms = the routed experts' launches); the product call at "
+                      "one GPU orders, plans and places in one or two launches and runs shared and routed tiles together; "
+                      "at more GPUs it overlaps the exchange with the shared expert",
         "layer_tflops_per_gpu": flops_mean / (step_ms * 1e-3) / 1e12,
         "layer_tensor_frac": flops_mean / (step_ms * 1e-3) / 1e12 / tensor_peak,
         "layer_algorithmic_gbs_per_gpu": bytes_mean / (step_ms * 1e-3) / 1e9,
@@ -689,7 +691,7 @@ def main():
                     help="N > 1: device-side NVLink exchange with the write-back fused into GEMM2 (default), the same "
                          "with a separate copy kernel, or the host-driven NCCL all-to-allv")
     ap.add_argument("--orientation", type=int, default=0, choices=(0, 1, 2, 3),
-                    help="grouped-GEMM kernel family: 0 chosen per call, 1 weights-as-A, 2 tokens-as-A, 3 tokens-as-A on CTA pairs")
+                    help="grouped-GEMM kernel family: 0 chosen per expert, 1 weights-as-A, 2 or 3 tokens-as-A on CTA pairs")
     ap.add_argument("--no-sweep", action="store_true")
     ap.add_argument("--no-cpu-baseline", action="store_true")
     args = ap.parse_args()

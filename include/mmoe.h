@@ -79,6 +79,7 @@ typedef struct MmoeLayout {
   int64_t pool_sf_rows;     /* row capacity (multiple of 128) of the pool SF chunk matrices */
   int64_t max_routes;       /* T * min(k, E/R): rows one rank can send */
   int64_t max_tiles;        /* capacity of the tile table */
+  int64_t shared_tile_sf;   /* int32 chunks of the shared expert's token scales: chunk j = tile j, element (chunk row, word) at word*rows + row */
 } MmoeLayout;
 
 /* Replaces `build_symm_buffer_layout` (backend/heuristics.py:504-674) / `SymmBuffer.__init__` sizing
@@ -271,12 +272,9 @@ int mmoe_read_status(const MmoeGeometry* geo, void* workspace, int32_t* words8, 
 
 /* Process-wide tuning of the tensor-core kernels (the reference keeps such knobs in `KernelOptions`,
  * backend/frontend.py:72-116).  `max_stages`: cap on the shared-memory pipeline depth of the weights-as-A kernels (0: no
- * cap).  `orientation`: 0 = chosen per call (weights-as-A kernels below about 80 expected rows per expert, tokens-as-A
- * kernels from there, and for the shared expert of a call with more than 128 tokens), 1 = weights-as-A always, 2 =
- * tokens-as-A wherever the geometry allows (intermediate >= 192, hidden >= 384), 3 = tokens-as-A on CTA pairs
- * (`tcgen05.mma.cta_group::2`) wherever the geometry and BLOCK_M (>= 128) allow; never chosen automatically: measured
- * on B200 it is slower than single CTAs at 120 to 480 rows per expert.  Every rank and every step of a call (planning, GEMM launches) must see the same
- * setting. */
+ * cap).  `orientation`: 0 = chosen per expert from the rows it received (weights-as-A kernels for few rows, tokens-as-A
+ * kernels on CTA pairs, `tcgen05.mma.cta_group::2`, for many), 1 = weights-as-A always, 2 or 3 = tokens-as-A always.  Every
+ * rank and every step of a call (planning, GEMM launches) must see the same setting. */
 int mmoe_set_tuning(int32_t max_stages, int32_t orientation);
 
 const char* mmoe_status_string(int code);

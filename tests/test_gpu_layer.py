@@ -353,3 +353,43 @@ def test_shared_expert_ahead_of_the_routed_plan(m, bm):
     _native.check(lib.mmoe_combine(geo, base, y.data_ptr(), m, sp))
     read_status(buf)
     assert torch.equal(y, y_whole)
+
+
+@pytest.mark.parametrize("m,rows", [(193, (193, 192, 1)), (260, (257, 256, 129, 81, 112)), (300, (300, 160, 161, 113, 80)),
+                                    (700, (700, 513, 512, 385, 225, 16)), (129, (129, 100, 17))])
+def test_tile_cuts_at_their_edges(m, rows):
+    """Experts with exactly the row counts at which the cut changes: one, two and three tiles of the weights-as-A kernels (80 /
+    112 rows each), the first pair, full and just overfull pairs, and a token that names one expert twice.  The single-GPU
+    forward (routes counted, planned and placed in two launches) against the oracle, and bit for bit against the general
+    sequence over receive counts."""
+    import ctypes
+    from vllm_plugin_b200 import api
+    from vllm_plugin_b200.backend import _native
+    from vllm_plugin_b200.backend.frontend import _weights_struct, check_mega_moe_arguments, read_status
+    layer = H.make_layer(512, 256, 8, 6, True, seed=41)
+    hid = O.make_hidden(m, layer.hidden, 3)
+    g = torch.Generator().manual_seed(m)
+    ids = torch.full((m, 6), -1, dtype=torch.int64)
+    for e, n in enumerate(rows):                               # expert e takes n of the m tokens, in slot e
+        ids[torch.randperm(m, generator=g)[:n], e % 6] = e + 1
+    ids[0, 5] = ids[0, 0]
+    w = torch.rand((m, 6), generator=g)
+    y_one, buf = H.run_layer(layer, hid, ids, w)
+    pool_one, act_one = buf.l1_acts.view(torch.uint8).clone(), buf.l2_acts.view(torch.uint8).clone()
+    met = O.parity_metrics(y_one.cpu(), H.oracle_layer(layer, hid, ids, w))
+    assert met["rel_l2"] <= 1e-3, met
+    dev = torch.device("cuda", 0)
+    l1, l2, sl1, sl2 = H.kernel_weights(layer, dev)
+    y = torch.empty_like(y_one)
+    s13, s2 = check_mega_moe_arguments(y, l1, l2, buf, sl1, sl2, None, (1, 1, 32), "swiglu", 10.0, True, 1.0, 0.0)
+    ws, opts = _weights_struct(l1, l2, sl1, sl2, s13, s2), _native.MmoeOptions(10.0, 1, 0, 2000, 0)
+    lib, geo, base = _native.load(), ctypes.byref(buf.geo), buf.base_ptr
+    sp = torch.cuda.current_stream(dev).cuda_stream
+    bm = api.stage_inputs_for_mega_moe(buf, hid.to(dev), ids.to(dev), w.to(dev))
+    _native.check(lib.mmoe_dispatch_count(geo, base, m, sp))
+    _native.check(lib.mmoe_dispatch_place(geo, base, m, bm, None, sp))
+    _native.check(lib.mmoe_experts(geo, base, ctypes.byref(ws), ctypes.byref(opts), m, bm, sp))
+    _native.check(lib.mmoe_combine(geo, base, y.data_ptr(), m, sp))
+    read_status(buf)
+    assert torch.equal(buf.l1_acts.view(torch.uint8), pool_one) and torch.equal(buf.l2_acts.view(torch.uint8), act_one)
+    assert torch.equal(y, y_one)

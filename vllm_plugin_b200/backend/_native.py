@@ -45,7 +45,8 @@ _LAYOUT_FIELDS = (
     "total_bytes", "x", "x_sf", "topk_idx", "topk_weights", "shared_x_sf", "shared_sf_rows", "send_count",
     "send_offset", "route_pos", "sorted_route", "sort_scratch", "recv_count", "plan", "send_x", "send_sf", "send_w",
     "recv_x", "recv_sf", "recv_w", "pool_x", "pool_sf", "pool_w", "pool_dst", "act_x", "act_sf", "shared_act_x",
-    "shared_act_sf", "ret", "ret_recv", "shared_out", "ep_sync", "status", "pool_rows", "pool_sf_rows", "max_routes", "max_tiles")
+    "shared_act_sf", "ret", "ret_recv", "shared_out", "ep_sync", "status", "pool_rows", "pool_sf_rows", "max_routes", "max_tiles",
+    "shared_tile_sf")
 
 
 class MmoeLayout(ctypes.Structure):

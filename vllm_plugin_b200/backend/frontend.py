@@ -40,9 +40,9 @@ class KernelOptions:
                                 # stream; False = one stream, separate copy kernel after GEMM2 (same result)
     status_poll_interval: int = 32   # eager calls between two non-blocking reads of the device status words (a bounded
                                      # wait that expired, an expert id out of range); 0 = never, 1 = every call
-    orientation: int = 0        # grouped-GEMM kernel family: 0 = chosen per call from the expected rows per expert,
-                                # 1 = weights-as-A (small token counts) always, 2 = tokens-as-A wherever the geometry
-                                # allows, 3 = tokens-as-A on CTA pairs; every rank of a group must use the same value
+    orientation: int = 0        # grouped-GEMM kernel family: 0 = chosen per expert from the rows it received, 1 =
+                                # weights-as-A (few rows) always, 2 or 3 = tokens-as-A on CTA pairs (many rows) always;
+                                # every rank of a group must use the same value
 
 
 _kernel_options = KernelOptions()

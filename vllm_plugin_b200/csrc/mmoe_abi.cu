@@ -82,6 +82,18 @@ int check_geometry(const MmoeGeometry* g) {
   return MMOE_OK;
 }
 
+// Experts with more rows than this run on CTA pairs (256 tokens x 256 weight rows per task), the others on the
+// weights-as-A kernels (tiles of at most 112 rows).  A pair spends 2 x 512 clk of SM time per 128-K stage and 256 weight rows
+// whatever its rows; a weights-as-A tile 430-500 clk, growing with them, so two of those (up to 224 rows) cost about the
+// same as a pair and a third one more.
+constexpr int kPairAbove = 192;
+
+// A pure function of the process-wide setting, so that the planning step and the GEMM launches of one call agree.
+int pair_above_of() {
+  const int forced = mmoe::tuned_orientation();
+  return forced == 0 ? kPairAbove : (forced == 1 ? mmoe::kNeverPair : 0);
+}
+
 int make_ctx(const MmoeGeometry* g, void* ws, mmoe::Ctx* c) {
   int rc = check_geometry(g);
   if (rc != MMOE_OK) return rc;
@@ -93,28 +105,8 @@ int make_ctx(const MmoeGeometry* g, void* ws, mmoe::Ctx* c) {
   c->ws = static_cast<char*>(ws);
   c->e_local = g->num_experts / g->num_ranks;
   c->kmax = g->num_topk < c->e_local ? g->num_topk : c->e_local;
+  c->pair_above = pair_above_of();
   return MMOE_OK;
-}
-
-// Which kernel family runs a tile list, hence how the list is cut.  A pure function of the call's geometry, token
-// count and BLOCK_M, so that the planning step and the GEMM launches of one call agree without talking to each other.
-// `early_shared`: the shared expert's tiles planned ahead of the routed ones (tile_select 2); otherwise the routed tiles
-// and the shared tiles planned with them.
-int choose_family(const MmoeGeometry* g, int m, int block_m, bool early_shared) {
-  // a half of each weight matrix must hold a 192-row box (more than one for the short last block of a CTA pair)
-  const bool fits = g->intermediate >= 192 && g->hidden / 2 >= 192;
-  const bool pair_ok = fits && block_m >= 128;        // two scale chunks per pool block: one per half of a pair
-  const int forced = mmoe::tuned_orientation();
-  if (!fits || forced == 1) return mmoe::kFamilyWeightsAsA;
-  if (forced == 2 || (forced == 3 && !pair_ok)) return mmoe::kFamilyTokensAsA;
-  if (forced == 3) return mmoe::kFamilyTokensAsAPair;
-  // CTA pairs are never chosen automatically: measured on B200 at 120 / 240 / 480 rows per expert a pair step takes
-  // 1.90 / 1.20 / 1.08 ms against 1.38 / 1.15 / 1.08 ms on single CTAs (the issuing thread pays two commits per stage)
-  if (early_shared) return m > 128 ? mmoe::kFamilyTokensAsA : mmoe::kFamilyWeightsAsA;
-  // expected rows per expert (the quantity BLOCK_M is chosen from): below ~80 the weights-as-A kernels, whose cost
-  // follows the token count, win (and stream more weight bytes per stage when the call is HBM-bound)
-  const double expected = (double)m * g->num_ranks * g->num_topk / g->num_experts;
-  return block_m >= 64 && expected >= 80.0 ? mmoe::kFamilyTokensAsA : mmoe::kFamilyWeightsAsA;
 }
 
 int check_tokens(const MmoeGeometry* g, int m) {
@@ -240,6 +232,7 @@ int mmoe_layout(const MmoeGeometry* g, MmoeLayout* out) {
   out->shared_out = take(shared ? T * H * 2 : 0);
   out->ep_sync = take(ep ? mmoe::ep_sync_bytes() : 0);
   out->status = take(64);
+  out->shared_tile_sf = take(shared ? mmoe::shared_chunk_rows(T) * (H / 128) * 4 : 0);
   out->total_bytes = off;
   out->pool_rows = pool_rows;
   out->pool_sf_rows = sf_rows;
@@ -419,7 +412,6 @@ int mmoe_dispatch_place(const MmoeGeometry* geo, void* workspace, int32_t num_to
   rc = check_tokens(geo, num_tokens);
   if (rc != MMOE_OK) return rc;
   if (!valid_block_m(block_m)) return fail(MMOE_ERR_INVALID_ARGUMENT, "block_m=%d is not a BLOCK_M value", block_m);
-  c.family = choose_family(geo, num_tokens, block_m, false);
   cudaError_t e = mmoe::launch_plan_place(c, num_tokens, block_m, stats, static_cast<cudaStream_t>(stream));
   return e == cudaSuccess ? MMOE_OK : cuda_fail(e, "dispatch_place launch");
 }
@@ -442,7 +434,6 @@ int mmoe_plan_shared(const MmoeGeometry* geo, void* workspace, int32_t num_token
   if (rc == MMOE_OK) rc = check_tokens(geo, num_tokens);
   if (rc != MMOE_OK) return rc;
   if (!valid_block_m(block_m)) return fail(MMOE_ERR_INVALID_ARGUMENT, "block_m=%d is not a BLOCK_M value", block_m);
-  c.family = choose_family(geo, num_tokens, block_m, true);
   cudaError_t e = mmoe::launch_shared_plan(c, num_tokens, block_m, static_cast<cudaStream_t>(stream));
   return e == cudaSuccess ? MMOE_OK : cuda_fail(e, "shared plan launch");
 }
@@ -504,8 +495,7 @@ int run_experts(const MmoeGeometry* geo, void* workspace, const void* const* pee
     if (!mmoe::tc_ready()) return fail(MMOE_ERR_NOT_PREPARED, "mmoe_prepare() must run on this device before the first launch");
     c.peer_ws = peers;
     c.tile_select = tile_select;
-    c.family = choose_family(geo, num_tokens, block_m, tile_select == 2);
-    e = mmoe::launch_experts_umma(c, *weights, o, num_tokens, block_m, st);
+      e = mmoe::launch_experts_umma(c, *weights, o, num_tokens, block_m, st);
     if (e == cudaSuccess && peers != nullptr) e = mmoe::launch_ep_signal_return(c, peers, timeout_ns, st);
   } else {
     return fail(MMOE_ERR_UNSUPPORTED, "engine=%d", o.engine);
@@ -538,54 +528,18 @@ int mmoe_forward(const MmoeGeometry* geo, void* workspace, const MmoeWeights* we
   mmoe::ChainScope chain(num_tokens <= 128);
   if (geo != nullptr && geo->num_ranks != 1)
     return fail(MMOE_ERR_INVALID_ARGUMENT, "mmoe_forward is the single-rank sequence; call mmoe_forward_ep for num_ranks > 1");
-  const bool decode = geo != nullptr && num_tokens > 0 && num_tokens <= 128 && geo->num_experts <= 512 &&
-                      valid_block_m(block_m) && workspace != nullptr;
-  // route ordering, plan and placement of the routed experts on stream `st`
-  auto dispatch = [&](void* st) -> int {
-    if (decode) {                       // one launch orders the routes and builds the plan
-      mmoe::Ctx c;
-      int r = make_ctx(geo, workspace, &c);
-      if (r != MMOE_OK) return r;
-      c.family = choose_family(geo, num_tokens, block_m, false);
-      cudaError_t e = mmoe::launch_route_plan_place_small(c, num_tokens, block_m, stats, static_cast<cudaStream_t>(st));
-      return e == cudaSuccess ? MMOE_OK : cuda_fail(e, "route/plan launch");
-    }
-    int r = mmoe_dispatch_count(geo, workspace, num_tokens, st);
-    if (r == MMOE_OK) r = mmoe_dispatch_place(geo, workspace, num_tokens, block_m, stats, st);
-    return r;
-  };
-  cudaStream_t main_stream = static_cast<cudaStream_t>(stream);
-  SideLane* lane = nullptr;
-  // (only past the decode sizes: at a handful of tokens the three extra launches cost more than the overlap gains --
-  // measured 61 -> 82 us at M=1, 1.742 -> 1.719 ms at M=3840)
-  if (geo != nullptr && opt != nullptr && opt->engine == 0 && geo->num_shared_experts > 0 && num_tokens > 128 &&
-      (opt->layer_mask == 0 || opt->layer_mask == 3)) {
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    cudaStreamIsCapturing(main_stream, &cap);
-    lane = side_lane(cap == cudaStreamCaptureStatusNone);
-  }
-  int rc;
-  if (lane == nullptr) {
-    rc = dispatch(stream);
-    if (rc == MMOE_OK) rc = mmoe_experts(geo, workspace, weights, opt, num_tokens, block_m, stream);
-    if (rc == MMOE_OK) rc = mmoe_combine_residual(geo, workspace, y_bf16, opt != nullptr ? opt->residual : nullptr, num_tokens, stream);
-    return rc;
-  }
-  // The shared expert needs only the staged tokens: its two GEMMs run here while the routed experts' ordering, plan
-  // and placement run on the library's second stream (fork / join with events, capturable).
-  cudaError_t e = cudaEventRecord(lane->fork, main_stream);
-  if (e == cudaSuccess) e = cudaStreamWaitEvent(lane->stream, lane->fork, 0);
-  if (e != cudaSuccess) return cuda_fail(e, "forking the dispatch stream");
-  mmoe::break_chain();                      // the side stream's first kernel follows an event, not a kernel
-  const int rc_side = dispatch(lane->stream);
-  e = cudaEventRecord(lane->join, lane->stream);
-  rc = mmoe_plan_shared(geo, workspace, num_tokens, block_m, stream);
-  if (rc == MMOE_OK) rc = run_experts(geo, workspace, nullptr, weights, opt, num_tokens, block_m, stream, 2);
-  if (e == cudaSuccess) e = cudaStreamWaitEvent(main_stream, lane->join, 0);
-  if (e != cudaSuccess) return cuda_fail(e, "joining the dispatch stream");
-  mmoe::break_chain();                      // the next kernel has two predecessors: launch it without the attribute
-  if (rc_side != MMOE_OK) return rc_side;
-  if (rc == MMOE_OK) rc = run_experts(geo, workspace, nullptr, weights, opt, num_tokens, block_m, stream, 1);
+  mmoe::Ctx c;
+  int rc = make_ctx(geo, workspace, &c);
+  if (rc == MMOE_OK) rc = check_tokens(geo, num_tokens);
+  if (rc != MMOE_OK) return rc;
+  if (!valid_block_m(block_m)) return fail(MMOE_ERR_INVALID_ARGUMENT, "block_m=%d is not a BLOCK_M value", block_m);
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  // route ordering, plan and placement: one launch up to 128 tokens, two beyond
+  const cudaError_t e = num_tokens > 0 && num_tokens <= 128 && geo->num_experts <= 512
+                            ? mmoe::launch_route_small(c, num_tokens, block_m, stats, st)
+                            : mmoe::launch_route_large(c, num_tokens, block_m, stats, st);
+  if (e != cudaSuccess) return cuda_fail(e, "route / plan / placement launch");
+  rc = mmoe_experts(geo, workspace, weights, opt, num_tokens, block_m, stream);
   if (rc == MMOE_OK) rc = mmoe_combine_residual(geo, workspace, y_bf16, opt != nullptr ? opt->residual : nullptr, num_tokens, stream);
   return rc;
 }
@@ -622,7 +576,6 @@ int mmoe_forward_ep(const MmoeGeometry* geo, void* workspace, const void* const*
   // ... while the shared expert, which needs only this rank's own tokens, runs both of its GEMMs here
   mmoe::Ctx c;
   rc = make_ctx(geo, workspace, &c);
-  if (rc == MMOE_OK) c.family = choose_family(geo, num_tokens, block_m, true);
   if (rc == MMOE_OK && mmoe::launch_shared_plan(c, num_tokens, block_m, main_stream) != cudaSuccess)
     rc = cuda_fail(cudaGetLastError(), "shared plan launch");
   if (rc == MMOE_OK) rc = run_experts(geo, workspace, nullptr, weights, opt, num_tokens, block_m, stream, 2);

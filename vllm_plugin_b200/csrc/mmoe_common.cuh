@@ -17,33 +17,42 @@ constexpr int kGroupK = 32;        // K elements per UE8M0 scale
 constexpr int kTileK = 128;        // K elements per pipeline stage = one packed scale word
 constexpr int kTileRows = 128;     // weight rows per tile (UMMA M)
 constexpr int kChunkRows = 128;    // token rows per scale-factor chunk (one 512-byte tcgen05.cp source per K stage)
-constexpr int kMaxTileTokens = 112;  // largest UMMA N of one task
-// Largest token tile of a BLOCK_M variant; an expert with more rows is cut into equal tiles.  BLOCK_M = 128 caps its
-// tiles at 80 rows: the 10 KB token slot buys a fifth pipeline stage.  192 / 240 keep 112 (the tensor-bound
-// expert-parallel shapes, where fewer and larger tiles matter more than pipeline depth).
-__host__ __device__ inline int max_tile_rows(int block_m) { return block_m <= 64 ? block_m : (block_m == 128 ? 80 : kMaxTileTokens); }
-// Kernel family of a launch, hence how its tile list is cut: weights-as-A kernels (tiles of at most max_tile_rows),
-// tokens-as-A kernels (tiles of up to 128 rows whatever BLOCK_M is), tokens-as-A kernels on CTA pairs (an even number of
-// tiles per expert: tiles 2j and 2j + 1 are the two halves of one pair task).
-enum { kFamilyWeightsAsA = 0, kFamilyTokensAsA = 1, kFamilyTokensAsAPair = 2 };
-constexpr int kTokenMajorTileRows = 128;
-__host__ __device__ inline int tile_cap(int block_m, int family) { return family != kFamilyWeightsAsA ? kTokenMajorTileRows : max_tile_rows(block_m); }
-// Scale-factor chunks (128 token rows each) reserved per pool block of a BLOCK_M variant: at least as many as the
-// tiles an expert's rows are cut into (ceil(n / max_tile_rows) <= ceil(n / block_m) * chunks_per_block for every n).
+constexpr int kSmallTileRows = 112;      // largest token tile of the weights-as-A kernels (UMMA N): four accumulators of 112 TMEM columns
+constexpr int kPairTileRows = 128;       // largest token tile of the tokens-as-A kernels (half of a CTA pair's 256 rows)
+// Which kernels run an expert depends on the rows it received in this call (see pair_above_default in mmoe_abi.cu).
+constexpr int kNeverPair = 0x7fffffff;
+
+// How the n rows of an expert are cut into tiles.  Up to `pair_above` rows: ceil(n / small_cap) equal tiles (rounded up to 16
+// rows) for the weights-as-A kernels.  Above: an even number of tiles of at most 128 rows, the two halves of CTA-pair tasks;
+// the second half of a single pair is empty when everything fits the first.  Cuts ignore the BLOCK_M boundaries of the pool.
+struct Cut {
+  int32_t parts, step;
+};
+__host__ __device__ inline Cut cut_rows(int n, int pair_above, int small_cap) {
+  if (n <= 0) return Cut{0, 16};
+  if (n > pair_above) {
+    if (n <= kPairTileRows) return Cut{2, kPairTileRows};
+    const int parts = 2 * ((n + 2 * kPairTileRows - 1) / (2 * kPairTileRows));
+    return Cut{parts, ((n + parts - 1) / parts + 15) & ~15};
+  }
+  const int parts = (n + small_cap - 1) / small_cap;
+  return Cut{parts, ((n + parts - 1) / parts + 15) & ~15};
+}
+// Scale-factor chunks (128 token rows each) reserved per pool block of a BLOCK_M variant: at least as many as the non-empty
+// tiles an expert's rows are cut into (small_cap >= 16 for BLOCK_M 16, >= 32 for 32, >= 64 for 64, >= 80 above).
 __host__ __device__ inline int chunks_per_block(int block_m) { return block_m <= 64 ? 1 : (block_m <= 192 ? 2 : 3); }
 constexpr int kSortChunkTokens = 128;
 constexpr int kSharedExpert = -2;  // MmoeTile::expert of a shared-expert tile
 
-// One unit of token rows handed to the grouped GEMMs: `n_valid` (<= 112) rows starting at `row0` of the token matrix
-// (pool rows for routed experts, token indices for the shared expert), whose scales live in chunk `sf_chunk`
-// starting at row `32 * sf_col` of that chunk.
+// One unit of token rows handed to the grouped GEMMs: `n_valid` rows starting at `row0` of the token matrix (pool rows for
+// routed experts, token indices for the shared expert), whose scales live in chunk `sf_chunk`.
 struct Tile {
   int32_t expert;    // local expert index, or kSharedExpert
   int32_t row0;
   int32_t n_valid;
   int32_t sf_chunk;
-  int32_t sf_col;    // 0 or 2: first 32-row group of the chunk this tile uses
-  int32_t pad[3];
+  int32_t part, parts;   // this tile is the part-th of the `parts` tiles of its expert
+  int32_t pad[2];
 };
 static_assert(sizeof(Tile) == 32, "tile record is 32 bytes");
 
@@ -55,7 +64,13 @@ struct PlanHeader {
   int32_t block_m;
   int32_t num_tokens;
   int32_t num_early_shared_tiles;   // shared-expert tiles written ahead of the routed plan, at the tail of the tile table
-  int32_t pad[9];
+  int32_t num_small_tiles;     // the first of the routed tiles: those of the weights-as-A kernels; the others are pair tiles
+  int32_t small_cap;           // rows a weights-as-A tile of this call may have
+  int32_t small_rows;          // rows of the largest one, rounded up to 16
+  int32_t shared_small;        // 1: the shared expert's tiles are weights-as-A tiles
+  int32_t early_small_rows;    // small_rows of the tiles written ahead (0: they are pair tiles)
+  int32_t ticket;              // blocks of the route-counting launch that have finished; zero between launches
+  int32_t pad[3];
 };
 static_assert(sizeof(PlanHeader) == 64, "plan header is 64 bytes");
 
@@ -73,6 +88,38 @@ struct PlanView {
 };
 
 __host__ __device__ inline int64_t align_up(int64_t a, int64_t b) { return (a + b - 1) / b * b; }
+
+// A contiguous run of the tile table, after `lead` further records that come first in the task order (the shared expert's).
+struct TileRange {
+  const Tile* tiles;
+  int32_t count;          // all records, the leading ones included
+  const Tile* lead_tiles;
+  int32_t lead;
+  __host__ __device__ const Tile& at(int i) const { return i < lead ? lead_tiles[i] : tiles[i - lead]; }
+};
+// The tiles a launch runs.  `select`: 0 = every tile of the plan, 1 = routed tiles only, 2 = the shared expert's tiles
+// planned ahead (at the tail of the table).  Table order: routed weights-as-A tiles, routed pair tiles, shared tiles.
+__host__ __device__ inline TileRange small_tiles(const PlanView& v, int select, bool has_shared, int64_t early_first, int early_cap) {
+  const PlanHeader& h = *v.hdr;
+  if (select == 2) {
+    const int n = has_shared && h.early_small_rows > 0 ? h.num_early_shared_tiles : 0;
+    return TileRange{v.tiles + early_first, n < 0 ? 0 : (n > early_cap ? early_cap : n), nullptr, 0};
+  }
+  const int lead = select == 0 && has_shared && h.shared_small ? h.num_shared_tiles : 0;   // a shared weight row has twice the bytes: first
+  return TileRange{v.tiles, h.num_small_tiles + lead, v.tiles + h.num_routed_tiles, lead};
+}
+__host__ __device__ inline TileRange pair_tiles(const PlanView& v, int select, bool has_shared, int64_t early_first, int early_cap) {
+  const PlanHeader& h = *v.hdr;
+  if (select == 2) {
+    const int n = has_shared && h.early_small_rows == 0 ? h.num_early_shared_tiles : 0;
+    return TileRange{v.tiles + early_first, n < 0 ? 0 : (n > early_cap ? early_cap : n), nullptr, 0};
+  }
+  const int n = h.num_routed_tiles - h.num_small_tiles + (select == 0 && has_shared && !h.shared_small ? h.num_shared_tiles : 0);
+  return TileRange{v.tiles + h.num_small_tiles, n, nullptr, 0};
+}
+
+// scale chunks of the shared expert's tokens: one per tile, whatever the cut
+__host__ __device__ inline int64_t shared_chunk_rows(int64_t max_tokens) { return (max_tokens / 64 + 2) * 128; }
 
 // tile records reserved for the shared expert of a call with at most `max_tokens` tokens (they sit at the tail of the
 // tile table when the shared expert is planned ahead of the routed experts)
@@ -185,7 +232,10 @@ struct Ctx {             // resolved pointers of one call
   int kmax;              // min(k, E/R)
   const void* const* peer_ws = nullptr;   // set by the call that fuses the write-back into GEMM2 (EP > 1)
   int tile_select = 0;                    // 0: every tile of the plan, 1: routed tiles only, 2: the early shared tiles only
-  int family = kFamilyWeightsAsA;         // kernel family the tiles this call plans / runs are cut for
+  int pair_above = kNeverPair;            // experts with more rows than this run on CTA pairs ...
+  // ... in a call of m tokens on this rank: with one rank and few tokens none does (not even one that a token names twice),
+  // and the call needs no pair launch
+  int pair_above_for(int m) const { return geo.num_ranks == 1 && m <= pair_above ? kNeverPair : pair_above; }
   template <typename T> T* at(int64_t off) const { return reinterpret_cast<T*>(ws + off); }
 };
 
@@ -238,6 +288,26 @@ cudaError_t launch_chained(void (*kernel)(KArgs...), dim3 grid, dim3 block, size
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(std::forward<Args>(args))...);
 }
 
+// the same for a kernel of CTA clusters
+template <typename... KArgs, typename... Args>
+cudaError_t launch_clustered(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, int cluster, cudaStream_t s, Args&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = cluster;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = take_chain_flag() ? 2 : 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(std::forward<Args>(args))...);
+}
+
 cudaError_t launch_stage(const Ctx& c, const void* hidden, const void* ids, int ids64, const float* w,
                          const uint8_t* pad, int m, int shared_bm, cudaStream_t s);
 cudaError_t launch_route_stage(const Ctx& c, const void* hidden, const void* ids, int ids64, const float* w,
@@ -248,7 +318,8 @@ cudaError_t launch_stage_nvfp4(const void* hidden, void* q_out, void* sf_out, fl
                                cudaStream_t s);
 cudaError_t launch_count_sort(const Ctx& c, int m, cudaStream_t s);
 cudaError_t launch_pack(const Ctx& c, int m, cudaStream_t s);
-cudaError_t launch_route_plan_place_small(const Ctx& c, int m, int block_m, int32_t* stats, cudaStream_t s);
+cudaError_t launch_route_small(const Ctx& c, int m, int block_m, int32_t* stats, cudaStream_t s);
+cudaError_t launch_route_large(const Ctx& c, int m, int block_m, int32_t* stats, cudaStream_t s);
 cudaError_t launch_plan_place(const Ctx& c, int m, int block_m, int32_t* stats, cudaStream_t s);
 cudaError_t launch_shared_plan(const Ctx& c, int m, int block_m, cudaStream_t s);
 cudaError_t launch_combine(const Ctx& c, void* y, const void* residual, int m, cudaStream_t s);
@@ -257,7 +328,7 @@ cudaError_t launch_experts_umma(const Ctx& c, const MmoeWeights& w, const MmoeOp
 int prepare_umma(const MmoeGeometry& geo);   // returns an MMOE_* code
 bool tc_ready();                             // prepare_umma() has run on the current device
 void set_tuning(int max_stages, int orientation);
-int tuned_orientation();                     // 0: per call, 1: weights-as-A, 2: tokens-as-A, 3: tokens-as-A on CTA pairs
+int tuned_orientation();                     // 0: per expert, 1: weights-as-A, 2 and 3: tokens-as-A on CTA pairs
 cudaError_t route_order_static(const int64_t* topk_idx, int m, int k, int num_experts, int32_t* send_count,
                                int32_t* send_offset, int32_t* route_pos, int32_t* sorted_route, cudaStream_t s);
 int route_order_static_max_tokens();

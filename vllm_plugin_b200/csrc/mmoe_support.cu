@@ -494,260 +494,440 @@ cudaError_t launch_pack(const Ctx& c, int m, cudaStream_t s) {
 }
 
 // =====================================================================================================================
-// Pool plan (one block).  Pool order: local experts ascending, each expert starting on a BLOCK_M boundary
+// Pool plan.  Pool order: local experts ascending, each expert starting on a BLOCK_M boundary
 // (backend/kernel/dispatch.py:431-447); inside an expert, source ranks ascending and each source's routes in its send
 // order (token, slot) -- a fixed order where the reference's is arrival order.
 // =====================================================================================================================
+struct PlanArgs {
+  int e_local, num_ranks, block_m, pair_above, m, has_shared;
+};
 
-// Shared expert: the call's own tokens in blocks of block_m rows; the scale chunks were written by the quantiser in the
-// layout the engine prescribes (128-row chunks inside each block, backend/staging.py:85-95), so a tile is one chunk, or
-// one of its two 64-row halves when the chunk holds more rows than a tile may.
-__device__ int emit_shared_tiles(Tile* out, int n, int block_m, int cap, bool pair) {
-  const int cpb = (block_m + kChunkRows - 1) / kChunkRows;
-  int count = 0;
-  for (int b = 0; b * block_m < n; ++b) {
-    const int in_block = min(block_m, n - b * block_m);
-    for (int s = 0; s < cpb; ++s) {
-      const int rows = min(kChunkRows, in_block - s * kChunkRows);
-      if (rows <= 0) break;
-      const int row0 = b * block_m + s * kChunkRows;
-      const int chunk = b * cpb + s;
-      if (rows > cap) {
-        out[count] = Tile{kSharedExpert, row0, 64, chunk, 0, {0, 0, 0}};
-        out[count + 1] = Tile{kSharedExpert, row0 + 64, rows - 64, chunk, 2, {0, 0, 0}};
-        count += 2;
-      } else {
-        out[count] = Tile{kSharedExpert, row0, rows, chunk, 0, {0, 0, 0}};
-        count += 1;
-      }
+// Exclusive prefix of one value pair per thread over the block (a multiple of 32 threads, at most 1024), with the totals.
+struct ScanPair {
+  uint64_t a;      // pool blocks | weights-as-A tiles << 21 | pair tiles << 42
+  int32_t b;       // rows
+};
+__device__ ScanPair block_scan_pair(ScanPair v, ScanPair* total) {
+  __shared__ uint64_t warp_a[33];
+  __shared__ int32_t warp_b[33];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+  uint64_t a = v.a;
+  int32_t b = v.b;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const uint64_t ta = __shfl_up_sync(0xffffffffu, a, d);
+    const int32_t tb = __shfl_up_sync(0xffffffffu, b, d);
+    if (lane >= d) { a += ta; b += tb; }
+  }
+  __syncthreads();                                   // an earlier scan's totals have been read
+  if (lane == 31) { warp_a[warp] = a; warp_b[warp] = b; }
+  __syncthreads();
+  if (warp == 0) {
+    const uint64_t wa = lane < nwarps ? warp_a[lane] : 0;
+    const int32_t wb = lane < nwarps ? warp_b[lane] : 0;
+    uint64_t sa = wa;
+    int32_t sb = wb;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const uint64_t ta = __shfl_up_sync(0xffffffffu, sa, d);
+      const int32_t tb = __shfl_up_sync(0xffffffffu, sb, d);
+      if (lane >= d) { sa += ta; sb += tb; }
     }
+    warp_a[lane] = sa - wa;
+    warp_b[lane] = sb - wb;
+    if (lane == 31) { warp_a[32] = sa; warp_b[32] = sb; }
   }
-  if (pair && (count & 1)) out[count++] = Tile{kSharedExpert, 0, 0, 0, 0, {0, 0, 0}};   // empty second half of the last pair
-  return count;
+  __syncthreads();
+  *total = ScanPair{warp_a[32], warp_b[32]};
+  return ScanPair{warp_a[warp] + a - v.a, warp_b[warp] + b - v.b};
 }
 
-// Routed expert: its n rows are contiguous in the pool, starting on a block_m boundary (pool block `first_block`).
-// They are cut into ceil(n / cap) equal tiles (rounded up to 16 rows) regardless of the block boundaries inside the
-// expert; for CTA pairs into an even number of them (the last may be empty), so that tiles 2j and 2j + 1 of the table
-// always belong to the same expert.  The scale chunks of the pool are this library's own: tile j of the expert uses chunk j of the
-// chunks reserved for the expert's blocks.
-__device__ __forceinline__ void tile_cut(int n, int cap, bool pair, int* parts_out, int* step_out) {
-  const int parts = pair ? 2 * ((n + 2 * cap - 1) / (2 * cap)) : (n + cap - 1) / cap;
-  *parts_out = parts;
-  *step_out = parts == 1 ? n : ((n + parts - 1) / parts + 15) & ~15;
+// The tiles of one expert (or of the shared expert) behind `out`.
+__device__ void emit_tiles(Tile* out, int expert, int row_base, int n, Cut cut, int chunk0) {
+  for (int j = 0; j < cut.parts; ++j) {
+    const int rows = max(0, min(cut.step, n - j * cut.step));
+    out[j] = Tile{expert, rows > 0 ? row_base + j * cut.step : row_base, rows, rows > 0 ? chunk0 + j : chunk0, j, cut.parts, {0, 0}};
+  }
 }
 
-__device__ int emit_tiles(Tile* out, int expert, int row_base, int n, int block_m, int cap, bool pair, int first_block,
-                          bool write) {
-  if (n <= 0) return 0;
-  int parts, step;
-  tile_cut(n, cap, pair, &parts, &step);
+// What the placement of an expert's rows needs, thread e holding expert e.
+struct ExpertPlan {
+  int block_off;     // first pool block
+  int row_off;       // rows of the experts before it
+  int small_cap;     // of the call
+  Cut cut;
+};
+
+// Builds the plan from the rows `n` of every expert, thread e holding expert e (0 past the last; e_local <= blockDim.x): tile
+// table, offsets and header, written by the blocks that pass `write`.  The whole block takes part.
+__device__ ExpertPlan build_plan(const PlanView& pv, int n, const PlanArgs& a, bool write) {
+  const int e = threadIdx.x;
+  __shared__ int s_rows;
+  if (threadIdx.x == 0) s_rows = 16;
+  // A weights-as-A stage holds five stages of up to 80 rows, or four of 112: 112 only when enough experts gain a tile by it.
+  const bool small = n > 0 && n <= a.pair_above;
+  const bool wide = small && ((n > 80 && n <= kSmallTileRows) || n > 160);
+  const int num_small = __syncthreads_count(small), num_wide = __syncthreads_count(wide);
+  const int cap = num_wide * 8 > num_small ? kSmallTileRows : 80;
+  const Cut cut = cut_rows(n, a.pair_above, cap);
+  const Cut shared_cut = cut_rows(a.has_shared ? a.m : 0, a.pair_above, cap);
+  const bool shared_small = a.m <= a.pair_above;
+  const int blocks = (n + a.block_m - 1) / a.block_m;
+  ScanPair total;
+  const ScanPair at = block_scan_pair(
+      ScanPair{static_cast<uint64_t>(blocks) | (static_cast<uint64_t>(small ? cut.parts : 0) << 21) |
+                   (static_cast<uint64_t>(small ? 0 : cut.parts) << 42), n}, &total);
+  const int block_off = static_cast<int>(at.a & 0x1FFFFF);
+  const int small_total = static_cast<int>((total.a >> 21) & 0x1FFFFF), pair_total = static_cast<int>(total.a >> 42);
   if (write) {
-    const int chunk0 = first_block * chunks_per_block(block_m);
-    for (int j = 0; j < parts; ++j)
-      out[j] = Tile{expert, row_base + j * step, max(0, min(step, n - j * step)), chunk0 + j, 0, {0, 0, 0}};
+    const int rows = small ? cut.step : 0;
+    const int warp_rows = __reduce_max_sync(0xffffffffu, rows);
+    if ((threadIdx.x & 31) == 0 && warp_rows > 0) atomicMax(&s_rows, warp_rows);
+    const int first_tile = small ? static_cast<int>((at.a >> 21) & 0x1FFFFF) : small_total + static_cast<int>(at.a >> 42);
+    if (e < a.e_local) {
+      pv.expert_total[e] = n;
+      pv.expert_block_off[e] = block_off;
+      pv.expert_tile_off[e] = first_tile;
+      emit_tiles(pv.tiles + first_tile, e, block_off * a.block_m, n, cut, block_off * chunks_per_block(a.block_m));
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      PlanHeader& h = *pv.hdr;
+      h.num_routed_tiles = small_total + pair_total;
+      h.num_shared_tiles = shared_cut.parts;
+      h.num_pool_blocks = static_cast<int>(total.a & 0x1FFFFF);
+      h.total_recv = total.b;
+      h.block_m = a.block_m;
+      h.num_tokens = a.m;
+      h.num_small_tiles = small_total;
+      h.small_cap = cap;
+      h.small_rows = max(s_rows, shared_small && a.has_shared ? shared_cut.step : 16);
+      h.shared_small = shared_small ? 1 : 0;
+      pv.expert_block_off[a.e_local] = h.num_pool_blocks;
+      pv.expert_tile_off[a.e_local] = h.num_routed_tiles;
+    }
+    if (a.has_shared)
+      for (int j = threadIdx.x; j < shared_cut.parts; j += blockDim.x) {
+        const int rows_j = max(0, min(shared_cut.step, a.m - j * shared_cut.step));
+        pv.tiles[small_total + pair_total + j] =
+            Tile{kSharedExpert, rows_j > 0 ? j * shared_cut.step : 0, rows_j, rows_j > 0 ? j : 0, j, shared_cut.parts, {0, 0}};
+      }
   }
-  return parts;
+  return ExpertPlan{block_off, at.b, cap, cut};
+}
+
+// Scale words of the call's own tokens in the chunks of the shared expert's tiles (chunk j = tile j), whole warps.
+struct SharedScales {
+  const int32_t* x_sf;
+  int32_t* out;          // nullptr: no shared expert
+  int64_t rows;
+};
+__device__ void place_shared_scales(const SharedScales& s, Cut cut, int t, int words) {
+  const int j = t / cut.step;
+  const int64_t pos = (int64_t)j * kChunkRows + chunk_pos(t - j * cut.step);
+  for (int w = threadIdx.x & 31; w < words; w += 32) s.out[w * s.rows + pos] = s.x_sf[(int64_t)t * words + w];
 }
 
 // The shared expert's tiles depend only on the token count, so they can be planned (and run) before the routed
 // experts' receive counts are known: written at the tail of the tile table, counted in the header.
-__global__ void shared_plan_kernel(char* __restrict__ plan_base, int e_local, int num_ranks, int m, int block_m,
-                                   int cap, int pair, int64_t first_tile) {
+__global__ void __launch_bounds__(256) shared_plan_kernel(char* __restrict__ plan_base, int e_local, int num_ranks, int m,
+                                                          int pair_above, int64_t first_tile, SharedScales scales, int words) {
   chain_begin();
-  if (threadIdx.x == 0 && blockIdx.x == 0) {
+  const Cut cut = cut_rows(m, pair_above, kSmallTileRows);
+  if (blockIdx.x == 0) {
     PlanView pv = plan_view(plan_base, e_local, num_ranks);
-    pv.hdr->num_early_shared_tiles = emit_shared_tiles(pv.tiles + first_tile, m, block_m, cap, pair != 0);
+    for (int j = threadIdx.x; j < cut.parts; j += blockDim.x) {
+      const int rows = max(0, min(cut.step, m - j * cut.step));
+      pv.tiles[first_tile + j] = Tile{kSharedExpert, rows > 0 ? j * cut.step : 0, rows, rows > 0 ? j : 0, j, cut.parts, {0, 0}};
+    }
+    if (threadIdx.x == 0) {
+      pv.hdr->num_early_shared_tiles = cut.parts;
+      pv.hdr->early_small_rows = m <= pair_above ? cut.step : 0;
+    }
   }
+  const int warps = (gridDim.x * blockDim.x) >> 5;
+  for (int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < m; t += warps) place_shared_scales(scales, cut, t, words);
 }
 
-__global__ void __launch_bounds__(1024) plan_kernel(
-    char* __restrict__ plan_base, const int32_t* __restrict__ recv_count, int32_t* __restrict__ stats, int e_local,
-    int num_ranks, int block_m, int cap, int pair, int m, int has_shared) {
+// General plan (any number of source ranks), one block: rows per expert from the receive counts, and for every (expert,
+// source) segment where it starts in the pool and in receive order.
+constexpr int kPlanThreads = 512;      // one thread per local expert
+__global__ void __launch_bounds__(kPlanThreads) plan_kernel(char* __restrict__ plan_base, const int32_t* __restrict__ recv_count,
+                                                            int32_t* __restrict__ stats, PlanArgs a) {
   chain_begin();
-  PlanView pv = plan_view(plan_base, e_local, num_ranks);
-  __shared__ int32_t s_blocks[513], s_tiles[513];
-  // per-source totals -> rank offsets in receive order
-  if (threadIdx.x <= num_ranks) {
-    // rank_off[r] = sum over sources < r of all their routes to this rank
-    int run = 0;
-    for (int r = 0; r < (int)threadIdx.x; ++r)
-      for (int e = 0; e < e_local; ++e) run += recv_count[r * e_local + e];
-    pv.rank_off[threadIdx.x] = run;
-    if ((int)threadIdx.x == num_ranks) pv.hdr->total_recv = run;
+  PlanView pv = plan_view(plan_base, a.e_local, a.num_ranks);
+  const int e = threadIdx.x;
+  int n = 0;
+  if (e < a.e_local)
+    for (int r = 0; r < a.num_ranks; ++r) n += recv_count[r * a.e_local + e];
+  if (stats != nullptr && e < a.e_local) stats[e] += n;      // cumulative per-expert receive statistics (dispatch.py:644-650)
+  const ExpertPlan ep = build_plan(pv, n, a, true);
+  int rank_off = 0, pool_row = ep.block_off * a.block_m;
+  for (int r = 0; r < a.num_ranks; ++r) {
+    const int c = e < a.e_local ? recv_count[r * a.e_local + e] : 0;
+    ScanPair total;
+    const ScanPair at = block_scan_pair(ScanPair{0, c}, &total);
+    if (e < a.e_local) {
+      pv.seg_recv_start[e * a.num_ranks + r] = rank_off + at.b;
+      pv.seg_pool_start[e * a.num_ranks + r] = pool_row;
+    }
+    if (e == 0) pv.rank_off[r] = rank_off;
+    rank_off += total.b;
+    pool_row += c;
   }
-  for (int e = threadIdx.x; e < e_local; e += blockDim.x) {
-    int tot = 0;
-    for (int r = 0; r < num_ranks; ++r) tot += recv_count[r * e_local + e];
-    pv.expert_total[e] = tot;
-    s_blocks[e] = (tot + block_m - 1) / block_m;
-    s_tiles[e] = emit_tiles(nullptr, e, 0, tot, block_m, cap, pair != 0, 0, false);
-    if (stats != nullptr) stats[e] += tot;      // cumulative per-expert receive statistics (dispatch.py:644-650)
-  }
-  __shared__ int32_t s_boff[514], s_toff[514];
-  block_exclusive_scan(s_blocks, s_boff, e_local);
-  block_exclusive_scan(s_tiles, s_toff, e_local);
-  for (int e = threadIdx.x; e <= e_local; e += blockDim.x) {
-    pv.expert_block_off[e] = s_boff[e];
-    pv.expert_tile_off[e] = s_toff[e];
-  }
-  if (threadIdx.x == 0) {
-    const int rt = s_toff[e_local];
-    pv.hdr->num_routed_tiles = rt;
-    pv.hdr->num_pool_blocks = s_boff[e_local];
-    pv.hdr->block_m = block_m;
-    pv.hdr->num_tokens = m;
-    // shared-expert tiles: the call's own tokens in blocks of block_m (chunk numbering of backend/staging.py:85-95)
-    int ns = 0;
-    if (has_shared) ns = emit_shared_tiles(pv.tiles + rt, m, block_m, cap, pair != 0);
-    pv.hdr->num_shared_tiles = ns;
+  if (e == 0) pv.rank_off[a.num_ranks] = rank_off;
+}
+
+// =====================================================================================================================
+// One GPU: route ordering, plan and placement without the detour over receive counts.  Same results as
+// sort_local/scan/place + plan_kernel + place_kernel (tested against them).
+// =====================================================================================================================
+constexpr int kRouteThreads = 512;     // one thread per expert in the plan, 16 warps that rank routes
+constexpr int kRouteWarps = kRouteThreads / 32;
+
+// Stable rank of up to kSortChunkTokens * k routes among the routes of the same expert, by the whole block: every warp ranks
+// a run of its own against its own counters (lanes with the same expert find each other with match.any), then each
+// expert's counters are summed over the warps.  ids[i] (0xFFFF = masked) -> rank[i]; returns thread e's expert total.
+// (One warp walking all routes took 10 us for 768; 16 warps take 2.)
+__device__ int block_rank_routes(const uint16_t* ids, int n, uint16_t* rank, uint16_t* warp_count, int num_experts) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int i = threadIdx.x; i < kRouteWarps * num_experts; i += kRouteThreads) warp_count[i] = 0;
+  __syncthreads();                                   // ids are in place too
+  const int run = ((n + kRouteWarps - 1) / kRouteWarps + 31) & ~31;
+  uint16_t* mine = warp_count + warp * num_experts;
+  const int end = min(n, (warp + 1) * run);
+  for (int base = warp * run; base < end; base += 32) {
+    const int i = base + lane;
+    const int e = i < end ? ids[i] : 0xFFFF;
+    const unsigned peers = __match_any_sync(0xffffffffu, e);
+    const int before = __popc(peers & ((1u << lane) - 1u));
+    const int start = e != 0xFFFF ? mine[e] : 0;
+    __syncwarp();
+    if (e != 0xFFFF && before == 0) mine[e] = static_cast<uint16_t>(start + __popc(peers));
+    __syncwarp();
+    if (i < end) rank[i] = static_cast<uint16_t>(start + before);
   }
   __syncthreads();
-  // per-source cumulative offsets over experts in receive order (one thread per source rank)
-  if ((int)threadIdx.x < num_ranks) {
-    const int r = threadIdx.x;
-    int run = pv.rank_off[r];
-    for (int e = 0; e < e_local; ++e) {
-      pv.seg_recv_start[e * num_ranks + r] = run;
-      run += recv_count[r * e_local + e];
+  int total = 0;
+  if ((int)threadIdx.x < num_experts)
+#pragma unroll
+    for (int w = 0; w < kRouteWarps; ++w) {
+      const int c = warp_count[w * num_experts + threadIdx.x];
+      warp_count[w * num_experts + threadIdx.x] = static_cast<uint16_t>(total);
+      total += c;
     }
-  }
-  for (int e = threadIdx.x; e < e_local; e += blockDim.x) {
-    int run = pv.expert_block_off[e] * block_m;
-    for (int r = 0; r < num_ranks; ++r) {
-      pv.seg_pool_start[e * num_ranks + r] = run;
-      run += recv_count[r * e_local + e];
-    }
-    emit_tiles(pv.tiles + pv.expert_tile_off[e], e, pv.expert_block_off[e] * block_m, pv.expert_total[e], block_m, cap,
-               pair != 0, pv.expert_block_off[e], true);
-  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < n; i += kRouteThreads)
+    if (ids[i] != 0xFFFF) rank[i] = static_cast<uint16_t>(rank[i] + warp_count[(i / run) * num_experts + ids[i]]);
+  __syncthreads();
+  return total;
 }
 
-// Decode path at EP1 (one chunk of at most 128 tokens): route ordering and pool plan in ONE single-block launch
-// instead of four, because at a handful of tokens the layer is bound by launch latency.  Same results as
-// sort_local/scan/place + plan_kernel (tested against them).
-// Placement arguments of route_plan_small_kernel (pool_x == nullptr: the placement kernel follows as its own launch)
-struct SmallPlace {
-  const uint4* src_x;
-  const int32_t* src_sf;
-  const float* src_w;
+struct RouteArgs {
+  const int64_t* topk_idx;
+  int32_t* route_pos;
+  int32_t* sorted_route;
+  int32_t* send_count;
+  int32_t* send_offset;
+  int32_t* recv_count;
+  int32_t* chunk_count;      // [chunks][E]
+  int32_t* stats;
+  int32_t* status;
+  char* plan;
+  const uint4* x;
+  const int32_t* x_sf;
+  const float* w;
   uint4* pool_x;
   int32_t* pool_sf;
   float* pool_w;
   int32_t* pool_dst;
   int64_t pool_sf_rows;
-  int h;
+  SharedScales shared;
+  int h, k;
+  PlanArgs a;
 };
 
-__global__ void __launch_bounds__(1024) route_plan_small_kernel(
-    const int64_t* __restrict__ topk_idx, int32_t* __restrict__ route_pos, int32_t* __restrict__ sorted_route,
-    int32_t* __restrict__ send_count, int32_t* __restrict__ send_offset, int32_t* __restrict__ recv_count,
-    char* __restrict__ plan_base, int32_t* __restrict__ stats, int32_t* __restrict__ status, int m, int k,
-    int num_experts, int block_m, int cap, int pair, int has_shared, SmallPlace place) {
+// everything of the plan that is the same for every caller with one source rank
+__device__ void write_single_rank_plan(const RouteArgs& r, const PlanView& pv, int n, const ExpertPlan& ep) {
+  const int e = threadIdx.x;
+  if (e < r.a.e_local) {
+    r.send_count[e] = n;
+    r.recv_count[e] = n;
+    r.send_offset[e] = ep.row_off;
+    pv.seg_pool_start[e] = ep.block_off * r.a.block_m;
+    pv.seg_recv_start[e] = ep.row_off;
+    if (r.stats != nullptr) r.stats[e] += n;         // cumulative per-expert receive statistics (dispatch.py:644-650)
+    if (e == r.a.e_local - 1) {
+      r.send_offset[r.a.e_local] = ep.row_off + n;
+      pv.rank_off[0] = 0;
+      pv.rank_off[1] = ep.row_off + n;
+    }
+  }
+}
+
+// Calls of at most 128 tokens: ONE launch.  Every block ranks the routes and builds the plan for itself in shared memory
+// (2-3 us, less than a second launch behind a grid-wide hand-over), block 0 writes it out, and each block places its share
+// of the routes, one warp per route.
+__global__ void __launch_bounds__(kRouteThreads) route_small_kernel(const RouteArgs r) {
   chain_begin();
   extern __shared__ int32_t sm[];
-  int32_t* ids = sm;                              // [m*k]
-  int32_t* hist = sm + kSortChunkTokens * k;      // [E]
-  int32_t* off = hist + num_experts;              // [E+1]  send offsets
-  int32_t* boff = off + num_experts + 1;          // [E+1]  pool block offsets
-  int32_t* toff = boff + num_experts + 1;         // [E+1]  tile offsets
-  PlanView pv = plan_view(plan_base, num_experts, 1);
-  const int n = m * k;
-  for (int e = threadIdx.x; e < num_experts; e += blockDim.x) hist[e] = 0;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    int64_t id = topk_idx[i];
-    if (id >= num_experts) { report_bad_index(status); id = -1; }
-    ids[i] = id < 0 ? -1 : static_cast<int32_t>(id);
+  const int E = r.a.e_local, n = r.a.m * r.k, n_even = (n + 1) & ~1;
+  int32_t* s_block = sm;                             // [E] first pool block
+  int32_t* s_off = s_block + E;                      // [E] send offset
+  int32_t* s_step = s_off + E;                       // [E] rows per tile
+  uint16_t* ids = reinterpret_cast<uint16_t*>(s_step + E);
+  uint16_t* rank = ids + n_even;
+  uint16_t* warp_count = rank + n_even;              // [16][E]
+  for (int i = threadIdx.x; i < n; i += kRouteThreads) {
+    int64_t id = r.topk_idx[i];
+    if (id >= E) { if (blockIdx.x == 0) report_bad_index(r.status); id = -1; }
+    ids[i] = id < 0 ? 0xFFFF : static_cast<uint16_t>(id);
   }
-  __syncthreads();
-  int32_t* rank = toff + num_experts + 1;         // [m*k]
-  if (threadIdx.x < 32) warp_rank_routes(ids, n, hist, rank);
-  __syncthreads();
-  int32_t* blocks = rank + kSortChunkTokens * k;  // [E] scratch of the scans
-  int32_t* tiles_n = blocks + num_experts;        // [E]
-  for (int e = threadIdx.x; e < num_experts; e += blockDim.x) {
-    const int tot = hist[e];
-    blocks[e] = (tot + block_m - 1) / block_m;
-    tiles_n[e] = emit_tiles(nullptr, e, 0, tot, block_m, cap, pair != 0, 0, false);
+  const int total = block_rank_routes(ids, n, rank, warp_count, E);
+  const PlanView pv = plan_view(r.plan, E, 1);
+  const ExpertPlan ep = build_plan(pv, total, r.a, blockIdx.x == 0);
+  if ((int)threadIdx.x < E) {
+    s_block[threadIdx.x] = ep.block_off;
+    s_off[threadIdx.x] = ep.row_off;
+    s_step[threadIdx.x] = ep.cut.step;
   }
-  block_exclusive_scan(hist, off, num_experts);
-  block_exclusive_scan(blocks, boff, num_experts);
-  block_exclusive_scan(tiles_n, toff, num_experts);
-  if (threadIdx.x == 0) {
-    const int to = toff[num_experts];
-    pv.hdr->num_routed_tiles = to;
-    pv.hdr->num_pool_blocks = boff[num_experts];
-    pv.hdr->total_recv = off[num_experts];
-    pv.hdr->block_m = block_m;
-    pv.hdr->num_tokens = m;
-    pv.hdr->num_shared_tiles = has_shared ? emit_shared_tiles(pv.tiles + to, m, block_m, cap, pair != 0) : 0;
-    pv.rank_off[0] = 0;
-    pv.rank_off[1] = off[num_experts];
-  }
+  if (blockIdx.x == 0) write_single_rank_plan(r, pv, total, ep);
   __syncthreads();
+  const int lane = threadIdx.x & 31, warps = gridDim.x * kRouteWarps;
+  const int vec = r.h / 16, words = r.h / kTileK, cpb = chunks_per_block(r.a.block_m);
+  for (int i = blockIdx.x * kRouteWarps + (threadIdx.x >> 5); i < n; i += warps) {
+    const int e = ids[i];
+    if (e == 0xFFFF) {
+      if (lane == 0) r.route_pos[i] = -1;
+      continue;
+    }
+    const int j = rank[i], t = i / r.k;
+    const int p = s_block[e] * r.a.block_m + j, part = j / s_step[e];
+    const uint4* src = r.x + (int64_t)t * vec;
+    uint4* dst = r.pool_x + (int64_t)p * vec;
+    for (int v0 = lane; v0 < vec; v0 += 128) {
+      uint4 q[4];
 #pragma unroll
-  for (int u = 0; u < 4; ++u) {
-    const int i = threadIdx.x + u * blockDim.x;
-    if (i < n) {
-      int pos = -1;
-      if (rank[i] >= 0) {
-        pos = off[ids[i]] + rank[i];
-        sorted_route[pos] = i;
-      }
-      route_pos[i] = pos;
+      for (int u = 0; u < 4; ++u)
+        if (v0 + 32 * u < vec) q[u] = src[v0 + 32 * u];
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (v0 + 32 * u < vec) dst[v0 + 32 * u] = q[u];
+    }
+    const int64_t pos = (int64_t)(s_block[e] * cpb + part) * kChunkRows + chunk_pos(j - part * s_step[e]);
+    for (int wd = lane; wd < words; wd += 32) r.pool_sf[wd * r.pool_sf_rows + pos] = r.x_sf[(int64_t)t * words + wd];
+    if (lane == 0) {
+      r.pool_w[p] = r.w[i];
+      r.pool_dst[p] = s_off[e] + j;
+      r.route_pos[i] = s_off[e] + j;
+      r.sorted_route[s_off[e] + j] = i;
     }
   }
-  for (int e = threadIdx.x; e < num_experts; e += blockDim.x) {
-    const int tot = hist[e];
-    send_count[e] = tot;
-    recv_count[e] = tot;
-    send_offset[e] = off[e];
-    pv.expert_total[e] = tot;
-    pv.expert_block_off[e] = boff[e];
-    pv.expert_tile_off[e] = toff[e];
-    pv.seg_pool_start[e] = boff[e] * block_m;
-    pv.seg_recv_start[e] = off[e];
-    if (stats != nullptr) stats[e] += tot;
-    emit_tiles(pv.tiles + toff[e], e, boff[e] * block_m, tot, block_m, cap, pair != 0, boff[e], true);
+  if (r.shared.out != nullptr) {
+    const Cut cut = cut_rows(r.a.m, r.a.pair_above, ep.small_cap);
+    for (int t = blockIdx.x * kRouteWarps + (threadIdx.x >> 5); t < r.a.m; t += warps) place_shared_scales(r.shared, cut, t, words);
   }
-  if (threadIdx.x == 0) {
-    send_offset[num_experts] = off[num_experts];
-    pv.expert_block_off[num_experts] = boff[num_experts];
-    pv.expert_tile_off[num_experts] = toff[num_experts];
+}
+
+// Larger calls, first of two launches: one block per 128 tokens ranks its routes; the last block to finish sums the chunks
+// and builds the plan.
+__global__ void __launch_bounds__(kRouteThreads) route_count_kernel(const RouteArgs r) {
+  chain_begin();
+  extern __shared__ int32_t sm[];
+  const int E = r.a.e_local, r0 = blockIdx.x * kSortChunkTokens * r.k;
+  const int n = max(0, min(kSortChunkTokens * r.k, r.a.m * r.k - r0)), n_even = (kSortChunkTokens * r.k + 1) & ~1;
+  uint16_t* ids = reinterpret_cast<uint16_t*>(sm);
+  uint16_t* rank = ids + n_even;
+  uint16_t* warp_count = rank + n_even;
+  for (int i = threadIdx.x; i < n; i += kRouteThreads) {
+    int64_t id = r.topk_idx[r0 + i];
+    if (id >= E) { report_bad_index(r.status); id = -1; }
+    ids[i] = id < 0 ? 0xFFFF : static_cast<uint16_t>(id);
   }
-  // A handful of routes: this block also places them (one warp per route), which saves the placement launch.  Route i
-  // of expert e with rank r among the expert's routes is pool row boff[e] * block_m + r, row r - j * step of the
-  // expert's tile j (the cut emit_tiles makes).
-  if (place.pool_x != nullptr) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
-    const int vec = place.h / 16, words = place.h / kTileK;
-    for (int i = warp; i < n; i += warps) {
-      if (rank[i] < 0) continue;
-      const int e = ids[i], r = rank[i];
-      int parts, step;
-      tile_cut(hist[e], cap, pair != 0, &parts, &step);
-      const int j = r / step;
-      const int p = boff[e] * block_m + r;
-      const int64_t src_row = i / k;
-      const uint4* src = place.src_x + src_row * vec;
-      uint4* dst = place.pool_x + (int64_t)p * vec;
-      for (int v0 = lane; v0 < vec; v0 += 128) {
-        uint4 q[4];
+  int total = block_rank_routes(ids, n, rank, warp_count, E);
+  for (int i = threadIdx.x; i < n; i += kRouteThreads) r.route_pos[r0 + i] = ids[i] == 0xFFFF ? -1 : rank[i];
+  const int e = threadIdx.x;
+  if (e < E) r.chunk_count[(int64_t)blockIdx.x * E + e] = total;
+  const PlanView pv = plan_view(r.plan, E, 1);
+  __shared__ int last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(&pv.hdr->ticket, 1) == (int)gridDim.x - 1;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  if (threadIdx.x == 0) pv.hdr->ticket = 0;
+  total = 0;
+  if (e < E)
+    for (int c0 = 0; c0 < (int)gridDim.x; c0 += 8) {         // eight independent loads in flight
+      int v[8];
 #pragma unroll
-        for (int u = 0; u < 4; ++u)
-          if (v0 + 32 * u < vec) q[u] = src[v0 + 32 * u];
+      for (int u = 0; u < 8; ++u) v[u] = c0 + u < (int)gridDim.x ? __ldcg(&r.chunk_count[(int64_t)(c0 + u) * E + e]) : 0;
 #pragma unroll
-        for (int u = 0; u < 4; ++u)
+      for (int u = 0; u < 8; ++u) {
+        if (c0 + u < (int)gridDim.x) r.chunk_count[(int64_t)(c0 + u) * E + e] = total;
+        total += v[u];
+      }
+    }
+  const ExpertPlan ep = build_plan(pv, total, r.a, true);
+  write_single_rank_plan(r, pv, total, ep);
+}
+
+// Second launch: one warp per token.  The token's FP8 row is read once and stored to the pool rows of all its routes; lane s
+// works out where route s goes.
+__global__ void __launch_bounds__(256) route_place_kernel(const RouteArgs r) {
+  chain_begin();
+  const PlanView pv = plan_view(r.plan, r.a.e_local, 1);
+  const int lane = threadIdx.x & 31, warps = (gridDim.x * blockDim.x) >> 5;
+  const int vec = r.h / 16, words = r.h / kTileK, cpb = chunks_per_block(r.a.block_m);
+  const int cap = pv.hdr->small_cap;
+  const Cut shared_cut = cut_rows(r.a.m, r.a.pair_above, cap);
+  for (int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < r.a.m; t += warps) {
+    int row = -1, sf_pos = 0;                          // lane s: pool row and scale position of route s
+    if (lane < r.k) {
+      const int i = t * r.k + lane;
+      const int64_t id = r.topk_idx[i];
+      int pos = -1;
+      if (id >= 0 && id < r.a.e_local) {
+        const int e = static_cast<int>(id);
+        const int j = r.chunk_count[(int64_t)(t / kSortChunkTokens) * r.a.e_local + e] + r.route_pos[i];
+        const int block = pv.expert_block_off[e];
+        const Cut cut = cut_rows(pv.expert_total[e], r.a.pair_above, cap);
+        const int part = j / cut.step;
+        pos = r.send_offset[e] + j;
+        row = block * r.a.block_m + j;
+        sf_pos = (block * cpb + part) * kChunkRows + chunk_pos(j - part * cut.step);
+        r.sorted_route[pos] = i;
+        r.pool_w[row] = r.w[i];
+        r.pool_dst[row] = pos;
+      }
+      r.route_pos[i] = pos;
+    }
+    const uint4* src = r.x + (int64_t)t * vec;
+    for (int base = 0; base < vec; base += 160) {
+      const int v0 = base + lane;
+      uint4 q[5];
+#pragma unroll
+      for (int u = 0; u < 5; ++u)
+        if (v0 + 32 * u < vec) q[u] = src[v0 + 32 * u];
+      for (int s = 0; s < r.k; ++s) {
+        const int p = __shfl_sync(0xffffffffu, row, s);
+        if (p < 0) continue;
+        uint4* dst = r.pool_x + (int64_t)p * vec;
+#pragma unroll
+        for (int u = 0; u < 5; ++u)
           if (v0 + 32 * u < vec) dst[v0 + 32 * u] = q[u];
       }
-      const int pos = (boff[e] * chunks_per_block(block_m) + j) * kChunkRows + chunk_pos(r - j * step);
-      for (int wd = lane; wd < words; wd += 32)
-        place.pool_sf[(int64_t)wd * place.pool_sf_rows + pos] = place.src_sf[src_row * words + wd];
-      if (lane == 0) {
-        place.pool_w[p] = place.src_w[i];
-        place.pool_dst[p] = off[e] + r;
+    }
+    for (int w0 = 0; w0 < words; w0 += 32) {
+      const int wd = w0 + lane;
+      const int32_t v = wd < words ? r.x_sf[(int64_t)t * words + wd] : 0;
+      for (int s = 0; s < r.k; ++s) {
+        const int p = __shfl_sync(0xffffffffu, row, s), pos = __shfl_sync(0xffffffffu, sf_pos, s);
+        if (p >= 0 && wd < words) r.pool_sf[wd * r.pool_sf_rows + pos] = v;
       }
     }
+    if (r.shared.out != nullptr) place_shared_scales(r.shared, shared_cut, t, words);
   }
 }
 
@@ -759,14 +939,19 @@ __global__ void __launch_bounds__(256) place_kernel(
     char* __restrict__ plan_base, const uint4* __restrict__ src_x, const int32_t* __restrict__ src_sf,
     const float* __restrict__ src_w, const int32_t* __restrict__ sorted_route, uint4* __restrict__ pool_x,
     int32_t* __restrict__ pool_sf, float* __restrict__ pool_w, int32_t* __restrict__ pool_dst, int64_t pool_sf_rows,
-    int e_local, int num_ranks, int h, int k, int direct) {
+    int e_local, int num_ranks, int h, int k, int direct, int pair_above, SharedScales shared) {
   chain_begin();
   PlanView pv = plan_view(plan_base, e_local, num_ranks);
   const int ntiles = pv.hdr->num_routed_tiles;
   const int block_m = pv.hdr->block_m;
   const int vec = h / 16, words = h / kTileK;
   const int warp_in_block = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
-  constexpr int kSlices = (kTokenMajorTileRows + 31) / 32;
+  if (shared.out != nullptr) {
+    const int m = pv.hdr->num_tokens;
+    const Cut cut = cut_rows(m, pair_above, pv.hdr->small_cap);
+    for (int t = blockIdx.x * warps + warp_in_block; t < m; t += gridDim.x * warps) place_shared_scales(shared, cut, t, words);
+  }
+  constexpr int kSlices = kPairTileRows / 32;
   for (int task = blockIdx.x; task < ntiles * kSlices; task += gridDim.x) {
     const int slice = task / ntiles, t = task - slice * ntiles;   // slice-major: the first slices are the populated ones
     const Tile tile = pv.tiles[t];
@@ -804,7 +989,7 @@ __global__ void __launch_bounds__(256) place_kernel(
         for (int u = 0; u < 4; ++u)
           if (v0 + 32 * u < vec) dst[v0 + 32 * u] = q[u];
       }
-      const int pos = tile.sf_chunk * kChunkRows + chunk_pos(tile.sf_col * 32 + i);
+      const int pos = tile.sf_chunk * kChunkRows + chunk_pos(i);
       for (int wd = lane; wd < words; wd += 32) pool_sf[(int64_t)wd * pool_sf_rows + pos] = src_sf[src_row * words + wd];
       if (lane == 0) {
         pool_w[p] = w;
@@ -814,47 +999,79 @@ __global__ void __launch_bounds__(256) place_kernel(
   }
 }
 
-// EP1, M <= 128: fused route ordering + plan; up to 128 routes the same block also places them, beyond that the
-// placement kernel follows
-cudaError_t launch_route_plan_place_small(const Ctx& c, int m, int block_m, int32_t* stats, cudaStream_t s) {
-  const int k = c.geo.num_topk, e = c.geo.num_experts;
-  const size_t smem = (size_t)(2 * kSortChunkTokens * k + 6 * e + 3) * sizeof(int32_t);
-  const bool place_here = m * k <= 128;
-  SmallPlace place = {};
-  if (place_here)
-    place = SmallPlace{c.at<uint4>(c.lay.x), c.at<int32_t>(c.lay.x_sf), c.at<float>(c.lay.topk_weights),
-                       c.at<uint4>(c.lay.pool_x), c.at<int32_t>(c.lay.pool_sf), c.at<float>(c.lay.pool_w),
-                       c.at<int32_t>(c.lay.pool_dst), c.lay.pool_sf_rows, c.geo.hidden};
-  launch_chained(route_plan_small_kernel, dim3(1), dim3(1024), smem, s, c.at<int64_t>(c.lay.topk_idx),
-                 c.at<int32_t>(c.lay.route_pos), c.at<int32_t>(c.lay.sorted_route), c.at<int32_t>(c.lay.send_count),
-                 c.at<int32_t>(c.lay.send_offset), c.at<int32_t>(c.lay.recv_count), c.ws + c.lay.plan, stats,
-                 c.at<int32_t>(c.lay.status), m, k, e, block_m, tile_cap(block_m, c.family),
-                 c.family == kFamilyTokensAsAPair, c.geo.num_shared_experts > 0, place);
-  if (!place_here)
-    launch_chained(place_kernel, dim3(148 * 2), dim3(256), 0, s, c.ws + c.lay.plan, c.at<uint4>(c.lay.x),
-                   c.at<int32_t>(c.lay.x_sf), c.at<float>(c.lay.topk_weights), c.at<int32_t>(c.lay.sorted_route),
-                   c.at<uint4>(c.lay.pool_x), c.at<int32_t>(c.lay.pool_sf), c.at<float>(c.lay.pool_w),
-                   c.at<int32_t>(c.lay.pool_dst), c.lay.pool_sf_rows, c.e_local, 1, c.geo.hidden, c.geo.num_topk, 1);
+namespace {
+PlanArgs plan_args(const Ctx& c, int m, int block_m) {
+  return PlanArgs{c.e_local, c.geo.num_ranks, block_m, c.pair_above_for(m), m, c.geo.num_shared_experts > 0 && m > 0 ? 1 : 0};
+}
+
+SharedScales shared_scales(const Ctx& c, int m) {
+  const bool on = c.geo.num_shared_experts > 0 && m > 0;
+  return SharedScales{c.at<int32_t>(c.lay.x_sf), on ? c.at<int32_t>(c.lay.shared_tile_sf) : nullptr, shared_chunk_rows(c.geo.num_max_tokens)};
+}
+
+RouteArgs route_args(const Ctx& c, int m, int block_m, int32_t* stats) {
+  RouteArgs r{};
+  r.topk_idx = c.at<int64_t>(c.lay.topk_idx);
+  r.route_pos = c.at<int32_t>(c.lay.route_pos);
+  r.sorted_route = c.at<int32_t>(c.lay.sorted_route);
+  r.send_count = c.at<int32_t>(c.lay.send_count);
+  r.send_offset = c.at<int32_t>(c.lay.send_offset);
+  r.recv_count = c.at<int32_t>(c.lay.recv_count);
+  r.chunk_count = c.at<int32_t>(c.lay.sort_scratch);
+  r.stats = stats;
+  r.status = c.at<int32_t>(c.lay.status);
+  r.plan = c.ws + c.lay.plan;
+  r.x = c.at<uint4>(c.lay.x);
+  r.x_sf = c.at<int32_t>(c.lay.x_sf);
+  r.w = c.at<float>(c.lay.topk_weights);
+  r.pool_x = c.at<uint4>(c.lay.pool_x);
+  r.pool_sf = c.at<int32_t>(c.lay.pool_sf);
+  r.pool_w = c.at<float>(c.lay.pool_w);
+  r.pool_dst = c.at<int32_t>(c.lay.pool_dst);
+  r.pool_sf_rows = c.lay.pool_sf_rows;
+  r.shared = shared_scales(c, m);
+  r.h = c.geo.hidden;
+  r.k = c.geo.num_topk;
+  r.a = plan_args(c, m, block_m);
+  return r;
+}
+}  // namespace
+
+cudaError_t launch_route_small(const Ctx& c, int m, int block_m, int32_t* stats, cudaStream_t s) {
+  const int n = m * c.geo.num_topk, e = c.geo.num_experts;
+  const size_t smem = (size_t)3 * e * 4 + (size_t)2 * ((n + 1) & ~1) * 2 + (size_t)kRouteWarps * e * 2;
+  launch_chained(route_small_kernel, dim3(std::min((n + kRouteWarps - 1) / kRouteWarps, 148)), dim3(kRouteThreads), smem, s,
+                 route_args(c, m, block_m, stats));
+  return cudaGetLastError();
+}
+
+cudaError_t launch_route_large(const Ctx& c, int m, int block_m, int32_t* stats, cudaStream_t s) {
+  const RouteArgs r = route_args(c, m, block_m, stats);
+  const int chunks = std::max(1, (m + kSortChunkTokens - 1) / kSortChunkTokens);
+  const size_t smem = (size_t)2 * ((kSortChunkTokens * r.k + 1) & ~1) * 2 + (size_t)kRouteWarps * r.a.e_local * 2;
+  launch_chained(route_count_kernel, dim3(chunks), dim3(kRouteThreads), smem, s, r);
+  if (m > 0) launch_chained(route_place_kernel, dim3(std::min((m + 7) / 8, 148 * 8)), dim3(256), 0, s, r);
   return cudaGetLastError();
 }
 
 cudaError_t launch_shared_plan(const Ctx& c, int m, int block_m, cudaStream_t s) {
-  launch_chained(shared_plan_kernel, dim3(1), dim3(32), 0, s, c.ws + c.lay.plan, c.e_local, c.geo.num_ranks, m, block_m,
-                                      tile_cap(block_m, c.family), c.family == kFamilyTokensAsAPair, c.lay.max_tiles - shared_tile_capacity(c.geo.num_max_tokens));
+  (void)block_m;
+  launch_chained(shared_plan_kernel, dim3(std::max(1, std::min((m + 7) / 8, 148 * 2))), dim3(256), 0, s, c.ws + c.lay.plan, c.e_local,
+                 c.geo.num_ranks, m, c.pair_above_for(m), c.lay.max_tiles - shared_tile_capacity(c.geo.num_max_tokens),
+                 shared_scales(c, m), c.geo.hidden / kTileK);
   return cudaGetLastError();
 }
 
 cudaError_t launch_plan_place(const Ctx& c, int m, int block_m, int32_t* stats, cudaStream_t s) {
   const int R = c.geo.num_ranks;
-  launch_chained(plan_kernel, dim3(1), dim3(1024), 0, s, c.ws + c.lay.plan, c.at<int32_t>(c.lay.recv_count), stats, c.e_local, R, block_m,
-                                 tile_cap(block_m, c.family), c.family == kFamilyTokensAsAPair, m,
-                                 c.geo.num_shared_experts > 0);
+  launch_chained(plan_kernel, dim3(1), dim3(kPlanThreads), 0, s, c.ws + c.lay.plan, c.at<int32_t>(c.lay.recv_count), stats,
+                 plan_args(c, m, block_m));
   const bool direct = R == 1;
   launch_chained(place_kernel, dim3(148 * 8), dim3(256), 0, s, c.ws + c.lay.plan, direct ? c.at<uint4>(c.lay.x) : c.at<uint4>(c.lay.recv_x),
       direct ? c.at<int32_t>(c.lay.x_sf) : c.at<int32_t>(c.lay.recv_sf),
       direct ? c.at<float>(c.lay.topk_weights) : c.at<float>(c.lay.recv_w), c.at<int32_t>(c.lay.sorted_route),
       c.at<uint4>(c.lay.pool_x), c.at<int32_t>(c.lay.pool_sf), c.at<float>(c.lay.pool_w), c.at<int32_t>(c.lay.pool_dst),
-      c.lay.pool_sf_rows, c.e_local, R, c.geo.hidden, c.geo.num_topk, direct ? 1 : 0);
+      c.lay.pool_sf_rows, c.e_local, R, c.geo.hidden, c.geo.num_topk, direct ? 1 : 0, c.pair_above_for(m), shared_scales(c, m));
   return cudaGetLastError();
 }
 
@@ -950,7 +1167,7 @@ __device__ __forceinline__ uint32_t weight_sf_byte(const int32_t* __restrict__ s
 
 __device__ __forceinline__ uint32_t token_sf_byte(const int32_t* __restrict__ sf, int64_t sf_rows, const Tile& tile,
                                                   int i, int g) {
-  const int pos = tile.sf_chunk * kChunkRows + chunk_pos(tile.sf_col * 32 + i);
+  const int pos = tile.sf_chunk * kChunkRows + chunk_pos(i);
   const uint32_t word = static_cast<uint32_t>(sf[(int64_t)(g / 4) * sf_rows + pos]);
   return (word >> (8 * (g % 4))) & 0xFFu;
 }
@@ -1014,7 +1231,7 @@ __global__ void __launch_bounds__(128) simt_l1_kernel(
       const int sf_exp = ue8m0_exp_of_amax(amax);
       act_x[(int64_t)(tile.row0 + i) * inter + c] = float_to_e4m3(__fmul_rn(act, ue8m0_inv(sf_exp)));
       if (lane == 0) {
-        const int pos = tile.sf_chunk * kChunkRows + chunk_pos(tile.sf_col * 32 + i);
+        const int pos = tile.sf_chunk * kChunkRows + chunk_pos(i);
         act_sf[((int64_t)(g_out / 4) * act_sf_rows + pos) * 4 + (g_out % 4)] = static_cast<uint8_t>(sf_exp);
       }
     }
@@ -1073,7 +1290,7 @@ cudaError_t launch_experts_simt(const Ctx& c, const MmoeWeights& w, const MmoeOp
                                         w.w2_slice_stride);
   if (c.geo.num_shared_experts > 0 && m > 0) {
     simt_l1_kernel<<<blocks, 128, 0, s>>>(plan, c.e_local, c.geo.num_ranks, 0, 1, c.at<uint8_t>(c.lay.x),
-                                          c.at<int32_t>(c.lay.shared_x_sf), c.lay.shared_sf_rows, nullptr,
+                                          c.at<int32_t>(c.lay.shared_tile_sf), shared_chunk_rows(c.geo.num_max_tokens), nullptr,
                                           static_cast<const uint8_t*>(w.shared_w13),
                                           static_cast<const int32_t*>(w.shared_w13_sf),
                                           c.at<uint8_t>(c.lay.shared_act_x), c.at<uint8_t>(c.lay.shared_act_sf),

@@ -214,22 +214,24 @@ int make_weight_map(CUtensorMap* map, bool fp4, const void* base, uint64_t k_ele
 int tc_num_sms();          // SM count of the device mmoe_prepare() ran on last (0 before)
 bool tc_ready();
 
+// scale words as a 2-D int32 map [columns, rows]: box `box_rows` consecutive words of one column
+int make_scale_map(CUtensorMap* map, const void* base, uint64_t rows, uint64_t columns, uint32_t box_rows);
+
 // parameters of one launch of the tokens-as-A kernels (mmoe_umma_tm.cu)
 struct TmParams {
-  CUtensorMap map_w_routed;        // box 192 rows x 128 K (96 rows for CTA pairs)
+  CUtensorMap map_w_routed;        // box 128 rows x 128 K
   CUtensorMap map_w_shared;
-  CUtensorMap map_tok_routed[2];   // boxes of 64 / 128 token rows
-  CUtensorMap map_tok_shared[2];
+  CUtensorMap map_wsf_routed;      // [E_l * K/128][rows_per_expert] scale words, 4x32 transposed per 128 rows; box 256
+  CUtensorMap map_wsf_shared;
+  CUtensorMap map_tsf_routed;      // token scale chunks, [K/128][chunk rows]; box 128
+  CUtensorMap map_tsf_shared;
+  CUtensorMap map_tok_routed[4];   // boxes of 32 / 64 / 96 / 128 token rows
+  CUtensorMap map_tok_shared[4];
   const char* plan;
-  const int32_t* wsf_routed;       // [E_l][K/128][rows_per_expert] scale words, 4x32 transposed per 128 rows
-  const int32_t* wsf_shared;
-  const int32_t* tsf_routed;       // token scale chunks: word w of chunk row r at w * tsf_rows + r
-  const int32_t* tsf_shared;
-  int64_t tsf_rows_routed, tsf_rows_shared;
   uint8_t* act_routed;             // layer-1 outputs
   uint8_t* act_shared;
-  uint8_t* act_sf_routed;
-  uint8_t* act_sf_shared;
+  int32_t* act_sf_routed;
+  int32_t* act_sf_shared;
   int64_t act_sf_rows_routed, act_sf_rows_shared;
   const float* pool_w;
   __nv_bfloat16* ret;              // layer-2 outputs
@@ -253,6 +255,6 @@ struct TmParams {
   int has_shared_weights;
 };
 cudaError_t tm_prepare();
-cudaError_t tm_launch(int layer, bool fused, int ctas, const TmParams& p, cudaStream_t s);   // ctas: 1, or 2 for CTA pairs
+cudaError_t tm_launch(int layer, bool fused, const TmParams& p, cudaStream_t s);
 
 }  // namespace mmoe

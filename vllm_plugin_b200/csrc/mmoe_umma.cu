@@ -38,6 +38,8 @@ namespace {
 
 constexpr int kThreads = 256;   // producer, MMA 0, 4 epilogue warps, MMA 1, scale arranger (layer 1)
 
+constexpr int kNumBoxes = kSmallTileRows / 16;
+
 struct UmmaParams {
   CUtensorMap map_w_routed;    // FP4 weights, box 128 K x 256 rows (layer 1: the 5-D de-interleaving form)
   CUtensorMap map_w_shared;    // E4M3 weights of the shared expert
@@ -63,7 +65,6 @@ struct UmmaParams {
   int tile_select;             // 0: every tile of the plan, 1: routed tiles only, 2: the early shared tiles only
   int64_t early_shared_first;  // index of the first early shared tile in the tile table
   int early_shared_cap;        // tile records reserved there
-  int fused_return;
   int ep_me;
   const int32_t* ep_totals;    // [32][32]: totals[s][d] = routes rank s sent to rank d in this call
   __nv_bfloat16* ep_ret_recv[32];
@@ -78,9 +79,9 @@ struct UmmaParams {
   float clamp;
   int fast_math;
   int has_shared_weights;
-  int num_stages;              // shared-memory pipeline depth in use (<= the compiled capacity)
-  CUtensorMap map_tok_routed_box[5];   // token maps with boxes of 16 / 32 / 64 / 80 / 128 rows
-  CUtensorMap map_tok_shared_box[5];
+  int max_stages;              // > 0: cap on the shared-memory pipeline depth
+  CUtensorMap map_tok_routed_box[kNumBoxes];   // token maps with boxes of 16, 32, ... 112 rows
+  CUtensorMap map_tok_shared_box[kNumBoxes];
 };
 
 struct Control {          // lives at the start of shared memory
@@ -104,28 +105,33 @@ static_assert(sizeof(Control) <= 1024, "control block");
 // channels, layer 2 two consecutive 128-row blocks of W2.  Two tiles per stage halve the per-byte cost of everything
 // that is paid per stage (barrier hand-offs, token tile, token scales) and give the two MMA-issuing warps one
 // accumulator each.
-template <int kLayer, int kBoxRows>
+//
+// The token slot of a stage is as large as the largest tile of the call (rounded up to 16 rows), which the plan records, so
+// one kernel serves every call: 6 stages at 16 rows, 5 at 32-80, 4 at 96 and 112.
+template <int kLayer>
 struct Shape {
-  static constexpr int kNCap = kBoxRows > kMaxTileTokens ? kMaxTileTokens : kBoxRows;   // accumulator columns per matrix (kBoxRows = largest tile)
   static constexpr int kABytes = 2 * kTileRows * kTileK;           // byte containers in shared memory
-  static constexpr int kBBytes = kBoxRows * kTileK;
   // scale area of a stage: [weight scales of the two tiles, 2 x 512][token scales 512][layer 1: stored-order scales
   // 1024].  Layer 2 receives the two 512-byte chunks in tensor-memory order.  Layer 1 receives them in stored (gate/up
   // interleaved) order and the scale arranger rewrites them into the first 1024 bytes.
   static constexpr int kSfBytes = 3 * 512 + (kLayer == 1 ? 1024 : 0);
-  static constexpr int kStageBytes = kABytes + kBBytes + kSfBytes;
-  static constexpr int kStagesRaw = (kSmemBudget - 1024) / kStageBytes;
-  static constexpr int kStages = kStagesRaw > 8 ? 8 : kStagesRaw;
-  static constexpr int kSmemBytes = 1024 + kStages * kStageBytes + 1024;   // control block + stages + alignment slack
-  static constexpr int kAccCols = 2 * kNCap;                        // TMEM columns of one accumulator stage
-  static constexpr int kSfCol = 2 * kAccCols;                       // scale region: A0, A1, token scales (one copy per MMA warp)
+  static constexpr int kMaxStages = 8;
+  static constexpr int kRingBytes = kSmemBudget - 1024;
+  static constexpr int kSmemBytes = 1024 + kRingBytes + 1024;      // control block + stages + alignment slack
+  static constexpr int kNCap = kSmallTileRows;                     // accumulator columns per weight tile
+  static constexpr int kAccCols = 2 * kNCap;                       // TMEM columns of one accumulator stage
+  static constexpr int kSfCol = 2 * kAccCols;                      // scale region: A0, A1, token scales (one copy per MMA warp)
+  __host__ __device__ static int stages(int tile_rows) {
+    const int n = kRingBytes / (kABytes + tile_rows * kTileK + kSfBytes);
+    return n < kMaxStages ? n : kMaxStages;
+  }
   static_assert(kSfCol + 16 <= (int)kTmemCols, "TMEM budget");
-  static_assert(kStages >= 3, "pipeline too shallow");
+  static_assert(kRingBytes / (kABytes + kSmallTileRows * kTileK + kSfBytes) >= 4, "pipeline too shallow");
   static_assert(kSmemBytes <= 227 * 1024, "shared memory budget");
 };
 
 // ---------------------------------------------------------------------------------------------------------------
-// The roles, each a function of (layer, largest token box, stage layout L).
+// The roles, each a function of (layer, stage layout L).
 // ---------------------------------------------------------------------------------------------------------------
 struct RoleState {                 // pipeline position of a role
   uint32_t stage = 0, phase = 0;   // position in the shared-memory ring
@@ -140,40 +146,49 @@ struct Cta {                       // where a role finds the CTA's resources
   uint8_t* sf_base;
   uint32_t tmem_base;
   uint32_t num_stages;
+  uint32_t b_bytes;                // token slot of a stage
 };
 
+// Tasks in order: tile by tile, or for an expert with several tiles weight block by weight block, so that the tiles of one
+// block read its weights while they are in L2.
 struct TaskList {
-  const Tile* tiles;
-  int64_t num_tasks;
+  TileRange range;
+  int num_tasks, n_blocks;
+  __device__ __forceinline__ const Tile& get(int task, int* nb) const {
+    const int i = task / n_blocks;
+    const Tile& t = range.at(i);
+    if (t.parts == 1) {
+      *nb = task - i * n_blocks;
+      return t;
+    }
+    const int first = i - t.part;
+    const int local = task - first * n_blocks;
+    *nb = local / t.parts;
+    return range.at(first + local - *nb * t.parts);
+  }
 };
 
-__device__ __forceinline__ TaskList task_list(const UmmaParams& p) {
-  PlanView pv = plan_view(const_cast<char*>(p.plan), p.e_local, p.num_ranks);
-  const int num_tiles = p.tile_select == 2
-                            ? (p.has_shared_weights ? max(0, min(pv.hdr->num_early_shared_tiles, p.early_shared_cap)) : 0)
-                            : pv.hdr->num_routed_tiles + (p.tile_select == 0 && p.has_shared_weights ? pv.hdr->num_shared_tiles : 0);
-  return TaskList{pv.tiles + (p.tile_select == 2 ? p.early_shared_first : 0), (int64_t)num_tiles * p.n_blocks};
+__device__ __forceinline__ TaskList task_list(const UmmaParams& p, const PlanView& pv) {
+  const TileRange r = small_tiles(pv, p.tile_select, p.has_shared_weights != 0, p.early_shared_first, p.early_shared_cap);
+  return TaskList{r, r.count * p.n_blocks, p.n_blocks};
 }
 
 // ------------------------------------------------------------------------------------------------ producer
 // One warp in step, one elected lane issues.  Everything that does not change inside a task is computed once per task; the
 // K loop only bumps 32-bit coordinates and two pointers, because such a loop runs at instruction latency, not throughput.
-template <int kLayer, int kBoxRows, typename L>
+template <int kLayer, typename L>
 __device__ __forceinline__ void sa_producer(const UmmaParams& p, const Cta& c, const TaskList& tl, Waiter& waiter,
                                             RoleState& st) {
   const int k_stages = p.k_dim / kTileK;
   const uint32_t full0 = smem_u32(&c.ctl->full[0]), empty0 = smem_u32(&c.ctl->empty[0]);
   const uint32_t sf_full0 = smem_u32(&c.ctl->sf_full[0]);
   const uint32_t a0 = smem_u32(c.a_base), b0 = smem_u32(c.b_base), sf0 = smem_u32(c.sf_base);
-  for (int64_t task = blockIdx.x; task < tl.num_tasks && st.ok; task += gridDim.x) {
-    const int tile_idx = static_cast<int>(task / p.n_blocks);
-    const int nb = static_cast<int>(task - (int64_t)tile_idx * p.n_blocks);
-    const Tile tile = tl.tiles[tile_idx];
+  for (int task = blockIdx.x; task < tl.num_tasks && st.ok; task += gridDim.x) {
+    int nb;
+    const Tile tile = tl.get(task, &nb);
     const bool shared = tile.expert == kSharedExpert;
-    // smallest token box that covers the tile (16 / 32 / 64 / 128 rows): fewer rows to move and to pad
-    const int n16 = (tile.n_valid + 15) & ~15;
-    const int box_sel = n16 <= 16 ? 0 : (n16 <= 32 ? 1 : (n16 <= 64 ? 2 : (n16 <= 80 ? 3 : 4)));   // never above kBoxRows
-    const uint32_t box_rows = box_sel == 3 ? 80u : (box_sel == 4 ? 128u : (16u << box_sel));
+    const int box_sel = (max(tile.n_valid, 1) - 1) >> 4;         // token box: n_valid rounded up to 16 rows
+    const uint32_t box_rows = 16u * (box_sel + 1);
     const CUtensorMap* wmap = shared ? &p.map_w_shared : &p.map_w_routed;
     const CUtensorMap* tmap = shared ? &p.map_tok_shared_box[box_sel] : &p.map_tok_routed_box[box_sel];
     const int e = shared ? 0 : tile.expert;
@@ -207,7 +222,7 @@ __device__ __forceinline__ void sa_producer(const UmmaParams& p, const Cta& c, c
         if (kLayer == 1) tma_load_5d(a_dst, wmap, k0, 0, group, 0, slice, bar);
         else tma_load_3d(a_dst, wmap, k0, row, slice, bar);
         if (kLayer == 2) bulk_load(sf_dst, wsf, 1024, bar);        // two chunks already in tensor-memory order
-        tma_load_2d(b0 + st.stage * L::kBBytes, tmap, k0, tile.row0, bar);
+        tma_load_2d(b0 + st.stage * c.b_bytes, tmap, k0, tile.row0, bar);
         bulk_load(sf_dst + 2 * 512, tsf, 512, bar);
       }
       __syncwarp();
@@ -237,7 +252,7 @@ __device__ __forceinline__ void sa_arrange_scales(const UmmaParams& p, const Cta
     const int r = 16 * ((m & 63) >> 3) + 8 * h + (m & 7);   // stored row inside its 128-row block
     src[t] = 128 * (m >> 6) + 4 * (r & 31) + (r >> 5);
   }
-  for (int64_t task = blockIdx.x; task < tl.num_tasks && st.ok; task += gridDim.x) {
+  for (int task = blockIdx.x; task < tl.num_tasks && st.ok; task += gridDim.x) {
     for (int kb = 0; kb < k_stages; ++kb) {
       // the stage's scales have landed, which also says that the MMAs which read the previous ones have retired
       if (!waiter.wait_uniform(sf_full0 + 8 * st.stage, st.phase)) { st.ok = false; break; }
@@ -259,7 +274,7 @@ __device__ __forceinline__ void sa_arrange_scales(const UmmaParams& p, const Cta
 // Two warps, one per weight tile / accumulator (h = 0, 1).  The whole warp walks the loop so that loop state stays
 // warp-uniform; one elected lane issues.  Each warp copies the scales it needs into its own TMEM columns, so no
 // ordering between the two warps' tensor-core instructions is needed.
-template <int kLayer, int kBoxRows, typename L>
+template <int kLayer, typename L>
 __device__ __forceinline__ void sa_mma(const UmmaParams& p, const Cta& c, const TaskList& tl, Waiter& waiter,
                                        RoleState& st, int h) {
   const int k_stages = p.k_dim / kTileK;
@@ -272,8 +287,9 @@ __device__ __forceinline__ void sa_mma(const UmmaParams& p, const Cta& c, const 
   const uint32_t sf_lo0 = (smem_u32(c.sf_base) & 0x3FFFFu) >> 4;
   const uint32_t sfa_col = c.tmem_base + L::kSfCol + 4 * h;
   const uint32_t sfb_col = c.tmem_base + L::kSfCol + 8 + 4 * h;
-  for (int64_t task = blockIdx.x; task < tl.num_tasks && st.ok; task += gridDim.x, ++st.it) {
-    const Tile tile = tl.tiles[task / p.n_blocks];
+  for (int task = blockIdx.x; task < tl.num_tasks && st.ok; task += gridDim.x, ++st.it) {
+    int nb;
+    const Tile tile = tl.get(task, &nb);
     const bool shared = tile.expert == kSharedExpert;
     const uint32_t acc_stage = st.it & 1u, acc_phase = (st.it >> 1) & 1u;
     if (!waiter.wait_uniform(smem_u32(&c.ctl->tmem_empty[acc_stage]), acc_phase ^ 1u)) { st.ok = false; break; }
@@ -281,12 +297,11 @@ __device__ __forceinline__ void sa_mma(const UmmaParams& p, const Cta& c, const 
     const uint32_t n = static_cast<uint32_t>((tile.n_valid + 15) & ~15);
     const uint32_t idesc0 = make_idesc(shared ? 0u : 5u, 0u, n, 0);
     const uint32_t d = c.tmem_base + acc_stage * L::kAccCols + h * L::kNCap;
-    const uint32_t sfb = sfb_col + tile.sf_col;
     for (int kb = 0; kb < k_stages; ++kb) {
       if (kLayer == 1 && !waiter.wait_uniform(sf_ready0 + 8 * st.stage, st.phase)) { st.ok = false; break; }
       if (!waiter.wait_uniform(full0 + 8 * st.stage, st.phase)) { st.ok = false; break; }
       const uint32_t a_lo = a_lo0 + st.stage * (L::kABytes >> 4);
-      const uint32_t b_lo = b_lo0 + st.stage * (L::kBBytes >> 4);
+      const uint32_t b_lo = b_lo0 + st.stage * (c.b_bytes >> 4);
       const uint32_t sf_lo = sf_lo0 + st.stage * (L::kSfBytes >> 4);
       if (elect_one()) {
         tc_cp_sf(sfa_col, sf_hi | (sf_lo + 32 * h));
@@ -295,7 +310,7 @@ __device__ __forceinline__ void sa_mma(const UmmaParams& p, const Cta& c, const 
         for (int k = 0; k < kTileK / 32; ++k)
           tc_mma(d, sw128_hi | (a_lo + 2 * k), sw128_hi | (b_lo + 2 * k),
                  idesc0 + k * ((1u << 4) | (1u << 29)),               // scale byte k of both operands
-                 sfa_col, sfb, (kb | k) != 0 ? 1u : 0u);
+                 sfa_col, sfb_col, (kb | k) != 0 ? 1u : 0u);
         tc_commit(empty0 + 8 * st.stage);            // shared memory of this stage is free once these MMAs retire
       }
       __syncwarp();
@@ -310,16 +325,16 @@ __device__ __forceinline__ void sa_mma(const UmmaParams& p, const Cta& c, const 
 // Four warps; a thread owns one weight row (accumulator lane), the columns are the tile's tokens.
 // kFused (layer 2, EP > 1): every output row goes to the rank its token came from; compiled as kernels of its own so
 // that the single-destination epilogue of the other cases keeps its shorter inner loop.
-template <int kLayer, int kBoxRows, typename L, bool kFused>
+template <int kLayer, typename L, bool kFused>
 __device__ __forceinline__ void sa_epilogue(const UmmaParams& p, const Cta& c, const TaskList& tl, Waiter& waiter,
                                             RoleState& st) {
   Control* ctl = c.ctl;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int q = warp & 3;                     // TMEM lane quadrant this warp may read
   const uint32_t lane_sel = static_cast<uint32_t>(q * 32) << 16;
-  for (int64_t task = blockIdx.x; task < tl.num_tasks && st.ok; task += gridDim.x, ++st.it) {
-    const Tile tile = tl.tiles[task / p.n_blocks];
-    const int nb = static_cast<int>(task % p.n_blocks);
+  for (int task = blockIdx.x; task < tl.num_tasks && st.ok; task += gridDim.x, ++st.it) {
+    int nb;
+    const Tile tile = tl.get(task, &nb);
     const bool shared = tile.expert == kSharedExpert;
     const uint32_t acc_stage = st.it & 1u, acc_phase = (st.it >> 1) & 1u;
     // Per-token side data of the tile (top-k weight / destination row), one coalesced load per 32 tokens issued
@@ -381,7 +396,7 @@ __device__ __forceinline__ void sa_epilogue(const UmmaParams& p, const Cta& c, c
         for (int j = 0; j < 16; ++j)
           if (i0 + j < tile.n_valid) act_col[(int64_t)(i0 + j) * p.inter] = static_cast<uint8_t>(g[j]);
         if (lane < 16 && i0 + lane < tile.n_valid)
-          sf_out[chunk_pos(tile.sf_col * 32 + i0 + lane) * 4] = static_cast<uint8_t>(my_sf);
+          sf_out[chunk_pos(i0 + lane) * 4] = static_cast<uint8_t>(my_sf);
       }
     } else if (!kFused) {
 #pragma unroll
@@ -429,17 +444,23 @@ __device__ __forceinline__ void sa_epilogue(const UmmaParams& p, const Cta& c, c
 }
 
 // ------------------------------------------------------------------------------------------------ set-up / teardown
+__device__ __forceinline__ uint8_t* sa_align(uint8_t* smem_raw) {
+  return smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+}
+
+// the stages behind the control block, for tiles of at most `tile_rows` rows
 template <typename L>
-__device__ __forceinline__ Cta sa_carve(uint8_t* smem_raw) {
-  const uint32_t raw = smem_u32(smem_raw);
-  uint8_t* smem = smem_raw + ((1024u - (raw & 1023u)) & 1023u);
+__device__ __forceinline__ Cta sa_carve(uint8_t* smem, int tile_rows, int max_stages) {
   Cta c;
+  int stages = L::stages(tile_rows);
+  if (max_stages > 0 && max_stages < stages) stages = max_stages;
+  c.num_stages = static_cast<uint32_t>(stages);
+  c.b_bytes = static_cast<uint32_t>(tile_rows * kTileK);
   c.ctl = reinterpret_cast<Control*>(smem);
   c.a_base = smem + 1024;
-  c.b_base = c.a_base + L::kStages * L::kABytes;
-  c.sf_base = c.b_base + L::kStages * L::kBBytes;
+  c.b_base = c.a_base + stages * L::kABytes;
+  c.sf_base = c.b_base + stages * c.b_bytes;
   c.tmem_base = 0;
-  c.num_stages = L::kStages;
   return c;
 }
 
@@ -447,7 +468,7 @@ __device__ __forceinline__ Cta sa_carve(uint8_t* smem_raw) {
 template <typename L>
 __device__ __forceinline__ void sa_setup(Control* ctl) {
   if (threadIdx.x == 0) {
-    for (int i = 0; i < L::kStages; ++i) {
+    for (int i = 0; i < L::kMaxStages; ++i) {
       mbar_init(smem_u32(&ctl->full[i]), 1);
       mbar_init(smem_u32(&ctl->empty[i]), 2);          // both MMA warps release a stage
       mbar_init(smem_u32(&ctl->sf_full[i]), 1);
@@ -484,13 +505,13 @@ __device__ __forceinline__ void sa_teardown(Control* ctl, uint32_t tmem_base) {
 }
 
 // One layer per launch.
-template <int kLayer, int kBoxRows, bool kFused = false>
+template <int kLayer, bool kFused = false>
 __global__ void __launch_bounds__(kThreads, 1) umma_kernel(const __grid_constant__ UmmaParams p) {
   static_assert(!kFused || kLayer == 2, "only GEMM2 writes rows back");
-  using L = Shape<kLayer, kBoxRows>;
+  using L = Shape<kLayer>;
   extern __shared__ uint8_t smem_raw[];
-  Cta c = sa_carve<L>(smem_raw);
-  Control* ctl = c.ctl;
+  uint8_t* smem = sa_align(smem_raw);
+  Control* ctl = reinterpret_cast<Control*>(smem);
   const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);   // warp-uniform for the compiler too
   chain_release();
   sa_setup<L>(ctl);
@@ -515,19 +536,21 @@ __global__ void __launch_bounds__(kThreads, 1) umma_kernel(const __grid_constant
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  const PlanView pv = plan_view(const_cast<char*>(p.plan), p.e_local, p.num_ranks);
+  const int tile_rows = max(16, min(kSmallTileRows, p.tile_select == 2 ? pv.hdr->early_small_rows : pv.hdr->small_rows));
+  Cta c = sa_carve<L>(smem, tile_rows, p.max_stages);
   c.tmem_base = __shfl_sync(0xffffffffu, ctl->tmem_base, 0);
-  c.num_stages = static_cast<uint32_t>(p.num_stages);
-  const TaskList tl = task_list(p);
+  const TaskList tl = task_list(p, pv);
   Waiter waiter{&ctl->abort_flag, p.status, global_timer() + static_cast<uint64_t>(p.timeout_ns), kLayer, warp};
   RoleState st;
   if (warp == 0) {
-    sa_producer<kLayer, kBoxRows, L>(p, c, tl, waiter, st);
+    sa_producer<kLayer, L>(p, c, tl, waiter, st);
   } else if (warp == 1 || warp == 6) {
-    sa_mma<kLayer, kBoxRows, L>(p, c, tl, waiter, st, warp == 1 ? 0 : 1);
+    sa_mma<kLayer, L>(p, c, tl, waiter, st, warp == 1 ? 0 : 1);
   } else if (warp == 7) {
     if (kLayer == 1) sa_arrange_scales<L>(p, c, tl, waiter, st);
   } else {
-    sa_epilogue<kLayer, kBoxRows, L, kFused>(p, c, tl, waiter, st);
+    sa_epilogue<kLayer, L, kFused>(p, c, tl, waiter, st);
   }
   sa_teardown(ctl, c.tmem_base);
 }
@@ -542,7 +565,7 @@ EncodeTiledFn g_encode = nullptr;
 constexpr int kMaxDevices = 64;
 int g_num_sms[kMaxDevices] = {};   // per device, 0 = mmoe_prepare() has not run there
 int g_tune_stages = 0;             // 0: every stage that fits
-int g_orientation = 0;             // 0: chosen per call, 1: weights-as-A, 2: tokens-as-A, 3: tokens-as-A on CTA pairs
+int g_orientation = 0;             // 0: chosen per expert, 1: weights-as-A, 2 and 3: tokens-as-A on CTA pairs
 
 int current_device() {
   int dev = -1;
@@ -568,44 +591,20 @@ int make_w13_map(CUtensorMap* map, bool fp4, const void* base, uint64_t k_elems,
   return r == CUDA_SUCCESS ? 0 : static_cast<int>(r);
 }
 
-template <int kLayer, int kBoxRows>
+template <int kLayer, bool kFused>
 cudaError_t prepare_one() {
-  cudaError_t e = cudaFuncSetAttribute(umma_kernel<kLayer, kBoxRows, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       Shape<kLayer, kBoxRows>::kSmemBytes);
-  if (e == cudaSuccess && kLayer == 2)
-    e = cudaFuncSetAttribute(umma_kernel<2, kBoxRows, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             Shape<2, kBoxRows>::kSmemBytes);
-  return e;
+  return cudaFuncSetAttribute(umma_kernel<kLayer, kFused>, cudaFuncAttributeMaxDynamicSharedMemorySize, Shape<kLayer>::kSmemBytes);
 }
 
-template <int kLayer, int kBoxRows>
-cudaError_t launch_one(const UmmaParams& p0, cudaStream_t s) {
-  using S = Shape<kLayer, kBoxRows>;
-  UmmaParams p = p0;
-  p.num_stages = g_tune_stages > 0 && g_tune_stages < S::kStages ? g_tune_stages : S::kStages;
-  const int grid = tc_num_sms();
-  if (kLayer == 2 && p.fused_return)
-    launch_chained(umma_kernel<2, kBoxRows, true>, dim3(grid), dim3(kThreads), Shape<2, kBoxRows>::kSmemBytes, s, p);
-  else
-    launch_chained(umma_kernel<kLayer, kBoxRows, false>, dim3(grid), dim3(kThreads), S::kSmemBytes, s, p);
+template <int kLayer, bool kFused>
+cudaError_t launch_layer(UmmaParams& p, cudaStream_t s) {
+  p.max_stages = g_tune_stages;
+  launch_chained(umma_kernel<kLayer, kFused>, dim3(tc_num_sms()), dim3(kThreads), Shape<kLayer>::kSmemBytes, s, p);
   return cudaGetLastError();
 }
 
-int box_rows_of(int block_m) { return block_m <= 16 ? 16 : (block_m <= 32 ? 32 : (block_m <= 64 ? 64 : (block_m == 128 ? 80 : 128))); }
-
-template <int kLayer>
-cudaError_t launch_layer(const UmmaParams& p, int box, cudaStream_t s) {
-  switch (box) {
-    case 16: return launch_one<kLayer, 16>(p, s);
-    case 32: return launch_one<kLayer, 32>(p, s);
-    case 64: return launch_one<kLayer, 64>(p, s);
-    case 80: return launch_one<kLayer, 80>(p, s);
-    default: return launch_one<kLayer, 128>(p, s);
-  }
-}
-
 // ---------------------------------------------------------------------------------------------------------------
-// Launch parameters that depend only on (workspace, weights, geometry, kernel family) -- above all the encoded tensor
+// Launch parameters that depend only on (workspace, weights, geometry) -- above all the encoded tensor
 // maps -- are built once and kept: a serving engine calls the layer with the same buffers thousands of times, and
 // encoding two dozen tensor maps per call costs more host time than the launches themselves.  What changes per call
 // (tile selection, options, peers) is patched into a copy.  The reference keeps the same kind of record per validated
@@ -616,7 +615,6 @@ struct PlanKey {
   const void* w[8];
   int64_t s13, s2;
   MmoeGeometry geo;
-  int family;
   int has_shared;
   int device;
   bool operator==(const PlanKey& o) const { return memcmp(this, &o, sizeof(PlanKey)) == 0; }
@@ -641,7 +639,6 @@ PlanKey make_key(const Ctx& c, const MmoeWeights& w, bool has_shared) {
   k.s13 = w.w13_slice_stride;
   k.s2 = w.w2_slice_stride;
   k.geo = c.geo;
-  k.family = c.family;
   k.has_shared = has_shared ? 1 : 0;
   k.device = current_device();
   return k;
@@ -650,34 +647,27 @@ PlanKey make_key(const Ctx& c, const MmoeWeights& w, bool has_shared) {
 // tokens-as-A form: both layers through mmoe_umma_tm.cu
 bool build_tm(const Ctx& c, const MmoeWeights& w, bool has_shared, TmParams* out) {
   const int h = c.geo.hidden, inter = c.geo.intermediate, el = c.e_local;
+  const int64_t shared_sf_rows = shared_chunk_rows(c.geo.num_max_tokens);
   TmParams p1{};
   int bad = 0;
-  const int ctas = c.family == kFamilyTokensAsAPair ? 2 : 1;
-  const uint32_t wbox = 192 / ctas;          // a CTA of a pair stages half of a task's weight rows
-  bad |= make_weight_map(&p1.map_w_routed, true, w.w13, h, (uint64_t)el * 2 * inter, w.w13_slice_stride, wbox);
-  if (has_shared) bad |= make_weight_map(&p1.map_w_shared, false, w.shared_w13, h, 2 * (uint64_t)inter, 0, wbox);
-  else p1.map_w_shared = p1.map_w_routed;
-  const uint32_t kBoxes[2] = {64, 128};
-  // a 128-row box may start up to 127 rows before the end of the token matrix; the rows past it are workspace bytes of
-  // the regions that follow (never stored anywhere: they only feed accumulator lanes of rows that do not exist)
-  const uint64_t x_rows = (uint64_t)c.geo.num_max_tokens + 128;
-  for (int b = 0; b < 2; ++b) {
-    bad |= make_token_map(&p1.map_tok_routed[b], c.ws + c.lay.pool_x, h, c.lay.pool_rows, kBoxes[b]);
-    if (has_shared) bad |= make_token_map(&p1.map_tok_shared[b], c.ws + c.lay.x, h, x_rows, kBoxes[b]);
-    else p1.map_tok_shared[b] = p1.map_tok_routed[b];
+  bad |= make_weight_map(&p1.map_w_routed, true, w.w13, h, (uint64_t)el * 2 * inter, w.w13_slice_stride, kTileRows);
+  bad |= make_scale_map(&p1.map_wsf_routed, w.w13_sf, 2 * (uint64_t)inter, (uint64_t)el * (h / kTileK), 256);
+  bad |= make_scale_map(&p1.map_tsf_routed, c.ws + c.lay.pool_sf, c.lay.pool_sf_rows, h / kTileK, kChunkRows);
+  for (int b = 0; b < 4; ++b)
+    bad |= make_token_map(&p1.map_tok_routed[b], c.ws + c.lay.pool_x, h, c.lay.pool_rows, 32 * (b + 1));
+  if (has_shared) {
+    bad |= make_weight_map(&p1.map_w_shared, false, w.shared_w13, h, 2 * (uint64_t)inter, 0, kTileRows);
+    bad |= make_scale_map(&p1.map_wsf_shared, w.shared_w13_sf, 2 * (uint64_t)inter, h / kTileK, 256);
+    bad |= make_scale_map(&p1.map_tsf_shared, c.ws + c.lay.shared_tile_sf, shared_sf_rows, h / kTileK, kChunkRows);
+    for (int b = 0; b < 4; ++b)
+      bad |= make_token_map(&p1.map_tok_shared[b], c.ws + c.lay.x, h, c.geo.num_max_tokens, 32 * (b + 1));
   }
   if (bad) return false;
   p1.plan = c.ws + c.lay.plan;
-  p1.wsf_routed = static_cast<const int32_t*>(w.w13_sf);
-  p1.wsf_shared = static_cast<const int32_t*>(w.shared_w13_sf);
-  p1.tsf_routed = c.at<int32_t>(c.lay.pool_sf);
-  p1.tsf_shared = c.at<int32_t>(c.lay.shared_x_sf);
-  p1.tsf_rows_routed = c.lay.pool_sf_rows;
-  p1.tsf_rows_shared = c.lay.shared_sf_rows;
   p1.act_routed = c.at<uint8_t>(c.lay.act_x);
   p1.act_shared = c.at<uint8_t>(c.lay.shared_act_x);
-  p1.act_sf_routed = c.at<uint8_t>(c.lay.act_sf);
-  p1.act_sf_shared = c.at<uint8_t>(c.lay.shared_act_sf);
+  p1.act_sf_routed = c.at<int32_t>(c.lay.act_sf);
+  p1.act_sf_shared = c.at<int32_t>(c.lay.shared_act_sf);
   p1.act_sf_rows_routed = c.lay.pool_sf_rows;
   p1.act_sf_rows_shared = c.lay.shared_sf_rows;
   p1.pool_w = c.at<float>(c.lay.pool_w);
@@ -694,19 +684,19 @@ bool build_tm(const Ctx& c, const MmoeWeights& w, bool has_shared, TmParams* out
   p1.early_shared_cap = static_cast<int>(shared_tile_capacity(c.geo.num_max_tokens));
 
   TmParams p2 = p1;
-  bad |= make_weight_map(&p2.map_w_routed, true, w.w2, inter, (uint64_t)el * h, w.w2_slice_stride, wbox);
-  if (has_shared) bad |= make_weight_map(&p2.map_w_shared, false, w.shared_w2, inter, (uint64_t)h, 0, wbox);
-  else p2.map_w_shared = p2.map_w_routed;
-  for (int b = 0; b < 2; ++b) {
-    bad |= make_token_map(&p2.map_tok_routed[b], c.ws + c.lay.act_x, inter, c.lay.pool_rows, kBoxes[b]);
-    if (has_shared) bad |= make_token_map(&p2.map_tok_shared[b], c.ws + c.lay.shared_act_x, inter, x_rows, kBoxes[b]);
-    else p2.map_tok_shared[b] = p2.map_tok_routed[b];
+  bad |= make_weight_map(&p2.map_w_routed, true, w.w2, inter, (uint64_t)el * h, w.w2_slice_stride, kTileRows);
+  bad |= make_scale_map(&p2.map_wsf_routed, w.w2_sf, h, (uint64_t)el * (inter / kTileK), 256);
+  bad |= make_scale_map(&p2.map_tsf_routed, c.ws + c.lay.act_sf, c.lay.pool_sf_rows, inter / kTileK, kChunkRows);
+  for (int b = 0; b < 4; ++b)
+    bad |= make_token_map(&p2.map_tok_routed[b], c.ws + c.lay.act_x, inter, c.lay.pool_rows, 32 * (b + 1));
+  if (has_shared) {
+    bad |= make_weight_map(&p2.map_w_shared, false, w.shared_w2, inter, (uint64_t)h, 0, kTileRows);
+    bad |= make_scale_map(&p2.map_wsf_shared, w.shared_w2_sf, h, inter / kTileK, 256);
+    bad |= make_scale_map(&p2.map_tsf_shared, c.ws + c.lay.shared_act_sf, c.lay.shared_sf_rows, inter / kTileK, kChunkRows);
+    for (int b = 0; b < 4; ++b)
+      bad |= make_token_map(&p2.map_tok_shared[b], c.ws + c.lay.shared_act_x, inter, c.geo.num_max_tokens + 128, 32 * (b + 1));
   }
   if (bad) return false;
-  p2.wsf_routed = static_cast<const int32_t*>(w.w2_sf);
-  p2.wsf_shared = static_cast<const int32_t*>(w.shared_w2_sf);
-  p2.tsf_routed = c.at<int32_t>(c.lay.act_sf);
-  p2.tsf_shared = c.at<int32_t>(c.lay.shared_act_sf);
   p2.ret = c.at<__nv_bfloat16>(c.lay.ret);
   p2.shared_out = c.at<__nv_bfloat16>(c.lay.shared_out);
   p2.pool_dst = c.at<int32_t>(c.lay.pool_dst);
@@ -725,11 +715,9 @@ bool build_sa(const Ctx& c, const MmoeWeights& w, bool has_shared, UmmaParams* o
   bad |= make_w13_map(&p1.map_w_routed, true, w.w13, h, (uint64_t)el * 2 * inter, w.w13_slice_stride);
   if (has_shared) bad |= make_w13_map(&p1.map_w_shared, false, w.shared_w13, h, 2 * (uint64_t)inter, 0);
   else p1.map_w_shared = p1.map_w_routed;
-  // token maps: one per box size a tile can pick (a launch never picks one above its kernel's own box)
-  const uint32_t kBoxes[5] = {16, 32, 64, 80, 128};
-  for (int b = 0; b < 5; ++b) {
-    bad |= make_token_map(&p1.map_tok_routed_box[b], c.ws + c.lay.pool_x, h, c.lay.pool_rows, kBoxes[b]);
-    if (has_shared) bad |= make_token_map(&p1.map_tok_shared_box[b], c.ws + c.lay.x, h, c.geo.num_max_tokens, kBoxes[b]);
+  for (int b = 0; b < kNumBoxes; ++b) {
+    bad |= make_token_map(&p1.map_tok_routed_box[b], c.ws + c.lay.pool_x, h, c.lay.pool_rows, 16 * (b + 1));
+    if (has_shared) bad |= make_token_map(&p1.map_tok_shared_box[b], c.ws + c.lay.x, h, c.geo.num_max_tokens, 16 * (b + 1));
     else p1.map_tok_shared_box[b] = p1.map_tok_routed_box[b];
   }
   if (bad) return false;
@@ -737,9 +725,9 @@ bool build_sa(const Ctx& c, const MmoeWeights& w, bool has_shared, UmmaParams* o
   p1.wsf_routed = static_cast<const int32_t*>(w.w13_sf);
   p1.wsf_shared = static_cast<const int32_t*>(w.shared_w13_sf);
   p1.tsf_routed = c.at<int32_t>(c.lay.pool_sf);
-  p1.tsf_shared = c.at<int32_t>(c.lay.shared_x_sf);
+  p1.tsf_shared = c.at<int32_t>(c.lay.shared_tile_sf);
   p1.tsf_rows_routed = c.lay.pool_sf_rows;
-  p1.tsf_rows_shared = c.lay.shared_sf_rows;
+  p1.tsf_rows_shared = shared_chunk_rows(c.geo.num_max_tokens);
   p1.act_routed = c.at<uint8_t>(c.lay.act_x);
   p1.act_shared = c.at<uint8_t>(c.lay.shared_act_x);
   p1.act_sf_routed = c.at<uint8_t>(c.lay.act_sf);
@@ -764,9 +752,9 @@ bool build_sa(const Ctx& c, const MmoeWeights& w, bool has_shared, UmmaParams* o
   bad |= make_weight_map(&p2.map_w_routed, true, w.w2, inter, (uint64_t)el * h, w.w2_slice_stride, 2 * kTileRows);
   if (has_shared) bad |= make_weight_map(&p2.map_w_shared, false, w.shared_w2, inter, (uint64_t)h, 0, 2 * kTileRows);
   else p2.map_w_shared = p2.map_w_routed;
-  for (int b = 0; b < 5; ++b) {
-    bad |= make_token_map(&p2.map_tok_routed_box[b], c.ws + c.lay.act_x, inter, c.lay.pool_rows, kBoxes[b]);
-    if (has_shared) bad |= make_token_map(&p2.map_tok_shared_box[b], c.ws + c.lay.shared_act_x, inter, c.geo.num_max_tokens, kBoxes[b]);
+  for (int b = 0; b < kNumBoxes; ++b) {
+    bad |= make_token_map(&p2.map_tok_routed_box[b], c.ws + c.lay.act_x, inter, c.lay.pool_rows, 16 * (b + 1));
+    if (has_shared) bad |= make_token_map(&p2.map_tok_shared_box[b], c.ws + c.lay.shared_act_x, inter, c.geo.num_max_tokens, 16 * (b + 1));
     else p2.map_tok_shared_box[b] = p2.map_tok_routed_box[b];
   }
   if (bad) return false;
@@ -774,6 +762,7 @@ bool build_sa(const Ctx& c, const MmoeWeights& w, bool has_shared, UmmaParams* o
   p2.wsf_shared = static_cast<const int32_t*>(w.shared_w2_sf);
   p2.tsf_routed = c.at<int32_t>(c.lay.act_sf);
   p2.tsf_shared = c.at<int32_t>(c.lay.shared_act_sf);
+  p2.tsf_rows_shared = c.lay.shared_sf_rows;
   p2.ret = c.at<__nv_bfloat16>(c.lay.ret);
   p2.shared_out = c.at<__nv_bfloat16>(c.lay.shared_out);
   p2.pool_dst = c.at<int32_t>(c.lay.pool_dst);
@@ -786,7 +775,7 @@ bool build_sa(const Ctx& c, const MmoeWeights& w, bool has_shared, UmmaParams* o
   return true;
 }
 
-// the kept record for (workspace, weights, geometry, family), built on first use; least recently used slot is replaced
+// the kept record for (workspace, weights, geometry), built on first use; least recently used slot is replaced
 const PlanEntry* cached_plan(const Ctx& c, const MmoeWeights& w, bool has_shared) {
   const PlanKey key = make_key(c, w, has_shared);
   std::lock_guard<std::mutex> lock(g_plan_mutex);
@@ -798,7 +787,7 @@ const PlanEntry* cached_plan(const Ctx& c, const MmoeWeights& w, bool has_shared
     }
     if (e.stamp < victim->stamp) victim = &e;
   }
-  const bool ok = c.family == kFamilyWeightsAsA ? build_sa(c, w, has_shared, victim->sa) : build_tm(c, w, has_shared, victim->tm);
+  const bool ok = build_sa(c, w, has_shared, victim->sa) && build_tm(c, w, has_shared, victim->tm);
   if (!ok) {
     victim->stamp = 0;
     return nullptr;
@@ -849,6 +838,17 @@ int make_weight_map(CUtensorMap* map, bool fp4, const void* base, uint64_t k_ele
   return r == CUDA_SUCCESS ? 0 : static_cast<int>(r);
 }
 
+int make_scale_map(CUtensorMap* map, const void* base, uint64_t rows, uint64_t columns, uint32_t box_rows) {
+  const cuuint64_t dims[2] = {rows, columns};
+  const cuuint64_t strides[1] = {rows * 4};
+  const cuuint32_t box[2] = {box_rows, 1};
+  const cuuint32_t estr[2] = {1, 1};
+  const CUresult r = g_encode(map, CU_TENSOR_MAP_DATA_TYPE_INT32, 2, const_cast<void*>(base), dims, strides, box, estr,
+                              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? 0 : static_cast<int>(r);
+}
+
 // Once per device (the dynamic shared-memory limits are per device) and outside stream capture.
 int prepare_umma(const MmoeGeometry& geo) {
   (void)geo;
@@ -866,16 +866,9 @@ int prepare_umma(const MmoeGeometry& geo) {
   int sms = 0;
   if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return MMOE_ERR_CUDA;
   cudaError_t e = cudaSuccess;
-  if (e == cudaSuccess) e = prepare_one<1, 16>();
-  if (e == cudaSuccess) e = prepare_one<1, 32>();
-  if (e == cudaSuccess) e = prepare_one<1, 64>();
-  if (e == cudaSuccess) e = prepare_one<1, 80>();
-  if (e == cudaSuccess) e = prepare_one<1, 128>();
-  if (e == cudaSuccess) e = prepare_one<2, 16>();
-  if (e == cudaSuccess) e = prepare_one<2, 32>();
-  if (e == cudaSuccess) e = prepare_one<2, 64>();
-  if (e == cudaSuccess) e = prepare_one<2, 80>();
-  if (e == cudaSuccess) e = prepare_one<2, 128>();
+  if (e == cudaSuccess) e = prepare_one<1, false>();
+  if (e == cudaSuccess) e = prepare_one<2, false>();
+  if (e == cudaSuccess) e = prepare_one<2, true>();
   if (e == cudaSuccess) e = tm_prepare();
   if (e != cudaSuccess) return MMOE_ERR_CUDA;
   g_num_sms[dev] = sms;
@@ -906,31 +899,23 @@ cudaError_t launch_experts_umma(const Ctx& c, const MmoeWeights& w, const MmoeOp
         p.ep_ret_recv[r] = reinterpret_cast<__nv_bfloat16*>(static_cast<char*>(const_cast<void*>(c.peer_ws[r])) + c.lay.ret_recv);
     }
   };
-  if (c.family != kFamilyWeightsAsA) {
-    const int ctas = c.family == kFamilyTokensAsAPair ? 2 : 1;
-    if (mask & 1) {
-      TmParams p = plan->tm[0];
-      patch(p, false);
-      e = tm_launch(1, false, ctas, p, s);
+  // Experts with many rows run on CTA pairs, the others on the weights-as-A kernels: which ones is in the plan.  The
+  // ahead-of-plan launch knows its own kind.
+  const int pair_above = c.pair_above_for(m);
+  const bool pairs = c.tile_select == 2 ? m > pair_above : pair_above != kNeverPair;
+  const bool small = c.tile_select == 2 ? !pairs : pair_above > 0;
+  for (int layer = 1; layer <= 2; ++layer) {
+    if ((mask & layer) == 0) continue;
+    if (e == cudaSuccess && pairs) {
+      TmParams p = plan->tm[layer - 1];
+      patch(p, layer == 2);
+      e = tm_launch(layer, layer == 2 && fused, p, s);
     }
-    if (e == cudaSuccess && (mask & 2)) {
-      TmParams p = plan->tm[1];
-      patch(p, true);
-      e = tm_launch(2, fused, ctas, p, s);
+    if (e == cudaSuccess && small) {
+      UmmaParams p = plan->sa[layer - 1];
+      patch(p, layer == 2);
+      e = layer == 1 ? launch_layer<1, false>(p, s) : fused ? launch_layer<2, true>(p, s) : launch_layer<2, false>(p, s);
     }
-    return e;
-  }
-  const int box = box_rows_of(block_m);
-  if (mask & 1) {
-    UmmaParams p = plan->sa[0];
-    patch(p, false);
-    e = launch_layer<1>(p, box, s);
-  }
-  if (e == cudaSuccess && (mask & 2)) {
-    UmmaParams p = plan->sa[1];
-    patch(p, true);
-    p.fused_return = fused ? 1 : 0;
-    e = launch_layer<2>(p, box, s);
   }
   return e;
 }
