@@ -43,11 +43,12 @@ bool take_chain_flag() {
 // Kernel (a): BF16 -> MXFP8 E4M3 with one UE8M0 scale per 32 elements, four scale bytes per int32 word.
 // Follows the reference quantiser (backend/staging.py:36-82): scale = 2^ceil(log2(max(amax, 1e-4) / 448)), exponent
 // clamped to [1, 254]; values multiplied by the exact reciprocal and rounded to nearest even.
-// One thread converts 8 elements (one 16-byte load, one 8-byte store); 4 threads share a scale, 16 a scale word.
+// A warp takes segments of 128 vectors of 8 elements: four independent 16-byte loads per lane, 4 lanes share a scale, 16 a
+// scale word.  HBM-bound: 3840 x 5120 (60 MB) took 30 us with one division per vector and single-value conversions.
 // =====================================================================================================================
-__device__ __forceinline__ void stage_vector(const uint4& raw, bool live, int64_t i, int vec_per_row, int h,
-                                             uint2* __restrict__ x_q, int32_t* __restrict__ x_sf,
-                                             int32_t* __restrict__ shared_sf, int64_t shared_rows, int shared_bm) {
+constexpr int kStageSegVec = 128;
+
+__device__ __forceinline__ void stage_vector(const uint4& raw, uint2* __restrict__ q_out, uint32_t* word_out) {
   const __nv_bfloat162* p = reinterpret_cast<const __nv_bfloat162*>(&raw);
   float v[8];
   float amax = 0.f;
@@ -61,37 +62,21 @@ __device__ __forceinline__ void stage_vector(const uint4& raw, bool live, int64_
   amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
   amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
   amax = fmaxf(amax, 1e-4f);
-  const uint32_t bits = __float_as_uint(__fdiv_rn(amax, 448.0f));
-  int e = static_cast<int>((bits >> 23) & 0xFFu) + ((bits & 0x7FFFFFu) != 0u);
-  e = min(max(e, 1), 254);
-  const float inv = __uint_as_float(static_cast<uint32_t>(254 - e) << 23);   // exact reciprocal of 2^(e-127), e in [1, 253]
-  const float inv_exact = e == 254 ? __fdiv_rn(1.0f, __uint_as_float(254u << 23)) : inv;
-  uint32_t lo = 0, hi = 0;
+  // ceil(log2(amax / 448)), 448 = 1.75 * 2^8: the exponent of amax, one more if its mantissa exceeds 1.75 (the carry of the
+  // addition), less 8.  An infinite amax gets the largest exponent.
+  const uint32_t bits = __float_as_uint(amax);
+  const int e = bits == 0x7F800000u ? 254 : static_cast<int>((bits + (0x7FFFFFu - (0x60u << 16))) >> 23) - 8;
+  const float inv = __uint_as_float(e == 254 ? 0x00400000u : static_cast<uint32_t>(254 - e) << 23);   // exactly 2^(127 - e)
+  uint32_t w[4];
 #pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    lo |= static_cast<uint32_t>(float_to_e4m3(__fmul_rn(v[j], inv_exact))) << (8 * j);
-    hi |= static_cast<uint32_t>(float_to_e4m3(__fmul_rn(v[4 + j], inv_exact))) << (8 * j);
-  }
-  if (live) x_q[i] = make_uint2(lo, hi);
-  // scale word: lanes 0,4,8,12 of each 16-lane group hold the four exponents
-  const int lane = threadIdx.x & 31;
-  const int base = lane & 16;
-  uint32_t word = static_cast<uint32_t>(__shfl_sync(0xffffffffu, e, base + 0));
-  word |= static_cast<uint32_t>(__shfl_sync(0xffffffffu, e, base + 4)) << 8;
-  word |= static_cast<uint32_t>(__shfl_sync(0xffffffffu, e, base + 8)) << 16;
-  word |= static_cast<uint32_t>(__shfl_sync(0xffffffffu, e, base + 12)) << 24;
-  if (live && (lane & 15) == 0) {
-    const int64_t t = i / vec_per_row;
-    const int w = static_cast<int>(i - t * vec_per_row) / 16;
-    x_sf[t * (h / kTileK) + w] = static_cast<int32_t>(word);
-    if (shared_bm > 0) {
-      // row of token t in the BLOCK_M-dependent shared-expert scale layout (backend/staging.py:85-95)
-      const int64_t mm = t % shared_bm;
-      const int64_t bm_al = (shared_bm + 127) / 128 * 128;
-      const int64_t row = (t / shared_bm) * bm_al + (mm / 128) * 128 + (mm % 32) * 4 + (mm % 128) / 32;
-      shared_sf[(int64_t)w * shared_rows + row] = static_cast<int32_t>(word);
-    }
-  }
+  for (int j = 0; j < 4; ++j)
+    w[j] = __nv_cvt_float2_to_fp8x2(make_float2(__fmul_rn(v[2 * j], inv), __fmul_rn(v[2 * j + 1], inv)), __NV_SATFINITE, __NV_E4M3);
+  *q_out = make_uint2(w[0] | (w[1] << 16), w[2] | (w[3] << 16));
+  // the four exponents of a 16-lane group, one per byte, in every lane of the group
+  uint32_t word = static_cast<uint32_t>(e) << (8 * ((threadIdx.x >> 2) & 3));
+  word |= __shfl_xor_sync(0xffffffffu, word, 4);
+  word |= __shfl_xor_sync(0xffffffffu, word, 8);
+  *word_out = word;
 }
 
 // Router in front of the quantiser (one warp per token): the k largest gate logits (ties: the lower expert id), weights =
@@ -149,26 +134,33 @@ __global__ void __launch_bounds__(256) stage_kernel(
     const void* __restrict__ ids_in, int ids64, const float* __restrict__ w_in, const uint8_t* __restrict__ pad,
     int64_t* __restrict__ ids_out, float* __restrict__ w_out, int m, int h, int k, RouterArgs router) {
   chain_begin();
-  const int vec_per_row = h / 8;
-  const int64_t total = (int64_t)m * vec_per_row;
+  const int vec_per_row = h / 8, segs = (vec_per_row + kStageSegVec - 1) / kStageSegVec, words = h / kTileK;
+  const int lane = threadIdx.x & 31;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int64_t total_padded = (total + 31) / 32 * 32;   // whole warps iterate together (shuffles inside)
-  // four independent 16-byte loads in flight per thread before any of them is consumed
-  for (int64_t i = tid; i < total_padded; i += 4 * stride) {
+  for (int64_t seg = tid >> 5; seg < (int64_t)m * segs; seg += stride >> 5) {
+    const int t = static_cast<int>(seg / segs);
+    const int v0 = static_cast<int>(seg - (int64_t)t * segs) * kStageSegVec + lane;
+    const uint4* row = hidden + (int64_t)t * vec_per_row;
     uint4 raw[4];
-    bool live[4], active[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) raw[u] = v0 + 32 * u < vec_per_row ? __ldcs(row + v0 + 32 * u) : make_uint4(0, 0, 0, 0);
+    // row of token t in the BLOCK_M-dependent shared-expert scale layout (backend/staging.py:85-95)
+    const int mm = shared_bm > 0 ? t % shared_bm : 0;
+    const int64_t shared_row = shared_bm > 0 ? (int64_t)(t / shared_bm) * ((shared_bm + 127) / 128 * 128) + (mm / 128) * 128 + (mm % 32) * 4 + (mm % 128) / 32 : 0;
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
-      const int64_t iu = i + u * stride;
-      active[u] = iu < total_padded;           // warp-uniform: stride and total_padded are multiples of 32
-      live[u] = iu < total;
-      raw[u] = make_uint4(0, 0, 0, 0);
-      if (live[u]) raw[u] = hidden[iu];
+      const int v = v0 + 32 * u;                     // rows are whole multiples of 32 vectors: a warp is in or out together
+      if (v >= vec_per_row) break;
+      uint2 q;
+      uint32_t word;
+      stage_vector(raw[u], &q, &word);
+      x_q[(int64_t)t * vec_per_row + v] = q;
+      if ((lane & 15) == 0) {
+        x_sf[(int64_t)t * words + v / 16] = static_cast<int32_t>(word);
+        if (shared_bm > 0) shared_sf[(int64_t)(v / 16) * shared_rows + shared_row] = static_cast<int32_t>(word);
+      }
     }
-#pragma unroll
-    for (int u = 0; u < 4; ++u)
-      if (active[u]) stage_vector(raw[u], live[u], i + u * stride, vec_per_row, h, x_q, x_sf, shared_sf, shared_rows, shared_bm);
   }
   if (router.logits != nullptr) {
     const int64_t warp = tid >> 5, warps = stride >> 5;
@@ -197,8 +189,8 @@ cudaError_t launch_route_stage(const Ctx& c, const void* hidden, const void* ids
                                cudaStream_t s) {
   if (m == 0) return cudaSuccess;
   const int h = c.geo.hidden;
-  const int64_t total = (int64_t)m * h / 8;
-  int blocks = static_cast<int>(std::min<int64_t>((total + 1023) / 1024, 148 * 8));
+  const int64_t segs = (int64_t)m * ((h / 8 + kStageSegVec - 1) / kStageSegVec);      // one warp each
+  int blocks = static_cast<int>(std::min<int64_t>((segs + 7) / 8, 148 * 8));
   if (blocks < 1) blocks = 1;
   const RouterArgs router{logits, num_logical, replica_count, replica_slots, max_copies};
   launch_chained(stage_kernel, dim3(blocks), dim3(256), 0, s, static_cast<const uint4*>(hidden), c.at<uint2>(c.lay.x), c.at<int32_t>(c.lay.x_sf),
@@ -1089,44 +1081,78 @@ __device__ __forceinline__ void add_bf16x8(float (&acc)[8], const uint4& v) {
   }
 }
 
+// A warp takes 64 vectors of 8 outputs of one token; a lane has the rows of up to eight slots of its two vectors in flight at
+// once (with one dependent load after the other 3840 x 5120 top-6, 315 MB, took 63 us).
+constexpr int kCombineSegVec = 64;
 __global__ void __launch_bounds__(256) combine_kernel(
     const uint4* __restrict__ rows, const int32_t* __restrict__ route_pos, const uint4* __restrict__ shared_out,
     const uint4* __restrict__ residual, uint4* __restrict__ y, int m, int h, int k) {
   chain_begin();
-  const int vec = h / 8;
-  const int64_t total = (int64_t)m * vec;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t t = i / vec;
-    const int v = static_cast<int>(i % vec);
-    float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    for (int s = 0; s < k; ++s) {
-      const int pos = route_pos[t * k + s];
-      if (pos >= 0) add_bf16x8(acc, rows[(int64_t)pos * vec + v]);
-    }
-    if (shared_out != nullptr) add_bf16x8(acc, shared_out[i]);
-    uint4 out;
-    __nv_bfloat162* o = reinterpret_cast<__nv_bfloat162*>(&out);
+  const int vec = h / 8, segs = (vec + kCombineSegVec - 1) / kCombineSegVec, lane = threadIdx.x & 31;
+  const int64_t warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  for (int64_t seg = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; seg < (int64_t)m * segs; seg += warps) {
+    const int t = static_cast<int>(seg / segs);
+    const int v0 = static_cast<int>(seg - (int64_t)t * segs) * kCombineSegVec + lane;
+    const bool both = v0 + 32 < vec;                 // rows are whole multiples of 32 vectors
+    const int my_pos = lane < k ? route_pos[(int64_t)t * k + lane] : -1;
+    const int64_t i = (int64_t)t * vec + v0;
+    uint4 sh[2], res[2];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) o[j] = __floats2bfloat162_rn(acc[2 * j], acc[2 * j + 1]);
-    if (residual != nullptr) {
-      // what the serving engine's separate BF16 addition leaves: the layer output rounded to BF16 first, then the sum
-      // of the two BF16 values rounded once more
-      const uint4 res = residual[i];
-      const __nv_bfloat162* r = reinterpret_cast<const __nv_bfloat162*>(&res);
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const float2 a = __bfloat1622float2(o[j]), b = __bfloat1622float2(r[j]);
-        o[j] = __floats2bfloat162_rn(__fadd_rn(a.x, b.x), __fadd_rn(a.y, b.y));
+    for (int u = 0; u < 2; ++u) {
+      sh[u] = res[u] = make_uint4(0, 0, 0, 0);
+      if (u == 0 || both) {
+        if (shared_out != nullptr) sh[u] = __ldcs(shared_out + i + 32 * u);
+        if (residual != nullptr) res[u] = residual[i + 32 * u];
       }
     }
-    y[i] = out;
+    float acc[2][8] = {};
+    for (int s0 = 0; s0 < k; s0 += 8) {
+      uint4 q[8][2];
+      bool valid[8];
+#pragma unroll
+      for (int s = 0; s < 8; ++s) {
+        const int pos = __shfl_sync(0xffffffffu, my_pos, (s0 + s) & 31);
+        valid[s] = s0 + s < k && pos >= 0;           // warp-uniform
+        if (valid[s]) {
+          const uint4* row = rows + (int64_t)pos * vec + v0;
+          q[s][0] = __ldcs(row);
+          if (both) q[s][1] = __ldcs(row + 32);
+        }
+      }
+#pragma unroll
+      for (int s = 0; s < 8; ++s)
+        if (valid[s]) {
+          add_bf16x8(acc[0], q[s][0]);
+          if (both) add_bf16x8(acc[1], q[s][1]);
+        }
+    }
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      if (u == 1 && !both) break;
+      if (shared_out != nullptr) add_bf16x8(acc[u], sh[u]);
+      uint4 out;
+      __nv_bfloat162* o = reinterpret_cast<__nv_bfloat162*>(&out);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) o[j] = __floats2bfloat162_rn(acc[u][2 * j], acc[u][2 * j + 1]);
+      if (residual != nullptr) {
+        // what the serving engine's separate BF16 addition leaves: the layer output rounded to BF16 first, then the sum
+        // of the two BF16 values rounded once more
+        const __nv_bfloat162* r = reinterpret_cast<const __nv_bfloat162*>(&res[u]);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const float2 a = __bfloat1622float2(o[j]), b = __bfloat1622float2(r[j]);
+          o[j] = __floats2bfloat162_rn(__fadd_rn(a.x, b.x), __fadd_rn(a.y, b.y));
+        }
+      }
+      y[i + 32 * u] = out;
+    }
   }
 }
 
 cudaError_t launch_combine(const Ctx& c, void* y, const void* residual, int m, cudaStream_t s) {
   if (m == 0) return cudaSuccess;
-  const int64_t total = (int64_t)m * c.geo.hidden / 8;
-  const int blocks = static_cast<int>(std::min<int64_t>((total + 255) / 256, 148 * 16));
+  const int64_t segs = (int64_t)m * ((c.geo.hidden / 8 + kCombineSegVec - 1) / kCombineSegVec);      // one warp each
+  const int blocks = static_cast<int>(std::min<int64_t>((segs + 7) / 8, 148 * 8));
   const uint4* rows = c.geo.num_ranks == 1 ? c.at<uint4>(c.lay.ret) : c.at<uint4>(c.lay.ret_recv);
   launch_chained(combine_kernel, dim3(blocks), dim3(256), 0, s, rows, c.at<int32_t>(c.lay.route_pos),
                                         c.geo.num_shared_experts > 0 ? c.at<uint4>(c.lay.shared_out) : nullptr,
