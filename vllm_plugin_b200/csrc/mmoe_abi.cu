@@ -277,7 +277,7 @@ int mmoe_prepare(const MmoeGeometry* geo, int32_t* block_ms, int32_t cap, int32_
 int mmoe_stage_inputs(const MmoeGeometry* geo, void* workspace, const void* hidden_bf16, const void* topk_ids,
                       int32_t ids_are_int64, const float* topk_weights, const uint8_t* is_padding, int32_t num_tokens,
                       int32_t shared_block_m, void* stream) {
-  mmoe::ChainScope chain(num_tokens <= 128);
+  mmoe::ChainScope chain(geo != nullptr && geo->num_ranks == 1);
   mmoe::Ctx c;
   int rc = make_ctx(geo, workspace, &c);
   if (rc != MMOE_OK) return rc;
@@ -298,7 +298,7 @@ int mmoe_route_stage_inputs(const MmoeGeometry* geo, void* workspace, const void
                             int32_t num_logical_experts, const int32_t* replica_count, const int32_t* replica_slots,
                             int32_t max_copies, const uint8_t* is_padding, int32_t num_tokens, int32_t shared_block_m,
                             void* stream) {
-  mmoe::ChainScope chain(num_tokens <= 128);
+  mmoe::ChainScope chain(geo != nullptr && geo->num_ranks == 1);
   mmoe::Ctx c;
   int rc = make_ctx(geo, workspace, &c);
   if (rc != MMOE_OK) return rc;
@@ -434,7 +434,7 @@ int mmoe_plan_shared(const MmoeGeometry* geo, void* workspace, int32_t num_token
   if (rc == MMOE_OK) rc = check_tokens(geo, num_tokens);
   if (rc != MMOE_OK) return rc;
   if (!valid_block_m(block_m)) return fail(MMOE_ERR_INVALID_ARGUMENT, "block_m=%d is not a BLOCK_M value", block_m);
-  cudaError_t e = mmoe::launch_shared_plan(c, num_tokens, block_m, static_cast<cudaStream_t>(stream));
+  cudaError_t e = mmoe::launch_shared_plan(c, num_tokens, static_cast<cudaStream_t>(stream));
   return e == cudaSuccess ? MMOE_OK : cuda_fail(e, "shared plan launch");
 }
 
@@ -525,7 +525,7 @@ int mmoe_combine(const MmoeGeometry* geo, void* workspace, void* y_bf16, int32_t
 
 int mmoe_forward(const MmoeGeometry* geo, void* workspace, const MmoeWeights* weights, const MmoeOptions* opt,
                  void* y_bf16, int32_t num_tokens, int32_t block_m, int32_t* stats, void* stream) {
-  mmoe::ChainScope chain(num_tokens <= 128);
+  mmoe::ChainScope chain(true);
   if (geo != nullptr && geo->num_ranks != 1)
     return fail(MMOE_ERR_INVALID_ARGUMENT, "mmoe_forward is the single-rank sequence; call mmoe_forward_ep for num_ranks > 1");
   mmoe::Ctx c;
@@ -534,8 +534,9 @@ int mmoe_forward(const MmoeGeometry* geo, void* workspace, const MmoeWeights* we
   if (rc != MMOE_OK) return rc;
   if (!valid_block_m(block_m)) return fail(MMOE_ERR_INVALID_ARGUMENT, "block_m=%d is not a BLOCK_M value", block_m);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  // route ordering, plan and placement: one launch up to 128 tokens, two beyond
-  const cudaError_t e = num_tokens > 0 && num_tokens <= 128 && geo->num_experts <= 512
+  // route ordering, plan and placement: one launch up to 128 tokens, two beyond (and where the pair kernels are forced on:
+  // those read the shared expert's scales from chunks that the larger form writes)
+  const cudaError_t e = num_tokens > 0 && num_tokens <= 128 && c.pair_above_for(num_tokens) == mmoe::kNeverPair
                             ? mmoe::launch_route_small(c, num_tokens, block_m, stats, st)
                             : mmoe::launch_route_large(c, num_tokens, block_m, stats, st);
   if (e != cudaSuccess) return cuda_fail(e, "route / plan / placement launch");
@@ -576,7 +577,7 @@ int mmoe_forward_ep(const MmoeGeometry* geo, void* workspace, const void* const*
   // ... while the shared expert, which needs only this rank's own tokens, runs both of its GEMMs here
   mmoe::Ctx c;
   rc = make_ctx(geo, workspace, &c);
-  if (rc == MMOE_OK && mmoe::launch_shared_plan(c, num_tokens, block_m, main_stream) != cudaSuccess)
+  if (rc == MMOE_OK && mmoe::launch_shared_plan(c, num_tokens, main_stream) != cudaSuccess)
     rc = cuda_fail(cudaGetLastError(), "shared plan launch");
   if (rc == MMOE_OK) rc = run_experts(geo, workspace, nullptr, weights, opt, num_tokens, block_m, stream, 2);
   // join (always, so that a capture is never left forked)

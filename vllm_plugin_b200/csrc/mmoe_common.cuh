@@ -22,6 +22,9 @@ constexpr int kPairTileRows = 128;       // largest token tile of the tokens-as-
 // Which kernels run an expert depends on the rows it received in this call (see pair_above_default in mmoe_abi.cu).
 constexpr int kNeverPair = 0x7fffffff;
 
+// Rows of a weights-as-A tile: five stages of up to 80 rows fit the shared memory, four of 112.
+constexpr int kDeepTileRows = 80;
+
 // How the n rows of an expert are cut into tiles.  Up to `pair_above` rows: ceil(n / small_cap) equal tiles (rounded up to 16
 // rows) for the weights-as-A kernels.  Above: an even number of tiles of at most 128 rows, the two halves of CTA-pair tasks;
 // the second half of a single pair is empty when everything fits the first.  Cuts ignore the BLOCK_M boundaries of the pool.
@@ -38,9 +41,18 @@ __host__ __device__ inline Cut cut_rows(int n, int pair_above, int small_cap) {
   const int parts = (n + small_cap - 1) / small_cap;
   return Cut{parts, ((n + parts - 1) / parts + 15) & ~15};
 }
+// The cut of the shared expert's m tokens: known to the host, so that its tiles need no plan.
+__host__ __device__ inline Cut shared_cut(int m, int pair_above) { return cut_rows(m, pair_above, kDeepTileRows); }
+// Cap of a call without pair tiles (also known to the host: the largest tile of such a call fixes its stage layout): no expert
+// has more rows than there are tokens unless a token names it twice, which then costs another tile.
+__host__ __device__ inline int small_only_cap(int m, int block_m) {
+  const int rows = (m + 15) & ~15, least = block_m < 64 ? block_m : 64;
+  return rows >= kDeepTileRows ? kDeepTileRows : (rows > least ? rows : least);
+}
+
 // Scale-factor chunks (128 token rows each) reserved per pool block of a BLOCK_M variant: at least as many as the non-empty
-// tiles an expert's rows are cut into (small_cap >= 16 for BLOCK_M 16, >= 32 for 32, >= 64 for 64, >= 80 above).
-__host__ __device__ inline int chunks_per_block(int block_m) { return block_m <= 64 ? 1 : (block_m <= 192 ? 2 : 3); }
+// tiles an expert's rows are cut into (small_cap >= 16 for BLOCK_M 16, >= 32 for 32, >= 64 for 64, >= 80 for 192 and 240).
+__host__ __device__ inline int chunks_per_block(int block_m) { return block_m <= 64 ? 1 : (block_m <= 128 ? 2 : 3); }
 constexpr int kSortChunkTokens = 128;
 constexpr int kSharedExpert = -2;  // MmoeTile::expert of a shared-expert tile
 
@@ -63,14 +75,11 @@ struct PlanHeader {
   int32_t total_recv;          // routes received by this rank
   int32_t block_m;
   int32_t num_tokens;
-  int32_t num_early_shared_tiles;   // shared-expert tiles written ahead of the routed plan, at the tail of the tile table
   int32_t num_small_tiles;     // the first of the routed tiles: those of the weights-as-A kernels; the others are pair tiles
   int32_t small_cap;           // rows a weights-as-A tile of this call may have
   int32_t small_rows;          // rows of the largest one, rounded up to 16
-  int32_t shared_small;        // 1: the shared expert's tiles are weights-as-A tiles
-  int32_t early_small_rows;    // small_rows of the tiles written ahead (0: they are pair tiles)
   int32_t ticket;              // blocks of the route-counting launch that have finished; zero between launches
-  int32_t pad[3];
+  int32_t pad[6];
 };
 static_assert(sizeof(PlanHeader) == 64, "plan header is 64 bytes");
 
@@ -89,40 +98,19 @@ struct PlanView {
 
 __host__ __device__ inline int64_t align_up(int64_t a, int64_t b) { return (a + b - 1) / b * b; }
 
-// A contiguous run of the tile table, after `lead` further records that come first in the task order (the shared expert's).
-struct TileRange {
-  const Tile* tiles;
-  int32_t count;          // all records, the leading ones included
-  const Tile* lead_tiles;
-  int32_t lead;
-  __host__ __device__ const Tile& at(int i) const { return i < lead ? lead_tiles[i] : tiles[i - lead]; }
+// The shared expert's tiles of a launch, in front of the routed ones and without a tile record.
+struct SharedTiles {
+  int32_t parts, step, m;       // parts 0: none in this launch
+  __host__ __device__ Tile at(int j) const {
+    const int rows = m - j * step < step ? m - j * step : step;
+    return rows > 0 ? Tile{kSharedExpert, j * step, rows, j, j, parts, {0, 0}} : Tile{kSharedExpert, 0, 0, 0, j, parts, {0, 0}};
+  }
 };
-// The tiles a launch runs.  `select`: 0 = every tile of the plan, 1 = routed tiles only, 2 = the shared expert's tiles
-// planned ahead (at the tail of the table).  Table order: routed weights-as-A tiles, routed pair tiles, shared tiles.
-__host__ __device__ inline TileRange small_tiles(const PlanView& v, int select, bool has_shared, int64_t early_first, int early_cap) {
-  const PlanHeader& h = *v.hdr;
-  if (select == 2) {
-    const int n = has_shared && h.early_small_rows > 0 ? h.num_early_shared_tiles : 0;
-    return TileRange{v.tiles + early_first, n < 0 ? 0 : (n > early_cap ? early_cap : n), nullptr, 0};
-  }
-  const int lead = select == 0 && has_shared && h.shared_small ? h.num_shared_tiles : 0;   // a shared weight row has twice the bytes: first
-  return TileRange{v.tiles, h.num_small_tiles + lead, v.tiles + h.num_routed_tiles, lead};
-}
-__host__ __device__ inline TileRange pair_tiles(const PlanView& v, int select, bool has_shared, int64_t early_first, int early_cap) {
-  const PlanHeader& h = *v.hdr;
-  if (select == 2) {
-    const int n = has_shared && h.early_small_rows == 0 ? h.num_early_shared_tiles : 0;
-    return TileRange{v.tiles + early_first, n < 0 ? 0 : (n > early_cap ? early_cap : n), nullptr, 0};
-  }
-  const int n = h.num_routed_tiles - h.num_small_tiles + (select == 0 && has_shared && !h.shared_small ? h.num_shared_tiles : 0);
-  return TileRange{v.tiles + h.num_small_tiles, n, nullptr, 0};
-}
 
 // scale chunks of the shared expert's tokens: one per tile, whatever the cut
 __host__ __device__ inline int64_t shared_chunk_rows(int64_t max_tokens) { return (max_tokens / 64 + 2) * 128; }
 
-// tile records reserved for the shared expert of a call with at most `max_tokens` tokens (they sit at the tail of the
-// tile table when the shared expert is planned ahead of the routed experts)
+// tile records reserved for the shared expert of a call with at most `max_tokens` tokens
 __host__ __device__ inline int64_t shared_tile_capacity(int64_t max_tokens) { return (max_tokens / 16 + 2) * 2; }
 
 __host__ __device__ inline int64_t plan_bytes(int e_local, int num_ranks, int64_t max_tiles) {
@@ -321,7 +309,7 @@ cudaError_t launch_pack(const Ctx& c, int m, cudaStream_t s);
 cudaError_t launch_route_small(const Ctx& c, int m, int block_m, int32_t* stats, cudaStream_t s);
 cudaError_t launch_route_large(const Ctx& c, int m, int block_m, int32_t* stats, cudaStream_t s);
 cudaError_t launch_plan_place(const Ctx& c, int m, int block_m, int32_t* stats, cudaStream_t s);
-cudaError_t launch_shared_plan(const Ctx& c, int m, int block_m, cudaStream_t s);
+cudaError_t launch_shared_plan(const Ctx& c, int m, cudaStream_t s);
 cudaError_t launch_combine(const Ctx& c, void* y, const void* residual, int m, cudaStream_t s);
 cudaError_t launch_experts_simt(const Ctx& c, const MmoeWeights& w, const MmoeOptions& o, int m, int block_m, cudaStream_t s);
 cudaError_t launch_experts_umma(const Ctx& c, const MmoeWeights& w, const MmoeOptions& o, int m, int block_m, cudaStream_t s);

@@ -546,7 +546,6 @@ __device__ void emit_tiles(Tile* out, int expert, int row_base, int n, Cut cut, 
 struct ExpertPlan {
   int block_off;     // first pool block
   int row_off;       // rows of the experts before it
-  int small_cap;     // of the call
   Cut cut;
 };
 
@@ -556,13 +555,14 @@ __device__ ExpertPlan build_plan(const PlanView& pv, int n, const PlanArgs& a, b
   const int e = threadIdx.x;
   __shared__ int s_rows;
   if (threadIdx.x == 0) s_rows = 16;
-  // A weights-as-A stage holds five stages of up to 80 rows, or four of 112: 112 only when enough experts gain a tile by it.
+  // With pair tiles in the call, weights-as-A tiles of 112 rows (four stages fit the shared memory) only when enough experts
+  // gain a tile by it, else of 80 (five stages).
   const bool small = n > 0 && n <= a.pair_above;
-  const bool wide = small && ((n > 80 && n <= kSmallTileRows) || n > 160);
+  const bool wide = small && ((n > kDeepTileRows && n <= kSmallTileRows) || n > 2 * kDeepTileRows);
   const int num_small = __syncthreads_count(small), num_wide = __syncthreads_count(wide);
-  const int cap = num_wide * 8 > num_small ? kSmallTileRows : 80;
+  const int cap = a.pair_above == kNeverPair ? small_only_cap(a.m, a.block_m) : (num_wide * 8 > num_small ? kSmallTileRows : kDeepTileRows);
   const Cut cut = cut_rows(n, a.pair_above, cap);
-  const Cut shared_cut = cut_rows(a.has_shared ? a.m : 0, a.pair_above, cap);
+  const Cut sh_cut = shared_cut(a.has_shared ? a.m : 0, a.pair_above);
   const bool shared_small = a.m <= a.pair_above;
   const int blocks = (n + a.block_m - 1) / a.block_m;
   ScanPair total;
@@ -586,26 +586,21 @@ __device__ ExpertPlan build_plan(const PlanView& pv, int n, const PlanArgs& a, b
     if (threadIdx.x == 0) {
       PlanHeader& h = *pv.hdr;
       h.num_routed_tiles = small_total + pair_total;
-      h.num_shared_tiles = shared_cut.parts;
+      h.num_shared_tiles = sh_cut.parts;
       h.num_pool_blocks = static_cast<int>(total.a & 0x1FFFFF);
       h.total_recv = total.b;
       h.block_m = a.block_m;
       h.num_tokens = a.m;
       h.num_small_tiles = small_total;
       h.small_cap = cap;
-      h.small_rows = max(s_rows, shared_small && a.has_shared ? shared_cut.step : 16);
-      h.shared_small = shared_small ? 1 : 0;
+      h.small_rows = max(s_rows, shared_small && a.has_shared ? sh_cut.step : 16);
       pv.expert_block_off[a.e_local] = h.num_pool_blocks;
       pv.expert_tile_off[a.e_local] = h.num_routed_tiles;
     }
-    if (a.has_shared)
-      for (int j = threadIdx.x; j < shared_cut.parts; j += blockDim.x) {
-        const int rows_j = max(0, min(shared_cut.step, a.m - j * shared_cut.step));
-        pv.tiles[small_total + pair_total + j] =
-            Tile{kSharedExpert, rows_j > 0 ? j * shared_cut.step : 0, rows_j, rows_j > 0 ? j : 0, j, shared_cut.parts, {0, 0}};
-      }
+    const SharedTiles shared{sh_cut.parts, sh_cut.step, a.m};
+    for (int j = threadIdx.x; j < sh_cut.parts; j += blockDim.x) pv.tiles[small_total + pair_total + j] = shared.at(j);
   }
-  return ExpertPlan{block_off, at.b, cap, cut};
+  return ExpertPlan{block_off, at.b, cut};
 }
 
 // Scale words of the call's own tokens in the chunks of the shared expert's tiles (chunk j = tile j), whole warps.
@@ -613,32 +608,21 @@ struct SharedScales {
   const int32_t* x_sf;
   int32_t* out;          // nullptr: no shared expert
   int64_t rows;
+  Cut cut;
 };
-__device__ void place_shared_scales(const SharedScales& s, Cut cut, int t, int words) {
+__device__ void place_shared_scales(const SharedScales& s, int t, int words) {
+  const Cut cut = s.cut;
   const int j = t / cut.step;
   const int64_t pos = (int64_t)j * kChunkRows + chunk_pos(t - j * cut.step);
   for (int w = threadIdx.x & 31; w < words; w += 32) s.out[w * s.rows + pos] = s.x_sf[(int64_t)t * words + w];
 }
 
-// The shared expert's tiles depend only on the token count, so they can be planned (and run) before the routed
-// experts' receive counts are known: written at the tail of the tile table, counted in the header.
-__global__ void __launch_bounds__(256) shared_plan_kernel(char* __restrict__ plan_base, int e_local, int num_ranks, int m,
-                                                          int pair_above, int64_t first_tile, SharedScales scales, int words) {
+// The shared expert's tiles depend only on the token count: with its scale chunks written it can run before the routed
+// experts' receive counts are known.
+__global__ void __launch_bounds__(256) shared_plan_kernel(int m, SharedScales scales, int words) {
   chain_begin();
-  const Cut cut = cut_rows(m, pair_above, kSmallTileRows);
-  if (blockIdx.x == 0) {
-    PlanView pv = plan_view(plan_base, e_local, num_ranks);
-    for (int j = threadIdx.x; j < cut.parts; j += blockDim.x) {
-      const int rows = max(0, min(cut.step, m - j * cut.step));
-      pv.tiles[first_tile + j] = Tile{kSharedExpert, rows > 0 ? j * cut.step : 0, rows, rows > 0 ? j : 0, j, cut.parts, {0, 0}};
-    }
-    if (threadIdx.x == 0) {
-      pv.hdr->num_early_shared_tiles = cut.parts;
-      pv.hdr->early_small_rows = m <= pair_above ? cut.step : 0;
-    }
-  }
   const int warps = (gridDim.x * blockDim.x) >> 5;
-  for (int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < m; t += warps) place_shared_scales(scales, cut, t, words);
+  for (int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < m; t += warps) place_shared_scales(scales, t, words);
 }
 
 // General plan (any number of source ranks), one block: rows per expert from the receive counts, and for every (expert,
@@ -759,9 +743,10 @@ __device__ void write_single_rank_plan(const RouteArgs& r, const PlanView& pv, i
 
 // Calls of at most 128 tokens: ONE launch.  Every block ranks the routes and builds the plan for itself in shared memory
 // (2-3 us, less than a second launch behind a grid-wide hand-over), block 0 writes it out, and each block places its share
-// of the routes, one warp per route.
+// of the routes, one warp per route.  The shared expert's scales are not placed: its GEMM1 gathers them itself.
 __global__ void __launch_bounds__(kRouteThreads) route_small_kernel(const RouteArgs r) {
-  chain_begin();
+  chain_wait();
+  chain_release();       // in this order: the GEMM1 launch starts knowing that the staging has completed
   extern __shared__ int32_t sm[];
   const int E = r.a.e_local, n = r.a.m * r.k, n_even = (n + 1) & ~1;
   int32_t* s_block = sm;                             // [E] first pool block
@@ -815,10 +800,6 @@ __global__ void __launch_bounds__(kRouteThreads) route_small_kernel(const RouteA
       r.sorted_route[s_off[e] + j] = i;
     }
   }
-  if (r.shared.out != nullptr) {
-    const Cut cut = cut_rows(r.a.m, r.a.pair_above, ep.small_cap);
-    for (int t = blockIdx.x * kRouteWarps + (threadIdx.x >> 5); t < r.a.m; t += warps) place_shared_scales(r.shared, cut, t, words);
-  }
 }
 
 // Larger calls, first of two launches: one block per 128 tokens ranks its routes; the last block to finish sums the chunks
@@ -836,6 +817,10 @@ __global__ void __launch_bounds__(kRouteThreads) route_count_kernel(const RouteA
     if (id >= E) { report_bad_index(r.status); id = -1; }
     ids[i] = id < 0 ? 0xFFFF : static_cast<uint16_t>(id);
   }
+  // scale chunks of the shared expert's tiles: written here because GEMM1 starts with them while the next launch still places
+  if (r.shared.out != nullptr)
+    for (int t = blockIdx.x * kSortChunkTokens + (threadIdx.x >> 5); t < min(r.a.m, (blockIdx.x + 1) * kSortChunkTokens); t += kRouteWarps)
+      place_shared_scales(r.shared, t, r.h / kTileK);
   int total = block_rank_routes(ids, n, rank, warp_count, E);
   for (int i = threadIdx.x; i < n; i += kRouteThreads) r.route_pos[r0 + i] = ids[i] == 0xFFFF ? -1 : rank[i];
   const int e = threadIdx.x;
@@ -868,12 +853,12 @@ __global__ void __launch_bounds__(kRouteThreads) route_count_kernel(const RouteA
 // Second launch: one warp per token.  The token's FP8 row is read once and stored to the pool rows of all its routes; lane s
 // works out where route s goes.
 __global__ void __launch_bounds__(256) route_place_kernel(const RouteArgs r) {
-  chain_begin();
+  chain_wait();
+  chain_release();       // in this order: the GEMM1 launch starts knowing that staging, counting and plan have completed
   const PlanView pv = plan_view(r.plan, r.a.e_local, 1);
   const int lane = threadIdx.x & 31, warps = (gridDim.x * blockDim.x) >> 5;
   const int vec = r.h / 16, words = r.h / kTileK, cpb = chunks_per_block(r.a.block_m);
   const int cap = pv.hdr->small_cap;
-  const Cut shared_cut = cut_rows(r.a.m, r.a.pair_above, cap);
   for (int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < r.a.m; t += warps) {
     int row = -1, sf_pos = 0;                          // lane s: pool row and scale position of route s
     if (lane < r.k) {
@@ -919,7 +904,6 @@ __global__ void __launch_bounds__(256) route_place_kernel(const RouteArgs r) {
         if (p >= 0 && wd < words) r.pool_sf[wd * r.pool_sf_rows + pos] = v;
       }
     }
-    if (r.shared.out != nullptr) place_shared_scales(r.shared, shared_cut, t, words);
   }
 }
 
@@ -931,7 +915,7 @@ __global__ void __launch_bounds__(256) place_kernel(
     char* __restrict__ plan_base, const uint4* __restrict__ src_x, const int32_t* __restrict__ src_sf,
     const float* __restrict__ src_w, const int32_t* __restrict__ sorted_route, uint4* __restrict__ pool_x,
     int32_t* __restrict__ pool_sf, float* __restrict__ pool_w, int32_t* __restrict__ pool_dst, int64_t pool_sf_rows,
-    int e_local, int num_ranks, int h, int k, int direct, int pair_above, SharedScales shared) {
+    int e_local, int num_ranks, int h, int k, int direct, SharedScales shared) {
   chain_begin();
   PlanView pv = plan_view(plan_base, e_local, num_ranks);
   const int ntiles = pv.hdr->num_routed_tiles;
@@ -940,8 +924,7 @@ __global__ void __launch_bounds__(256) place_kernel(
   const int warp_in_block = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
   if (shared.out != nullptr) {
     const int m = pv.hdr->num_tokens;
-    const Cut cut = cut_rows(m, pair_above, pv.hdr->small_cap);
-    for (int t = blockIdx.x * warps + warp_in_block; t < m; t += gridDim.x * warps) place_shared_scales(shared, cut, t, words);
+    for (int t = blockIdx.x * warps + warp_in_block; t < m; t += gridDim.x * warps) place_shared_scales(shared, t, words);
   }
   constexpr int kSlices = kPairTileRows / 32;
   for (int task = blockIdx.x; task < ntiles * kSlices; task += gridDim.x) {
@@ -998,7 +981,8 @@ PlanArgs plan_args(const Ctx& c, int m, int block_m) {
 
 SharedScales shared_scales(const Ctx& c, int m) {
   const bool on = c.geo.num_shared_experts > 0 && m > 0;
-  return SharedScales{c.at<int32_t>(c.lay.x_sf), on ? c.at<int32_t>(c.lay.shared_tile_sf) : nullptr, shared_chunk_rows(c.geo.num_max_tokens)};
+  return SharedScales{c.at<int32_t>(c.lay.x_sf), on ? c.at<int32_t>(c.lay.shared_tile_sf) : nullptr, shared_chunk_rows(c.geo.num_max_tokens),
+                      shared_cut(m, c.pair_above_for(m))};
 }
 
 RouteArgs route_args(const Ctx& c, int m, int block_m, int32_t* stats) {
@@ -1046,11 +1030,10 @@ cudaError_t launch_route_large(const Ctx& c, int m, int block_m, int32_t* stats,
   return cudaGetLastError();
 }
 
-cudaError_t launch_shared_plan(const Ctx& c, int m, int block_m, cudaStream_t s) {
-  (void)block_m;
-  launch_chained(shared_plan_kernel, dim3(std::max(1, std::min((m + 7) / 8, 148 * 2))), dim3(256), 0, s, c.ws + c.lay.plan, c.e_local,
-                 c.geo.num_ranks, m, c.pair_above_for(m), c.lay.max_tiles - shared_tile_capacity(c.geo.num_max_tokens),
-                 shared_scales(c, m), c.geo.hidden / kTileK);
+cudaError_t launch_shared_plan(const Ctx& c, int m, cudaStream_t s) {
+  if (m == 0 || c.geo.num_shared_experts == 0) return cudaSuccess;
+  launch_chained(shared_plan_kernel, dim3(std::max(1, std::min((m + 7) / 8, 148 * 2))), dim3(256), 0, s, m, shared_scales(c, m),
+                 c.geo.hidden / kTileK);
   return cudaGetLastError();
 }
 
@@ -1063,7 +1046,7 @@ cudaError_t launch_plan_place(const Ctx& c, int m, int block_m, int32_t* stats, 
       direct ? c.at<int32_t>(c.lay.x_sf) : c.at<int32_t>(c.lay.recv_sf),
       direct ? c.at<float>(c.lay.topk_weights) : c.at<float>(c.lay.recv_w), c.at<int32_t>(c.lay.sorted_route),
       c.at<uint4>(c.lay.pool_x), c.at<int32_t>(c.lay.pool_sf), c.at<float>(c.lay.pool_w), c.at<int32_t>(c.lay.pool_dst),
-      c.lay.pool_sf_rows, c.e_local, R, c.geo.hidden, c.geo.num_topk, direct ? 1 : 0, c.pair_above_for(m), shared_scales(c, m));
+      c.lay.pool_sf_rows, c.e_local, R, c.geo.hidden, c.geo.num_topk, direct ? 1 : 0, shared_scales(c, m));
   return cudaGetLastError();
 }
 
@@ -1237,7 +1220,9 @@ __global__ void __launch_bounds__(128) simt_l1_kernel(
       const uint8_t* xr = tok_x + (int64_t)(tile.row0 + i) * h;
       float accg = 0.f, accu = 0.f;
       for (int g = 0; g < h / 32; ++g) {
-        const float sx = ue8m0_to_float(token_sf_byte(tok_sf, tok_sf_rows, tile, i, g));
+        // (the shared expert's tokens: the staged scale rows themselves)
+        const float sx = ue8m0_to_float(shared ? (static_cast<uint32_t>(tok_sf[(int64_t)(tile.row0 + i) * (h / kTileK) + g / 4]) >> (8 * (g % 4))) & 0xFFu
+                                               : token_sf_byte(tok_sf, tok_sf_rows, tile, i, g));
         const float sg = ue8m0_to_float(weight_sf_byte(wsf, 2 * inter, row_g, g));
         const float su = ue8m0_to_float(weight_sf_byte(wsf, 2 * inter, row_u, g));
         float dg, du;
@@ -1316,7 +1301,7 @@ cudaError_t launch_experts_simt(const Ctx& c, const MmoeWeights& w, const MmoeOp
                                         w.w2_slice_stride);
   if (c.geo.num_shared_experts > 0 && m > 0) {
     simt_l1_kernel<<<blocks, 128, 0, s>>>(plan, c.e_local, c.geo.num_ranks, 0, 1, c.at<uint8_t>(c.lay.x),
-                                          c.at<int32_t>(c.lay.shared_tile_sf), shared_chunk_rows(c.geo.num_max_tokens), nullptr,
+                                          c.at<int32_t>(c.lay.x_sf), 0, nullptr,
                                           static_cast<const uint8_t*>(w.shared_w13),
                                           static_cast<const int32_t*>(w.shared_w13_sf),
                                           c.at<uint8_t>(c.lay.shared_act_x), c.at<uint8_t>(c.lay.shared_act_sf),

@@ -237,9 +237,8 @@ struct TmParams {
   __nv_bfloat16* ret;              // layer-2 outputs
   __nv_bfloat16* shared_out;
   const int32_t* pool_dst;
-  int tile_select;                 // 0: every tile of the plan, 1: routed tiles only, 2: the early shared tiles only
-  int64_t early_shared_first;
-  int early_shared_cap;
+  SharedTiles shared_tiles;        // run first
+  int with_routed;                 // 0: only those
   int ep_me;                       // fused write-back (layer 2, EP > 1)
   const int32_t* ep_totals;
   __nv_bfloat16* ep_ret_recv[32];
@@ -252,7 +251,6 @@ struct TmParams {
   int hidden, inter;
   float clamp;
   int fast_math;
-  int has_shared_weights;
 };
 cudaError_t tm_prepare();
 cudaError_t tm_launch(int layer, bool fused, const TmParams& p, cudaStream_t s);

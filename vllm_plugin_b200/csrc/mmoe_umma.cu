@@ -47,7 +47,7 @@ struct UmmaParams {
   const int32_t* wsf_routed;   // [E_l][K/128][rows_per_expert] scale words, 4x32 transposed per 128 rows
   const int32_t* wsf_shared;
   const int32_t* tsf_routed;   // token scale chunks: word w of chunk row r at w * tsf_rows + r
-  const int32_t* tsf_shared;
+  const int32_t* tsf_shared;   // layer 2 only
   int64_t tsf_rows_routed, tsf_rows_shared;
   // layer-1 outputs
   uint8_t* act_routed;
@@ -62,9 +62,11 @@ struct UmmaParams {
   const int32_t* pool_dst;
   // layer 2 at EP > 1 with the write-back fused in: an output row goes straight into the `ret_recv` of the rank its
   // token came from (plain peer stores over NVLink), at that rank's send position
-  int tile_select;             // 0: every tile of the plan, 1: routed tiles only, 2: the early shared tiles only
-  int64_t early_shared_first;  // index of the first early shared tile in the tile table
-  int early_shared_cap;        // tile records reserved there
+  SharedTiles shared_tiles;    // run first
+  int with_routed;             // 0: only those
+  int tile_rows;               // > 0: rows of the call's largest tile, known to the host; 0: in the plan
+  int skip_wait;               // 1: what this launch reads was complete before the launch in front of it let it start
+  const int32_t* x_sf;         // layer 1: the staged tokens' scale words [T][K/128], gathered for the shared expert's tiles
   int ep_me;
   const int32_t* ep_totals;    // [32][32]: totals[s][d] = routes rank s sent to rank d in this call
   __nv_bfloat16* ep_ret_recv[32];
@@ -78,7 +80,6 @@ struct UmmaParams {
   int hidden, inter;
   float clamp;
   int fast_math;
-  int has_shared_weights;
   int max_stages;              // > 0: cap on the shared-memory pipeline depth
   CUtensorMap map_tok_routed_box[kNumBoxes];   // token maps with boxes of 16, 32, ... 112 rows
   CUtensorMap map_tok_shared_box[kNumBoxes];
@@ -149,43 +150,67 @@ struct Cta {                       // where a role finds the CTA's resources
   uint32_t b_bytes;                // token slot of a stage
 };
 
-// Tasks in order: tile by tile, or for an expert with several tiles weight block by weight block, so that the tiles of one
-// block read its weights while they are in L2.
-struct TaskList {
-  TileRange range;
-  int num_tasks, n_blocks;
-  __device__ __forceinline__ const Tile& get(int task, int* nb) const {
-    const int i = task / n_blocks;
-    const Tile& t = range.at(i);
-    if (t.parts == 1) {
-      *nb = task - i * n_blocks;
-      return t;
+// The task list of one CTA as a role walks it.  First the shared expert's tasks, which need nothing but the staged tokens and
+// the host's count of them; then -- after what precedes this launch in the stream has completed -- the routed tiles of the
+// plan.  In the single-GPU decode call the shared expert's GEMM1 thus runs beside the route ordering.
+// Tile by tile, or for an expert with several tiles weight block by weight block, so that the tiles of a block read its
+// weights while they are in L2.  After the first round the CTAs take their tasks in the opposite order: the first ones,
+// whose shared tasks have twice the weight bytes, are not also the ones with a task more in the last round.
+struct TaskWalk {
+  const UmmaParams& p;
+  int shared_tasks, routed_tasks, round;
+  bool waited;
+  const Tile* tiles;
+  Tile tile;               // current task
+  int nb;
+  __device__ __forceinline__ TaskWalk(const UmmaParams& params, bool has_waited)
+      : p(params), shared_tasks(params.shared_tiles.parts * params.n_blocks), routed_tasks(0), round(0), waited(false), tiles(nullptr) {
+    if (has_waited) load_plan();
+  }
+  __device__ __forceinline__ void load_plan() {
+    if (!p.skip_wait) chain_wait();
+    const PlanView pv = plan_view(const_cast<char*>(p.plan), p.e_local, p.num_ranks);
+    tiles = pv.tiles;
+    routed_tasks = p.with_routed ? pv.hdr->num_small_tiles * p.n_blocks : 0;
+    waited = true;
+  }
+  // true: tile and nb are the next task's
+  __device__ __forceinline__ bool next() {
+    int task = round == 0 ? blockIdx.x : (round + 1) * gridDim.x - 1 - blockIdx.x;
+    ++round;
+    if (task < shared_tasks) {
+      nb = task / p.shared_tiles.parts;
+      tile = p.shared_tiles.at(task - nb * p.shared_tiles.parts);
+      return true;
     }
-    const int first = i - t.part;
-    const int local = task - first * n_blocks;
-    *nb = local / t.parts;
-    return range.at(first + local - *nb * t.parts);
+    if (!waited) load_plan();
+    task -= shared_tasks;
+    if (task >= routed_tasks) return false;
+    const int i = task / p.n_blocks;
+    tile = tiles[i];
+    nb = task - i * p.n_blocks;
+    if (tile.parts > 1) {
+      const int first = i - tile.part, local = task - first * p.n_blocks;
+      nb = local / tile.parts;
+      tile = tiles[first + local - nb * tile.parts];
+    }
+    return true;
   }
 };
-
-__device__ __forceinline__ TaskList task_list(const UmmaParams& p, const PlanView& pv) {
-  const TileRange r = small_tiles(pv, p.tile_select, p.has_shared_weights != 0, p.early_shared_first, p.early_shared_cap);
-  return TaskList{r, r.count * p.n_blocks, p.n_blocks};
-}
 
 // ------------------------------------------------------------------------------------------------ producer
 // One warp in step, one elected lane issues.  Everything that does not change inside a task is computed once per task; the
 // K loop only bumps 32-bit coordinates and two pointers, because such a loop runs at instruction latency, not throughput.
 template <int kLayer, typename L>
-__device__ __forceinline__ void sa_producer(const UmmaParams& p, const Cta& c, const TaskList& tl, Waiter& waiter,
+__device__ __forceinline__ void sa_producer(const UmmaParams& p, const Cta& c, TaskWalk walk, Waiter& waiter,
                                             RoleState& st) {
   const int k_stages = p.k_dim / kTileK;
   const uint32_t full0 = smem_u32(&c.ctl->full[0]), empty0 = smem_u32(&c.ctl->empty[0]);
   const uint32_t sf_full0 = smem_u32(&c.ctl->sf_full[0]);
   const uint32_t a0 = smem_u32(c.a_base), b0 = smem_u32(c.b_base), sf0 = smem_u32(c.sf_base);
-  for (int task = blockIdx.x; task < tl.num_tasks && st.ok; task += gridDim.x) {
-    int nb;
-    const Tile tile = tl.get(task, &nb);
+  while (st.ok && walk.next()) {
+    const Tile tile = walk.tile;
+    const int nb = walk.nb;
     const bool shared = tile.expert == kSharedExpert;
     const int box_sel = (max(tile.n_valid, 1) - 1) >> 4;         // token box: n_valid rounded up to 16 rows
     const uint32_t box_rows = 16u * (box_sel + 1);
@@ -205,7 +230,8 @@ __device__ __forceinline__ void sa_producer(const UmmaParams& p, const Cta& c, c
     const int64_t tsf_rows = shared ? p.tsf_rows_shared : p.tsf_rows_routed;
     const int32_t* tsf = (shared ? p.tsf_shared : p.tsf_routed) + (int64_t)tile.sf_chunk * kChunkRows;
     const uint32_t a_tx = shared ? 2 * kTileRows * kTileK : kTileRows * kTileK;   // packed FP4 counts its global bytes
-    const uint32_t tx = a_tx + box_rows * kTileK + 512 + (kLayer == 1 ? 0 : 1024);
+    const bool gathered = kLayer == 1 && shared;          // token scales come from the scale arranger
+    const uint32_t tx = a_tx + box_rows * kTileK + (gathered ? 0 : 512) + (kLayer == 1 ? 0 : 1024);
     int k0 = 0;
     for (int kb = 0; kb < k_stages; ++kb, k0 += kTileK, wsf += p.rows_per_expert, tsf += tsf_rows) {
       if (!waiter.wait_uniform(empty0 + 8 * st.stage, st.phase ^ 1u)) { st.ok = false; break; }
@@ -223,7 +249,7 @@ __device__ __forceinline__ void sa_producer(const UmmaParams& p, const Cta& c, c
         else tma_load_3d(a_dst, wmap, k0, row, slice, bar);
         if (kLayer == 2) bulk_load(sf_dst, wsf, 1024, bar);        // two chunks already in tensor-memory order
         tma_load_2d(b0 + st.stage * c.b_bytes, tmap, k0, tile.row0, bar);
-        bulk_load(sf_dst + 2 * 512, tsf, 512, bar);
+        if (!gathered) bulk_load(sf_dst + 2 * 512, tsf, 512, bar);
       }
       __syncwarp();
       if (++st.stage == c.num_stages) { st.stage = 0; st.phase ^= 1u; }
@@ -238,7 +264,7 @@ __device__ __forceinline__ void sa_producer(const UmmaParams& p, const Cta& c, c
 // On the MMA warps' path this work was a third of a stage's issue time (about 230 of 700 clk, and a stage is 580 clk of
 // HBM time at the clock a power-capped B200 runs this kernel at).
 template <typename L>
-__device__ __forceinline__ void sa_arrange_scales(const UmmaParams& p, const Cta& c, const TaskList& tl, Waiter& waiter,
+__device__ __forceinline__ void sa_arrange_scales(const UmmaParams& p, const Cta& c, TaskWalk walk, Waiter& waiter,
                                                   RoleState& st) {
   const int lane = threadIdx.x & 31;
   const int k_stages = p.k_dim / kTileK;
@@ -252,7 +278,19 @@ __device__ __forceinline__ void sa_arrange_scales(const UmmaParams& p, const Cta
     const int r = 16 * ((m & 63) >> 3) + 8 * h + (m & 7);   // stored row inside its 128-row block
     src[t] = 128 * (m >> 6) + 4 * (r & 31) + (r >> 5);
   }
-  for (int task = blockIdx.x; task < tl.num_tasks && st.ok; task += gridDim.x) {
+  while (st.ok && walk.next()) {
+    // The shared expert's token scales are gathered here, word kb of the staged scale rows (chunk position 4 (i % 32) + i / 32
+    // for token i), two stages ahead: its tiles then need no placement, only the staging.
+    const bool shared = walk.tile.expert == kSharedExpert;
+    const int32_t* x_sf = p.x_sf + (int64_t)(walk.tile.row0 + lane) * k_stages;
+    uint32_t ahead[2][4] = {};
+    auto gather = [&](uint32_t (&w)[4], int kb) {
+#pragma unroll
+      for (int a = 0; a < 4; ++a)
+        w[a] = shared && kb < k_stages && lane + 32 * a < walk.tile.n_valid ? __ldg(x_sf + 32 * a * k_stages + kb) : 0u;
+    };
+    gather(ahead[0], 0);
+    gather(ahead[1], 1);
     for (int kb = 0; kb < k_stages; ++kb) {
       // the stage's scales have landed, which also says that the MMAs which read the previous ones have retired
       if (!waiter.wait_uniform(sf_full0 + 8 * st.stage, st.phase)) { st.ok = false; break; }
@@ -262,6 +300,12 @@ __device__ __forceinline__ void sa_arrange_scales(const UmmaParams& p, const Cta
       for (int t = 0; t < 8; ++t) v[t] = area[3 * 128 + src[t]];
 #pragma unroll
       for (int t = 0; t < 8; ++t) area[lane + 32 * t] = v[t];
+      if (shared) {
+        *reinterpret_cast<uint4*>(area + 2 * 128 + 4 * lane) = make_uint4(ahead[0][0], ahead[0][1], ahead[0][2], ahead[0][3]);
+#pragma unroll
+        for (int a = 0; a < 4; ++a) ahead[0][a] = ahead[1][a];
+        gather(ahead[1], kb + 2);
+      }
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // generic writes -> visible to tcgen05.cp
       __syncwarp();
       if (elect_one()) mbar_arrive(sf_ready0 + 8 * st.stage);
@@ -275,7 +319,7 @@ __device__ __forceinline__ void sa_arrange_scales(const UmmaParams& p, const Cta
 // warp-uniform; one elected lane issues.  Each warp copies the scales it needs into its own TMEM columns, so no
 // ordering between the two warps' tensor-core instructions is needed.
 template <int kLayer, typename L>
-__device__ __forceinline__ void sa_mma(const UmmaParams& p, const Cta& c, const TaskList& tl, Waiter& waiter,
+__device__ __forceinline__ void sa_mma(const UmmaParams& p, const Cta& c, TaskWalk walk, Waiter& waiter,
                                        RoleState& st, int h) {
   const int k_stages = p.k_dim / kTileK;
   const uint32_t full0 = smem_u32(&c.ctl->full[0]), sf_ready0 = smem_u32(&c.ctl->sf_ready[0]);
@@ -287,9 +331,8 @@ __device__ __forceinline__ void sa_mma(const UmmaParams& p, const Cta& c, const 
   const uint32_t sf_lo0 = (smem_u32(c.sf_base) & 0x3FFFFu) >> 4;
   const uint32_t sfa_col = c.tmem_base + L::kSfCol + 4 * h;
   const uint32_t sfb_col = c.tmem_base + L::kSfCol + 8 + 4 * h;
-  for (int task = blockIdx.x; task < tl.num_tasks && st.ok; task += gridDim.x, ++st.it) {
-    int nb;
-    const Tile tile = tl.get(task, &nb);
+  for (; st.ok && walk.next(); ++st.it) {
+    const Tile tile = walk.tile;
     const bool shared = tile.expert == kSharedExpert;
     const uint32_t acc_stage = st.it & 1u, acc_phase = (st.it >> 1) & 1u;
     if (!waiter.wait_uniform(smem_u32(&c.ctl->tmem_empty[acc_stage]), acc_phase ^ 1u)) { st.ok = false; break; }
@@ -326,15 +369,15 @@ __device__ __forceinline__ void sa_mma(const UmmaParams& p, const Cta& c, const 
 // kFused (layer 2, EP > 1): every output row goes to the rank its token came from; compiled as kernels of its own so
 // that the single-destination epilogue of the other cases keeps its shorter inner loop.
 template <int kLayer, typename L, bool kFused>
-__device__ __forceinline__ void sa_epilogue(const UmmaParams& p, const Cta& c, const TaskList& tl, Waiter& waiter,
+__device__ __forceinline__ void sa_epilogue(const UmmaParams& p, const Cta& c, TaskWalk walk, Waiter& waiter,
                                             RoleState& st) {
   Control* ctl = c.ctl;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int q = warp & 3;                     // TMEM lane quadrant this warp may read
   const uint32_t lane_sel = static_cast<uint32_t>(q * 32) << 16;
-  for (int task = blockIdx.x; task < tl.num_tasks && st.ok; task += gridDim.x, ++st.it) {
-    int nb;
-    const Tile tile = tl.get(task, &nb);
+  for (; st.ok && walk.next(); ++st.it) {
+    const Tile tile = walk.tile;
+    const int nb = walk.nb;
     const bool shared = tile.expert == kSharedExpert;
     const uint32_t acc_stage = st.it & 1u, acc_phase = (st.it >> 1) & 1u;
     // Per-token side data of the tile (top-k weight / destination row), one coalesced load per 32 tokens issued
@@ -516,8 +559,10 @@ __global__ void __launch_bounds__(kThreads, 1) umma_kernel(const __grid_constant
   chain_release();
   sa_setup<L>(ctl);
   // Everything above touches only this CTA's own shared and tensor memory, so it may run while the kernel before this
-  // one in the stream is still running; everything below reads what that kernel wrote.
-  chain_wait();
+  // one in the stream is still running.  GEMM1 of a call without pair tiles goes on with the shared expert: its launch is let
+  // start by the route ordering's blocks once they have seen the staging complete.
+  const bool early = kLayer == 1 && p.tile_rows > 0;
+  if (!early && !p.skip_wait) chain_wait();
   if (kFused) {
     if (threadIdx.x == 0) ctl->out_base[32] = p.shared_out;
     const int t = threadIdx.x - 32;
@@ -536,22 +581,23 @@ __global__ void __launch_bounds__(kThreads, 1) umma_kernel(const __grid_constant
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const PlanView pv = plan_view(const_cast<char*>(p.plan), p.e_local, p.num_ranks);
-  const int tile_rows = max(16, min(kSmallTileRows, p.tile_select == 2 ? pv.hdr->early_small_rows : pv.hdr->small_rows));
+  const int tile_rows = p.tile_rows > 0 ? p.tile_rows
+                                       : max(16, min(kSmallTileRows, plan_view(const_cast<char*>(p.plan), p.e_local, p.num_ranks).hdr->small_rows));
   Cta c = sa_carve<L>(smem, tile_rows, p.max_stages);
   c.tmem_base = __shfl_sync(0xffffffffu, ctl->tmem_base, 0);
-  const TaskList tl = task_list(p, pv);
+  const TaskWalk walk(p, !early);
   Waiter waiter{&ctl->abort_flag, p.status, global_timer() + static_cast<uint64_t>(p.timeout_ns), kLayer, warp};
   RoleState st;
   if (warp == 0) {
-    sa_producer<kLayer, L>(p, c, tl, waiter, st);
+    sa_producer<kLayer, L>(p, c, walk, waiter, st);
   } else if (warp == 1 || warp == 6) {
-    sa_mma<kLayer, L>(p, c, tl, waiter, st, warp == 1 ? 0 : 1);
+    sa_mma<kLayer, L>(p, c, walk, waiter, st, warp == 1 ? 0 : 1);
   } else if (warp == 7) {
-    if (kLayer == 1) sa_arrange_scales<L>(p, c, tl, waiter, st);
+    if (kLayer == 1) sa_arrange_scales<L>(p, c, walk, waiter, st);
   } else {
-    sa_epilogue<kLayer, L, kFused>(p, c, tl, waiter, st);
+    sa_epilogue<kLayer, L, kFused>(p, c, walk, waiter, st);
   }
+  chain_wait();       // a CTA that has not waited yet must not end before what precedes the launch
   sa_teardown(ctl, c.tmem_base);
 }
 
@@ -679,9 +725,6 @@ bool build_tm(const Ctx& c, const MmoeWeights& w, bool has_shared, TmParams* out
   p1.routed_sliced = w.w13_slice_stride > 0 ? 1 : 0;
   p1.hidden = h;
   p1.inter = inter;
-  p1.has_shared_weights = has_shared ? 1 : 0;
-  p1.early_shared_first = c.lay.max_tiles - shared_tile_capacity(c.geo.num_max_tokens);
-  p1.early_shared_cap = static_cast<int>(shared_tile_capacity(c.geo.num_max_tokens));
 
   TmParams p2 = p1;
   bad |= make_weight_map(&p2.map_w_routed, true, w.w2, inter, (uint64_t)el * h, w.w2_slice_stride, kTileRows);
@@ -725,9 +768,8 @@ bool build_sa(const Ctx& c, const MmoeWeights& w, bool has_shared, UmmaParams* o
   p1.wsf_routed = static_cast<const int32_t*>(w.w13_sf);
   p1.wsf_shared = static_cast<const int32_t*>(w.shared_w13_sf);
   p1.tsf_routed = c.at<int32_t>(c.lay.pool_sf);
-  p1.tsf_shared = c.at<int32_t>(c.lay.shared_tile_sf);
+  p1.x_sf = c.at<int32_t>(c.lay.x_sf);
   p1.tsf_rows_routed = c.lay.pool_sf_rows;
-  p1.tsf_rows_shared = shared_chunk_rows(c.geo.num_max_tokens);
   p1.act_routed = c.at<uint8_t>(c.lay.act_x);
   p1.act_shared = c.at<uint8_t>(c.lay.shared_act_x);
   p1.act_sf_routed = c.at<uint8_t>(c.lay.act_sf);
@@ -744,9 +786,6 @@ bool build_sa(const Ctx& c, const MmoeWeights& w, bool has_shared, UmmaParams* o
   p1.n_blocks = inter / kTileRows;
   p1.hidden = h;
   p1.inter = inter;
-  p1.has_shared_weights = has_shared ? 1 : 0;
-  p1.early_shared_first = c.lay.max_tiles - shared_tile_capacity(c.geo.num_max_tokens);
-  p1.early_shared_cap = static_cast<int>(shared_tile_capacity(c.geo.num_max_tokens));
 
   UmmaParams p2 = p1;
   bad |= make_weight_map(&p2.map_w_routed, true, w.w2, inter, (uint64_t)el * h, w.w2_slice_stride, 2 * kTileRows);
@@ -891,7 +930,7 @@ cudaError_t launch_experts_umma(const Ctx& c, const MmoeWeights& w, const MmoeOp
     p.timeout_ns = timeout_ns;
     p.clamp = o.activation_clamp;
     p.fast_math = o.fast_math;
-    p.tile_select = c.tile_select;
+    p.with_routed = c.tile_select != 2 ? 1 : 0;
     if (layer2 && fused) {
       p.ep_me = c.geo.rank;
       p.ep_totals = reinterpret_cast<const int32_t*>(c.ws + c.lay.ep_sync + ep_totals_offset());
@@ -899,21 +938,30 @@ cudaError_t launch_experts_umma(const Ctx& c, const MmoeWeights& w, const MmoeOp
         p.ep_ret_recv[r] = reinterpret_cast<__nv_bfloat16*>(static_cast<char*>(const_cast<void*>(c.peer_ws[r])) + c.lay.ret_recv);
     }
   };
-  // Experts with many rows run on CTA pairs, the others on the weights-as-A kernels: which ones is in the plan.  The
-  // ahead-of-plan launch knows its own kind.
+  // Experts with many rows run on CTA pairs, the others on the weights-as-A kernels: which ones is in the plan.  The shared
+  // expert is one or the other by the call's token count.
   const int pair_above = c.pair_above_for(m);
-  const bool pairs = c.tile_select == 2 ? m > pair_above : pair_above != kNeverPair;
-  const bool small = c.tile_select == 2 ? !pairs : pair_above > 0;
+  const bool with_shared = has_shared && c.tile_select != 1;
+  const Cut cut = shared_cut(with_shared ? m : 0, pair_above);
+  const SharedTiles shared{cut.parts, cut.step, m}, none{0, 16, 0};
+  const bool shared_pairs = m > pair_above;
+  const bool pairs = c.tile_select == 2 ? with_shared && shared_pairs : pair_above != kNeverPair;
+  const bool small = c.tile_select == 2 ? with_shared && !shared_pairs : pair_above > 0;
   for (int layer = 1; layer <= 2; ++layer) {
     if ((mask & layer) == 0) continue;
     if (e == cudaSuccess && pairs) {
       TmParams p = plan->tm[layer - 1];
       patch(p, layer == 2);
+      p.shared_tiles = shared_pairs ? shared : none;
       e = tm_launch(layer, layer == 2 && fused, p, s);
     }
     if (e == cudaSuccess && small) {
       UmmaParams p = plan->sa[layer - 1];
       patch(p, layer == 2);
+      p.shared_tiles = shared_pairs ? none : shared;
+      p.tile_rows = c.tile_select == 2 ? cut.step : (pairs ? 0 : small_only_cap(m, block_m));
+      // The pair launch in front reads and writes nothing that this one does, and lets it start only after its own wait.
+      p.skip_wait = pairs ? 1 : 0;
       e = layer == 1 ? launch_layer<1, false>(p, s) : fused ? launch_layer<2, true>(p, s) : launch_layer<2, false>(p, s);
     }
   }

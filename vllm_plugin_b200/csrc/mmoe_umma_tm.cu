@@ -128,6 +128,51 @@ __device__ __forceinline__ void pair_load_3d(uint32_t dst, const CUtensorMap* ma
       : "memory");
 }
 
+// The task list of one unit as a role walks it: first the shared expert's tasks, which need nothing but the staged tokens
+// and are on the host's count of tokens, then -- once everything before this launch in the stream has completed -- the pair
+// tiles of the plan.  In GEMM1 of the single-GPU call the placement of the routed rows, and the launch itself, hide behind
+// the shared expert this way.
+struct PairWalk {
+  const TmParams& p;
+  uint32_t cta;
+  int n_blocks, task, stride;
+  bool waited;
+  int routed_tiles;
+  const Tile* tiles;
+  Tile tile;              // this CTA's half of the current task
+  int peer_valid, nb;     // rows of the other half; weight block
+  __device__ __forceinline__ PairWalk(const TmParams& params, uint32_t cta_rank, bool has_waited)
+      : p(params), cta(cta_rank), n_blocks(params.rows_per_expert / kTmN), task(blockIdx.x / 2), stride(gridDim.x / 2),
+        waited(false), routed_tiles(0), tiles(nullptr) {
+    if (has_waited) load_plan();
+  }
+  __device__ __forceinline__ void load_plan() {
+    chain_wait();
+    const PlanView pv = plan_view(const_cast<char*>(p.plan), p.e_local, p.num_ranks);
+    tiles = pv.tiles + pv.hdr->num_small_tiles;
+    routed_tiles = p.with_routed ? pv.hdr->num_routed_tiles - pv.hdr->num_small_tiles : 0;
+    waited = true;
+  }
+  // true: tile, peer_valid and nb are the next task's
+  __device__ __forceinline__ bool next() {
+    const int t = task;
+    task += stride;
+    const int pair = t / n_blocks, first = p.shared_tiles.parts / 2;
+    nb = t - pair * n_blocks;
+    if (pair < first) {
+      tile = p.shared_tiles.at(2 * pair + static_cast<int>(cta));
+      peer_valid = p.shared_tiles.at(2 * pair + static_cast<int>(cta ^ 1u)).n_valid;
+      return true;
+    }
+    if (!waited) load_plan();
+    const int i = 2 * (pair - first);
+    if (i >= routed_tiles) return false;
+    tile = tiles[i + cta];
+    peer_valid = tiles[i + (cta ^ 1u)].n_valid;
+    return true;
+  }
+};
+
 // token box of a tile: the smallest of 32 / 64 / 96 / 128 rows that covers it
 __device__ __forceinline__ int tm_box(int n_valid) { return n_valid <= 32 ? 0 : (n_valid - 1) >> 5; }
 
@@ -173,8 +218,6 @@ __global__ void __launch_bounds__(kTmThreads, 1) tm_kernel(const __grid_constant
 
   const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   const uint32_t cta = cluster_ctarank();                         // 0 = leader
-  const int unit = blockIdx.x / 2, num_units = gridDim.x / 2;     // a unit is a CTA pair
-  chain_release();
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < kTmStages; ++i) {
@@ -190,9 +233,11 @@ __global__ void __launch_bounds__(kTmThreads, 1) tm_kernel(const __grid_constant
     asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&ctl->tmem_base)), "r"(kTmemCols) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
   }
-  // Everything above touches only this CTA's own shared and tensor memory, so it may run while the kernel before this
-  // one in the stream is still running; everything below reads what that kernel wrote.
-  chain_wait();
+  // Everything above touches only this CTA's own shared and tensor memory.  GEMM2, and GEMM1 behind an ordinary launch, wait
+  // here for everything before them; GEMM1 in a programmatic chain starts when the blocks of the placement have all started,
+  // i.e. after the launches before it (staging, counting) have completed, and waits when it comes to the routed tiles.
+  // Only then does it let the next launch start.
+  if (kLayer == 2) chain_wait();
   if (kFused) {
     const int t = threadIdx.x - 32;
     if (t >= 0 && t < p.num_ranks) {
@@ -212,11 +257,7 @@ __global__ void __launch_bounds__(kTmThreads, 1) tm_kernel(const __grid_constant
   cluster_sync_all();                       // the peer's barriers are initialised before anything arrives on them
   tc_fence_after();
   const uint32_t tmem_base = __shfl_sync(0xffffffffu, ctl->tmem_base, 0);
-  PlanView pv = plan_view(const_cast<char*>(p.plan), p.e_local, p.num_ranks);
-  const TileRange range = pair_tiles(pv, p.tile_select, p.has_shared_weights != 0, p.early_shared_first, p.early_shared_cap);
-  const Tile* tiles = range.tiles;          // tiles 2j and 2j + 1 are the halves of pair j
-  const int n_blocks = p.rows_per_expert / kTmN;
-  const int num_tasks = range.count / 2 * n_blocks;
+  PairWalk walk(p, cta, kLayer == 2);
   const int k_stages = p.k_dim / kTileK;
 
   Waiter waiter{&ctl->abort_flag, p.status, global_timer() + static_cast<uint64_t>(p.timeout_ns), 20 + kLayer, warp};
@@ -230,11 +271,14 @@ __global__ void __launch_bounds__(kTmThreads, 1) tm_kernel(const __grid_constant
     const uint32_t a0 = smem_u32(a_base), b0 = smem_u32(b_base), sf0 = smem_u32(sf_base);
     const uint32_t leader_full0 = map_to_cta(full0, 0);
     const int half = p.rows_per_expert / 2;
-    bool ok = true;
-    for (int task = unit; task < num_tasks && ok; task += num_units) {
-      const int pair = task / n_blocks, nb = task - pair * n_blocks;
-      const Tile tile = tiles[2 * pair + cta];
-      const int peer_valid = tiles[2 * pair + (cta ^ 1u)].n_valid;
+    bool ok = true, released = false;
+    while (ok && walk.next()) {
+      const Tile tile = walk.tile;
+      const int nb = walk.nb;
+      if (!released && walk.waited) {
+        chain_release();
+        released = true;
+      }
       const bool shared = tile.expert == kSharedExpert;
       const int e = shared ? 0 : tile.expert;
       const int r0 = nb * kTmN + static_cast<int>(cta) * (kTmN / 2);     // this CTA's 128 stored weight rows: inside one slice
@@ -247,7 +291,7 @@ __global__ void __launch_bounds__(kTmThreads, 1) tm_kernel(const __grid_constant
       const int box = tm_box(tile.n_valid);
       const CUtensorMap* tmap = shared ? &p.map_tok_shared[box] : &p.map_tok_routed[box];
       // what both CTAs' copies add up to, counted on the leader's barrier; packed FP4 counts its global bytes
-      const uint32_t tx = static_cast<uint32_t>((box + tm_box(peer_valid) + 2) * 32 * kTileK) +
+      const uint32_t tx = static_cast<uint32_t>((box + tm_box(walk.peer_valid) + 2) * 32 * kTileK) +
                           (shared ? kTmN * kTileK : kTmN * kTileK / 2) + 2 * kTmSfBytes;
       const int wsf_col = nb * kTmN, tsf_col = tile.sf_chunk * kChunkRows;
       int wsf_row = e * k_stages;
@@ -275,8 +319,8 @@ __global__ void __launch_bounds__(kTmThreads, 1) tm_kernel(const __grid_constant
       const uint32_t a_lo0 = (smem_u32(a_base) & 0x3FFFFu) >> 4;
       const uint32_t b_lo0 = (smem_u32(b_base) & 0x3FFFFu) >> 4;
       const uint32_t sf_lo0 = (smem_u32(sf_base) & 0x3FFFFu) >> 4;
-      for (int task = unit; task < num_tasks && ok; task += num_units, ++it) {
-        const bool shared = tiles[2 * (task / n_blocks)].expert == kSharedExpert;
+      for (; ok && walk.next(); ++it) {
+        const bool shared = walk.tile.expert == kSharedExpert;
         // M = 256 over the pair; idesc field [24,29) = M >> 4
         const uint32_t idesc0 = make_idesc(0u, shared ? 0u : 5u, static_cast<uint32_t>(kTmN), 0) + ((128u >> 4) << 24);
         const uint32_t d = tmem_base + (it & 1u) * kTmAccStride;
@@ -319,9 +363,9 @@ __global__ void __launch_bounds__(kTmThreads, 1) tm_kernel(const __grid_constant
     const uint32_t overlap_free_leader = map_to_cta(smem_u32(&ctl->overlap_free), 0);
     uint32_t it = 0;
     bool ok = true;
-    for (int task = unit; task < num_tasks && ok; task += num_units, ++it) {
-      const int pair = task / n_blocks, nb = task - pair * n_blocks;
-      const Tile tile = tiles[2 * pair + cta];
+    for (; ok && walk.next(); ++it) {
+      const Tile tile = walk.tile;
+      const int nb = walk.nb;
       const bool shared = tile.expert == kSharedExpert;
       const uint32_t acc = it & 1u;
       const bool live = i < tile.n_valid;
@@ -417,6 +461,7 @@ __global__ void __launch_bounds__(kTmThreads, 1) tm_kernel(const __grid_constant
   }
 
   // ---------------------------------------------------------------------------------------------------- teardown
+  chain_wait();                             // a unit without routed tasks must not end before what precedes the launch
   __syncwarp();
   if (ctl->abort_flag != 0) {
     // abandoned call: give copies that are still in flight time to land in this CTA's shared memory before it exits
