@@ -419,7 +419,8 @@ int mmoe_dispatch_place(const MmoeGeometry* geo, void* workspace, int32_t num_to
 namespace {
 // `peers` != NULL: EP > 1 with the write-back fused into GEMM2, followed by barrier 2
 int run_experts(const MmoeGeometry* geo, void* workspace, const void* const* peers, const MmoeWeights* weights,
-                const MmoeOptions* opt, int32_t num_tokens, int32_t block_m, void* stream, int tile_select = 0);
+                const MmoeOptions* opt, int32_t num_tokens, int32_t block_m, void* stream, int tile_select = 0,
+                bool route_in_gemm = false, int32_t* stats = nullptr);
 
 }  // namespace
 
@@ -460,7 +461,8 @@ int mmoe_experts_ep_return(const MmoeGeometry* geo, void* workspace, const void*
 
 namespace {
 int run_experts(const MmoeGeometry* geo, void* workspace, const void* const* peers, const MmoeWeights* weights,
-                const MmoeOptions* opt, int32_t num_tokens, int32_t block_m, void* stream, int tile_select) {
+                const MmoeOptions* opt, int32_t num_tokens, int32_t block_m, void* stream, int tile_select, bool route_in_gemm,
+                int32_t* stats) {
   mmoe::Ctx c;
   int rc = make_ctx(geo, workspace, &c);
   if (rc != MMOE_OK) return rc;
@@ -495,6 +497,8 @@ int run_experts(const MmoeGeometry* geo, void* workspace, const void* const* pee
     if (!mmoe::tc_ready()) return fail(MMOE_ERR_NOT_PREPARED, "mmoe_prepare() must run on this device before the first launch");
     c.peer_ws = peers;
     c.tile_select = tile_select;
+    c.route_in_gemm = route_in_gemm;
+    c.stats = stats;
       e = mmoe::launch_experts_umma(c, *weights, o, num_tokens, block_m, st);
     if (e == cudaSuccess && peers != nullptr) e = mmoe::launch_ep_signal_return(c, peers, timeout_ns, st);
   } else {
@@ -534,13 +538,17 @@ int mmoe_forward(const MmoeGeometry* geo, void* workspace, const MmoeWeights* we
   if (rc != MMOE_OK) return rc;
   if (!valid_block_m(block_m)) return fail(MMOE_ERR_INVALID_ARGUMENT, "block_m=%d is not a BLOCK_M value", block_m);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  // route ordering, plan and placement: one launch up to 128 tokens, two beyond (and where the pair kernels are forced on:
-  // those read the shared expert's scales from chunks that the larger form writes)
-  const cudaError_t e = num_tokens > 0 && num_tokens <= 128 && c.pair_above_for(num_tokens) == mmoe::kNeverPair
-                            ? mmoe::launch_route_small(c, num_tokens, block_m, stats, st)
-                            : mmoe::launch_route_large(c, num_tokens, block_m, stats, st);
-  if (e != cudaSuccess) return cuda_fail(e, "route / plan / placement launch");
-  rc = mmoe_experts(geo, workspace, weights, opt, num_tokens, block_m, stream);
+  // route ordering, plan and placement: inside the GEMM launches up to kStagedTokens tokens, one launch up to 128, two beyond
+  // (and where the pair kernels are forced on: those read the shared expert's scales from chunks that the larger form writes)
+  const bool small_only = num_tokens > 0 && c.pair_above_for(num_tokens) == mmoe::kNeverPair;
+  const bool in_gemm = small_only && num_tokens <= mmoe::kStagedTokens && block_m <= mmoe::kStagedTokens && opt != nullptr &&
+                       opt->engine == 0 && (opt->layer_mask == 0 || opt->layer_mask == 3);
+  if (!in_gemm) {
+    const cudaError_t e = small_only && num_tokens <= 128 ? mmoe::launch_route_small(c, num_tokens, block_m, stats, st)
+                                                          : mmoe::launch_route_large(c, num_tokens, block_m, stats, st);
+    if (e != cudaSuccess) return cuda_fail(e, "route / plan / placement launch");
+  }
+  rc = run_experts(geo, workspace, nullptr, weights, opt, num_tokens, block_m, stream, 0, in_gemm, stats);
   if (rc == MMOE_OK) rc = mmoe_combine_residual(geo, workspace, y_bf16, opt != nullptr ? opt->residual : nullptr, num_tokens, stream);
   return rc;
 }

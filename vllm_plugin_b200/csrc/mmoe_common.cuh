@@ -43,6 +43,9 @@ __host__ __device__ inline Cut cut_rows(int n, int pair_above, int small_cap) {
 }
 // The cut of the shared expert's m tokens: known to the host, so that its tiles need no plan.
 __host__ __device__ inline Cut shared_cut(int m, int pair_above) { return cut_rows(m, pair_above, kDeepTileRows); }
+// GEMM1 of a call of at most this many tokens on one GPU multiplies every expert that is hit with all staged tokens and orders
+// the routes itself (an UMMA takes 16 token columns at least).
+constexpr int kStagedTokens = 16;
 // Cap of a call without pair tiles (also known to the host: the largest tile of such a call fixes its stage layout): no expert
 // has more rows than there are tokens unless a token names it twice, which then costs another tile.
 __host__ __device__ inline int small_only_cap(int m, int block_m) {
@@ -79,7 +82,8 @@ struct PlanHeader {
   int32_t small_cap;           // rows a weights-as-A tile of this call may have
   int32_t small_rows;          // rows of the largest one, rounded up to 16
   int32_t ticket;              // blocks of the route-counting launch that have finished; zero between launches
-  int32_t pad[6];
+  int32_t routed;              // 1 while a GEMM1 launch that orders the routes itself has the plan complete; GEMM2 clears it
+  int32_t pad[5];
 };
 static_assert(sizeof(PlanHeader) == 64, "plan header is 64 bytes");
 
@@ -218,6 +222,8 @@ struct Ctx {             // resolved pointers of one call
   char* ws;
   int e_local;
   int kmax;              // min(k, E/R)
+  int32_t* stats = nullptr;               // cumulative receive counts, for a GEMM1 launch that orders the routes itself ...
+  bool route_in_gemm = false;             // ... which it does when this is set
   const void* const* peer_ws = nullptr;   // set by the call that fuses the write-back into GEMM2 (EP > 1)
   int tile_select = 0;                    // 0: every tile of the plan, 1: routed tiles only, 2: the early shared tiles only
   int pair_above = kNeverPair;            // experts with more rows than this run on CTA pairs ...

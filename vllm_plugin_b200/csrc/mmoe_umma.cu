@@ -55,18 +55,35 @@ struct UmmaParams {
   uint8_t* act_sf_routed;      // byte view of the activation scale chunks
   uint8_t* act_sf_shared;
   int64_t act_sf_rows_routed, act_sf_rows_shared;
-  const float* pool_w;
+  float* pool_w;
   // layer-2 outputs
   __nv_bfloat16* ret;
   __nv_bfloat16* shared_out;
-  const int32_t* pool_dst;
+  int32_t* pool_dst;
   // layer 2 at EP > 1 with the write-back fused in: an output row goes straight into the `ret_recv` of the rank its
   // token came from (plain peer stores over NVLink), at that rank's send position
   SharedTiles shared_tiles;    // run first
   int with_routed;             // 0: only those
   int tile_rows;               // > 0: rows of the call's largest tile, known to the host; 0: in the plan
+  int early;                   // 1: the launch in front lets this one start when the staged tokens (layer 1) / the plan (layer 2) are complete
   int skip_wait;               // 1: what this launch reads was complete before the launch in front of it let it start
-  const int32_t* x_sf;         // layer 1: the staged tokens' scale words [T][K/128], gathered for the shared expert's tiles
+  const int32_t* x_sf;         // layer 1: the staged tokens' scale words [T][K/128], gathered for tiles of staged tokens
+  // kernels of calls of at most kStagedTokens tokens: every routed tile of layer 1 is the staged tokens themselves (see TaskWalk)
+  const int64_t* topk_idx;
+  int32_t* sorted_route;
+  int num_routes, topk;
+  // ... and with route_here the launch also orders the routes and builds the plan (layer 1) / places the rows (layer 2)
+  int route_here;
+  const float* topk_weights;
+  int32_t* route_pos;
+  int32_t* send_count;
+  int32_t* send_offset;
+  int32_t* recv_count;
+  int32_t* stats;
+  const uint4* x;
+  uint4* pool_x;
+  int32_t* pool_sf;
+  int64_t pool_sf_rows;
   int ep_me;
   const int32_t* ep_totals;    // [32][32]: totals[s][d] = routes rank s sent to rank d in this call
   __nv_bfloat16* ep_ret_recv[32];
@@ -94,6 +111,7 @@ struct Control {          // lives at the start of shared memory
   uint64_t tmem_empty[2];
   uint32_t tmem_base;
   volatile int32_t abort_flag;
+  uint32_t hit[16];       // layer 1 with staged tokens: bit e = some token is routed to expert e
   // layer 2 with the write-back fused in: where output rows go.  slot s < 32: `ret_recv` of source rank s, slot 32: the
   // shared expert's (local) output
   __nv_bfloat16* out_base[33];
@@ -156,22 +174,53 @@ struct Cta {                       // where a role finds the CTA's resources
 // Tile by tile, or for an expert with several tiles weight block by weight block, so that the tiles of a block read its
 // weights while they are in L2.  After the first round the CTAs take their tasks in the opposite order: the first ones,
 // whose shared tasks have twice the weight bytes, are not also the ones with a task more in the last round.
+//
+// GEMM1 of at most 16 tokens needs no placed rows either: an UMMA takes 16 token columns at least, so every expert that some
+// token is routed to multiplies all staged tokens, and the epilogue takes the columns of the tokens routed to it.  Which
+// experts those are every CTA reads from the route table itself; only the epilogue waits for the plan.
+template <bool kStaged>
 struct TaskWalk {
   const UmmaParams& p;
-  int shared_tasks, routed_tasks, round;
+  const uint32_t* hit;
+  int hit_experts;
+  int n_blocks, shared_tasks, routed_tasks, round;
   bool waited;
   const Tile* tiles;
   Tile tile;               // current task
   int nb;
-  __device__ __forceinline__ TaskWalk(const UmmaParams& params, bool has_waited)
-      : p(params), shared_tasks(params.shared_tiles.parts * params.n_blocks), routed_tasks(0), round(0), waited(false), tiles(nullptr) {
-    if (has_waited) load_plan();
+  // `plan_ready`: the plan is complete, without a wait
+  __device__ __forceinline__ TaskWalk(const UmmaParams& params, const uint32_t* hit_words, bool plan_ready, int blocks_per_tile)
+      : p(params), hit(hit_words), hit_experts(0), n_blocks(blocks_per_tile), shared_tasks(params.shared_tiles.parts * blocks_per_tile),
+        routed_tasks(0), round(0),
+        waited(false), tiles(nullptr) {
+    if (kStaged) {
+      hit_experts = __reduce_add_sync(0xffffffffu, (threadIdx.x & 31) < 16 ? __popc(hit[threadIdx.x & 15]) : 0);
+      routed_tasks = p.with_routed ? hit_experts * n_blocks : 0;
+    } else if (plan_ready) {
+      load_plan(true);
+    }
   }
-  __device__ __forceinline__ void load_plan() {
-    if (!p.skip_wait) chain_wait();
+  // i-th expert (ascending) with a bit in `hit`; whole warp
+  __device__ __forceinline__ int hit_expert(int i) const {
+    const int lane = threadIdx.x & 31;
+    uint32_t word = lane < 16 ? hit[lane] : 0u;
+    const int mine = __popc(word);
+    int before = mine;
+#pragma unroll
+    for (int d = 1; d < 16; d <<= 1) {
+      const int t = __shfl_up_sync(0xffffffffu, before, d);
+      if (lane >= d) before += t;
+    }
+    before -= mine;
+    const int owner = __ffs(__ballot_sync(0xffffffffu, i >= before && i < before + mine)) - 1;
+    for (int drop = i - before; drop > 0 && lane == owner; --drop) word &= word - 1;
+    return __shfl_sync(0xffffffffu, 32 * lane + __ffs(word) - 1, owner);
+  }
+  __device__ __forceinline__ void load_plan(bool ready) {
+    if (!ready) chain_wait();
     const PlanView pv = plan_view(const_cast<char*>(p.plan), p.e_local, p.num_ranks);
     tiles = pv.tiles;
-    routed_tasks = p.with_routed ? pv.hdr->num_small_tiles * p.n_blocks : 0;
+    routed_tasks = p.with_routed ? pv.hdr->num_small_tiles * n_blocks : 0;
     waited = true;
   }
   // true: tile and nb are the next task's
@@ -183,14 +232,21 @@ struct TaskWalk {
       tile = p.shared_tiles.at(task - nb * p.shared_tiles.parts);
       return true;
     }
-    if (!waited) load_plan();
     task -= shared_tasks;
+    if (kStaged) {
+      if (task >= routed_tasks) return false;
+      const int u = task / n_blocks;
+      nb = task - u * n_blocks;
+      tile = Tile{hit_expert(u), 0, p.shared_tiles.m, 0, 0, 1, {0, 0}};
+      return true;
+    }
+    if (!waited) load_plan(false);
     if (task >= routed_tasks) return false;
-    const int i = task / p.n_blocks;
+    const int i = task / n_blocks;
     tile = tiles[i];
-    nb = task - i * p.n_blocks;
+    nb = task - i * n_blocks;
     if (tile.parts > 1) {
-      const int first = i - tile.part, local = task - first * p.n_blocks;
+      const int first = i - tile.part, local = task - first * n_blocks;
       nb = local / tile.parts;
       tile = tiles[first + local - nb * tile.parts];
     }
@@ -198,24 +254,171 @@ struct TaskWalk {
   }
 };
 
+// ------------------------------------------------------------------------------------------------ routing in the launch
+// Calls of at most kStagedTokens tokens: the last CTA's epilogue warps, idle until its first accumulator 15 us later, order the
+// routes and build the plan, which only epilogues and GEMM2 need.  A launch of its own took 8-20 us in front of GEMM1: little
+// work, but every instruction line comes from DRAM (each call streams its weights through the L2), so what counts is that
+// the code is short.  Pool blocks and tiles have 16 rows here, hence one tile per block.
+constexpr int kRouteThreads = 128;
+constexpr int kMaxHereRoutes = kStagedTokens * 31, kMaxHereExperts = 512;
+struct alignas(16) RouteScratch {
+  uint32_t count[kMaxHereExperts];
+  uint32_t before[kMaxHereExperts];      // rows | blocks << 16 of the experts before it
+  uint16_t ids[kMaxHereRoutes + 16];
+  uint32_t warp_sum[4];
+};
+static_assert(6 * (Shape<1>::kABytes + kStagedTokens * kTileK + Shape<1>::kSfBytes) + sizeof(RouteScratch) <= Shape<1>::kRingBytes &&
+                  Shape<1>::kRingBytes / (Shape<1>::kABytes + kStagedTokens * kTileK + Shape<1>::kSfBytes) == 6,
+              "the scratch lives behind the six stages of a 16-row ring");
+__device__ __forceinline__ void route_barrier() { asm volatile("bar.sync 1, %0;" ::"n"(kRouteThreads) : "memory"); }
+
+__device__ __noinline__ void sa_route(const UmmaParams& p, RouteScratch& s, int t) {
+  const int E = p.e_local, n = p.num_routes, lane = t & 31;
+#pragma unroll 1
+  for (int e = t; e < kMaxHereExperts; e += kRouteThreads) s.count[e] = 0u;
+  route_barrier();
+#pragma unroll 1
+  for (int i = t; i < n; i += kRouteThreads) {
+    const int64_t id = p.topk_idx[i];
+    if (id >= E) report_bad_index(p.status);
+    s.ids[i] = id >= 0 && id < E ? static_cast<uint16_t>(id) : 0xFFFF;
+    if (id >= 0 && id < E) atomicAdd(&s.count[id], 1u);
+  }
+  route_barrier();
+  uint4 c = reinterpret_cast<const uint4*>(s.count)[t];        // this thread's four experts
+  c.x |= ((c.x + 15) >> 4) << 16;
+  c.y |= ((c.y + 15) >> 4) << 16;
+  c.z |= ((c.z + 15) >> 4) << 16;
+  c.w |= ((c.w + 15) >> 4) << 16;
+  const uint32_t sum = c.x + c.y + c.z + c.w;
+  uint32_t incl = sum;
+#pragma unroll 1
+  for (int d = 1; d < 32; d <<= 1) {
+    const uint32_t o = __shfl_up_sync(0xffffffffu, incl, d);
+    if (lane >= d) incl += o;
+  }
+  if (lane == 31) s.warp_sum[t >> 5] = incl;
+  route_barrier();
+  uint32_t at = incl - sum, total = 0;
+#pragma unroll 1
+  for (int w = 0; w < 4; ++w) {
+    if (w < (t >> 5)) at += s.warp_sum[w];
+    total += s.warp_sum[w];
+  }
+  reinterpret_cast<uint4*>(s.before)[t] = make_uint4(at, at + c.x, at + c.x + c.y, at + c.x + c.y + c.z);
+  route_barrier();
+  const PlanView pv = plan_view(const_cast<char*>(p.plan), E, 1);
+#pragma unroll 1
+  for (int e = t; e <= E; e += kRouteThreads) {
+    const uint32_t off = e < E ? s.before[e] : total;
+    const int row = static_cast<int>(off & 0xFFFF), block = static_cast<int>(off >> 16);
+    p.send_offset[e] = row;
+    pv.expert_block_off[e] = block;
+    pv.expert_tile_off[e] = block;
+    if (e == E) break;
+    const int n_e = static_cast<int>(s.count[e]);
+    p.send_count[e] = n_e;
+    p.recv_count[e] = n_e;
+    pv.expert_total[e] = n_e;
+    pv.seg_pool_start[e] = block * kStagedTokens;
+    pv.seg_recv_start[e] = row;
+    if (p.stats != nullptr && n_e > 0) atomicAdd(&p.stats[e], n_e);      // cumulative per-expert receive statistics (dispatch.py:644-650)
+    const int parts = (n_e + kStagedTokens - 1) / kStagedTokens;
+#pragma unroll 1
+    for (int j = 0; j < parts; ++j)
+      pv.tiles[block + j] = Tile{e, (block + j) * kStagedTokens, min(kStagedTokens, n_e - j * kStagedTokens), block + j, j, parts, {0, 0}};
+  }
+  if (t == 0) {
+    const int rows = static_cast<int>(total & 0xFFFF), tiles = static_cast<int>(total >> 16);
+    int32_t* h = reinterpret_cast<int32_t*>(pv.hdr);       // the fields in order
+    reinterpret_cast<int4*>(h)[0] = make_int4(tiles, p.shared_tiles.parts, tiles, rows);
+    reinterpret_cast<int4*>(h)[1] = make_int4(kStagedTokens, p.shared_tiles.m, tiles, kStagedTokens);
+    h[8] = kStagedTokens;
+    pv.rank_off[0] = 0;
+    pv.rank_off[1] = rows;
+    if (p.shared_tiles.parts > 0) pv.tiles[tiles] = p.shared_tiles.at(0);
+  }
+#pragma unroll 1
+  for (int i = t; i < n; i += kRouteThreads) {
+    const uint32_t e = s.ids[i];
+    int pos = -1;
+    if (e != 0xFFFFu) {
+      uint32_t rank = 0;
+#pragma unroll 1
+      for (int o = 0; o < i; ++o) rank += s.ids[o] == e ? 1u : 0u;
+      pos = static_cast<int>((s.before[e] & 0xFFFF) + rank);
+      const int row = static_cast<int>((s.before[e] >> 16) * kStagedTokens + rank);
+      p.sorted_route[pos] = i;
+      p.pool_w[row] = p.topk_weights[i];
+      p.pool_dst[row] = pos;
+    }
+    p.route_pos[i] = pos;
+  }
+  __threadfence();
+  route_barrier();
+  if (t == 0) asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(&pv.hdr->routed), "r"(1) : "memory");
+}
+
+// Layer 2 of such a call: the placed rows and scales, which nothing in the call reads, by the warp that layer 1 uses for scales.
+__device__ __noinline__ void sa_place(const UmmaParams& p) {
+  const int lane = threadIdx.x & 31, vec = p.hidden / 16, words = p.hidden / kTileK;
+  const PlanView pv = plan_view(const_cast<char*>(p.plan), p.e_local, 1);
+  for (int i = blockIdx.x; i < p.num_routes; i += gridDim.x) {
+    const int pos = p.route_pos[i];
+    if (pos < 0) continue;
+    const int e = static_cast<int>(p.topk_idx[i]), r = pos - p.send_offset[e], t = i / p.topk, block = pv.expert_block_off[e];
+    const uint4* src = p.x + (int64_t)t * vec;
+    uint4* dst = p.pool_x + (int64_t)(block * kStagedTokens + r) * vec;
+#pragma unroll 1
+    for (int v = lane; v < vec; v += 32) dst[v] = src[v];
+    int32_t* sf = p.pool_sf + (int64_t)(block + r / kStagedTokens) * kChunkRows + chunk_pos(r % kStagedTokens);
+#pragma unroll 1
+    for (int w = lane; w < words; w += 32) sf[w * p.pool_sf_rows] = p.x_sf[(int64_t)t * words + w];
+  }
+}
+
+// waits until the plan is complete, whole warp; false when the call is being abandoned
+__device__ __forceinline__ bool sa_wait_plan(const UmmaParams& p, Waiter& waiter) {
+  if (!p.route_here) {
+    chain_wait();
+    return true;
+  }
+  const int32_t* flag = &plan_view(const_cast<char*>(p.plan), p.e_local, p.num_ranks).hdr->routed;
+  for (uint32_t spin = 0;; ++spin) {
+    int32_t v;
+    asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(flag) : "memory");
+    if (__any_sync(0xffffffffu, v != 0)) {
+      asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(flag) : "memory");   // by every lane
+      return true;
+    }
+    if ((spin & 63u) == 63u && __any_sync(0xffffffffu, waiter.abandoned())) return false;
+    __nanosleep(100);
+  }
+}
+
 // ------------------------------------------------------------------------------------------------ producer
 // One warp in step, one elected lane issues.  Everything that does not change inside a task is computed once per task; the
 // K loop only bumps 32-bit coordinates and two pointers, because such a loop runs at instruction latency, not throughput.
-template <int kLayer, typename L>
-__device__ __forceinline__ void sa_producer(const UmmaParams& p, const Cta& c, TaskWalk walk, Waiter& waiter,
+template <int kLayer, typename L, bool kStaged>
+__device__ __forceinline__ void sa_producer(const UmmaParams& p, const Cta& c, TaskWalk<kStaged && kLayer == 1> walk, bool early, int ready, Waiter& waiter,
                                             RoleState& st) {
   const int k_stages = p.k_dim / kTileK;
   const uint32_t full0 = smem_u32(&c.ctl->full[0]), empty0 = smem_u32(&c.ctl->empty[0]);
   const uint32_t sf_full0 = smem_u32(&c.ctl->sf_full[0]);
   const uint32_t a0 = smem_u32(c.a_base), b0 = smem_u32(c.b_base), sf0 = smem_u32(c.sf_base);
+  // GEMM2 behind a GEMM1 that ordered the routes starts while that is still running: the weights of its first stages do not depend on that, so
+  // they are requested before the wait, the activations after it.
+  bool ahead = kStaged && kLayer == 2 && early;
+  // `ready`: stages of the first task whose weights have been requested already
   while (st.ok && walk.next()) {
     const Tile tile = walk.tile;
     const int nb = walk.nb;
     const bool shared = tile.expert == kSharedExpert;
+    const bool staged = kLayer == 1 && (shared || kStaged);     // the token tile is rows of the staged tokens
     const int box_sel = (max(tile.n_valid, 1) - 1) >> 4;         // token box: n_valid rounded up to 16 rows
     const uint32_t box_rows = 16u * (box_sel + 1);
     const CUtensorMap* wmap = shared ? &p.map_w_shared : &p.map_w_routed;
-    const CUtensorMap* tmap = shared ? &p.map_tok_shared_box[box_sel] : &p.map_tok_routed_box[box_sel];
+    const CUtensorMap* tmap = shared || staged ? &p.map_tok_shared_box[box_sel] : &p.map_tok_routed_box[box_sel];
     const int e = shared ? 0 : tile.expert;
     // The 256 stored weight rows of the task.  Layer 1 reads W13 in its stored order [g0..7, u0..7, g8..15, ...]
     // through a 5-D map (K, row in group of 8, group of 16 rows, gate/up, slice): one box of 8 x 16 x 2 lands the
@@ -229,31 +432,57 @@ __device__ __forceinline__ void sa_producer(const UmmaParams& p, const Cta& c, T
     const int32_t* wsf = (shared ? p.wsf_shared : p.wsf_routed) + (int64_t)e * k_stages * p.rows_per_expert + r0;
     const int64_t tsf_rows = shared ? p.tsf_rows_shared : p.tsf_rows_routed;
     const int32_t* tsf = (shared ? p.tsf_shared : p.tsf_routed) + (int64_t)tile.sf_chunk * kChunkRows;
-    const uint32_t a_tx = shared ? 2 * kTileRows * kTileK : kTileRows * kTileK;   // packed FP4 counts its global bytes
-    const bool gathered = kLayer == 1 && shared;          // token scales come from the scale arranger
-    const uint32_t tx = a_tx + box_rows * kTileK + (gathered ? 0 : 512) + (kLayer == 1 ? 0 : 1024);
+    const uint32_t w_tx = (shared ? 2 * kTileRows * kTileK : kTileRows * kTileK) + (kLayer == 1 ? 0 : 1024);   // packed FP4 counts its global bytes
+    const uint32_t t_tx = box_rows * kTileK + (staged ? 0 : 512);     // scales of staged tokens come from the scale arranger
+    auto load_weights = [&](uint32_t stage, int k0, const int32_t* sf) {
+      const uint32_t bar = full0 + 8 * stage;
+      if (kLayer == 1) {
+        tma_load_5d(a0 + stage * L::kABytes, wmap, k0, 0, group, 0, slice, bar);
+      } else {
+        tma_load_3d(a0 + stage * L::kABytes, wmap, k0, row, slice, bar);
+        bulk_load(sf0 + stage * L::kSfBytes, sf, 1024, bar);       // two chunks already in tensor-memory order
+      }
+    };
+    if (kStaged && ahead) {
+      ready = min(static_cast<int>(c.num_stages), k_stages);
+      if (elect_one())
+        for (int kb = 0; kb < ready; ++kb) {
+          mbar_expect_tx_only(full0 + 8 * kb, w_tx);
+          load_weights(kb, kb * kTileK, wsf + (int64_t)kb * p.rows_per_expert);
+        }
+      __syncwarp();
+      chain_wait();
+      ahead = false;
+    }
     int k0 = 0;
     for (int kb = 0; kb < k_stages; ++kb, k0 += kTileK, wsf += p.rows_per_expert, tsf += tsf_rows) {
       if (!waiter.wait_uniform(empty0 + 8 * st.stage, st.phase ^ 1u)) { st.ok = false; break; }
       const uint32_t bar = full0 + 8 * st.stage;
-      const uint32_t a_dst = a0 + st.stage * L::kABytes;
-      const uint32_t sf_dst = sf0 + st.stage * L::kSfBytes;
       if (elect_one()) {
-        if (kLayer == 1) {
+        if (kLayer == 1 && (!kStaged || kb >= ready)) {
           // scales of the 256 stored rows, rearranged by the scale arranger: their own barrier, first in the queue
           mbar_expect_tx(sf_full0 + 8 * st.stage, 1024);
-          bulk_load(sf_dst + 3 * 512, wsf, 1024, sf_full0 + 8 * st.stage);
+          bulk_load(sf0 + st.stage * L::kSfBytes + 3 * 512, wsf, 1024, sf_full0 + 8 * st.stage);
         }
-        mbar_expect_tx(bar, tx);
-        if (kLayer == 1) tma_load_5d(a_dst, wmap, k0, 0, group, 0, slice, bar);
-        else tma_load_3d(a_dst, wmap, k0, row, slice, bar);
-        if (kLayer == 2) bulk_load(sf_dst, wsf, 1024, bar);        // two chunks already in tensor-memory order
+        if (kStaged && kb < ready) {
+          mbar_expect_tx(bar, t_tx);
+        } else {
+          mbar_expect_tx(bar, w_tx + t_tx);
+          load_weights(st.stage, k0, wsf);
+        }
         tma_load_2d(b0 + st.stage * c.b_bytes, tmap, k0, tile.row0, bar);
-        if (!gathered) bulk_load(sf_dst + 2 * 512, tsf, 512, bar);
+        if (!staged) bulk_load(sf0 + st.stage * L::kSfBytes + 2 * 512, tsf, 512, bar);
       }
       __syncwarp();
       if (++st.stage == c.num_stages) { st.stage = 0; st.phase ^= 1u; }
     }
+    ready = 0;
+  }
+  // A GEMM1 that orders the routes lets GEMM2 start once this CTA has nothing left to request and knows the plan to be complete,
+  // which is what GEMM2 counts on.
+  if (kStaged && kLayer == 1 && p.route_here) {
+    if (!sa_wait_plan(p, waiter)) st.ok = false;
+    chain_release();
   }
 }
 
@@ -263,8 +492,8 @@ __device__ __forceinline__ void sa_producer(const UmmaParams& p, const Cta& c, T
 // transpose inside each 128-row block); the accumulators want the scales of 128 gate (h = 0) and 128 up (h = 1) channels.
 // On the MMA warps' path this work was a third of a stage's issue time (about 230 of 700 clk, and a stage is 580 clk of
 // HBM time at the clock a power-capped B200 runs this kernel at).
-template <typename L>
-__device__ __forceinline__ void sa_arrange_scales(const UmmaParams& p, const Cta& c, TaskWalk walk, Waiter& waiter,
+template <typename L, bool kStaged>
+__device__ __forceinline__ void sa_arrange_scales(const UmmaParams& p, const Cta& c, TaskWalk<kStaged> walk, Waiter& waiter,
                                                   RoleState& st) {
   const int lane = threadIdx.x & 31;
   const int k_stages = p.k_dim / kTileK;
@@ -279,15 +508,15 @@ __device__ __forceinline__ void sa_arrange_scales(const UmmaParams& p, const Cta
     src[t] = 128 * (m >> 6) + 4 * (r & 31) + (r >> 5);
   }
   while (st.ok && walk.next()) {
-    // The shared expert's token scales are gathered here, word kb of the staged scale rows (chunk position 4 (i % 32) + i / 32
-    // for token i), two stages ahead: its tiles then need no placement, only the staging.
-    const bool shared = walk.tile.expert == kSharedExpert;
+    // The scales of staged tokens are gathered here, word kb of the staged scale rows (chunk position 4 (i % 32) + i / 32
+    // for token i), two stages ahead: such tiles need no placement, only the staging.
+    const bool staged = walk.tile.expert == kSharedExpert || kStaged;
     const int32_t* x_sf = p.x_sf + (int64_t)(walk.tile.row0 + lane) * k_stages;
     uint32_t ahead[2][4] = {};
     auto gather = [&](uint32_t (&w)[4], int kb) {
 #pragma unroll
       for (int a = 0; a < 4; ++a)
-        w[a] = shared && kb < k_stages && lane + 32 * a < walk.tile.n_valid ? __ldg(x_sf + 32 * a * k_stages + kb) : 0u;
+        w[a] = staged && kb < k_stages && lane + 32 * a < walk.tile.n_valid ? __ldg(x_sf + 32 * a * k_stages + kb) : 0u;
     };
     gather(ahead[0], 0);
     gather(ahead[1], 1);
@@ -300,7 +529,7 @@ __device__ __forceinline__ void sa_arrange_scales(const UmmaParams& p, const Cta
       for (int t = 0; t < 8; ++t) v[t] = area[3 * 128 + src[t]];
 #pragma unroll
       for (int t = 0; t < 8; ++t) area[lane + 32 * t] = v[t];
-      if (shared) {
+      if (staged) {
         *reinterpret_cast<uint4*>(area + 2 * 128 + 4 * lane) = make_uint4(ahead[0][0], ahead[0][1], ahead[0][2], ahead[0][3]);
 #pragma unroll
         for (int a = 0; a < 4; ++a) ahead[0][a] = ahead[1][a];
@@ -318,8 +547,8 @@ __device__ __forceinline__ void sa_arrange_scales(const UmmaParams& p, const Cta
 // Two warps, one per weight tile / accumulator (h = 0, 1).  The whole warp walks the loop so that loop state stays
 // warp-uniform; one elected lane issues.  Each warp copies the scales it needs into its own TMEM columns, so no
 // ordering between the two warps' tensor-core instructions is needed.
-template <int kLayer, typename L>
-__device__ __forceinline__ void sa_mma(const UmmaParams& p, const Cta& c, TaskWalk walk, Waiter& waiter,
+template <int kLayer, typename L, bool kStaged>
+__device__ __forceinline__ void sa_mma(const UmmaParams& p, const Cta& c, TaskWalk<kStaged && kLayer == 1> walk, Waiter& waiter,
                                        RoleState& st, int h) {
   const int k_stages = p.k_dim / kTileK;
   const uint32_t full0 = smem_u32(&c.ctl->full[0]), sf_ready0 = smem_u32(&c.ctl->sf_ready[0]);
@@ -368,17 +597,73 @@ __device__ __forceinline__ void sa_mma(const UmmaParams& p, const Cta& c, TaskWa
 // Four warps; a thread owns one weight row (accumulator lane), the columns are the tile's tokens.
 // kFused (layer 2, EP > 1): every output row goes to the rank its token came from; compiled as kernels of its own so
 // that the single-destination epilogue of the other cases keeps its shorter inner loop.
-template <int kLayer, typename L, bool kFused>
-__device__ __forceinline__ void sa_epilogue(const UmmaParams& p, const Cta& c, TaskWalk walk, Waiter& waiter,
+// Tiles of at most this many rows leave column by column in a rolled loop: the unrolled batches of 16 columns are 16 KB of
+// instructions, which a call that has just streamed its weights through the L2 fetches from DRAM line by line (9 us at one
+// token), and with a token or two per expert most of their columns are padding.
+constexpr int kThinRows = 8;
+
+// GEMM1 epilogue of one column: this warp's 32 channels of one token, in a rolled loop
+__device__ __forceinline__ int sa_l1_column(const UmmaParams& p, uint32_t taddr, uint32_t up_offset, float wt, uint8_t* out) {
+  const uint32_t g = tc_ld1(taddr), u = tc_ld1(taddr + up_offset);
+  tc_ld_wait();
+  const float a = p.fast_math != 0 ? swiglu_act_t<true>(__uint_as_float(g), __uint_as_float(u), wt, p.clamp)
+                                   : swiglu_act_t<false>(__uint_as_float(g), __uint_as_float(u), wt, p.clamp);
+  const int sf_exp = ue8m0_exp_of_amax(warp_max_nonneg(fabsf(a)));
+  *out = float_to_e4m3(__fmul_rn(a, ue8m0_inv(sf_exp)));
+  return sf_exp;
+}
+
+// GEMM1 epilogue of a routed task whose columns are the staged tokens: every pool row of the expert takes the column of its
+// token.
+template <typename L>
+__device__ __forceinline__ bool sa_epilogue_staged(const UmmaParams& p, const Cta& c, const Tile& tile, int nb, Waiter& waiter, RoleState& st) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, q = warp & 3;
+  const uint32_t acc_stage = st.it & 1u, acc_phase = (st.it >> 1) & 1u;
+  const PlanView pv = plan_view(const_cast<char*>(p.plan), p.e_local, p.num_ranks);
+  const int n = pv.expert_total[tile.expert];
+  const Tile first = pv.tiles[pv.expert_tile_off[tile.expert]];
+  auto token_of = [&](int r) { return r < n ? p.sorted_route[p.pool_dst[first.row0 + r]] / p.topk : 0; };
+  int token = token_of(lane);
+  float weight = lane < n ? p.pool_w[first.row0 + lane] : 0.f;
+  if (!waiter.wait_warp(smem_u32(&c.ctl->tmem_full[acc_stage]), acc_phase)) return false;
+  tc_fence_after();
+  const uint32_t d0 = c.tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc_stage * L::kAccCols;
+  uint8_t* out = p.act_routed + (int64_t)first.row0 * p.inter + nb * kTileRows + q * 32 + lane;
+  // scale byte of (row r, channel group nb*4+q): word nb of the row's chunk (one per 16 rows), byte q
+  uint8_t* sf_out = p.act_sf_routed + ((int64_t)nb * p.act_sf_rows_routed + (int64_t)first.sf_chunk * kChunkRows) * 4 + q;
+#pragma unroll 1
+  for (int r = 0; r < n; ++r, out += p.inter) {
+    if (r > 0 && (r & 31) == 0) {                    // more than 32 rows: tokens that name the expert several times
+      token = token_of(r + lane);
+      weight = r + lane < n ? p.pool_w[first.row0 + r + lane] : 0.f;
+    }
+    const int j = __shfl_sync(0xffffffffu, token, r & 31);
+    const int sf_exp = sa_l1_column(p, d0 + j, L::kNCap, __shfl_sync(0xffffffffu, weight, r & 31), out);
+    if (lane == 0) sf_out[((r / kStagedTokens) * kChunkRows + chunk_pos(r % kStagedTokens)) * 4] = static_cast<uint8_t>(sf_exp);
+  }
+  tc_fence_before();
+  mbar_arrive(smem_u32(&c.ctl->tmem_empty[acc_stage]));
+  return true;
+}
+
+template <int kLayer, typename L, bool kFused, bool kStaged>
+__device__ __forceinline__ void sa_epilogue(const UmmaParams& p, const Cta& c, TaskWalk<kStaged && kLayer == 1> walk, Waiter& waiter,
                                             RoleState& st) {
   Control* ctl = c.ctl;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int q = warp & 3;                     // TMEM lane quadrant this warp may read
   const uint32_t lane_sel = static_cast<uint32_t>(q * 32) << 16;
+  bool plan_known = false;
   for (; st.ok && walk.next(); ++st.it) {
     const Tile tile = walk.tile;
     const int nb = walk.nb;
     const bool shared = tile.expert == kSharedExpert;
+    if (kStaged && kLayer == 1 && !shared) {
+      if (!plan_known && !sa_wait_plan(p, waiter)) { st.ok = false; break; }
+      plan_known = true;
+      if (!sa_epilogue_staged<L>(p, c, tile, nb, waiter, st)) { st.ok = false; break; }
+      continue;
+    }
     const uint32_t acc_stage = st.it & 1u, acc_phase = (st.it >> 1) & 1u;
     // Per-token side data of the tile (top-k weight / destination row), one coalesced load per 32 tokens issued
     // before the accumulator is awaited; tokens read it by shuffle.
@@ -412,7 +697,13 @@ __device__ __forceinline__ void sa_epilogue(const UmmaParams& p, const Cta& c, T
       // scale byte of (token i, channel group nb*4+q): word nb of the chunk row, byte q
       uint8_t* sf_out = act_sf + ((int64_t)nb * sf_rows + (int64_t)tile.sf_chunk * kChunkRows) * 4 + q;
       uint8_t* act_col = act + (int64_t)tile.row0 * p.inter + row;
-      for (int i0 = 0; i0 < n16; i0 += 16) {
+      if (tile.n_valid <= kThinRows) {
+#pragma unroll 1
+        for (int i = 0; i < tile.n_valid; ++i, act_col += p.inter) {
+          const int sf_exp = sa_l1_column(p, d0 + i, L::kNCap, __shfl_sync(0xffffffffu, wv[0], i), act_col);
+          if (lane == 0) sf_out[chunk_pos(i) * 4] = static_cast<uint8_t>(sf_exp);
+        }
+      } else for (int i0 = 0; i0 < n16; i0 += 16) {
         uint32_t g[16], u[16];
         tc_ld16(d0 + i0, g);
         tc_ld16(d0 + L::kNCap + i0, u);
@@ -440,6 +731,16 @@ __device__ __forceinline__ void sa_epilogue(const UmmaParams& p, const Cta& c, T
           if (i0 + j < tile.n_valid) act_col[(int64_t)(i0 + j) * p.inter] = static_cast<uint8_t>(g[j]);
         if (lane < 16 && i0 + lane < tile.n_valid)
           sf_out[chunk_pos(i0 + lane) * 4] = static_cast<uint8_t>(my_sf);
+      }
+    } else if (!kFused && tile.n_valid <= kThinRows) {
+      __nv_bfloat16* out = (shared ? p.shared_out : p.ret) + nb * 2 * kTileRows + q * 32 + lane;
+#pragma unroll 1
+      for (int i = 0; i < tile.n_valid; ++i) {
+        const uint32_t v0 = tc_ld1(d0 + i), v1 = tc_ld1(d0 + L::kNCap + i);
+        tc_ld_wait();
+        __nv_bfloat16* o = out + (int64_t)__shfl_sync(0xffffffffu, dv[0], i) * p.hidden;
+        o[0] = __float2bfloat16_rn(__uint_as_float(v0));
+        o[kTileRows] = __float2bfloat16_rn(__uint_as_float(v1));
       }
     } else if (!kFused) {
 #pragma unroll
@@ -522,6 +823,7 @@ __device__ __forceinline__ void sa_setup(Control* ctl) {
       mbar_init(smem_u32(&ctl->tmem_empty[i]), 128);
     }
     ctl->abort_flag = 0;
+    for (int i = 0; i < 16; ++i) ctl->hit[i] = 0u;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if ((threadIdx.x >> 5) == 1) {
@@ -547,8 +849,27 @@ __device__ __forceinline__ void sa_teardown(Control* ctl, uint32_t tmem_base) {
   }
 }
 
+// Layer 1, before anything has been waited for: weights and scales of the first stages of a CTA's shared task, by the producer
+// warp (it has initialised the barriers itself).  Returns the number of stages.
+template <typename L>
+__device__ __forceinline__ int sa_request_shared(const UmmaParams& p, const Cta& c) {
+  const int nb = static_cast<int>(blockIdx.x) / p.shared_tiles.parts, stages = min(static_cast<int>(c.num_stages), p.k_dim / kTileK);
+  __syncwarp();
+  if (elect_one())
+#pragma unroll 1
+    for (int kb = 0; kb < stages; ++kb) {
+      const uint32_t bar = smem_u32(&c.ctl->full[kb]), sf_bar = smem_u32(&c.ctl->sf_full[kb]);
+      mbar_expect_tx(sf_bar, 1024);
+      bulk_load(smem_u32(c.sf_base) + kb * L::kSfBytes + 3 * 512, p.wsf_shared + (int64_t)kb * p.rows_per_expert + 2 * nb * kTileRows, 1024, sf_bar);
+      mbar_expect_tx_only(bar, 2 * kTileRows * kTileK);
+      tma_load_5d(smem_u32(c.a_base) + kb * L::kABytes, &p.map_w_shared, kb * kTileK, 0, 2 * nb * kTileRows / 16, 0, 0, bar);
+    }
+  __syncwarp();
+  return stages;
+}
+
 // One layer per launch.
-template <int kLayer, bool kFused = false>
+template <int kLayer, bool kFused, bool kStaged>
 __global__ void __launch_bounds__(kThreads, 1) umma_kernel(const __grid_constant__ UmmaParams p) {
   static_assert(!kFused || kLayer == 2, "only GEMM2 writes rows back");
   using L = Shape<kLayer>;
@@ -556,13 +877,29 @@ __global__ void __launch_bounds__(kThreads, 1) umma_kernel(const __grid_constant
   uint8_t* smem = sa_align(smem_raw);
   Control* ctl = reinterpret_cast<Control*>(smem);
   const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);   // warp-uniform for the compiler too
-  chain_release();
+  if (kLayer == 2 || !kStaged || !p.route_here) chain_release();
   sa_setup<L>(ctl);
   // Everything above touches only this CTA's own shared and tensor memory, so it may run while the kernel before this
   // one in the stream is still running.  GEMM1 of a call without pair tiles goes on with the shared expert: its launch is let
-  // start by the route ordering's blocks once they have seen the staging complete.
-  const bool early = kLayer == 1 && p.tile_rows > 0;
-  if (!early && !p.skip_wait) chain_wait();
+  // start by the route ordering's blocks once they have seen the staging complete.  GEMM2 behind a GEMM1 that orders the routes
+  // itself starts when all CTAs of that have seen the plan complete.
+  const bool early = p.early != 0;
+  if (warp == 0 && elect_one()) {
+    prefetch_map(&p.map_w_routed);
+    prefetch_map(&p.map_w_shared);
+  }
+  // (a GEMM1 that orders the routes follows the staging itself; the shared expert's weights do not wait even for that)
+  int ready = 0;
+  if (kStaged && kLayer == 1 && p.route_here && warp == 0 && static_cast<int>(blockIdx.x) < p.shared_tiles.parts * p.n_blocks)
+    ready = sa_request_shared<L>(p, sa_carve<L>(smem, p.tile_rows, p.max_stages));
+  if ((!early || (kStaged && kLayer == 1 && p.route_here)) && !p.skip_wait) chain_wait();
+  if (kStaged && kLayer == 1) {
+    __syncthreads();                         // the words are zero
+    for (int i = threadIdx.x; i < p.num_routes; i += kThreads) {
+      const int64_t id = p.topk_idx[i];
+      if (id >= 0 && id < p.e_local) atomicOr(&ctl->hit[id >> 5], 1u << (id & 31));
+    }
+  }
   if (kFused) {
     if (threadIdx.x == 0) ctl->out_base[32] = p.shared_out;
     const int t = threadIdx.x - 32;
@@ -585,19 +922,24 @@ __global__ void __launch_bounds__(kThreads, 1) umma_kernel(const __grid_constant
                                        : max(16, min(kSmallTileRows, plan_view(const_cast<char*>(p.plan), p.e_local, p.num_ranks).hdr->small_rows));
   Cta c = sa_carve<L>(smem, tile_rows, p.max_stages);
   c.tmem_base = __shfl_sync(0xffffffffu, ctl->tmem_base, 0);
-  const TaskWalk walk(p, !early);
+  const TaskWalk<kStaged && kLayer == 1> walk(p, ctl->hit, kLayer == 2 || !early, p.n_blocks);
   Waiter waiter{&ctl->abort_flag, p.status, global_timer() + static_cast<uint64_t>(p.timeout_ns), kLayer, warp};
   RoleState st;
   if (warp == 0) {
-    sa_producer<kLayer, L>(p, c, walk, waiter, st);
+    sa_producer<kLayer, L, kStaged>(p, c, walk, early, ready, waiter, st);
   } else if (warp == 1 || warp == 6) {
-    sa_mma<kLayer, L>(p, c, walk, waiter, st, warp == 1 ? 0 : 1);
+    sa_mma<kLayer, L, kStaged>(p, c, walk, waiter, st, warp == 1 ? 0 : 1);
   } else if (warp == 7) {
-    if (kLayer == 1) sa_arrange_scales<L>(p, c, walk, waiter, st);
+    if constexpr (kLayer == 1) sa_arrange_scales<L, kStaged>(p, c, walk, waiter, st);
+    else if (kStaged && p.route_here) sa_place(p);
   } else {
-    sa_epilogue<kLayer, L, kFused>(p, c, walk, waiter, st);
+    if (kStaged && kLayer == 1 && p.route_here && blockIdx.x == gridDim.x - 1)
+      sa_route(p, *reinterpret_cast<RouteScratch*>(c.sf_base + c.num_stages * L::kSfBytes), static_cast<int>(threadIdx.x) - 64);
+    sa_epilogue<kLayer, L, kFused, kStaged>(p, c, walk, waiter, st);
   }
   chain_wait();       // a CTA that has not waited yet must not end before what precedes the launch
+  if (kStaged && kLayer == 2 && p.route_here && blockIdx.x == 0 && threadIdx.x == 0)      // GEMM1 has completed: nobody looks at the flag any more
+    plan_view(const_cast<char*>(p.plan), p.e_local, p.num_ranks).hdr->routed = 0;
   sa_teardown(ctl, c.tmem_base);
 }
 
@@ -637,15 +979,15 @@ int make_w13_map(CUtensorMap* map, bool fp4, const void* base, uint64_t k_elems,
   return r == CUDA_SUCCESS ? 0 : static_cast<int>(r);
 }
 
-template <int kLayer, bool kFused>
+template <int kLayer, bool kFused, bool kStaged>
 cudaError_t prepare_one() {
-  return cudaFuncSetAttribute(umma_kernel<kLayer, kFused>, cudaFuncAttributeMaxDynamicSharedMemorySize, Shape<kLayer>::kSmemBytes);
+  return cudaFuncSetAttribute(umma_kernel<kLayer, kFused, kStaged>, cudaFuncAttributeMaxDynamicSharedMemorySize, Shape<kLayer>::kSmemBytes);
 }
 
-template <int kLayer, bool kFused>
+template <int kLayer, bool kFused, bool kStaged>
 cudaError_t launch_layer(UmmaParams& p, cudaStream_t s) {
   p.max_stages = g_tune_stages;
-  launch_chained(umma_kernel<kLayer, kFused>, dim3(tc_num_sms()), dim3(kThreads), Shape<kLayer>::kSmemBytes, s, p);
+  launch_chained(umma_kernel<kLayer, kFused, kStaged>, dim3(tc_num_sms()), dim3(kThreads), Shape<kLayer>::kSmemBytes, s, p);
   return cudaGetLastError();
 }
 
@@ -760,8 +1102,7 @@ bool build_sa(const Ctx& c, const MmoeWeights& w, bool has_shared, UmmaParams* o
   else p1.map_w_shared = p1.map_w_routed;
   for (int b = 0; b < kNumBoxes; ++b) {
     bad |= make_token_map(&p1.map_tok_routed_box[b], c.ws + c.lay.pool_x, h, c.lay.pool_rows, 16 * (b + 1));
-    if (has_shared) bad |= make_token_map(&p1.map_tok_shared_box[b], c.ws + c.lay.x, h, c.geo.num_max_tokens, 16 * (b + 1));
-    else p1.map_tok_shared_box[b] = p1.map_tok_routed_box[b];
+    bad |= make_token_map(&p1.map_tok_shared_box[b], c.ws + c.lay.x, h, c.geo.num_max_tokens, 16 * (b + 1));
   }
   if (bad) return false;
   p1.plan = c.ws + c.lay.plan;
@@ -769,6 +1110,19 @@ bool build_sa(const Ctx& c, const MmoeWeights& w, bool has_shared, UmmaParams* o
   p1.wsf_shared = static_cast<const int32_t*>(w.shared_w13_sf);
   p1.tsf_routed = c.at<int32_t>(c.lay.pool_sf);
   p1.x_sf = c.at<int32_t>(c.lay.x_sf);
+  p1.topk_idx = c.at<int64_t>(c.lay.topk_idx);
+  p1.sorted_route = c.at<int32_t>(c.lay.sorted_route);
+  p1.pool_dst = c.at<int32_t>(c.lay.pool_dst);
+  p1.topk = c.geo.num_topk;
+  p1.topk_weights = c.at<float>(c.lay.topk_weights);
+  p1.route_pos = c.at<int32_t>(c.lay.route_pos);
+  p1.send_count = c.at<int32_t>(c.lay.send_count);
+  p1.send_offset = c.at<int32_t>(c.lay.send_offset);
+  p1.recv_count = c.at<int32_t>(c.lay.recv_count);
+  p1.x = c.at<uint4>(c.lay.x);
+  p1.pool_x = c.at<uint4>(c.lay.pool_x);
+  p1.pool_sf = c.at<int32_t>(c.lay.pool_sf);
+  p1.pool_sf_rows = c.lay.pool_sf_rows;
   p1.tsf_rows_routed = c.lay.pool_sf_rows;
   p1.act_routed = c.at<uint8_t>(c.lay.act_x);
   p1.act_shared = c.at<uint8_t>(c.lay.shared_act_x);
@@ -905,9 +1259,11 @@ int prepare_umma(const MmoeGeometry& geo) {
   int sms = 0;
   if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return MMOE_ERR_CUDA;
   cudaError_t e = cudaSuccess;
-  if (e == cudaSuccess) e = prepare_one<1, false>();
-  if (e == cudaSuccess) e = prepare_one<2, false>();
-  if (e == cudaSuccess) e = prepare_one<2, true>();
+  if (e == cudaSuccess) e = prepare_one<1, false, false>();
+  if (e == cudaSuccess) e = prepare_one<1, false, true>();
+  if (e == cudaSuccess) e = prepare_one<2, false, false>();
+  if (e == cudaSuccess) e = prepare_one<2, true, false>();
+  if (e == cudaSuccess) e = prepare_one<2, false, true>();
   if (e == cudaSuccess) e = tm_prepare();
   if (e != cudaSuccess) return MMOE_ERR_CUDA;
   g_num_sms[dev] = sms;
@@ -947,6 +1303,7 @@ cudaError_t launch_experts_umma(const Ctx& c, const MmoeWeights& w, const MmoeOp
   const bool shared_pairs = m > pair_above;
   const bool pairs = c.tile_select == 2 ? with_shared && shared_pairs : pair_above != kNeverPair;
   const bool small = c.tile_select == 2 ? with_shared && !shared_pairs : pair_above > 0;
+  const bool staged = !pairs && !fused && c.tile_select != 2 && m > 0 && m <= kStagedTokens && block_m <= kStagedTokens;
   for (int layer = 1; layer <= 2; ++layer) {
     if ((mask & layer) == 0) continue;
     if (e == cudaSuccess && pairs) {
@@ -962,7 +1319,14 @@ cudaError_t launch_experts_umma(const Ctx& c, const MmoeWeights& w, const MmoeOp
       p.tile_rows = c.tile_select == 2 ? cut.step : (pairs ? 0 : small_only_cap(m, block_m));
       // The pair launch in front reads and writes nothing that this one does, and lets it start only after its own wait.
       p.skip_wait = pairs ? 1 : 0;
-      e = layer == 1 ? launch_layer<1, false>(p, s) : fused ? launch_layer<2, true>(p, s) : launch_layer<2, false>(p, s);
+      p.early = !pairs && c.tile_select == 0 && !fused && (layer == 1 || c.route_in_gemm) ? 1 : 0;
+      p.num_routes = m * c.geo.num_topk;
+      p.route_here = c.route_in_gemm ? 1 : 0;
+      p.stats = c.stats;
+      // (instances of their own for the calls that route in the launch: the others keep the shorter code)
+      if (layer == 1) e = staged ? launch_layer<1, false, true>(p, s) : launch_layer<1, false, false>(p, s);
+      else if (fused) e = launch_layer<2, true, false>(p, s);
+      else e = staged ? launch_layer<2, false, true>(p, s) : launch_layer<2, false, false>(p, s);
     }
   }
   return e;
