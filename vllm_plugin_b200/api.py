@@ -10,6 +10,9 @@ from __future__ import annotations
 
 from typing import Any, Optional, Tuple, Union
 
+# implementations of the per-step functions, looked up once (a function-local import costs about a microsecond per call)
+_mega_moe = _stage = _route_and_stage = None
+
 
 def get_symm_buffer_for_mega_moe(group, num_experts: int, num_max_tokens_per_rank: int, num_topk: int, hidden: int,
                                  intermediate_hidden: int, num_shared_experts: int = 0,
@@ -40,11 +43,12 @@ def fp8_fp4_mega_moe(y, l1_weights: Tuple[Any, Any], l2_weights: Tuple[Any, Any]
                      activation_beta: float = 0.0, *, residual=None):
     """Fused MegaMoE for one rank.  The BLOCK_M variant is selected from ``y.size(0)`` of this call.  ``residual``
     (keyword only, an addition to the reference's signature): BF16 ``(M, H)`` added to the output in the combine pass."""
-    from .backend.frontend import fp8_fp4_mega_moe as _impl
-
-    return _impl(y, l1_weights, l2_weights, sym_buffer, shared_l1_weights, shared_l2_weights,
-                 cumulative_local_expert_recv_stats, recipe, activation, activation_clamp, fast_math, activation_alpha,
-                 activation_beta, residual=residual)
+    global _mega_moe
+    if _mega_moe is None:
+        from .backend.frontend import fp8_fp4_mega_moe as _mega_moe
+    return _mega_moe(y, l1_weights, l2_weights, sym_buffer, shared_l1_weights, shared_l2_weights,
+                     cumulative_local_expert_recv_stats, recipe, activation, activation_clamp, fast_math, activation_alpha,
+                     activation_beta, residual=residual)
 
 
 def get_block_m_for_mega_moe(num_ranks: int, num_experts: int, num_max_tokens_per_rank: int, num_tokens: int,
@@ -78,9 +82,10 @@ def get_unsupported_reason_for_mega_moe(num_ranks: int, num_experts: int, num_ma
 def stage_inputs_for_mega_moe(sym_buffer, hidden_states, topk_ids, topk_weights, *, is_padding=None,
                               block_m: Optional[int] = None) -> int:
     """Quantise and stage one call's inputs into ``sym_buffer`` (one CUDA launch); returns the BLOCK_M used."""
-    from .backend.staging import stage_inputs as _impl
-
-    return _impl(sym_buffer, hidden_states, topk_ids, topk_weights, is_padding=is_padding, block_m=block_m)
+    global _stage
+    if _stage is None:
+        from .backend.staging import stage_inputs as _stage
+    return _stage(sym_buffer, hidden_states, topk_ids, topk_weights, is_padding=is_padding, block_m=block_m)
 
 
 def route_and_stage_inputs_for_mega_moe(sym_buffer, hidden_states, router_logits, *, replica_map=None, is_padding=None,
@@ -88,9 +93,10 @@ def route_and_stage_inputs_for_mega_moe(sym_buffer, hidden_states, router_logits
     """Router (top-k by logit, softmax over the selected, optional logical -> physical replica choice) fused in front of
     the input staging: one CUDA launch; returns the BLOCK_M used.  Not part of the reference's surface: there the
     serving engine routes before it calls the layer."""
-    from .backend.staging import route_and_stage_inputs as _impl
-
-    return _impl(sym_buffer, hidden_states, router_logits, replica_map=replica_map, is_padding=is_padding, block_m=block_m)
+    global _route_and_stage
+    if _route_and_stage is None:
+        from .backend.staging import route_and_stage_inputs as _route_and_stage
+    return _route_and_stage(sym_buffer, hidden_states, router_logits, replica_map=replica_map, is_padding=is_padding, block_m=block_m)
 
 
 def prepare_megamoe_nvfp4_inputs(hidden_states, global_scale: float, out=None):

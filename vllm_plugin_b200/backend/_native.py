@@ -65,6 +65,7 @@ class MmoeOptions(ctypes.Structure):
 
 
 _lib: Optional[ctypes.CDLL] = None
+_raw_stream = None
 
 
 def library_path() -> str:
@@ -120,6 +121,15 @@ def load() -> ctypes.CDLL:
             fn.restype = ctypes.c_int
     _lib = lib
     return lib
+
+
+def raw_stream(device_index: int) -> int:
+    """Handle of the current stream of a CUDA device (without building a ``torch.cuda.Stream`` around it)."""
+    global _raw_stream
+    if _raw_stream is None:
+        import torch
+        _raw_stream = torch._C._cuda_getCurrentRawStream
+    return _raw_stream(device_index)
 
 
 def check(code: int) -> None:

@@ -18,6 +18,7 @@ from __future__ import annotations
 import ctypes
 import dataclasses
 import math
+import operator
 from typing import Any, Dict, Optional, Tuple
 
 import torch
@@ -86,6 +87,18 @@ def get_block_m_for_mega_moe(num_ranks: int, num_experts: int, num_max_tokens_pe
     if _kernel_options.block_m > 0:
         return _kernel_options.block_m
     return _h.get_block_m_for_mega_moe(num_ranks, num_experts, num_max_tokens_per_rank, num_tokens, num_topk, mma_type)
+
+
+def call_block_m(sym_buffer, num_tokens: int) -> int:
+    """BLOCK_M of a call on ``sym_buffer``, remembered per token count."""
+    if _kernel_options.block_m > 0:
+        return _kernel_options.block_m
+    block_m = sym_buffer.block_m_of.get(num_tokens)
+    if block_m is None:
+        block_m = sym_buffer.block_m_of[num_tokens] = _h.get_block_m_for_mega_moe(
+            sym_buffer.num_ranks, sym_buffer.num_experts, sym_buffer.num_max_tokens_per_rank, num_tokens, sym_buffer.num_topk,
+            sym_buffer.mma_type)
+    return block_m
 
 
 def precompile_mega_moe_variants(num_ranks: int, num_experts: int, num_max_tokens_per_rank: int, num_topk: int,
@@ -226,14 +239,11 @@ class _CallRecord:
     """What the last validated call on a buffer established: the tensor objects it checked (kept alive, so that their
     identities cannot be reused), the structures built from them, and the status poll state."""
 
-    __slots__ = ("tensors", "addresses", "weights", "stats", "options_key", "options", "peers", "variants_ready")
+    __slots__ = ("tensors", "present", "addresses", "weights", "weights_ref", "options_key", "options", "options_ref", "peers",
+                 "variants_ready")
 
     def matches(self, tensors) -> bool:
-        kept = self.tensors
-        for a, b, addr in zip(tensors, kept, self.addresses):
-            if a is not b or (a is not None and a.data_ptr() != addr):
-                return False
-        return True
+        return all(map(operator.is_, tensors, self.tensors)) and [t.data_ptr() for t in self.present] == self.addresses
 
 
 class _StatusPoll:
@@ -273,8 +283,10 @@ def _validate(y, l1_weights, l2_weights, sym_buffer, shared_l1_weights, shared_l
                                        activation_beta)
     rec = _CallRecord()
     rec.tensors = tensors
-    rec.addresses = tuple(t.data_ptr() if t is not None else 0 for t in tensors)
+    rec.present = [t for t in tensors if t is not None]
+    rec.addresses = [t.data_ptr() for t in rec.present]
     rec.weights = _weights_struct(l1_weights, l2_weights, shared_l1_weights, shared_l2_weights, s13, s2)
+    rec.weights_ref = ctypes.byref(rec.weights)
     rec.options_key = None
     rec.options = None
     rec.peers = None
@@ -301,9 +313,9 @@ def fp8_fp4_mega_moe(y: torch.Tensor, l1_weights, l2_weights, sym_buffer, shared
                shared_l1_weights[1] if shared_l1_weights is not None else None,
                shared_l2_weights[0] if shared_l2_weights is not None else None,
                shared_l2_weights[1] if shared_l2_weights is not None else None, stats)
-    rec = getattr(sym_buffer, "_call_record", None)
+    rec = sym_buffer._call_record
     m = y.size(0)
-    if (rec is None or not rec.matches(tensors) or tuple(recipe) != (1, 1, 32) or activation != "swiglu"
+    if (rec is None or not rec.matches(tensors) or (recipe != (1, 1, 32) and tuple(recipe) != (1, 1, 32)) or activation != "swiglu"
             or activation_alpha != 1.0 or activation_beta != 0.0):
         rec = _validate(y, l1_weights, l2_weights, sym_buffer, shared_l1_weights, shared_l2_weights, stats, recipe,
                         activation, activation_clamp, fast_math, activation_alpha, activation_beta, tensors)
@@ -324,6 +336,7 @@ def fp8_fp4_mega_moe(y: torch.Tensor, l1_weights, l2_weights, sym_buffer, shared
     if rec.options_key != key:
         rec.options = _native.MmoeOptions(float(activation_clamp) if activation_clamp is not None else math.inf,
                                           1 if fast_math else 0, _engine, ko.timeout_ms)
+        rec.options_ref = ctypes.byref(rec.options)
         rec.options_key = key
     capturing = torch.cuda.is_current_stream_capturing()
     if not rec.variants_ready and _engine == _native.ENGINE_TENSOR_CORE and not capturing:
@@ -333,20 +346,17 @@ def fp8_fp4_mega_moe(y: torch.Tensor, l1_weights, l2_weights, sym_buffer, shared
         rec.variants_ready = True
     poll = None
     if ko.status_poll_interval > 0 and not capturing:
-        poll = getattr(sym_buffer, "_status_poll", None)
+        poll = sym_buffer._status_poll
         if poll is None:
             poll = sym_buffer._status_poll = _StatusPoll(sym_buffer)
         poll.before_call(sym_buffer)
     lib = _native.load()
-    bm = get_block_m_for_mega_moe(sym_buffer.num_ranks, sym_buffer.num_experts, sym_buffer.num_max_tokens_per_rank, m,
-                                  sym_buffer.num_topk, sym_buffer.mma_type)
-    rec.options.residual = residual.data_ptr() if residual is not None and m > 0 else None
-    res_ptr = rec.options.residual
-    w, opts = ctypes.byref(rec.weights), ctypes.byref(rec.options)
+    bm = call_block_m(sym_buffer, m)
+    res_ptr = rec.options.residual = residual.data_ptr() if residual is not None and m > 0 else None
+    w, opts, g = rec.weights_ref, rec.options_ref, sym_buffer.geo_ref
     stats_ptr = stats.data_ptr() if stats is not None else None
-    stream = torch.cuda.current_stream(y.device).cuda_stream
+    stream = _native.raw_stream(y.get_device())
     ws = sym_buffer.base_ptr
-    g = ctypes.byref(sym_buffer.geo)
     if sym_buffer.num_ranks == 1:
         _native.check(lib.mmoe_forward(g, ws, w, opts, y.data_ptr(), m, bm, stats_ptr, stream))
     elif rec.peers is not None and ko.ep_transport == "peer":

@@ -8,7 +8,6 @@ a Triton kernel and its fallback a torch implementation; here the CUDA kernel is
 
 from __future__ import annotations
 
-import ctypes
 from typing import Optional, Tuple
 
 import torch
@@ -24,8 +23,9 @@ def get_shared_sf_rows(num_tokens: int, block_m: int, device=None) -> torch.Tens
     return (t // block_m) * align(block_m, 128) + (m // 128) * 128 + (m % 32) * 4 + (m % 128) // 32
 
 
-def _stream_ptr(device) -> int:
-    return torch.cuda.current_stream(device).cuda_stream
+def _block_m_of(sym_buffer, num_tokens: int) -> int:
+    from .frontend import call_block_m
+    return call_block_m(sym_buffer, num_tokens)
 
 
 def stage_inputs(sym_buffer, hidden_states: torch.Tensor, topk_ids: torch.Tensor, topk_weights: torch.Tensor, *,
@@ -35,10 +35,7 @@ def stage_inputs(sym_buffer, hidden_states: torch.Tensor, topk_ids: torch.Tensor
     num_tokens, hidden_size = hidden_states.shape
     assert num_tokens <= sym_buffer.num_max_tokens_per_rank, "num_tokens must be <= num_max_tokens_per_rank"
     if block_m is None:
-        from .frontend import get_block_m_for_mega_moe
-        block_m = get_block_m_for_mega_moe(sym_buffer.num_ranks, sym_buffer.num_experts,
-                                           sym_buffer.num_max_tokens_per_rank, num_tokens, sym_buffer.num_topk,
-                                           sym_buffer.mma_type)
+        block_m = _block_m_of(sym_buffer, num_tokens)
     if num_tokens == 0:
         return block_m
     if hidden_size % 128 != 0 or hidden_size != sym_buffer.hidden:
@@ -57,16 +54,17 @@ def stage_inputs(sym_buffer, hidden_states: torch.Tensor, topk_ids: torch.Tensor
     ids = topk_ids.contiguous()
     if ids.dtype not in (torch.int32, torch.int64):
         ids = ids.to(torch.int64)
-    w = topk_weights.to(torch.float32).contiguous()
+    w = topk_weights if topk_weights.dtype == torch.float32 else topk_weights.to(torch.float32)
+    w = w.contiguous()
     pad_ptr = None
     if is_padding is not None:
         pad = is_padding[:num_tokens].to(torch.uint8).contiguous()
         pad_ptr = pad.data_ptr()
     lib = _native.load()
     _native.check(lib.mmoe_stage_inputs(
-        ctypes.byref(sym_buffer.geo), sym_buffer.base_ptr, hidden_states.data_ptr(), ids.data_ptr(),
+        sym_buffer.geo_ref, sym_buffer.base_ptr, hidden_states.data_ptr(), ids.data_ptr(),
         1 if ids.dtype == torch.int64 else 0, w.data_ptr(), pad_ptr, num_tokens,
-        block_m if sym_buffer.num_shared_experts > 0 else 0, _stream_ptr(hidden_states.device)))
+        block_m if sym_buffer.num_shared_experts > 0 else 0, _native.raw_stream(hidden_states.get_device())))
     return block_m
 
 
@@ -80,10 +78,7 @@ def route_and_stage_inputs(sym_buffer, hidden_states: torch.Tensor, router_logit
     num_tokens, hidden_size = hidden_states.shape
     assert num_tokens <= sym_buffer.num_max_tokens_per_rank, "num_tokens must be <= num_max_tokens_per_rank"
     if block_m is None:
-        from .frontend import get_block_m_for_mega_moe
-        block_m = get_block_m_for_mega_moe(sym_buffer.num_ranks, sym_buffer.num_experts,
-                                           sym_buffer.num_max_tokens_per_rank, num_tokens, sym_buffer.num_topk,
-                                           sym_buffer.mma_type)
+        block_m = _block_m_of(sym_buffer, num_tokens)
     if num_tokens == 0:
         return block_m
     if hidden_size != sym_buffer.hidden or hidden_states.dtype != torch.bfloat16 or not hidden_states.is_cuda:
@@ -106,9 +101,9 @@ def route_and_stage_inputs(sym_buffer, hidden_states: torch.Tensor, router_logit
         pad_ptr = pad.data_ptr()
     lib = _native.load()
     _native.check(lib.mmoe_route_stage_inputs(
-        ctypes.byref(sym_buffer.geo), sym_buffer.base_ptr, hidden_states.data_ptr(), logits.data_ptr(), logits.shape[1],
+        sym_buffer.geo_ref, sym_buffer.base_ptr, hidden_states.data_ptr(), logits.data_ptr(), logits.shape[1],
         count_ptr, slots_ptr, copies, pad_ptr, num_tokens, block_m if sym_buffer.num_shared_experts > 0 else 0,
-        _stream_ptr(hidden_states.device)))
+        _native.raw_stream(hidden_states.get_device())))
     return block_m
 
 
@@ -129,7 +124,7 @@ def prepare_megamoe_nvfp4_inputs(hidden_states: torch.Tensor, global_scale: floa
     q, sf = out
     assert q.is_contiguous() and sf.is_contiguous() and q.shape == (m, h // 2) and sf.shape == (m, h // 16)
     _native.check(_native.load().mmoe_stage_inputs_nvfp4(hidden_states.data_ptr(), float(global_scale), q.data_ptr(),
-                                                         sf.data_ptr(), m, h, _stream_ptr(hidden_states.device)))
+                                                         sf.data_ptr(), m, h, _native.raw_stream(hidden_states.get_device())))
     return q, sf
 
 

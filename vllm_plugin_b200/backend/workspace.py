@@ -13,8 +13,9 @@ on ANY rank, every rank falls back together to ordinary device memory and the ho
 
 from __future__ import annotations
 
+import ctypes
 import warnings
-from typing import Optional, Union
+from typing import Dict, Optional, Union
 
 import torch
 
@@ -60,6 +61,12 @@ class SymmBuffer:
         self.geo = _native.MmoeGeometry(group.size(), group.rank(), num_experts, num_topk, hidden, intermediate_hidden,
                                         num_shared_experts, self.num_max_tokens_per_rank)
         self.layout = _native.layout_of(self.geo)
+        # per-step lookups kept out of the call path: the geometry as the library takes it, BLOCK_M by token count
+        self.num_ranks = group.size()
+        self.geo_ref = ctypes.byref(self.geo)
+        self.block_m_of: Dict[int, int] = {}
+        self._call_record = None
+        self._status_poll = None
         if device is None:
             device = torch.device("cuda", torch.cuda.current_device())
         self.device = device
@@ -167,10 +174,6 @@ class SymmBuffer:
     @property
     def rank(self) -> int:
         return self.group.rank()
-
-    @property
-    def num_ranks(self) -> int:
-        return self.group.size()
 
     @property
     def base_ptr(self) -> int:

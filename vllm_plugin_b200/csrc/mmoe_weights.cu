@@ -34,7 +34,7 @@ __global__ void __launch_bounds__(256) interleave_rows_kernel(const uint4* __res
       uint4 q[4];
 #pragma unroll
       for (int u = 0; u < 4; ++u)
-        if (v0 + 32 * u < vec) q[u] = s[v0 + 32 * u];
+        if (v0 + 32 * u < vec) q[u] = __ldcs(s + v0 + 32 * u);
 #pragma unroll
       for (int u = 0; u < 4; ++u)
         if (v0 + 32 * u < vec) d[v0 + 32 * u] = q[u];
@@ -84,7 +84,9 @@ constexpr int kSplitPieceVec = 1024;
 __global__ void __launch_bounds__(256) split_halves_kernel(const uint4* __restrict__ src, uint4* __restrict__ dst,
                                                            int num_halves, int64_t half_vec, int64_t slice_vec) {
   const int64_t pieces_per_half = (half_vec + kSplitPieceVec - 1) / kSplitPieceVec;
-  for (int64_t piece = blockIdx.x; piece < num_halves * pieces_per_half; piece += gridDim.x) {
+  const int64_t pieces = num_halves * pieces_per_half;
+  for (int64_t i = blockIdx.x; i < pieces; i += gridDim.x) {
+    const int64_t piece = pieces - 1 - i;                // from the end: what a transform in front has written last is still in L2
     const int64_t half = piece / pieces_per_half;        // 2 g + h, in source order
     const int64_t v0 = (piece - half * pieces_per_half) * kSplitPieceVec + threadIdx.x;
     const uint4* s = src + half * half_vec;
