@@ -205,10 +205,10 @@ int mmoe_dispatch_place(const MmoeGeometry* geo, void* workspace, int32_t num_to
 int mmoe_experts(const MmoeGeometry* geo, void* workspace, const MmoeWeights* weights, const MmoeOptions* opt,
                  int32_t num_tokens, int32_t block_m, void* stream);
 /* The two halves of `mmoe_experts` that `mmoe_forward_ep` runs on either side of the join, exported for hosts that build
- * their own overlap (and so that the split can be checked on one GPU): `mmoe_plan_shared` plans the shared expert's
- * tiles from the token count alone (before any receive count is known); `mmoe_experts_select` runs both GEMMs over
+ * their own overlap (and so that the split can be checked on one GPU): `mmoe_plan_shared` writes the scale chunks of the
+ * shared expert's tiles, which depend on the token count alone (before any receive count is known); `mmoe_experts_select` runs both GEMMs over
  * `tile_select` = 0 every tile of the plan (= `mmoe_experts`), 1 the routed tiles only, 2 the shared expert's tiles
- * written by `mmoe_plan_shared`.  Selections 1 and 2 together leave exactly what selection 0 leaves.  Corresponds to
+ * (after `mmoe_plan_shared`).  Selections 1 and 2 together leave exactly what selection 0 leaves.  Corresponds to
  * the reference scheduling shared-expert blocks ahead of the routed ones (backend/kernel/scheduler.py:250-259). */
 int mmoe_plan_shared(const MmoeGeometry* geo, void* workspace, int32_t num_tokens, int32_t block_m, void* stream);
 int mmoe_experts_select(const MmoeGeometry* geo, void* workspace, const MmoeWeights* weights, const MmoeOptions* opt,
@@ -229,21 +229,21 @@ int mmoe_combine(const MmoeGeometry* geo, void* workspace, void* y_bf16, int32_t
  * one read and one write of [num_tokens, H].  NULL residual: plain combine. */
 int mmoe_combine_residual(const MmoeGeometry* geo, void* workspace, void* y_bf16, const void* residual_bf16,
                           int32_t num_tokens, void* stream);
-/* EP1 convenience: count, place, experts, combine.  Past the decode sizes (num_tokens > 128, with a shared expert) the
- * routed experts' ordering, plan and placement run on the library's second stream while the shared expert's GEMMs run
- * on `stream` (fork / join with events, capturable); same result as the separate calls.  Up to 128 tokens the call is
- * one stream and five or six launches: one block orders the routes, builds the plan and (up to 128 routes) places the
- * rows; the kernels are launched as a programmatic chain, so that each one's launch and set-up overlap its
- * predecessor (MMOE_DISABLE_CHAINED_LAUNCH=1 in the environment, read once per process: ordinary launches).
- * Threading: the second stream and its two events exist once per device; call mmoe_forward / mmoe_forward_ep for one
- * device from one host thread at a time. */
+/* EP1 convenience: count, place, experts, combine; same result as the separate calls.  One stream, one programmatic chain
+ * of launches, so that each one's launch and set-up overlap its predecessor (MMOE_DISABLE_CHAINED_LAUNCH=1 in the
+ * environment, read once per process: ordinary launches).  Up to 16 tokens (BLOCK_M 16) three launches: GEMM1 orders the
+ * routes itself and takes the staged tokens as they are.  Up to 128 tokens four: one launch orders the routes, builds
+ * the plan and places the rows in front of GEMM1, GEMM2 and combine.  Past that ordering and placement are two launches, and
+ * past 192 tokens each GEMM is two: the experts with many rows on CTA pairs, the others on the weights-as-A kernels.  The
+ * shared expert's tiles come first in GEMM1, which starts with them while the rows are still being placed. */
 int mmoe_forward(const MmoeGeometry* geo, void* workspace, const MmoeWeights* weights, const MmoeOptions* opt,
                  void* y_bf16, int32_t num_tokens, int32_t block_m, int32_t* stats, void* stream);
 
 /* EP>1 convenience, device-side transport: count, exchange, place, experts with the fused write-back, combine.  The
  * exchange of counts and rows runs on a second stream of the library (created by `mmoe_prepare`) while the shared
  * expert, which needs only this rank's own tokens, runs both of its GEMMs on `stream`; the two streams fork and join
- * with events, so the whole call can be captured in a CUDA graph.  Same result as the separate calls.  Corresponds to
+ * with events, so the whole call can be captured in a CUDA graph.  Same result as the separate calls.  The second stream
+ * and its two events exist once per device: make these calls for one device from one host thread at a time.  Corresponds to
  * the reference scheduling the shared expert into the dispatch gap (backend/kernel/scheduler.py:250-259). */
 int mmoe_forward_ep(const MmoeGeometry* geo, void* workspace, const void* const* peer_workspaces,
                     const MmoeWeights* weights, const MmoeOptions* opt, void* y_bf16, int32_t num_tokens, int32_t block_m,

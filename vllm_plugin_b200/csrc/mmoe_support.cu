@@ -17,7 +17,6 @@ namespace mmoe {
 // the attribute off for the whole process (every launch then waits for the full completion of its predecessor).
 // ---------------------------------------------------------------------------------------------------------------------
 namespace {
-thread_local bool g_break_chain = false;
 thread_local bool g_chain_scope = false;   // inside a ChainScope(true) of this thread
 bool chaining_enabled() {
   static const bool on = [] {
@@ -31,13 +30,7 @@ bool chaining_enabled() {
 ChainScope::ChainScope(bool on) : saved_(g_chain_scope) { g_chain_scope = on && chaining_enabled(); }
 ChainScope::~ChainScope() { g_chain_scope = saved_; }
 
-void break_chain() { g_break_chain = true; }
-
-bool take_chain_flag() {
-  const bool broken = g_break_chain;
-  g_break_chain = false;
-  return g_chain_scope && !broken;
-}
+bool chained() { return g_chain_scope; }
 
 // =====================================================================================================================
 // Kernel (a): BF16 -> MXFP8 E4M3 with one UE8M0 scale per 32 elements, four scale bytes per int32 word.

@@ -15,6 +15,7 @@
 //              issues 4 UMMAs per stage, committing the stage's shared memory back to the producer and the finished
 //              accumulator to the epilogue
 //   warps 2-5  epilogue: TMEM -> registers (thread = weight row, columns = tokens), fused math, global stores
+//   warp 7     layer 1: brings a stage's weight scales from stored into tensor-memory order ahead of the MMA warps
 //
 // Persistent CTAs (one per SM) walk a static task list (tile, 128-row weight block); TMEM accumulators are double
 // buffered so the epilogue of task i overlaps the loads and MMAs of task i+1.  Every wait is bounded: when the budget
@@ -23,8 +24,7 @@
 //
 // Expert parallelism: layer 2 has a second form (kFused) whose epilogue stores every BF16 row straight into the buffer
 // of the rank the token came from (plain peer stores over NVLink, no TMA from or to peer memory), and `tile_select`
-// restricts a launch to the routed tiles or to the shared expert's tiles planned ahead, so that the shared expert can
-// run while the dispatch is still in flight on another stream.
+// restricts a launch to the routed tiles or to the shared expert's, so that the shared expert can run while the dispatch is still in flight on another stream.
 #include <string.h>
 
 #include <mutex>
