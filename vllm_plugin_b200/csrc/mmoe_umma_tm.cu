@@ -31,7 +31,7 @@
 //              containers on the way into shared memory) and the two scale chunks; every copy signals the LEADER's barrier
 //              (.cta_group::2), and none uses cluster multicast
 //   warp 1     issuer (leader): scale copies into TMEM, UMMAs, one commit that frees the stage in both CTAs
-//   warps 2-5  epilogue (both CTAs)
+//   warps 2-9  epilogue (both CTAs; layer 2: warps 2-5)
 //
 // Copies and tensor-core instructions are issued by one elected lane of a warp that walks its loop in step (all lanes wait,
 // elect.sync around the issue): operands then stay in uniform registers.  From a lane that alone runs the loop a stage took
@@ -48,7 +48,11 @@ namespace mmoe {
 
 namespace {
 
-constexpr int kTmThreads = 192;
+// Epilogue warps.  Layer 1 has two per scheduler, each with half of the columns: one alone runs at the latency of its own
+// instructions, and with the IEEE sigmoid (fast_math off) that is longer than the 22 thousand clk of a task's UMMAs (2800
+// tokens, 48 experts: 1304 us with one, 1024 with two).  Layer 2 only converts and stores, and has no shared memory left for more staging blocks.
+__host__ __device__ constexpr int tm_epilogue_warps(int layer) { return layer == 1 ? 8 : 4; }
+constexpr int tm_threads(int layer) { return 64 + 32 * tm_epilogue_warps(layer); }
 constexpr int kTmN = 256;                          // weight rows of a task (UMMA N)
 constexpr int kTmRows = 128;                       // token rows of a tile (UMMA M per CTA)
 constexpr int kTmABytes = kTmRows * kTileK;        // 16 KB
@@ -205,7 +209,7 @@ __device__ __forceinline__ int tm_l1_group(const uint32_t (&v)[64], float wt, fl
 }
 
 template <int kLayer, bool kFused>
-__global__ void __launch_bounds__(kTmThreads, 1) tm_kernel(const __grid_constant__ TmParams p) {
+__global__ void __launch_bounds__(tm_threads(kLayer), 1) tm_kernel(const __grid_constant__ TmParams p) {
   static_assert(!kFused || kLayer == 2, "only GEMM2 writes rows back");
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
@@ -225,7 +229,7 @@ __global__ void __launch_bounds__(kTmThreads, 1) tm_kernel(const __grid_constant
       mbar_init(smem_u32(&ctl->empty[i]), 1);
     }
     for (int i = 0; i < 2; ++i) mbar_init(smem_u32(&ctl->tmem_full[i]), 1);
-    mbar_init(smem_u32(&ctl->overlap_free), 8);                   // one arrival per epilogue warp of the pair
+    mbar_init(smem_u32(&ctl->overlap_free), 2 * tm_epilogue_warps(kLayer));   // one arrival per epilogue warp of the pair
     ctl->abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -324,8 +328,8 @@ __global__ void __launch_bounds__(kTmThreads, 1) tm_kernel(const __grid_constant
         // M = 256 over the pair; idesc field [24,29) = M >> 4
         const uint32_t idesc0 = make_idesc(0u, shared ? 0u : 5u, static_cast<uint32_t>(kTmN), 0) + ((128u >> 4) << 24);
         const uint32_t d = tmem_base + (it & 1u) * kTmAccStride;
-        // The previous task's overlapped columns have been read.  The epilogue takes tasks in order, so this task's own
-        // columns, last used two tasks ago, are free as well.
+        // Every epilogue warp has read its first columns of the previous task, the overlapped ones among them.  They take
+        // tasks in order, so this task's own columns, last used two tasks ago, are free as well.
         if (it > 0 && !waiter.wait_uniform(smem_u32(&ctl->overlap_free), (it - 1u) & 1u)) { ok = false; break; }
         tc_fence_after();
         for (int kb = 0; kb < k_stages; ++kb) {
@@ -401,12 +405,13 @@ __global__ void __launch_bounds__(kTmThreads, 1) tm_kernel(const __grid_constant
       if (!waiter.wait_warp(smem_u32(&ctl->tmem_full[acc]), (it >> 1) & 1u)) { ok = false; break; }
       tc_fence_after();
       const uint32_t d0 = tmem_base + lane_sel + acc * kTmAccStride;
-      // the 64-column group with the 32 overlapped columns comes first: columns 224-255 of accumulator 0, 0-31 of 1
-      const int first = acc == 0 ? 3 : 0;
+      // the 64-column group with the 32 overlapped columns comes first: columns 224-255 of accumulator 0, 0-31 of 1; in layer 1
+      // warps 2-5 take groups 0 and 1, warps 6-9 groups 2 and 3
+      const int first = acc == 0 ? 3 : 0, side = (warp - 2) >> 2;
       uint32_t sf_word = 0;
 #pragma unroll 1
-      for (int step = 0; step < 4; ++step) {
-        const int g = (first + step) & 3;
+      for (int step = 0; step < 16 / tm_epilogue_warps(kLayer); ++step) {
+        const int g = kLayer == 1 ? 2 * side + ((first + step) & 1) : (first + step) & 3;
         uint32_t v[64];
         tc_ld32(d0 + 64 * g, v);
         tc_ld32(d0 + 64 * g + 32, v + 32);
@@ -419,7 +424,7 @@ __global__ void __launch_bounds__(kTmThreads, 1) tm_kernel(const __grid_constant
         if (kLayer == 1) {
           uint32_t w[8];
           const int sf_exp = p.fast_math != 0 ? tm_l1_group<true>(v, wt, p.clamp, w) : tm_l1_group<false>(v, wt, p.clamp, w);
-          sf_word |= static_cast<uint32_t>(sf_exp) << (8 * g);
+          sf_word |= static_cast<uint32_t>(sf_exp) << (8 * (g & 1));
           if (live) {
             uint4* dst = reinterpret_cast<uint4*>((shared ? p.act_shared : p.act_routed) + row * p.inter + nb * (kTmN / 2) + 32 * g);
             dst[0] = make_uint4(w[0], w[1], w[2], w[3]);
@@ -452,10 +457,10 @@ __global__ void __launch_bounds__(kTmThreads, 1) tm_kernel(const __grid_constant
         }
       }
       if (kLayer == 1 && live) {
-        // the task's 128 channels are one scale word of layer 2's K dimension
+        // the task's 128 channels are one scale word of layer 2's K dimension, half of it from each of the row's two threads
         int32_t* act_sf = shared ? p.act_sf_shared : p.act_sf_routed;
         const int64_t sf_rows = shared ? p.act_sf_rows_shared : p.act_sf_rows_routed;
-        act_sf[nb * sf_rows + (int64_t)tile.sf_chunk * kChunkRows + chunk_pos(i)] = static_cast<int32_t>(sf_word);
+        reinterpret_cast<uint16_t*>(act_sf + nb * sf_rows + (int64_t)tile.sf_chunk * kChunkRows + chunk_pos(i))[side] = static_cast<uint16_t>(sf_word);
       }
     }
   }
@@ -492,7 +497,7 @@ cudaError_t tm_prepare() {
 cudaError_t tm_launch(int layer, bool fused, const TmParams& p, cudaStream_t s) {
   const int grid = tc_num_sms() & ~1;
   if (grid <= 0) return cudaErrorNotReady;
-  const dim3 g(grid), b(kTmThreads);
+  const dim3 g(grid), b(tm_threads(layer));
   if (layer == 1) return launch_clustered(tm_kernel<1, false>, g, b, tm_smem_bytes(1), 2, s, p);
   return fused ? launch_clustered(tm_kernel<2, true>, g, b, tm_smem_bytes(2), 2, s, p)
                : launch_clustered(tm_kernel<2, false>, g, b, tm_smem_bytes(2), 2, s, p);
