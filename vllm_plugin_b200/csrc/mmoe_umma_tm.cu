@@ -404,6 +404,12 @@ __global__ void __launch_bounds__(tm_threads(kLayer), 1) tm_kernel(const __grid_
       }
       if (!waiter.wait_warp(smem_u32(&ctl->tmem_full[acc]), (it >> 1) & 1u)) { ok = false; break; }
       tc_fence_after();
+      // None of this warp's rows is a token: nothing to do (350 rows per expert, fast_math off: 1035 -> 913 us).
+      if (q * 32 >= tile.n_valid) {
+        tc_fence_before();
+        if (lane == 0) mbar_arrive_cluster(overlap_free_leader);
+        continue;
+      }
       const uint32_t d0 = tmem_base + lane_sel + acc * kTmAccStride;
       // the 64-column group with the 32 overlapped columns comes first: columns 224-255 of accumulator 0, 0-31 of 1; in layer 1
       // warps 2-5 take groups 0 and 1, warps 6-9 groups 2 and 3
