@@ -356,10 +356,10 @@ def test_shared_expert_ahead_of_the_routed_plan(m, bm):
 
 
 @pytest.mark.parametrize("m,rows", [(193, (193, 192, 1)), (260, (257, 256, 129, 81, 112)), (300, (300, 160, 161, 113, 80)),
-                                    (700, (700, 513, 512, 385, 225, 16)), (129, (129, 100, 17))])
+                                    (700, (700, 513, 512, 385, 225, 16)), (400, (337, 336, 258, 305, 400)), (129, (129, 100, 17))])
 def test_tile_cuts_at_their_edges(m, rows):
     """Experts with exactly the row counts at which the cut changes: one, two and three tiles of the weights-as-A kernels (80 /
-    112 rows each), the first pair, full and just overfull pairs, and a token that names one expert twice.  The single-GPU
+    112 rows each), the first pair, full and just overfull pairs, the rows past one pair that go back to three tiles, and a token that names one expert twice.  The single-GPU
     forward (routes counted, planned and placed in two launches) against the oracle, and bit for bit against the general
     sequence over receive counts."""
     import ctypes

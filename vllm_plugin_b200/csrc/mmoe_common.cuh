@@ -19,21 +19,28 @@ constexpr int kTileRows = 128;     // weight rows per tile (UMMA M)
 constexpr int kChunkRows = 128;    // token rows per scale-factor chunk (one 512-byte tcgen05.cp source per K stage)
 constexpr int kSmallTileRows = 112;      // largest token tile of the weights-as-A kernels (UMMA N): four accumulators of 112 TMEM columns
 constexpr int kPairTileRows = 128;       // largest token tile of the tokens-as-A kernels (half of a CTA pair's 256 rows)
-// Which kernels run an expert depends on the rows it received in this call (see pair_above_default in mmoe_abi.cu).
 constexpr int kNeverPair = 0x7fffffff;
 
 // Rows of a weights-as-A tile: five stages of up to 80 rows fit the shared memory, four of 112.
 constexpr int kDeepTileRows = 80;
 
-// How the n rows of an expert are cut into tiles.  Up to `pair_above` rows: ceil(n / small_cap) equal tiles (rounded up to 16
-// rows) for the weights-as-A kernels.  Above: an even number of tiles of at most 128 rows, the two halves of CTA-pair tasks;
-// the second half of a single pair is empty when everything fits the first.  Cuts ignore the BLOCK_M boundaries of the pool.
+// Which kernels run a routed expert depends on the rows it received in this call: above `pair_above` (see kPairAbove) the CTA
+// pairs, except where they would start a second task for at most 80 rows.  A pair task takes 2 x 562 clk of SM time per stage
+// however few its rows, three weights-as-A tiles of up to 112 rows take about 1450 together: 270 rows per expert (48 experts)
+// 791 -> 683 us, 330 rows 873 -> 768, 281 rows (16 experts) 325 -> 302; at 400 rows four tiles lose (930 -> 957).
+__host__ __device__ inline bool on_pairs(int n, int pair_above) {
+  return n > pair_above && (pair_above == 0 || n <= 2 * kPairTileRows || n > 3 * kSmallTileRows);
+}
+
+// How the n rows of an expert are cut into tiles.  Weights-as-A kernels: ceil(n / small_cap) equal tiles (rounded up to 16
+// rows).  Pairs: an even number of tiles of at most 128 rows, the two halves of CTA-pair tasks; the second half
+// of a single pair is empty when everything fits the first.  Cuts ignore the BLOCK_M boundaries of the pool.
 struct Cut {
   int32_t parts, step;
 };
-__host__ __device__ inline Cut cut_rows(int n, int pair_above, int small_cap) {
+__host__ __device__ inline Cut cut_rows(int n, bool pairs, int small_cap) {
   if (n <= 0) return Cut{0, 16};
-  if (n > pair_above) {
+  if (pairs) {
     if (n <= kPairTileRows) return Cut{2, kPairTileRows};
     const int parts = 2 * ((n + 2 * kPairTileRows - 1) / (2 * kPairTileRows));
     return Cut{parts, ((n + parts - 1) / parts + 15) & ~15};
@@ -42,7 +49,7 @@ __host__ __device__ inline Cut cut_rows(int n, int pair_above, int small_cap) {
   return Cut{parts, ((n + parts - 1) / parts + 15) & ~15};
 }
 // The cut of the shared expert's m tokens: known to the host, so that its tiles need no plan.
-__host__ __device__ inline Cut shared_cut(int m, int pair_above) { return cut_rows(m, pair_above, kDeepTileRows); }
+__host__ __device__ inline Cut shared_cut(int m, int pair_above) { return cut_rows(m, m > pair_above, kDeepTileRows); }
 // GEMM1 of a call of at most this many tokens on one GPU multiplies every expert that is hit with all staged tokens and orders
 // the routes itself (an UMMA takes 16 token columns at least).
 constexpr int kStagedTokens = 16;
