@@ -1,0 +1,35 @@
+// Prints what the host-side rules of a call decide (csrc/mmoe_common.cuh), for the CPU tests.  Host code only.
+#include <stdio.h>
+#include <string.h>
+
+#include "../vllm_plugin_b200/csrc/mmoe_common.cuh"
+
+using namespace mmoe;
+
+static const int kBlockMs[] = {16, 32, 64, 128, 192, 240};
+
+// forms <ranks> <pair_above> <tile_select> <peers> <block_m> <m> <pairs> <small> <staged>
+static void forms() {
+  for (int ranks : {1, 2, 8})
+    for (int pair_above : {192, kNeverPair, 0})
+      for (int select : {0, 1, 2})
+        for (int peers : {0, 1})
+          for (int block_m : kBlockMs)
+            for (int m : {0, 1, 7, 15, 16, 17, 64, 128, 129, 192, 193, 1000, 3840}) {
+              static const void* peer[8] = {};
+              Ctx c{};
+              c.geo = MmoeGeometry{ranks, 0, 384, 6, 5120, 2304, 1, 3840};
+              c.pair_above = pair_above;
+              c.tile_select = select;
+              c.peer_ws = peers ? peer : nullptr;
+              const GemmForms f = gemm_forms(c, m, select != 1 && m > 0);
+              printf("forms %d %d %d %d %d %d %d %d %d\n", ranks, pair_above, select, peers, block_m, m, f.pairs, f.small,
+                     staged_tokens(c, m, block_m));
+            }
+}
+
+int main(int argc, char** argv) {
+  for (int i = 1; i < argc; ++i)
+    if (strcmp(argv[i], "forms") == 0) forms();
+  return 0;
+}

@@ -1,0 +1,41 @@
+"""The host-side rules that choose how a call is run (``csrc/mmoe_common.cuh``), compiled for the host and checked over
+everything they accept.  No GPU involved."""
+
+import os
+import shutil
+import subprocess
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+NEVER = 0x7fffffff
+
+
+@pytest.fixture(scope="module")
+def rules(tmp_path_factory):
+    """``rules("forms")`` -> the table's rows as tuples of integers."""
+    nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
+    if not os.path.exists(nvcc):
+        pytest.skip("nvcc is not installed")
+    exe = str(tmp_path_factory.mktemp("rules") / "dispatch_rules")
+    subprocess.run([nvcc, "-std=c++17", "-Wno-deprecated-gpu-targets", "-o", exe, os.path.join(ROOT, "tests", "dispatch_rules.cpp")],
+                   check=True, capture_output=True)
+
+    def table(name):
+        text = subprocess.run([exe, name], check=True, capture_output=True, text=True).stdout
+        rows = [tuple(int(v) for v in line.split()[1:]) for line in text.splitlines()]
+        assert rows
+        return rows
+
+    return table
+
+
+def test_staged_tokens_replace_placed_rows_on_one_gpu_only(rules):
+    """GEMM1 may multiply this rank's staged tokens only where every row is one of them: one rank, the routed tiles in the
+    launch, no expert on the pair kernels, at most 16 tokens in pool blocks of 16."""
+    for ranks, pair_above, select, peers, block_m, m, pairs, small, staged in rules("forms"):
+        case = (ranks, pair_above, select, peers, block_m, m)
+        want = ranks == 1 and select != 2 and pair_above != 0 and 1 <= m <= 16 and block_m == 16
+        assert staged == want, case
+        if staged:
+            assert small and not pairs, case

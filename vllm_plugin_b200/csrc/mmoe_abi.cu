@@ -542,8 +542,8 @@ int mmoe_forward(const MmoeGeometry* geo, void* workspace, const MmoeWeights* we
   // route ordering, plan and placement: inside the GEMM launches up to kStagedTokens tokens, one launch up to 128, two beyond
   // (and where the pair kernels are forced on: those read the shared expert's scales from chunks that the larger form writes)
   const bool small_only = num_tokens > 0 && c.pair_above_for(num_tokens) == mmoe::kNeverPair;
-  const bool in_gemm = small_only && num_tokens <= mmoe::kStagedTokens && block_m <= mmoe::kStagedTokens && opt != nullptr &&
-                       opt->engine == 0 && (opt->layer_mask == 0 || opt->layer_mask == 3);
+  const bool in_gemm = mmoe::staged_tokens(c, num_tokens, block_m) && opt != nullptr && opt->engine == 0 &&
+                       (opt->layer_mask == 0 || opt->layer_mask == 3);
   if (!in_gemm) {
     const cudaError_t e = small_only && num_tokens <= 128 ? mmoe::launch_route_small(c, num_tokens, block_m, stats, st)
                                                           : mmoe::launch_route_large(c, num_tokens, block_m, stats, st);

@@ -51,7 +51,7 @@ __host__ __device__ inline Cut cut_rows(int n, bool pairs, int small_cap) {
 // The cut of the shared expert's m tokens: known to the host, so that its tiles need no plan.
 __host__ __device__ inline Cut shared_cut(int m, int pair_above) { return cut_rows(m, m > pair_above, kDeepTileRows); }
 // GEMM1 of a call of at most this many tokens on one GPU multiplies every expert that is hit with all staged tokens and orders
-// the routes itself (an UMMA takes 16 token columns at least).
+// the routes itself (an UMMA takes 16 token columns at least); see staged_tokens().
 constexpr int kStagedTokens = 16;
 // Cap of a call without pair tiles (also known to the host: the largest tile of such a call fixes its stage layout): no expert
 // has more rows than there are tokens unless a token names it twice, which then costs another tile.
@@ -238,7 +238,25 @@ struct Ctx {             // resolved pointers of one call
   // and the call needs no pair launch
   int pair_above_for(int m) const { return geo.num_ranks == 1 && m <= pair_above ? kNeverPair : pair_above; }
   template <typename T> T* at(int64_t off) const { return reinterpret_cast<T*>(ws + off); }
+  bool fused() const { return peer_ws != nullptr && geo.num_ranks > 1 && tile_select != 2; }
 };
+
+// The GEMM launches of a call of m tokens: on CTA pairs, on the weights-as-A kernels, or both in this order.
+struct GemmForms {
+  bool pairs, small;
+};
+inline GemmForms gemm_forms(const Ctx& c, int m, bool with_shared) {
+  const int pair_above = c.pair_above_for(m);
+  if (c.tile_select == 2) return GemmForms{with_shared && m > pair_above, with_shared && m <= pair_above};
+  return GemmForms{pair_above != kNeverPair, pair_above > 0};
+}
+
+// Whether GEMM1 of such a call takes the staged tokens as they are instead of the rows of the pool.  With more than one rank the
+// rows come from other ranks and the route table names experts of all of them: only one GPU's call may.
+inline bool staged_tokens(const Ctx& c, int m, int block_m) {
+  return c.geo.num_ranks == 1 && c.tile_select != 2 && c.pair_above_for(m) == kNeverPair && m > 0 && m <= kStagedTokens &&
+         block_m <= kStagedTokens;
+}
 
 
 // ---------------------------------------------------------------------------------------------------------------------

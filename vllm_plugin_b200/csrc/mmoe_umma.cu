@@ -1277,7 +1277,7 @@ cudaError_t launch_experts_umma(const Ctx& c, const MmoeWeights& w, const MmoeOp
   const int64_t timeout_ns = (o.timeout_ms > 0 ? (int64_t)o.timeout_ms : 2000) * 1000000ll;
   const PlanEntry* plan = cached_plan(c, w, has_shared);
   if (plan == nullptr) return cudaErrorInvalidValue;
-  const bool fused = c.peer_ws != nullptr && c.geo.num_ranks > 1 && c.tile_select != 2;
+  const bool fused = c.fused();
   const int mask = o.layer_mask == 0 ? 3 : o.layer_mask;
   cudaError_t e = cudaSuccess;
 
@@ -1301,9 +1301,8 @@ cudaError_t launch_experts_umma(const Ctx& c, const MmoeWeights& w, const MmoeOp
   const Cut cut = shared_cut(with_shared ? m : 0, pair_above);
   const SharedTiles shared{cut.parts, cut.step, m}, none{0, 16, 0};
   const bool shared_pairs = m > pair_above;
-  const bool pairs = c.tile_select == 2 ? with_shared && shared_pairs : pair_above != kNeverPair;
-  const bool small = c.tile_select == 2 ? with_shared && !shared_pairs : pair_above > 0;
-  const bool staged = !pairs && !fused && c.tile_select != 2 && m > 0 && m <= kStagedTokens && block_m <= kStagedTokens;
+  const auto [pairs, small] = gemm_forms(c, m, with_shared);
+  const bool staged = staged_tokens(c, m, block_m);
   for (int layer = 1; layer <= 2; ++layer) {
     if ((mask & layer) == 0) continue;
     if (e == cudaSuccess && pairs) {
