@@ -319,6 +319,44 @@ def test_cuda_graph_replay_of_every_variant():
         assert_parity(y, H.oracle_layer(layer, hid_b, ids, w), f"graph replay m={m}")
 
 
+@pytest.mark.parametrize("m", [1, 16, 17, 200])
+def test_calls_in_flight_together_on_two_streams(m):
+    """Two buffers, two streams, and a third stream whose matrix products take SMs away from both: the CTAs of a call may start
+    one by one, and every call leaves bit for bit what it leaves alone."""
+    from vllm_plugin_b200 import api
+    layer = H.make_layer(512, 256, 32, 6, True, seed=41)
+    weights = H.kernel_weights(layer, "cuda")
+    lanes = []
+    for lane in range(2):
+        hid = O.make_hidden(m, layer.hidden, 50 + lane)
+        ids, w = O.make_routing(m, 32, 6, 60 + lane, zipf_s=1.2, mask_frac=0.05)
+        want, buf = H.run_layer(layer, hid, ids, w, weights=weights)
+        x, ids, w = hid.cuda(), ids.cuda(), w.cuda()
+        ys = [torch.empty_like(want) for _ in range(20)]
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            for y in ys:
+                api.stage_inputs_for_mega_moe(buf, x, ids, w)
+                api.fp8_fp4_mega_moe(y, weights[0], weights[1], buf, weights[2], weights[3], activation_clamp=10.0)
+        lanes.append((graph, torch.cuda.Stream(), ys, want, buf, (x, ids, w)))
+    a = torch.randn(2048, 2048, device="cuda", dtype=torch.bfloat16)
+    other = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    for _ in range(5):
+        with torch.cuda.stream(other):
+            for _ in range(20):
+                a @ a
+        for graph, stream, *_ in lanes:
+            with torch.cuda.stream(stream):
+                graph.replay()
+    torch.cuda.synchronize()
+    for _, _, ys, want, buf, _ in lanes:
+        api.read_status(buf)
+        for i, y in enumerate(ys):
+            assert torch.equal(y, want), i
+
+
 @pytest.mark.parametrize("m,bm", [(7, 16), (130, 32), (300, 128), (300, 192)])
 def test_shared_expert_ahead_of_the_routed_plan(m, bm):
     """The split the expert-parallel forward uses, on one GPU: shared expert planned and run first (both GEMMs), routed

@@ -90,7 +90,8 @@ struct PlanHeader {
   int32_t small_rows;          // rows of the largest one, rounded up to 16
   int32_t ticket;              // blocks of the route-counting launch that have finished; zero between launches
   int32_t routed;              // 1 while a GEMM1 launch that orders the routes itself has the plan complete; GEMM2 clears it
-  int32_t pad[5];
+  uint32_t claims;             // CTAs of that GEMM1 launch that have asked to do it, modulo its grid: zero between launches
+  int32_t pad[4];
 };
 static_assert(sizeof(PlanHeader) == 64, "plan header is 64 bytes");
 

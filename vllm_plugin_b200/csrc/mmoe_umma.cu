@@ -112,6 +112,7 @@ struct Control {          // lives at the start of shared memory
   uint32_t tmem_base;
   volatile int32_t abort_flag;
   uint32_t hit[16];       // layer 1 with staged tokens: bit e = some token is routed to expert e
+  uint32_t routes_here;   // ... and this CTA orders the routes
   // layer 2 with the write-back fused in: where output rows go.  slot s < 32: `ret_recv` of source rank s, slot 32: the
   // shared expert's (local) output
   __nv_bfloat16* out_base[33];
@@ -255,8 +256,9 @@ struct TaskWalk {
 };
 
 // ------------------------------------------------------------------------------------------------ routing in the launch
-// Calls of at most kStagedTokens tokens: the last CTA's epilogue warps, idle until its first accumulator 15 us later, order the
-// routes and build the plan, which only epilogues and GEMM2 need.  A launch of its own took 8-20 us in front of GEMM1: little
+// Calls of at most kStagedTokens tokens: the epilogue warps of the first CTA to ask, idle until its first accumulator 15 us
+// later, order the routes and build the plan, which only epilogues and GEMM2 need.  All other CTAs wait for that one, so it has
+// to be one that runs: a CTA takes an SM to itself, and work on other streams may hold any of them back for as long as it likes.  A launch of its own took 8-20 us in front of GEMM1: little
 // work, but every instruction line comes from DRAM (each call streams its weights through the L2), so what counts is that
 // the code is short.  Pool blocks and tiles have 16 rows here, hence one tile per block.
 constexpr int kRouteThreads = 128;
@@ -271,6 +273,16 @@ static_assert(6 * (Shape<1>::kABytes + kStagedTokens * kTileK + Shape<1>::kSfByt
                   Shape<1>::kRingBytes / (Shape<1>::kABytes + kStagedTokens * kTileK + Shape<1>::kSfBytes) == 6,
               "the scratch lives behind the six stages of a 16-row ring");
 __device__ __forceinline__ void route_barrier() { asm volatile("bar.sync 1, %0;" ::"n"(kRouteThreads) : "memory"); }
+
+// whether this CTA is the first of its launch to ask; all epilogue threads of every CTA, once
+__device__ __forceinline__ bool sa_claim_route(const UmmaParams& p, Control* ctl, int t) {
+  if (t == 0) {
+    uint32_t* claims = &plan_view(const_cast<char*>(p.plan), p.e_local, p.num_ranks).hdr->claims;
+    ctl->routes_here = atomicInc(claims, gridDim.x - 1) == 0 ? 1u : 0u;
+  }
+  route_barrier();
+  return ctl->routes_here != 0;
+}
 
 __device__ __noinline__ void sa_route(const UmmaParams& p, RouteScratch& s, int t) {
   const int E = p.e_local, n = p.num_routes, lane = t & 31;
@@ -933,8 +945,9 @@ __global__ void __launch_bounds__(kThreads, 1) umma_kernel(const __grid_constant
     if constexpr (kLayer == 1) sa_arrange_scales<L, kStaged>(p, c, walk, waiter, st);
     else if (kStaged && p.route_here) sa_place(p);
   } else {
-    if (kStaged && kLayer == 1 && p.route_here && blockIdx.x == gridDim.x - 1)
-      sa_route(p, *reinterpret_cast<RouteScratch*>(c.sf_base + c.num_stages * L::kSfBytes), static_cast<int>(threadIdx.x) - 64);
+    const int t = static_cast<int>(threadIdx.x) - 64;
+    if (kStaged && kLayer == 1 && p.route_here && sa_claim_route(p, ctl, t))
+      sa_route(p, *reinterpret_cast<RouteScratch*>(c.sf_base + c.num_stages * L::kSfBytes), t);
     sa_epilogue<kLayer, L, kFused, kStaged>(p, c, walk, waiter, st);
   }
   chain_wait();       // a CTA that has not waited yet must not end before what precedes the launch
