@@ -3,6 +3,7 @@
 #include <string.h>
 
 #include "../vllm_plugin_b200/csrc/mmoe_common.cuh"
+#include "../vllm_plugin_b200/csrc/mmoe_plan_cache.h"
 
 using namespace mmoe;
 
@@ -28,8 +29,36 @@ static void forms() {
             }
 }
 
+// cache <keys in turn> <rounds> <built> <built from a sibling> <wrong values>, with 4 workspaces and room for 16
+static void cache() {
+  struct Key {
+    int ws, layer;
+    bool operator==(const Key& o) const { return ws == o.ws && layer == o.layer; }
+    bool same_workspace(const Key& o) const { return ws == o.ws; }
+  };
+  for (int keys : {1, 3, 15, 16, 17, 40}) {
+    PlanCache<Key, int, 16> plans;
+    int built = 0, siblings = 0, wrong = 0;
+    const Key first{0, 0};
+    const std::shared_ptr<const int> held = plans.get(first, [&](const int*) { ++built; return std::make_shared<int>(0); });
+    for (int round = 0; round < 3; ++round)
+      for (int i = 0; i < keys; ++i) {
+        const Key key{i % 4, i};
+        plans.get(Key{9, 9}, [](const int*) { return std::shared_ptr<int>(); });     // fails: not kept
+        const auto v = plans.get(key, [&](const int* sibling) {
+          ++built;
+          if (sibling != nullptr) siblings += *sibling % 4 == key.ws ? 1 : 1000;
+          return std::make_shared<int>(i);
+        });
+        wrong += v == nullptr || *v != i;
+      }
+    printf("cache %d 3 %d %d %d\n", keys, built, siblings, wrong + (*held != 0));
+  }
+}
+
 int main(int argc, char** argv) {
   for (int i = 1; i < argc; ++i)
     if (strcmp(argv[i], "forms") == 0) forms();
+    else if (strcmp(argv[i], "cache") == 0) cache();
   return 0;
 }

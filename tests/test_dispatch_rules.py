@@ -39,3 +39,12 @@ def test_staged_tokens_replace_placed_rows_on_one_gpu_only(rules):
         assert staged == want, case
         if staged:
             assert small and not pairs, case
+
+
+def test_launch_parameters_are_kept_for_every_layer_of_a_model(rules):
+    """Keys that take turns are built once as long as they fit, from the parameters of a key with the same workspace where
+    there is one; a value that was handed out stays valid when its entry is replaced."""
+    for keys, rounds, built, siblings, wrong in rules("cache"):
+        assert wrong == 0
+        assert built == (keys if keys <= 16 else rounds * keys), keys
+        assert siblings == built - min(keys, 4), keys

@@ -25,7 +25,7 @@ def needs_build() -> bool:
     out = lib_path()
     if not os.path.exists(out):
         return True
-    newest = max(os.path.getmtime(os.path.join(HERE, f)) for f in os.listdir(HERE) if f.endswith((".cu", ".cuh")))
+    newest = max(os.path.getmtime(os.path.join(HERE, f)) for f in os.listdir(HERE) if f.endswith((".cu", ".cuh", ".h")))
     header = os.path.join(os.path.dirname(os.path.dirname(HERE)), "include", "mmoe.h")
     return max(newest, os.path.getmtime(header)) > os.path.getmtime(out)
 

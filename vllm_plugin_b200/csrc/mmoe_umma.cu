@@ -27,9 +27,10 @@
 // restricts a launch to the routed tiles or to the shared expert's, so that the shared expert can run while the dispatch is still in flight on another stream.
 #include <string.h>
 
-#include <mutex>
+#include <memory>
 #include <type_traits>
 
+#include "mmoe_plan_cache.h"
 #include "mmoe_tc.cuh"
 
 namespace mmoe {
@@ -1005,11 +1006,13 @@ cudaError_t launch_layer(UmmaParams& p, cudaStream_t s) {
 }
 
 // ---------------------------------------------------------------------------------------------------------------
-// Launch parameters that depend only on (workspace, weights, geometry) -- above all the encoded tensor
-// maps -- are built once and kept: a serving engine calls the layer with the same buffers thousands of times, and
-// encoding two dozen tensor maps per call costs more host time than the launches themselves.  What changes per call
-// (tile selection, options, peers) is patched into a copy.  The reference keeps the same kind of record per validated
-// call (backend/frontend.py:650-754).
+// Launch parameters that depend only on (workspace, weights, geometry) -- above all the encoded tensor maps, 32 for the
+// weights-as-A kernels and 28 for the pairs -- are built once and kept: a serving engine calls its layers with the same buffers
+// thousands of times.  What changes per call (tile selection, options, peers) is patched into a copy.  The reference keeps the
+// same kind of record per validated call (backend/frontend.py:650-754).
+//
+// A model's layers share one workspace: the parameters of a second layer begin as a copy of the first one's and only the 4 (8)
+// maps of its weights are encoded.  Each kernel family is built when a call first launches it.  256 layers fit (2.6 MB).
 // ---------------------------------------------------------------------------------------------------------------
 struct PlanKey {
   const void* ws;
@@ -1019,17 +1022,15 @@ struct PlanKey {
   int has_shared;
   int device;
   bool operator==(const PlanKey& o) const { return memcmp(this, &o, sizeof(PlanKey)) == 0; }
+  bool same_workspace(const PlanKey& o) const {
+    return ws == o.ws && has_shared == o.has_shared && device == o.device && memcmp(&geo, &o.geo, sizeof geo) == 0;
+  }
 };
-struct PlanEntry {
-  PlanKey key;
-  uint64_t stamp = 0;          // 0 = empty
-  UmmaParams sa[2];
-  TmParams tm[2];
-};
-constexpr int kPlanCacheSize = 16;
-PlanEntry g_plans[kPlanCacheSize];
-uint64_t g_plan_clock = 0;
-std::mutex g_plan_mutex;
+constexpr int kPlanCacheSize = 256;
+struct SaPlan { UmmaParams layer[2]; };
+struct TmPlan { TmParams layer[2]; };
+PlanCache<PlanKey, SaPlan, kPlanCacheSize> g_sa_plans;
+PlanCache<PlanKey, TmPlan, kPlanCacheSize> g_tm_plans;
 
 PlanKey make_key(const Ctx& c, const MmoeWeights& w, bool has_shared) {
   PlanKey k;
@@ -1045,25 +1046,12 @@ PlanKey make_key(const Ctx& c, const MmoeWeights& w, bool has_shared) {
   return k;
 }
 
-// tokens-as-A form: both layers through mmoe_umma_tm.cu
-bool build_tm(const Ctx& c, const MmoeWeights& w, bool has_shared, TmParams* out) {
+// Pair kernels: what depends on the workspace alone ...
+bool set_workspace(const Ctx& c, bool has_shared, TmPlan* plan) {
   const int h = c.geo.hidden, inter = c.geo.intermediate, el = c.e_local;
   const int64_t shared_sf_rows = shared_chunk_rows(c.geo.num_max_tokens);
-  TmParams p1{};
-  int bad = 0;
-  bad |= make_weight_map(&p1.map_w_routed, true, w.w13, h, (uint64_t)el * 2 * inter, w.w13_slice_stride, kTileRows);
-  bad |= make_scale_map(&p1.map_wsf_routed, w.w13_sf, 2 * (uint64_t)inter, (uint64_t)el * (h / kTileK), 256);
-  bad |= make_scale_map(&p1.map_tsf_routed, c.ws + c.lay.pool_sf, c.lay.pool_sf_rows, h / kTileK, kChunkRows);
-  for (int b = 0; b < 4; ++b)
-    bad |= make_token_map(&p1.map_tok_routed[b], c.ws + c.lay.pool_x, h, c.lay.pool_rows, 32 * (b + 1));
-  if (has_shared) {
-    bad |= make_weight_map(&p1.map_w_shared, false, w.shared_w13, h, 2 * (uint64_t)inter, 0, kTileRows);
-    bad |= make_scale_map(&p1.map_wsf_shared, w.shared_w13_sf, 2 * (uint64_t)inter, h / kTileK, 256);
-    bad |= make_scale_map(&p1.map_tsf_shared, c.ws + c.lay.shared_tile_sf, shared_sf_rows, h / kTileK, kChunkRows);
-    for (int b = 0; b < 4; ++b)
-      bad |= make_token_map(&p1.map_tok_shared[b], c.ws + c.lay.x, h, c.geo.num_max_tokens, 32 * (b + 1));
-  }
-  if (bad) return false;
+  TmParams& p1 = plan->layer[0];
+  TmParams& p2 = plan->layer[1];
   p1.plan = c.ws + c.lay.plan;
   p1.act_routed = c.at<uint8_t>(c.lay.act_x);
   p1.act_shared = c.at<uint8_t>(c.lay.shared_act_x);
@@ -1077,50 +1065,56 @@ bool build_tm(const Ctx& c, const MmoeWeights& w, bool has_shared, TmParams* out
   p1.num_ranks = c.geo.num_ranks;
   p1.k_dim = h;
   p1.rows_per_expert = 2 * inter;
-  p1.routed_sliced = w.w13_slice_stride > 0 ? 1 : 0;
   p1.hidden = h;
   p1.inter = inter;
-
-  TmParams p2 = p1;
-  bad |= make_weight_map(&p2.map_w_routed, true, w.w2, inter, (uint64_t)el * h, w.w2_slice_stride, kTileRows);
-  bad |= make_scale_map(&p2.map_wsf_routed, w.w2_sf, h, (uint64_t)el * (inter / kTileK), 256);
-  bad |= make_scale_map(&p2.map_tsf_routed, c.ws + c.lay.act_sf, c.lay.pool_sf_rows, inter / kTileK, kChunkRows);
-  for (int b = 0; b < 4; ++b)
-    bad |= make_token_map(&p2.map_tok_routed[b], c.ws + c.lay.act_x, inter, c.lay.pool_rows, 32 * (b + 1));
-  if (has_shared) {
-    bad |= make_weight_map(&p2.map_w_shared, false, w.shared_w2, inter, (uint64_t)h, 0, kTileRows);
-    bad |= make_scale_map(&p2.map_wsf_shared, w.shared_w2_sf, h, inter / kTileK, 256);
-    bad |= make_scale_map(&p2.map_tsf_shared, c.ws + c.lay.shared_act_sf, c.lay.shared_sf_rows, inter / kTileK, kChunkRows);
-    for (int b = 0; b < 4; ++b)
-      bad |= make_token_map(&p2.map_tok_shared[b], c.ws + c.lay.shared_act_x, inter, c.geo.num_max_tokens + 128, 32 * (b + 1));
-  }
-  if (bad) return false;
+  p2 = p1;
   p2.ret = c.at<__nv_bfloat16>(c.lay.ret);
   p2.shared_out = c.at<__nv_bfloat16>(c.lay.shared_out);
   p2.pool_dst = c.at<int32_t>(c.lay.pool_dst);
   p2.k_dim = inter;
   p2.rows_per_expert = h;
+  int bad = make_scale_map(&p1.map_tsf_routed, c.ws + c.lay.pool_sf, c.lay.pool_sf_rows, h / kTileK, kChunkRows);
+  bad |= make_scale_map(&p2.map_tsf_routed, c.ws + c.lay.act_sf, c.lay.pool_sf_rows, inter / kTileK, kChunkRows);
+  for (int b = 0; b < 4; ++b) {
+    bad |= make_token_map(&p1.map_tok_routed[b], c.ws + c.lay.pool_x, h, c.lay.pool_rows, 32 * (b + 1));
+    bad |= make_token_map(&p2.map_tok_routed[b], c.ws + c.lay.act_x, inter, c.lay.pool_rows, 32 * (b + 1));
+  }
+  if (has_shared) {
+    bad |= make_scale_map(&p1.map_tsf_shared, c.ws + c.lay.shared_tile_sf, shared_sf_rows, h / kTileK, kChunkRows);
+    bad |= make_scale_map(&p2.map_tsf_shared, c.ws + c.lay.shared_act_sf, c.lay.shared_sf_rows, inter / kTileK, kChunkRows);
+    for (int b = 0; b < 4; ++b) {
+      bad |= make_token_map(&p1.map_tok_shared[b], c.ws + c.lay.x, h, c.geo.num_max_tokens, 32 * (b + 1));
+      bad |= make_token_map(&p2.map_tok_shared[b], c.ws + c.lay.shared_act_x, inter, c.geo.num_max_tokens + 128, 32 * (b + 1));
+    }
+  }
+  return bad == 0;
+}
+// ... and what depends on the weights
+bool set_weights(const Ctx& c, const MmoeWeights& w, bool has_shared, TmPlan* plan) {
+  const int h = c.geo.hidden, inter = c.geo.intermediate, el = c.e_local;
+  TmParams& p1 = plan->layer[0];
+  TmParams& p2 = plan->layer[1];
+  p1.routed_sliced = w.w13_slice_stride > 0 ? 1 : 0;
   p2.routed_sliced = w.w2_slice_stride > 0 ? 1 : 0;
-  out[0] = p1;
-  out[1] = p2;
-  return true;
+  int bad = make_weight_map(&p1.map_w_routed, true, w.w13, h, (uint64_t)el * 2 * inter, w.w13_slice_stride, kTileRows);
+  bad |= make_scale_map(&p1.map_wsf_routed, w.w13_sf, 2 * (uint64_t)inter, (uint64_t)el * (h / kTileK), 256);
+  bad |= make_weight_map(&p2.map_w_routed, true, w.w2, inter, (uint64_t)el * h, w.w2_slice_stride, kTileRows);
+  bad |= make_scale_map(&p2.map_wsf_routed, w.w2_sf, h, (uint64_t)el * (inter / kTileK), 256);
+  if (has_shared) {
+    bad |= make_weight_map(&p1.map_w_shared, false, w.shared_w13, h, 2 * (uint64_t)inter, 0, kTileRows);
+    bad |= make_scale_map(&p1.map_wsf_shared, w.shared_w13_sf, 2 * (uint64_t)inter, h / kTileK, 256);
+    bad |= make_weight_map(&p2.map_w_shared, false, w.shared_w2, inter, (uint64_t)h, 0, kTileRows);
+    bad |= make_scale_map(&p2.map_wsf_shared, w.shared_w2_sf, h, inter / kTileK, 256);
+  }
+  return bad == 0;
 }
 
-bool build_sa(const Ctx& c, const MmoeWeights& w, bool has_shared, UmmaParams* out) {
+// The same two steps for the weights-as-A kernels.
+bool set_workspace(const Ctx& c, bool has_shared, SaPlan* plan) {
   const int h = c.geo.hidden, inter = c.geo.intermediate, el = c.e_local;
-  UmmaParams p1{};
-  int bad = 0;
-  bad |= make_w13_map(&p1.map_w_routed, true, w.w13, h, (uint64_t)el * 2 * inter, w.w13_slice_stride);
-  if (has_shared) bad |= make_w13_map(&p1.map_w_shared, false, w.shared_w13, h, 2 * (uint64_t)inter, 0);
-  else p1.map_w_shared = p1.map_w_routed;
-  for (int b = 0; b < kNumBoxes; ++b) {
-    bad |= make_token_map(&p1.map_tok_routed_box[b], c.ws + c.lay.pool_x, h, c.lay.pool_rows, 16 * (b + 1));
-    bad |= make_token_map(&p1.map_tok_shared_box[b], c.ws + c.lay.x, h, c.geo.num_max_tokens, 16 * (b + 1));
-  }
-  if (bad) return false;
+  UmmaParams& p1 = plan->layer[0];
+  UmmaParams& p2 = plan->layer[1];
   p1.plan = c.ws + c.lay.plan;
-  p1.wsf_routed = static_cast<const int32_t*>(w.w13_sf);
-  p1.wsf_shared = static_cast<const int32_t*>(w.shared_w13_sf);
   p1.tsf_routed = c.at<int32_t>(c.lay.pool_sf);
   p1.x_sf = c.at<int32_t>(c.lay.x_sf);
   p1.topk_idx = c.at<int64_t>(c.lay.topk_idx);
@@ -1149,58 +1143,63 @@ bool build_sa(const Ctx& c, const MmoeWeights& w, bool has_shared, UmmaParams* o
   p1.num_ranks = c.geo.num_ranks;
   p1.k_dim = h;
   p1.rows_per_expert = 2 * inter;
-  p1.routed_sliced = w.w13_slice_stride > 0 ? 1 : 0;
   p1.n_blocks = inter / kTileRows;
   p1.hidden = h;
   p1.inter = inter;
-
-  UmmaParams p2 = p1;
-  bad |= make_weight_map(&p2.map_w_routed, true, w.w2, inter, (uint64_t)el * h, w.w2_slice_stride, 2 * kTileRows);
-  if (has_shared) bad |= make_weight_map(&p2.map_w_shared, false, w.shared_w2, inter, (uint64_t)h, 0, 2 * kTileRows);
-  else p2.map_w_shared = p2.map_w_routed;
-  for (int b = 0; b < kNumBoxes; ++b) {
-    bad |= make_token_map(&p2.map_tok_routed_box[b], c.ws + c.lay.act_x, inter, c.lay.pool_rows, 16 * (b + 1));
-    if (has_shared) bad |= make_token_map(&p2.map_tok_shared_box[b], c.ws + c.lay.shared_act_x, inter, c.geo.num_max_tokens, 16 * (b + 1));
-    else p2.map_tok_shared_box[b] = p2.map_tok_routed_box[b];
-  }
-  if (bad) return false;
-  p2.wsf_routed = static_cast<const int32_t*>(w.w2_sf);
-  p2.wsf_shared = static_cast<const int32_t*>(w.shared_w2_sf);
+  p2 = p1;
   p2.tsf_routed = c.at<int32_t>(c.lay.act_sf);
   p2.tsf_shared = c.at<int32_t>(c.lay.shared_act_sf);
   p2.tsf_rows_shared = c.lay.shared_sf_rows;
   p2.ret = c.at<__nv_bfloat16>(c.lay.ret);
   p2.shared_out = c.at<__nv_bfloat16>(c.lay.shared_out);
-  p2.pool_dst = c.at<int32_t>(c.lay.pool_dst);
   p2.k_dim = inter;
   p2.rows_per_expert = h;
-  p2.routed_sliced = w.w2_slice_stride > 0 ? 1 : 0;
   p2.n_blocks = h / (2 * kTileRows);
-  out[0] = p1;
-  out[1] = p2;
-  return true;
+  int bad = 0;
+  for (int b = 0; b < kNumBoxes; ++b) {
+    bad |= make_token_map(&p1.map_tok_routed_box[b], c.ws + c.lay.pool_x, h, c.lay.pool_rows, 16 * (b + 1));
+    bad |= make_token_map(&p1.map_tok_shared_box[b], c.ws + c.lay.x, h, c.geo.num_max_tokens, 16 * (b + 1));
+    bad |= make_token_map(&p2.map_tok_routed_box[b], c.ws + c.lay.act_x, inter, c.lay.pool_rows, 16 * (b + 1));
+    if (has_shared) bad |= make_token_map(&p2.map_tok_shared_box[b], c.ws + c.lay.shared_act_x, inter, c.geo.num_max_tokens, 16 * (b + 1));
+    else p2.map_tok_shared_box[b] = p2.map_tok_routed_box[b];
+  }
+  return bad == 0;
+}
+bool set_weights(const Ctx& c, const MmoeWeights& w, bool has_shared, SaPlan* plan) {
+  const int h = c.geo.hidden, inter = c.geo.intermediate, el = c.e_local;
+  UmmaParams& p1 = plan->layer[0];
+  UmmaParams& p2 = plan->layer[1];
+  p1.wsf_routed = static_cast<const int32_t*>(w.w13_sf);
+  p1.wsf_shared = static_cast<const int32_t*>(w.shared_w13_sf);
+  p2.wsf_routed = static_cast<const int32_t*>(w.w2_sf);
+  p2.wsf_shared = static_cast<const int32_t*>(w.shared_w2_sf);
+  p1.routed_sliced = w.w13_slice_stride > 0 ? 1 : 0;
+  p2.routed_sliced = w.w2_slice_stride > 0 ? 1 : 0;
+  int bad = make_w13_map(&p1.map_w_routed, true, w.w13, h, (uint64_t)el * 2 * inter, w.w13_slice_stride);
+  bad |= make_weight_map(&p2.map_w_routed, true, w.w2, inter, (uint64_t)el * h, w.w2_slice_stride, 2 * kTileRows);
+  if (has_shared) {
+    bad |= make_w13_map(&p1.map_w_shared, false, w.shared_w13, h, 2 * (uint64_t)inter, 0);
+    bad |= make_weight_map(&p2.map_w_shared, false, w.shared_w2, inter, (uint64_t)h, 0, 2 * kTileRows);
+  } else {
+    p1.map_w_shared = p1.map_w_routed;
+    p2.map_w_shared = p2.map_w_routed;
+  }
+  return bad == 0;
 }
 
-// the kept record for (workspace, weights, geometry), built on first use; least recently used slot is replaced
-const PlanEntry* cached_plan(const Ctx& c, const MmoeWeights& w, bool has_shared) {
-  const PlanKey key = make_key(c, w, has_shared);
-  std::lock_guard<std::mutex> lock(g_plan_mutex);
-  PlanEntry* victim = &g_plans[0];
-  for (PlanEntry& e : g_plans) {
-    if (e.stamp != 0 && e.key == key) {
-      e.stamp = ++g_plan_clock;
-      return &e;
-    }
-    if (e.stamp < victim->stamp) victim = &e;
-  }
-  const bool ok = build_sa(c, w, has_shared, victim->sa) && build_tm(c, w, has_shared, victim->tm);
-  if (!ok) {
-    victim->stamp = 0;
+// the kept parameters of (workspace, weights, geometry), built on first use; null when the driver refuses a map or the host is
+// out of memory
+template <typename Plan, typename Cache>
+std::shared_ptr<const Plan> kept_plan(Cache& cache, const PlanKey& key, const Ctx& c, const MmoeWeights& w, bool has_shared) {
+  try {
+    return cache.get(key, [&](const Plan* sibling) -> std::shared_ptr<const Plan> {
+      const std::shared_ptr<Plan> plan = sibling != nullptr ? std::make_shared<Plan>(*sibling) : std::make_shared<Plan>();
+      if (sibling == nullptr && !set_workspace(c, has_shared, plan.get())) return nullptr;
+      return set_weights(c, w, has_shared, plan.get()) ? plan : nullptr;
+    });
+  } catch (...) {
     return nullptr;
   }
-  victim->key = key;
-  victim->stamp = ++g_plan_clock;
-  return victim;
 }
 
 }  // namespace
@@ -1288,8 +1287,6 @@ cudaError_t launch_experts_umma(const Ctx& c, const MmoeWeights& w, const MmoeOp
   if (!tc_ready()) return cudaErrorNotReady;
   const bool has_shared = c.geo.num_shared_experts > 0 && w.shared_w13 != nullptr && m > 0;
   const int64_t timeout_ns = (o.timeout_ms > 0 ? (int64_t)o.timeout_ms : 2000) * 1000000ll;
-  const PlanEntry* plan = cached_plan(c, w, has_shared);
-  if (plan == nullptr) return cudaErrorInvalidValue;
   const bool fused = c.fused();
   const int mask = o.layer_mask == 0 ? 3 : o.layer_mask;
   cudaError_t e = cudaSuccess;
@@ -1316,16 +1313,21 @@ cudaError_t launch_experts_umma(const Ctx& c, const MmoeWeights& w, const MmoeOp
   const bool shared_pairs = m > pair_above;
   const auto [pairs, small] = gemm_forms(c, m, with_shared);
   const bool staged = staged_tokens(c, m, block_m);
+  const PlanKey key = make_key(c, w, has_shared);
+  std::shared_ptr<const TmPlan> tm_plan;
+  std::shared_ptr<const SaPlan> sa_plan;
+  if (pairs && (tm_plan = kept_plan<TmPlan>(g_tm_plans, key, c, w, has_shared)) == nullptr) return cudaErrorInvalidValue;
+  if (small && (sa_plan = kept_plan<SaPlan>(g_sa_plans, key, c, w, has_shared)) == nullptr) return cudaErrorInvalidValue;
   for (int layer = 1; layer <= 2; ++layer) {
     if ((mask & layer) == 0) continue;
     if (e == cudaSuccess && pairs) {
-      TmParams p = plan->tm[layer - 1];
+      TmParams p = tm_plan->layer[layer - 1];
       patch(p, layer == 2);
       p.shared_tiles = shared_pairs ? shared : none;
       e = tm_launch(layer, layer == 2 && fused, p, s);
     }
     if (e == cudaSuccess && small) {
-      UmmaParams p = plan->sa[layer - 1];
+      UmmaParams p = sa_plan->layer[layer - 1];
       patch(p, layer == 2);
       p.shared_tiles = shared_pairs ? none : shared;
       p.tile_rows = c.tile_select == 2 ? cut.step : (pairs ? 0 : small_only_cap(m, block_m));
