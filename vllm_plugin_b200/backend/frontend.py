@@ -8,9 +8,9 @@ At EP > 1 the default transport is the device-side exchange over NVLink peer mem
 pushed into the peers' symmetric workspaces, GEMM2 writing its rows straight back to the rank they came from); the
 host-driven alternative issues the same three exchanges as ``torch.distributed`` all-to-allv calls on the caller's group.
 
-Like the reference (``frontend.py:650-754``) a call with the tensors of the previous call skips the argument checks: the
-record of the last validated call is kept on the buffer, and a call whose weight tensors are the same objects at the same
-addresses goes straight to the launch.
+Like the reference (``frontend.py:650-754``) a call with the tensors of an earlier call skips the argument checks: the
+buffer keeps a record per set of weights (the layers of a model share one buffer), and a call whose tensors are the same
+objects at the same addresses goes straight to the launch.
 """
 
 from __future__ import annotations
@@ -19,6 +19,7 @@ import ctypes
 import dataclasses
 import math
 import operator
+import weakref
 from typing import Any, Dict, Optional, Tuple
 
 import torch
@@ -235,15 +236,42 @@ def exchange_rows(group, dst: torch.Tensor, src: torch.Tensor, dst_splits, src_s
     dist.all_to_all_single(d, s, list(dst_splits), list(src_splits), group=group)
 
 
-class _CallRecord:
-    """What the last validated call on a buffer established: the tensor objects it checked (kept alive, so that their
-    identities cannot be reused), the structures built from them, and the status poll state."""
+_MAX_CALL_RECORDS = 256      # per buffer
 
-    __slots__ = ("tensors", "present", "addresses", "weights", "weights_ref", "options_key", "options", "options_ref", "peers",
+
+def _absent():
+    return None
+
+
+class _CallRecord:
+    """What a validated call on a buffer established: the tensor objects it checked, the structures built from them.  The
+    tensors are held weakly -- weights that the program gives up are not kept alive here -- and an identity cannot be reused
+    unnoticed: the reference to an object that is gone yields ``None``."""
+
+    __slots__ = ("refs", "addresses", "weights", "weights_ref", "options_key", "options", "options_ref", "peers",
                  "variants_ready")
 
+    def __init__(self, tensors):
+        self.refs = [_absent if t is None else weakref.ref(t) for t in tensors]
+        self.addresses = [t.data_ptr() for t in tensors if t is not None]
+
     def matches(self, tensors) -> bool:
-        return all(map(operator.is_, tensors, self.tensors)) and [t.data_ptr() for t in self.present] == self.addresses
+        return (all(map(operator.is_, tensors, [r() for r in self.refs]))
+                and [t.data_ptr() for t in tensors if t is not None] == self.addresses)
+
+
+def _keep_record(records: Dict[Tuple[int, int], _CallRecord], key: Tuple[int, int], rec: _CallRecord, owners) -> None:
+    """Put ``rec`` among the records of a buffer until one of its ``owners`` dies, the tensors whose ids are the key."""
+    if key not in records and len(records) >= _MAX_CALL_RECORDS:
+        records.pop(next(iter(records)), None)
+
+    def drop(_, records=records, key=key):
+        records.pop(key, None)
+
+    for i, t in owners:
+        if t is not None:
+            rec.refs[i] = weakref.ref(t, drop)
+    records[key] = rec
 
 
 class _StatusPoll:
@@ -281,10 +309,7 @@ def _validate(y, l1_weights, l2_weights, sym_buffer, shared_l1_weights, shared_l
     s13, s2 = check_mega_moe_arguments(y, l1_weights, l2_weights, sym_buffer, shared_l1_weights, shared_l2_weights,
                                        stats, recipe, activation, activation_clamp, fast_math, activation_alpha,
                                        activation_beta)
-    rec = _CallRecord()
-    rec.tensors = tensors
-    rec.present = [t for t in tensors if t is not None]
-    rec.addresses = [t.data_ptr() for t in rec.present]
+    rec = _CallRecord(tensors)
     rec.weights = _weights_struct(l1_weights, l2_weights, shared_l1_weights, shared_l2_weights, s13, s2)
     rec.weights_ref = ctypes.byref(rec.weights)
     rec.options_key = None
@@ -313,13 +338,14 @@ def fp8_fp4_mega_moe(y: torch.Tensor, l1_weights, l2_weights, sym_buffer, shared
                shared_l1_weights[1] if shared_l1_weights is not None else None,
                shared_l2_weights[0] if shared_l2_weights is not None else None,
                shared_l2_weights[1] if shared_l2_weights is not None else None, stats)
-    rec = sym_buffer._call_record
+    key = (id(tensors[0]), id(stats))
+    rec = sym_buffer._call_records.get(key)
     m = y.size(0)
     if (rec is None or not rec.matches(tensors) or (recipe != (1, 1, 32) and tuple(recipe) != (1, 1, 32)) or activation != "swiglu"
             or activation_alpha != 1.0 or activation_beta != 0.0):
         rec = _validate(y, l1_weights, l2_weights, sym_buffer, shared_l1_weights, shared_l2_weights, stats, recipe,
                         activation, activation_clamp, fast_math, activation_alpha, activation_beta, tensors)
-        sym_buffer._call_record = rec
+        _keep_record(sym_buffer._call_records, key, rec, ((0, tensors[0]), (8, stats)))
     else:
         # the record vouches for everything but the output tensor and the clamp
         assert y.dim() == 2 and y.size(1) == sym_buffer.hidden and y.dtype == torch.bfloat16 and y.is_contiguous(), \

@@ -65,7 +65,7 @@ class SymmBuffer:
         self.num_ranks = group.size()
         self.geo_ref = ctypes.byref(self.geo)
         self.block_m_of: Dict[int, int] = {}
-        self._call_record = None
+        self._call_records: Dict = {}      # validated calls by weight set
         self._status_poll = None
         if device is None:
             device = torch.device("cuda", torch.cuda.current_device())
