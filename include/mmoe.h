@@ -18,6 +18,11 @@
 extern "C" {
 #endif
 
+/* Version of the structures and functions below, raised whenever one of them changes: a structure that grows is written past
+ * its end for a host compiled against the earlier header.  Compare with mmoe_abi_version() before anything else.
+ * 3: MmoeOptions.residual.  4: MmoeLayout.shared_tile_sf, mmoe_split_halves. */
+#define MMOE_ABI_VERSION 4
+
 enum {
   MMOE_OK = 0,
   MMOE_ERR_INVALID_ARGUMENT = 1,  /* maps to AssertionError / ValueError on the Python side */
@@ -279,7 +284,7 @@ int mmoe_set_tuning(int32_t max_stages, int32_t orientation);
 
 const char* mmoe_status_string(int code);
 const char* mmoe_last_error(void);   /* detail of the last failure on this thread */
-int mmoe_abi_version(void);
+int mmoe_abi_version(void);           /* MMOE_ABI_VERSION of the library as built */
 
 #ifdef __cplusplus
 }

@@ -56,9 +56,15 @@ static void cache() {
   }
 }
 
+// abi <version> <bytes of MmoeGeometry> <MmoeLayout> <MmoeWeights> <MmoeOptions>
+static void abi() {
+  printf("abi %d %zu %zu %zu %zu\n", MMOE_ABI_VERSION, sizeof(MmoeGeometry), sizeof(MmoeLayout), sizeof(MmoeWeights), sizeof(MmoeOptions));
+}
+
 int main(int argc, char** argv) {
   for (int i = 1; i < argc; ++i)
     if (strcmp(argv[i], "forms") == 0) forms();
     else if (strcmp(argv[i], "cache") == 0) cache();
+    else if (strcmp(argv[i], "abi") == 0) abi();
   return 0;
 }

@@ -48,3 +48,15 @@ def test_launch_parameters_are_kept_for_every_layer_of_a_model(rules):
         assert wrong == 0
         assert built == (keys if keys <= 16 else rounds * keys), keys
         assert siblings == built - min(keys, 4), keys
+
+
+# sizes of the structures that cross the C boundary, by the version of the interface: a change needs a new version
+ABI_SIZES = {3: (32, 37 * 8, 80, 32), 4: (32, 38 * 8, 80, 32)}
+
+
+def test_structures_of_the_c_interface_and_its_version(rules):
+    import ctypes
+    from vllm_plugin_b200.backend import _native
+    (version, *sizes), = rules("abi")
+    assert tuple(sizes) == ABI_SIZES[version]
+    assert tuple(sizes) == tuple(ctypes.sizeof(s) for s in (_native.MmoeGeometry, _native.MmoeLayout, _native.MmoeWeights, _native.MmoeOptions))

@@ -105,7 +105,8 @@ def test_library_exports_every_declared_symbol():
     lib = ctypes.CDLL(_native.library_path())
     for name in declared:
         assert hasattr(lib, name), name
-    assert _native.load().mmoe_abi_version() == 3
+    version = int(re.search(r"#define MMOE_ABI_VERSION (\d+)", header).group(1))
+    assert _native.load().mmoe_abi_version() == version == _native.ABI_VERSION
 
 
 def test_layout_is_consistent():

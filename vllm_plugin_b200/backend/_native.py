@@ -21,6 +21,8 @@ MMOE_ERR_ARCH = 4
 MMOE_ERR_NOT_PREPARED = 5
 MMOE_ERR_DEVICE_TIMEOUT = 6
 
+ABI_VERSION = 4          # of include/mmoe.h, whose structures are mirrored below
+
 ENGINE_TENSOR_CORE = 0
 ENGINE_SCALAR_VALIDATION = 1
 
@@ -82,6 +84,10 @@ def load() -> ctypes.CDLL:
             f"{_LIB_PATH} is missing: build it with `python vllm_plugin_b200/csrc/build.py` (nvcc, sm_100a). "
             "The MegaMoE backend has no CPU or PyTorch fallback.")
     lib = ctypes.CDLL(_LIB_PATH)
+    version = lib.mmoe_abi_version()
+    if version != ABI_VERSION:
+        raise RuntimeError(f"{_LIB_PATH} has ABI version {version}, this package needs {ABI_VERSION}: rebuild it with "
+                           "`python vllm_plugin_b200/csrc/build.py`.")
     vp, i32 = ctypes.c_void_p, ctypes.c_int32
     geo_p = ctypes.POINTER(MmoeGeometry)
     lib.mmoe_layout.argtypes = [geo_p, ctypes.POINTER(MmoeLayout)]

@@ -128,7 +128,7 @@ float bf16_round_host(float v) {
 
 extern "C" {
 
-int mmoe_abi_version(void) { return 3; }
+int mmoe_abi_version(void) { return MMOE_ABI_VERSION; }
 
 int mmoe_set_tuning(int32_t max_stages, int32_t orientation) {
   if (max_stages < 0 || max_stages == 1) return fail(MMOE_ERR_INVALID_ARGUMENT, "max_stages=%d must be 0 or >= 2", max_stages);
