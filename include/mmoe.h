@@ -236,7 +236,8 @@ int mmoe_combine_residual(const MmoeGeometry* geo, void* workspace, void* y_bf16
                           int32_t num_tokens, void* stream);
 /* EP1 convenience: count, place, experts, combine; same result as the separate calls.  One stream, one programmatic chain
  * of launches, so that each one's launch and set-up overlap its predecessor (MMOE_DISABLE_CHAINED_LAUNCH=1 in the
- * environment, read once per process: ordinary launches).  Up to 16 tokens (BLOCK_M 16) three launches: GEMM1 orders the
+ * environment, read once per process: ordinary launches).  The first kernel of the chain reads nothing before everything in front
+ * of the call has ended, whether or not the kernel in front triggers its successors early.  Up to 16 tokens (BLOCK_M 16) three launches: GEMM1 orders the
  * routes itself and takes the staged tokens as they are.  Up to 128 tokens four: one launch orders the routes, builds
  * the plan and places the rows in front of GEMM1, GEMM2 and combine.  Past that ordering and placement are two launches, and
  * past 192 tokens each GEMM is two: the experts with many rows on CTA pairs, the others on the weights-as-A kernels.  The

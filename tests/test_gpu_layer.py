@@ -357,6 +357,56 @@ def test_calls_in_flight_together_on_two_streams(m):
             assert torch.equal(y, want), i
 
 
+@pytest.fixture(scope="module")
+def late_write(tmp_path_factory):
+    import ctypes
+    import os
+    import shutil
+    import subprocess
+    nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
+    if not os.path.exists(nvcc):
+        pytest.skip("nvcc is not installed")
+    so = str(tmp_path_factory.mktemp("late") / "late_writer.so")
+    subprocess.run([nvcc, "-gencode", "arch=compute_100a,code=sm_100a", "-shared", "-Xcompiler", "-fPIC", "-o", so,
+                    os.path.join(os.path.dirname(__file__), "late_writer.cu")], check=True, capture_output=True)
+    fn = ctypes.CDLL(so).late_write
+    fn.argtypes = [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int64, ctypes.c_int64, ctypes.c_void_p]
+    return fn
+
+
+@pytest.mark.parametrize("what", ["shared w13", "shared w13 scales", "w13", "w2"])
+@pytest.mark.parametrize("m", [1, 16, 100, 300])
+def test_nothing_is_read_before_a_predecessor_that_triggers_early_has_ended(late_write, m, what):
+    """Weights rewritten by a kernel in front of the call that lets the call's first kernel start at once and writes 300 us
+    later: the output is that of the new weights."""
+    from vllm_plugin_b200 import api
+    layer = H.make_layer(shared=True, seed=61, **SMALL)
+    other = H.make_layer(shared=True, seed=62, **SMALL)
+    weights, fresh = H.kernel_weights(layer, "cuda"), H.kernel_weights(other, "cuda")
+    i, j = {"shared w13": (2, 0), "shared w13 scales": (2, 1), "w13": (0, 0), "w2": (1, 0)}[what]
+    target = weights[i][j]
+    source = fresh[i][j] if j == 0 else target + 0x01010101        # every scale doubled
+    old, nbytes = target.clone(), target.numel() * target.element_size()
+    assert target.stride() == source.stride()
+    hid = O.make_hidden(m, layer.hidden, 1)
+    ids, w = O.make_routing(m, layer.num_experts, layer.num_topk, 2)
+    y_old, buf = H.run_layer(layer, hid, ids, w, weights=weights)
+    target.copy_(source)
+    want, _ = H.run_layer(layer, hid, ids, w, weights=weights, buf=buf)
+    assert not torch.equal(want, y_old)
+    x, ids, w = hid.cuda(), ids.cuda(), w.cuda()
+    y = torch.empty_like(want)
+    stream = torch.cuda.current_stream().cuda_stream
+    for _ in range(3):
+        target.copy_(old)
+        torch.cuda.synchronize()
+        assert late_write(target.data_ptr(), source.data_ptr(), nbytes, 300_000, stream) == 0
+        api.stage_inputs_for_mega_moe(buf, x, ids, w)
+        api.fp8_fp4_mega_moe(y, weights[0], weights[1], buf, weights[2], weights[3], activation_clamp=10.0)
+        api.read_status(buf)
+        assert torch.equal(y, want)
+
+
 @pytest.mark.parametrize("m,bm", [(7, 16), (130, 32), (300, 128), (300, 192)])
 def test_shared_expert_ahead_of_the_routed_plan(m, bm):
     """The split the expert-parallel forward uses, on one GPU: shared expert planned and run first (both GEMMs), routed

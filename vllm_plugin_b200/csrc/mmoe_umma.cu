@@ -862,7 +862,7 @@ __device__ __forceinline__ void sa_teardown(Control* ctl, uint32_t tmem_base) {
   }
 }
 
-// Layer 1, before anything has been waited for: weights and scales of the first stages of a CTA's shared task, by the producer
+// Layer 1, before the route table has been read: weights and scales of the first stages of a CTA's shared task, by the producer
 // warp (it has initialised the barriers itself).  Returns the number of stages.
 template <typename L>
 __device__ __forceinline__ int sa_request_shared(const UmmaParams& p, const Cta& c) {
@@ -901,11 +901,12 @@ __global__ void __launch_bounds__(kThreads, 1) umma_kernel(const __grid_constant
     prefetch_map(&p.map_w_routed);
     prefetch_map(&p.map_w_shared);
   }
-  // (a GEMM1 that orders the routes follows the staging itself; the shared expert's weights do not wait even for that)
+  if ((!early || (kStaged && kLayer == 1 && p.route_here)) && !p.skip_wait) chain_wait();
+  // GEMM1 that orders the routes follows the staging itself, whose predecessors may be anything: not even weights are read
+  // ahead of the wait, but the shared expert's ahead of the route table.
   int ready = 0;
   if (kStaged && kLayer == 1 && p.route_here && warp == 0 && static_cast<int>(blockIdx.x) < p.shared_tiles.parts * p.n_blocks)
     ready = sa_request_shared<L>(p, sa_carve<L>(smem, p.tile_rows, p.max_stages));
-  if ((!early || (kStaged && kLayer == 1 && p.route_here)) && !p.skip_wait) chain_wait();
   if (kStaged && kLayer == 1) {
     __syncthreads();                         // the words are zero
     for (int i = threadIdx.x; i < p.num_routes; i += kThreads) {
