@@ -56,6 +56,22 @@ static void cache() {
   }
 }
 
+// cuts <block_m> <pair tiles> <cap> <n> <parts> <step> <non-empty tiles> <scale chunks of the expert's blocks>
+static void cuts() {
+  for (int block_m : kBlockMs) {
+    bool caps[kSmallTileRows + 1] = {};
+    for (int m = 0; m <= 300; ++m) caps[small_only_cap(m, block_m)] = true;
+    caps[kDeepTileRows] = caps[kSmallTileRows] = true;                 // calls with pair tiles
+    for (int cap = 0; cap <= kSmallTileRows; ++cap)
+      for (int n = 1; caps[cap] && n <= 1100; ++n)
+        for (int pairs = 0; pairs <= 1; ++pairs) {
+          const Cut c = cut_rows(n, pairs != 0, cap);
+          printf("cuts %d %d %d %d %d %d %d %d\n", block_m, pairs, cap, n, c.parts, c.step, (n + c.step - 1) / c.step,
+                 (n + block_m - 1) / block_m * chunks_per_block(block_m));
+        }
+  }
+}
+
 // abi <version> <bytes of MmoeGeometry> <MmoeLayout> <MmoeWeights> <MmoeOptions>
 static void abi() {
   printf("abi %d %zu %zu %zu %zu\n", MMOE_ABI_VERSION, sizeof(MmoeGeometry), sizeof(MmoeLayout), sizeof(MmoeWeights), sizeof(MmoeOptions));
@@ -66,5 +82,6 @@ int main(int argc, char** argv) {
     if (strcmp(argv[i], "forms") == 0) forms();
     else if (strcmp(argv[i], "cache") == 0) cache();
     else if (strcmp(argv[i], "abi") == 0) abi();
+    else if (strcmp(argv[i], "cuts") == 0) cuts();
   return 0;
 }

@@ -60,3 +60,12 @@ def test_structures_of_the_c_interface_and_its_version(rules):
     (version, *sizes), = rules("abi")
     assert tuple(sizes) == ABI_SIZES[version]
     assert tuple(sizes) == tuple(ctypes.sizeof(s) for s in (_native.MmoeGeometry, _native.MmoeLayout, _native.MmoeWeights, _native.MmoeOptions))
+
+
+def test_cuts_fit_their_tiles_and_scale_chunks(rules):
+    """However many rows an expert has (more than there are tokens, when tokens name it twice or come from other ranks): its
+    tiles cover them, are no larger than the kernels' tiles, and no more than the scale chunks reserved for its pool blocks."""
+    for block_m, pairs, cap, n, parts, step, tiles, chunks in rules("cuts"):
+        case = (block_m, pairs, cap, n)
+        assert step % 16 == 0 and step <= (128 if pairs else cap) and parts * step >= n and tiles <= parts, case
+        assert tiles <= chunks, case

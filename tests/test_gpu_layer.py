@@ -357,6 +357,25 @@ def test_calls_in_flight_together_on_two_streams(m):
             assert torch.equal(y, want), i
 
 
+@pytest.mark.parametrize("bm", [16, 128, 192, 240])
+def test_few_tokens_that_name_an_expert_many_times(bm):
+    """40 tokens, nearly all six slots of each on one expert: up to 239 rows in a call that is sized for 40 per expert."""
+    from vllm_plugin_b200 import api
+    layer = H.make_layer(512, 256, 8, 6, True, seed=17)
+    hid = O.make_hidden(40, layer.hidden, 4)
+    _, w = O.make_routing(40, 8, 6, 5)
+    for rows, expert in ((40, 2), (20, 3), (13, 3)):
+        ids = torch.full((40, 6), 4, dtype=torch.int64)
+        ids[:rows] = expert
+        ids[39, 5] = 5
+        api.set_kernel_options(block_m=bm)
+        try:
+            y, _ = H.run_layer(layer, hid, ids, w)
+        finally:
+            api.set_kernel_options(block_m=0)
+        assert_parity(y, H.oracle_layer(layer, hid, ids, w), f"block_m {bm} rows {rows}")
+
+
 @pytest.fixture(scope="module")
 def late_write(tmp_path_factory):
     import ctypes

@@ -54,9 +54,10 @@ __host__ __device__ inline Cut shared_cut(int m, int pair_above) { return cut_ro
 // the routes itself (an UMMA takes 16 token columns at least); see staged_tokens().
 constexpr int kStagedTokens = 16;
 // Cap of a call without pair tiles (also known to the host: the largest tile of such a call fixes its stage layout): no expert
-// has more rows than there are tokens unless a token names it twice, which then costs another tile.
+// has more rows than there are tokens unless a token names it twice, which then costs another tile.  An expert of any size has
+// to fit the scale chunks of its pool blocks, see chunks_per_block().
 __host__ __device__ inline int small_only_cap(int m, int block_m) {
-  const int rows = (m + 15) & ~15, least = block_m < 64 ? block_m : 64;
+  const int rows = (m + 15) & ~15, least = block_m <= 64 ? block_m : (block_m <= 128 ? 64 : kDeepTileRows);
   return rows >= kDeepTileRows ? kDeepTileRows : (rows > least ? rows : least);
 }
 
