@@ -20,6 +20,7 @@ static void forms() {
               static const void* peer[8] = {};
               Ctx c{};
               c.geo = MmoeGeometry{ranks, 0, 384, 6, 5120, 2304, 1, 3840};
+              c.e_local = 384 / ranks;
               c.pair_above = pair_above;
               c.tile_select = select;
               c.peer_ws = peers ? peer : nullptr;

@@ -41,6 +41,23 @@ def test_staged_tokens_replace_placed_rows_on_one_gpu_only(rules):
             assert small and not pairs, case
 
 
+def test_pair_launches_of_small_calls(rules):
+    """No launch on CTA pairs where none can be worth it: one GPU with no more tokens than the line, several ranks with few
+    routes (6 per token, 192 or 48 of 384 experts here) -- but a rank without tokens, or with the pair kernels forced on, keeps
+    them.  The shared expert by itself takes one launch, by its own tokens."""
+    for ranks, pair_above, select, peers, block_m, m, pairs, small, staged in rules("forms"):
+        case = (ranks, pair_above, select, peers, block_m, m)
+        if select == 2:
+            assert (pairs, small) == ((1, 0) if m > pair_above else (0, 1) if m > 0 else (0, 0)), case
+        elif pair_above == NEVER:
+            assert (pairs, small) == (0, 1), case
+        elif ranks == 1:
+            assert (pairs, small) == (m > pair_above, pair_above > 0 or m == 0), case
+        else:
+            few = pair_above > 0 and 0 < 6 * m <= min(3072, 96 * (384 // ranks))
+            assert (pairs, small) == (not few, pair_above > 0), case
+
+
 def test_launch_parameters_are_kept_for_every_layer_of_a_model(rules):
     """Keys that take turns are built once as long as they fit, from the parameters of a key with the same workspace where
     there is one; a value that was handed out stays valid when its entry is replaced."""

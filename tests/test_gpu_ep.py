@@ -129,7 +129,7 @@ def run_ranks_in_turn(layer, hids, ids, ws, orientation=0):
 
 
 @pytest.mark.parametrize("orientation", [0, 1])
-@pytest.mark.parametrize("tokens", [(5, 9), (16, 1), (0, 12), (17, 16), (3, 400), (16, 2, 7, 1)])
+@pytest.mark.parametrize("tokens", [(5, 9), (16, 1), (0, 12), (17, 16), (3, 400), (120, 500), (16, 2, 7, 1)])
 def test_ranks_in_turn_match_the_oracle(tokens, orientation):
     """The layer's kernels at EP 2 and 4 without the transport: per rank a handful of tokens of its own, and rows of other
     ranks that it has never staged."""

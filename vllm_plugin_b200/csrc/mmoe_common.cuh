@@ -236,9 +236,20 @@ struct Ctx {             // resolved pointers of one call
   const void* const* peer_ws = nullptr;   // set by the call that fuses the write-back into GEMM2 (EP > 1)
   int tile_select = 0;                    // 0: every tile of the plan, 1: routed tiles only, 2: the early shared tiles only
   int pair_above = kNeverPair;            // experts with more rows than this run on CTA pairs ...
-  // ... in a call of m tokens on this rank: with one rank and few tokens none does (not even one that a token names twice),
-  // and the call needs no pair launch
-  int pair_above_for(int m) const { return geo.num_ranks == 1 && m <= pair_above ? kNeverPair : pair_above; }
+  // ... in a call of m tokens on this rank: in a small one none does, and the call needs no pair launch.  On one GPU a call is
+  // small when no expert can have that many rows (but for tokens that name one twice).
+  // With several ranks the host knows only its own tokens and takes the others to have as many, as the choice of BLOCK_M does;
+  // a rank without tokens knows nothing.  Two empty pair launches cost 7.3 us, which hot experts have to earn back.  GEMMs of
+  // one rank of 8, 48 experts each, Zipf(1.2) / even popularity, never -> with pairs: 64 tokens 164 -> 172 / 171 -> 178 us,
+  // 256: 208 -> 217 / 198 -> 216, 512: 254 -> 271 / 215 -> 230, 1024: 357 -> 354 / 330 -> 340, 1920: 545 -> 477 / 525 -> 442.
+  // One of 2 (192 experts), 512 tokens: 624 -> 625 / 616 -> 626.  16 experts, top-3, 512 tokens (96 rows each): 135 -> 145 /
+  // 139 -> 142.  A rank that misjudges the others is slower by the same measure, not wrong.
+  static constexpr int kFewRoutes = 3072, kFewRows = 96;
+  int pair_above_for(int m) const {
+    if (geo.num_ranks == 1) return m <= pair_above ? kNeverPair : pair_above;
+    const int64_t routes = (int64_t)m * geo.num_topk;
+    return pair_above > 0 && m > 0 && routes <= kFewRoutes && routes <= (int64_t)kFewRows * e_local ? kNeverPair : pair_above;
+  }
   template <typename T> T* at(int64_t off) const { return reinterpret_cast<T*>(ws + off); }
   bool fused() const { return peer_ws != nullptr && geo.num_ranks > 1 && tile_select != 2; }
 };
@@ -248,8 +259,9 @@ struct GemmForms {
   bool pairs, small;
 };
 inline GemmForms gemm_forms(const Ctx& c, int m, bool with_shared) {
+  // the shared expert by itself takes one launch in either form
+  if (c.tile_select == 2) return GemmForms{with_shared && m > c.pair_above, with_shared && m <= c.pair_above};
   const int pair_above = c.pair_above_for(m);
-  if (c.tile_select == 2) return GemmForms{with_shared && m > pair_above, with_shared && m <= pair_above};
   return GemmForms{pair_above != kNeverPair, pair_above > 0};
 }
 

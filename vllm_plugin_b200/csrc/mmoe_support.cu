@@ -548,12 +548,12 @@ __device__ ExpertPlan build_plan(const PlanView& pv, int n, const PlanArgs& a, b
   const int e = threadIdx.x;
   __shared__ int s_rows;
   if (threadIdx.x == 0) s_rows = 16;
-  // With pair tiles in the call, weights-as-A tiles of 112 rows (four stages fit the shared memory) only when enough experts
-  // gain a tile by it, else of 80 (five stages).
+  // With pair tiles in the call or rows from other ranks, weights-as-A tiles of 112 rows (four stages fit the shared memory) only
+  // when enough experts gain a tile by it, else of 80 (five stages).
   const bool small = n > 0 && !on_pairs(n, a.pair_above);
   const bool wide = small && ((n > kDeepTileRows && n <= kSmallTileRows) || n > 2 * kDeepTileRows);
   const int num_small = __syncthreads_count(small), num_wide = __syncthreads_count(wide);
-  const int cap = a.pair_above == kNeverPair ? small_only_cap(a.m, a.block_m) : (num_wide * 8 > num_small ? kSmallTileRows : kDeepTileRows);
+  const int cap = a.pair_above == kNeverPair && a.num_ranks == 1 ? small_only_cap(a.m, a.block_m) : (num_wide * 8 > num_small ? kSmallTileRows : kDeepTileRows);
   const Cut cut = cut_rows(n, n > 0 && !small, cap);
   const Cut sh_cut = shared_cut(a.has_shared ? a.m : 0, a.pair_above);
   const bool shared_small = a.m <= a.pair_above;
@@ -973,10 +973,10 @@ PlanArgs plan_args(const Ctx& c, int m, int block_m) {
   return PlanArgs{c.e_local, c.geo.num_ranks, block_m, c.pair_above_for(m), m, c.geo.num_shared_experts > 0 && m > 0 ? 1 : 0};
 }
 
-SharedScales shared_scales(const Ctx& c, int m) {
+SharedScales shared_scales(const Ctx& c, int m, int pair_above) {
   const bool on = c.geo.num_shared_experts > 0 && m > 0;
   return SharedScales{c.at<int32_t>(c.lay.x_sf), on ? c.at<int32_t>(c.lay.shared_tile_sf) : nullptr, shared_chunk_rows(c.geo.num_max_tokens),
-                      shared_cut(m, c.pair_above_for(m))};
+                      shared_cut(m, pair_above)};
 }
 
 RouteArgs route_args(const Ctx& c, int m, int block_m, int32_t* stats) {
@@ -999,7 +999,7 @@ RouteArgs route_args(const Ctx& c, int m, int block_m, int32_t* stats) {
   r.pool_w = c.at<float>(c.lay.pool_w);
   r.pool_dst = c.at<int32_t>(c.lay.pool_dst);
   r.pool_sf_rows = c.lay.pool_sf_rows;
-  r.shared = shared_scales(c, m);
+  r.shared = shared_scales(c, m, c.pair_above_for(m));
   r.h = c.geo.hidden;
   r.k = c.geo.num_topk;
   r.a = plan_args(c, m, block_m);
@@ -1026,7 +1026,7 @@ cudaError_t launch_route_large(const Ctx& c, int m, int block_m, int32_t* stats,
 
 cudaError_t launch_shared_plan(const Ctx& c, int m, cudaStream_t s) {
   if (m == 0 || c.geo.num_shared_experts == 0) return cudaSuccess;
-  launch_chained(shared_plan_kernel, dim3(std::max(1, std::min((m + 7) / 8, 148 * 2))), dim3(256), 0, s, m, shared_scales(c, m),
+  launch_chained(shared_plan_kernel, dim3(std::max(1, std::min((m + 7) / 8, 148 * 2))), dim3(256), 0, s, m, shared_scales(c, m, c.pair_above),
                  c.geo.hidden / kTileK);
   return cudaGetLastError();
 }
@@ -1040,7 +1040,7 @@ cudaError_t launch_plan_place(const Ctx& c, int m, int block_m, int32_t* stats, 
       direct ? c.at<int32_t>(c.lay.x_sf) : c.at<int32_t>(c.lay.recv_sf),
       direct ? c.at<float>(c.lay.topk_weights) : c.at<float>(c.lay.recv_w), c.at<int32_t>(c.lay.sorted_route),
       c.at<uint4>(c.lay.pool_x), c.at<int32_t>(c.lay.pool_sf), c.at<float>(c.lay.pool_w), c.at<int32_t>(c.lay.pool_dst),
-      c.lay.pool_sf_rows, c.e_local, R, c.geo.hidden, c.geo.num_topk, direct ? 1 : 0, shared_scales(c, m));
+      c.lay.pool_sf_rows, c.e_local, R, c.geo.hidden, c.geo.num_topk, direct ? 1 : 0, shared_scales(c, m, c.pair_above_for(m)));
   return cudaGetLastError();
 }
 

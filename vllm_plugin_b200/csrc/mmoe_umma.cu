@@ -1307,7 +1307,7 @@ cudaError_t launch_experts_umma(const Ctx& c, const MmoeWeights& w, const MmoeOp
   };
   // Experts with many rows run on CTA pairs, the others on the weights-as-A kernels: which ones is in the plan.  The shared
   // expert is one or the other by the call's token count.
-  const int pair_above = c.pair_above_for(m);
+  const int pair_above = c.tile_select == 2 ? c.pair_above : c.pair_above_for(m);
   const bool with_shared = has_shared && c.tile_select != 1;
   const Cut cut = shared_cut(with_shared ? m : 0, pair_above);
   const SharedTiles shared{cut.parts, cut.step, m}, none{0, 16, 0};
@@ -1331,10 +1331,10 @@ cudaError_t launch_experts_umma(const Ctx& c, const MmoeWeights& w, const MmoeOp
       UmmaParams p = sa_plan->layer[layer - 1];
       patch(p, layer == 2);
       p.shared_tiles = shared_pairs ? none : shared;
-      p.tile_rows = c.tile_select == 2 ? cut.step : (pairs ? 0 : small_only_cap(m, block_m));
+      p.tile_rows = c.tile_select == 2 ? cut.step : (pairs || c.geo.num_ranks > 1 ? 0 : small_only_cap(m, block_m));
       // The pair launch in front reads and writes nothing that this one does, and lets it start only after its own wait.
       p.skip_wait = pairs ? 1 : 0;
-      p.early = !pairs && c.tile_select == 0 && !fused && (layer == 1 || c.route_in_gemm) ? 1 : 0;
+      p.early = c.geo.num_ranks == 1 && !pairs && c.tile_select == 0 && (layer == 1 || c.route_in_gemm) ? 1 : 0;
       p.num_routes = m * c.geo.num_topk;
       p.route_here = c.route_in_gemm ? 1 : 0;
       p.stats = c.stats;
