@@ -189,7 +189,7 @@ def test_admission_gate_and_library_agree_on_the_kernel_limits():
 def test_call_records_of_many_weight_sets_on_one_buffer(monkeypatch):
     """Every layer of a model finds the record of its own last call on the shared buffer; a record neither keeps tensors
     alive nor outlives them, and a tensor whose storage was replaced is not vouched for."""
-    import gc
+    import weakref
     from vllm_plugin_b200.backend import frontend as F
     layers = [tuple(torch.empty(4) for _ in range(8)) + (None,) for _ in range(40)]
     layers[3] = layers[3][:4] + (None,) * 4 + (torch.empty(2),)           # no shared expert, receive counts wanted
@@ -204,16 +204,18 @@ def test_call_records_of_many_weight_sets_on_one_buffer(monkeypatch):
             rec = lookup(tensors)
             assert (rec is None) == (turn == 0)
             if rec is None:
-                F._keep_record(records, (id(tensors[0]), id(tensors[8])), F._CallRecord(tensors), ((0, tensors[0]), (8, tensors[8])))
+                F._keep_record(records, (id(tensors[0]), id(tensors[8])), F._CallRecord(tensors))
     assert lookup(layers[5][:2] + layers[6][2:]) is None                  # another tensor among them
     layers[7][4].data = torch.empty(64)
     assert lookup(layers[7]) is None
+    gone = [weakref.ref(t) for t in layers[0] if t is not None]
     del tensors, rec
     layers.pop(0)
-    layers[2] = layers[2][:8] + (None,)                                   # the counts of the layer without a shared expert die
-    gc.collect()
-    assert len(records) == 38
-    monkeypatch.setattr(F, "_MAX_CALL_RECORDS", 38)
-    extra = (torch.empty(4),) * 8 + (None,)
-    F._keep_record(records, (id(extra[0]), id(None)), F._CallRecord(extra), ((0, extra[0]), (8, None)))
-    assert len(records) == 38 and lookup(extra) is not None
+    assert all(r() is None for r in gone)
+    monkeypatch.setattr(F, "_MAX_CALL_RECORDS", 40)
+    for n in (40, 40, 40):                                                # the dead one goes first, then the oldest
+        extra = (torch.empty(4),) * 8 + (None,)
+        layers.append(extra)
+        F._keep_record(records, (id(extra[0]), id(None)), F._CallRecord(extra))
+        assert len(records) == n and lookup(extra) is not None
+    assert [lookup(t) is not None for t in layers[:4]] == [False, False, True, True]

@@ -260,17 +260,13 @@ class _CallRecord:
                 and [t.data_ptr() for t in tensors if t is not None] == self.addresses)
 
 
-def _keep_record(records: Dict[Tuple[int, int], _CallRecord], key: Tuple[int, int], rec: _CallRecord, owners) -> None:
-    """Put ``rec`` among the records of a buffer until one of its ``owners`` dies, the tensors whose ids are the key."""
-    if key not in records and len(records) >= _MAX_CALL_RECORDS:
-        records.pop(next(iter(records)), None)
-
-    def drop(_, records=records, key=key):
-        records.pop(key, None)
-
-    for i, t in owners:
-        if t is not None:
-            rec.refs[i] = weakref.ref(t, drop)
+def _keep_record(records: Dict[Tuple[int, int], _CallRecord], key: Tuple[int, int], rec: _CallRecord) -> None:
+    """Put ``rec`` among the records of a buffer; when they are too many those of weights that are gone give way, or else the
+    oldest."""
+    records.pop(key, None)
+    if len(records) >= _MAX_CALL_RECORDS:
+        for k in [k for k, r in records.items() if r.refs[0]() is None] or [next(iter(records))]:
+            del records[k]
     records[key] = rec
 
 
@@ -345,7 +341,7 @@ def fp8_fp4_mega_moe(y: torch.Tensor, l1_weights, l2_weights, sym_buffer, shared
             or activation_alpha != 1.0 or activation_beta != 0.0):
         rec = _validate(y, l1_weights, l2_weights, sym_buffer, shared_l1_weights, shared_l2_weights, stats, recipe,
                         activation, activation_clamp, fast_math, activation_alpha, activation_beta, tensors)
-        _keep_record(sym_buffer._call_records, key, rec, ((0, tensors[0]), (8, stats)))
+        _keep_record(sym_buffer._call_records, key, rec)
     else:
         # the record vouches for everything but the output tensor and the clamp
         assert y.dim() == 2 and y.size(1) == sym_buffer.hidden and y.dtype == torch.bfloat16 and y.is_contiguous(), \
