@@ -73,6 +73,15 @@ static void cuts() {
   }
 }
 
+// pairs <pair_above> <cap> <n> <on pairs> <tiles if not> <pair tasks if so>
+static void pairs() {
+  for (int pair_above : {192, kNeverPair, 0})
+    for (int cap : {kDeepTileRows, kSmallTileRows})
+      for (int n = 1; n <= 1100; ++n)
+        printf("pairs %d %d %d %d %d %d\n", pair_above, cap, n, on_pairs(n, pair_above, cap), cut_rows(n, false, cap).parts,
+               cut_rows(n, true, cap).parts / 2);
+}
+
 // abi <version> <bytes of MmoeGeometry> <MmoeLayout> <MmoeWeights> <MmoeOptions>
 static void abi() {
   printf("abi %d %zu %zu %zu %zu\n", MMOE_ABI_VERSION, sizeof(MmoeGeometry), sizeof(MmoeLayout), sizeof(MmoeWeights), sizeof(MmoeOptions));
@@ -84,5 +93,6 @@ int main(int argc, char** argv) {
     else if (strcmp(argv[i], "cache") == 0) cache();
     else if (strcmp(argv[i], "abi") == 0) abi();
     else if (strcmp(argv[i], "cuts") == 0) cuts();
+    else if (strcmp(argv[i], "pairs") == 0) pairs();
   return 0;
 }

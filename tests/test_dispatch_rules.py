@@ -86,3 +86,16 @@ def test_cuts_fit_their_tiles_and_scale_chunks(rules):
         case = (block_m, pairs, cap, n)
         assert step % 16 == 0 and step <= (128 if pairs else cap) and parts * step >= n and tiles <= parts, case
         assert tiles <= chunks, case
+
+
+def test_experts_just_past_one_pair_task(rules):
+    """Above the line experts run on pairs, unless a second task would be nearly empty and the weights-as-A kernels take no more
+    than four tiles of 80 rows, or three of 112, instead -- in the call's own tile size."""
+    for pair_above, cap, n, on_pairs, tiles, tasks in rules("pairs"):
+        case = (pair_above, cap, n)
+        if pair_above != 192:
+            assert on_pairs == (pair_above == 0), case
+        elif n <= 192 or 256 < n <= (320 if cap == 80 else 336):
+            assert not on_pairs and tiles <= (4 if cap == 80 else 3), case
+        else:
+            assert on_pairs, case

@@ -357,6 +357,26 @@ def test_calls_in_flight_together_on_two_streams(m):
             assert torch.equal(y, want), i
 
 
+@pytest.mark.parametrize("cold", [28, 2])
+def test_experts_just_past_one_pair_task(cold):
+    """321, 320 and 257 rows beside experts of a few rows: with many of those the tiles have 80 rows and 321 are a second pair
+    task, with few of them 112 rows and all three experts are cut into three tiles."""
+    layer = H.make_layer(512, 256, 32, 6, True, seed=43)
+    m = 340
+    hid = O.make_hidden(m, layer.hidden, 3)
+    ids = torch.full((m, 6), -1, dtype=torch.int64)
+    for slot, n in enumerate((321, 320, 257)):
+        ids[m - n:, slot] = slot + 1
+    for t in range(3 * cold):
+        ids[t, 3] = 4 + t % cold
+    w = torch.rand((m, 6), generator=torch.Generator().manual_seed(1))
+    y, buf = H.run_layer(layer, hid, ids, w)
+    words = buf.plan_words.cpu().tolist()
+    tiles, small, cap = words[0], words[6], words[7]
+    assert (small, cap, tiles - small) == ((cold + 8, 80, 4) if cold == 28 else (cold + 9, 112, 0))
+    assert_parity(y, H.oracle_layer(layer, hid, ids, w), f"cold {cold}")
+
+
 @pytest.mark.parametrize("bm", [16, 128, 192, 240])
 def test_few_tokens_that_name_an_expert_many_times(bm):
     """40 tokens, nearly all six slots of each on one expert: up to 239 rows in a call that is sized for 40 per expert."""

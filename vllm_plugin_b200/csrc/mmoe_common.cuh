@@ -25,11 +25,15 @@ constexpr int kNeverPair = 0x7fffffff;
 constexpr int kDeepTileRows = 80;
 
 // Which kernels run a routed expert depends on the rows it received in this call: above `pair_above` (see kPairAbove) the CTA
-// pairs, except where they would start a second task for at most 80 rows.  A pair task takes 2 x 562 clk of SM time per stage
-// however few its rows, three weights-as-A tiles of up to 112 rows take about 1450 together: 270 rows per expert (48 experts)
-// 791 -> 683 us, 330 rows 873 -> 768, 281 rows (16 experts) 325 -> 302; at 400 rows four tiles lose (930 -> 957).
-__host__ __device__ inline bool on_pairs(int n, int pair_above) {
-  return n > pair_above && (pair_above == 0 || n <= 2 * kPairTileRows || n > 3 * kSmallTileRows);
+// pairs, except where they would start a second task for at most 80 rows and the weights-as-A kernels, whose tiles have up to
+// `small_cap` rows in this call, take at most four tiles instead.  A pair task takes 2 x 562 clk of SM time per stage however few
+// its rows, a tile 430-500.  Three tiles of 112: 280 rows on each of 48 experts 727 -> 608 us, 336 rows 789 -> 667; at 400
+// rows four lose (930 -> 957).  Four tiles of 80, a few such experts among cold ones: 12 x 280 rows among 97 experts
+// 463.5 -> 453.6, 40 x 300 among 384 1745 -> 1647, 5 x 320 among 48 281.7 -> 258.7.  Five tiles, 321 to 336 rows, lose: 12 x 322
+// among 97 477.2 -> 484.6, 12 x 336 479.3 -> 489.3; 40 among 384 and 5 among 48 within 2 %.
+__host__ __device__ inline bool on_pairs(int n, int pair_above, int small_cap) {
+  const int few_tiles = small_cap >= kSmallTileRows ? 3 * kSmallTileRows : 4 * kDeepTileRows;
+  return n > pair_above && (pair_above == 0 || n <= 2 * kPairTileRows || n > few_tiles);
 }
 
 // How the n rows of an expert are cut into tiles.  Weights-as-A kernels: ceil(n / small_cap) equal tiles (rounded up to 16

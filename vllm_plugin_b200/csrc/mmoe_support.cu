@@ -550,10 +550,11 @@ __device__ ExpertPlan build_plan(const PlanView& pv, int n, const PlanArgs& a, b
   if (threadIdx.x == 0) s_rows = 16;
   // With pair tiles in the call or rows from other ranks, weights-as-A tiles of 112 rows (four stages fit the shared memory) only
   // when enough experts gain a tile by it, else of 80 (five stages).
-  const bool small = n > 0 && !on_pairs(n, a.pair_above);
-  const bool wide = small && ((n > kDeepTileRows && n <= kSmallTileRows) || n > 2 * kDeepTileRows);
-  const int num_small = __syncthreads_count(small), num_wide = __syncthreads_count(wide);
+  const bool may_be_small = n > 0 && !on_pairs(n, a.pair_above, kSmallTileRows);
+  const bool wide = may_be_small && ((n > kDeepTileRows && n <= kSmallTileRows) || n > 2 * kDeepTileRows);
+  const int num_small = __syncthreads_count(may_be_small), num_wide = __syncthreads_count(wide);
   const int cap = a.pair_above == kNeverPair && a.num_ranks == 1 ? small_only_cap(a.m, a.block_m) : (num_wide * 8 > num_small ? kSmallTileRows : kDeepTileRows);
+  const bool small = n > 0 && !on_pairs(n, a.pair_above, cap);
   const Cut cut = cut_rows(n, n > 0 && !small, cap);
   const Cut sh_cut = shared_cut(a.has_shared ? a.m : 0, a.pair_above);
   const bool shared_small = a.m <= a.pair_above;
@@ -863,7 +864,7 @@ __global__ void __launch_bounds__(256) route_place_kernel(const RouteArgs r) {
         const int j = r.chunk_count[(int64_t)(t / kSortChunkTokens) * r.a.e_local + e] + r.route_pos[i];
         const int block = pv.expert_block_off[e];
         const int total = pv.expert_total[e];
-        const Cut cut = cut_rows(total, on_pairs(total, r.a.pair_above), cap);
+        const Cut cut = cut_rows(total, on_pairs(total, r.a.pair_above, cap), cap);
         const int part = j / cut.step;
         pos = r.send_offset[e] + j;
         row = block * r.a.block_m + j;
