@@ -72,15 +72,12 @@ def test_every_block_m_variant(bm):
 
 @pytest.mark.parametrize("geom", [dict(hidden=512, inter=256, num_experts=8, num_topk=2),
                                   dict(hidden=1024, inter=384, num_experts=4, num_topk=2)])
-@pytest.mark.parametrize("orientation", [2, 3])
 @pytest.mark.parametrize("bm", [16, 64, 128, 192, 240])
-def test_tokens_as_a_kernels_every_block_m(geom, bm, orientation):
-    """The tokens-as-A kernel family forced on (it is otherwise chosen from the expected rows per expert): tiles of up
-    to 128 rows under every BLOCK_M pool layout, weight blocks of 192 stored rows with the short last block of a half
-    (64 or 128 rows, loaded through the shifted box), scale chunks starting at row 0 and 64 of a 128-row chunk, the
-    shared expert's tiles, masked routes and experts without tokens.  Orientation 3 runs them on CTA pairs (two tiles of
-    an expert per task, an empty second tile where an expert has an odd number; BLOCK_M < 128 falls back to single
-    CTAs).  Against the oracle, and against the weights-as-A kernels on the same inputs."""
+def test_tokens_as_a_kernels_every_block_m(geom, bm):
+    """The CTA-pair kernels forced on (they otherwise get the experts with many rows): tiles of up to 128 rows under every
+    BLOCK_M pool layout, 256-row weight blocks of which each CTA of the pair loads half, an empty second tile where an expert's
+    rows fit the first, scale chunks of blocks that a tile does not follow, the shared expert's tiles, masked routes and experts
+    without tokens.  Against the oracle, and against the weights-as-A kernels on the same inputs."""
     from vllm_plugin_b200 import api
     layer = H.make_layer(shared=True, seed=21, **geom)
     m = 600
@@ -89,7 +86,7 @@ def test_tokens_as_a_kernels_every_block_m(geom, bm, orientation):
     ids[ids == 1] = -1                                      # an expert that receives nothing
     api.set_kernel_options(block_m=bm)
     try:
-        y_tm, buf = H.run_layer(layer, hid, ids, w, orientation=orientation)
+        y_tm, buf = H.run_layer(layer, hid, ids, w, orientation=2)
         assert buf.plan_tables()[0]["block_m"] == bm
         y_sa, _ = H.run_layer(layer, hid, ids, w, orientation=1)
     finally:
@@ -104,8 +101,8 @@ def test_tokens_as_a_kernels_every_block_m(geom, bm, orientation):
 @pytest.mark.parametrize("orientation", [2, 3])
 @pytest.mark.parametrize("m", [1, 40, 129, 700])
 def test_tokens_as_a_kernels_token_counts_and_options(m, orientation):
-    """Forced tokens-as-A kernels over small and ragged token counts (tiles of 1..128 rows, the 64-row token box), with
-    the two-slice weight form, without clamp, and with the IEEE sigmoid."""
+    """Forced pair kernels (2 and 3 name the same form) over small and ragged token counts (tiles of 1..128 rows, token boxes of
+    32 to 128 rows), with the two-slice weight form, without clamp, and with the IEEE sigmoid."""
     layer = H.make_layer(shared=True, seed=23, hidden=1024, inter=512, num_experts=4, num_topk=2)
     hid = (O.make_hidden(m, layer.hidden, 1).float() * 3).to(torch.bfloat16)
     ids, w = O.make_routing(m, layer.num_experts, layer.num_topk, 2, mask_frac=0.1 if m > 1 else 0.0)
@@ -355,6 +352,55 @@ def test_calls_in_flight_together_on_two_streams(m):
         api.read_status(buf)
         for i, y in enumerate(ys):
             assert torch.equal(y, want), i
+
+
+@pytest.mark.parametrize("geom", [dict(hidden=512, inter=256, num_experts=8, num_topk=6),
+                                  dict(hidden=512, inter=256, num_experts=40, num_topk=31),
+                                  dict(hidden=256, inter=128, num_experts=512, num_topk=6)])
+@pytest.mark.parametrize("m", [1, 15, 16, 17])
+def test_staged_tokens_equal_placed_rows(geom, m):
+    """Calls of at most 16 tokens in pool blocks of 16 rows multiply the staged tokens as they are and order the routes inside
+    GEMM1; with blocks of 32 rows the same call places its rows first.  Bit for bit the same output rows, counts and ``y``, at
+    the largest numbers of routes and experts too, when all slots of a token name one expert (more than 32 rows of 16 tokens),
+    and with ids past the last expert, which are counted and masked."""
+    from vllm_plugin_b200 import api
+    layer = H.make_layer(shared=True, seed=71, **geom)
+    e, k = layer.num_experts, layer.num_topk
+    weights = H.kernel_weights(layer, "cuda")
+    hid = O.make_hidden(m, layer.hidden, 3)
+    ids, w = O.make_routing(m, e, k, 4, zipf_s=1.2, mask_frac=0.1)
+    repeated = ids[:, :1].clamp(min=0).expand(m, k).clone()
+    repeated[0] = e - 1
+    beyond = ids.clone()
+    beyond[0, 0], beyond[m - 1, k - 1] = e, 2 ** 40
+    for case, valid in ((ids, ids), (repeated, repeated), (beyond, torch.where(beyond >= e, -1, beyond))):
+        got = []
+        for bm in (16, 32):
+            api.set_kernel_options(block_m=bm)
+            stats = torch.zeros(e, dtype=torch.int32, device="cuda")
+            buf = None
+            try:
+                if case is beyond:
+                    buf = got[0][1] if got else H.run_layer(layer, hid, valid, w, weights=weights)[1]
+                    with pytest.raises(AssertionError, match="expert ids"):
+                        H.run_layer(layer, hid, case, w, weights=weights, buf=buf)
+                    y = torch.empty((m, layer.hidden), dtype=torch.bfloat16, device="cuda")
+                    api.stage_inputs_for_mega_moe(buf, hid.cuda(), case.cuda(), w.cuda())
+                    api.fp8_fp4_mega_moe(y, weights[0], weights[1], buf, weights[2], weights[3], stats, activation_clamp=10.0)
+                    with pytest.raises(AssertionError, match="2 expert ids"):
+                        api.read_status(buf)
+                else:
+                    y, buf = H.run_layer(layer, hid, case, w, weights=weights, stats=stats, buf=buf)
+            finally:
+                api.set_kernel_options(block_m=0)
+            rows = int((valid >= 0).sum())
+            assert torch.equal(stats.cpu().long(), torch.bincount(valid[valid >= 0], minlength=e))
+            got.append((y, buf, buf.ret[:rows].clone(), buf.route_pos[:m].clone(), buf.sorted_route[:rows].clone(), stats))
+        for a, b in zip(got[0][2:], got[1][2:]):
+            assert torch.equal(a, b)
+        assert torch.equal(got[0][0], got[1][0])
+        if e <= 40:
+            assert_parity(got[0][0], H.oracle_layer(layer, hid, valid, w), f"m {m} e {e}")
 
 
 @pytest.mark.parametrize("cold", [28, 2])
