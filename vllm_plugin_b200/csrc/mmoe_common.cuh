@@ -278,12 +278,14 @@ inline bool staged_tokens(const Ctx& c, int m, int block_m) {
 
 
 // ---------------------------------------------------------------------------------------------------------------------
-// Programmatic dependent launch.  The kernels of one call form a chain on a stream; each of them begins with
-// chain_begin(): it lets the NEXT kernel of the stream be scheduled as soon as every block of this one has started
-// (so that kernel's launch latency and set-up -- barrier initialisation, tensor-memory allocation -- overlap this
-// kernel's run) and then waits until everything BEFORE this kernel in the stream has completed and its memory is
-// visible.  A kernel must not touch global memory before chain_begin().  The wait is transitive: the next kernel's
-// wait ends only when this grid has completed, and this grid completes only after its own wait has.  Both
+// Programmatic dependent launch.  The kernels of one call form a chain on a stream.  chain_release() lets the NEXT kernel of
+// the stream be scheduled as soon as every block of this one has come to it or ended (so that kernel's launch latency and
+// set-up -- barrier initialisation, tensor-memory allocation -- overlap this kernel's run); chain_wait() waits until
+// everything BEFORE this kernel in the stream has completed and its memory is visible.  Most kernels begin with both, in this
+// order (chain_begin()), and touch no global memory before.  The wait is transitive: the next kernel's wait ends only when
+// this grid has completed, and this grid completes only after its own wait has.  A kernel of this library that waits first
+// and releases then tells its successor more: what precedes IT has completed when the successor starts, which may use that
+// without a wait.  Nothing is taken to be complete about a kernel from elsewhere, which may release as early as it likes.  Both
 // instructions do nothing in a kernel that was launched without the attribute below.
 // ---------------------------------------------------------------------------------------------------------------------
 __device__ __forceinline__ void chain_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }

@@ -61,8 +61,6 @@ struct UmmaParams {
   __nv_bfloat16* ret;
   __nv_bfloat16* shared_out;
   int32_t* pool_dst;
-  // layer 2 at EP > 1 with the write-back fused in: an output row goes straight into the `ret_recv` of the rank its
-  // token came from (plain peer stores over NVLink), at that rank's send position
   SharedTiles shared_tiles;    // run first
   int with_routed;             // 0: only those
   int tile_rows;               // > 0: rows of the call's largest tile, known to the host; 0: in the plan
@@ -85,6 +83,8 @@ struct UmmaParams {
   uint4* pool_x;
   int32_t* pool_sf;
   int64_t pool_sf_rows;
+  // layer 2 at EP > 1 with the write-back fused in: an output row goes straight into the `ret_recv` of the rank its
+  // token came from (plain peer stores over NVLink), at that rank's send position
   int ep_me;
   const int32_t* ep_totals;    // [32][32]: totals[s][d] = routes rank s sent to rank d in this call
   __nv_bfloat16* ep_ret_recv[32];
