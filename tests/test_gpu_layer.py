@@ -125,6 +125,19 @@ def test_options_fast_math_clamp_and_localized_weights():
     assert torch.equal(y0, y1)
 
 
+@pytest.mark.parametrize("hidden", [256, 512, 768, 1280])
+@pytest.mark.parametrize("m", [3, 60, 260])
+def test_two_slice_weights_of_any_hidden_size(hidden, m):
+    """Slices of W2 with an odd number of 128-row blocks: a task of 256 rows reaches from one slice into the other."""
+    layer = H.make_layer(hidden, 256, 4, 2, True, seed=10)
+    hid = O.make_hidden(m, hidden, 1)
+    ids, w = O.make_routing(m, 4, 2, 2)
+    y0, _ = H.run_layer(layer, hid, ids, w)
+    y1, _ = H.run_layer(layer, hid, ids, w, localized=True)
+    assert torch.equal(y0, y1)
+    assert_parity(y0, H.oracle_layer(layer, hid, ids, w), f"hidden {hidden} m {m}")
+
+
 def test_masked_tokens_padding_and_empty_call():
     layer = H.make_layer(shared=False, seed=11, **SMALL)
     m = 20

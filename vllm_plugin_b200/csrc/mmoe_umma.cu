@@ -94,6 +94,7 @@ struct UmmaParams {
   int k_dim;                   // reduction length: H (layer 1) or I (layer 2)
   int rows_per_expert;         // 2I (layer 1) or H (layer 2)
   int routed_sliced;           // 1: routed weights are [2, E_l, rows/2, K/2] (two slices), 0: [E_l, rows, K/2]
+  int routed_halves;           // layer 2: 1 when a slice is not whole 256-row blocks; the map's box is 128 rows then
   int n_blocks;                // 128-row weight blocks per tile: I/128 (layer 1) or H/128 (layer 2)
   int hidden, inter;
   float clamp;
@@ -442,6 +443,11 @@ __device__ __forceinline__ void sa_producer(const UmmaParams& p, const Cta& c, T
     const int slice = sliced ? r0 / rows_slice : 0;
     const int row = e * rows_slice + r0 % rows_slice;
     const int group = row / 16;
+    // Layer 2 with slices of an odd number of 128-row blocks: the task's two blocks are loaded one by one, the second may be in
+    // the other slice.
+    const bool halves = kLayer == 2 && sliced && p.routed_halves != 0;
+    const int slice2 = halves ? (r0 + kTileRows) / rows_slice : 0;
+    const int row2 = halves ? e * rows_slice + (r0 + kTileRows) % rows_slice : 0;
     const int32_t* wsf = (shared ? p.wsf_shared : p.wsf_routed) + (int64_t)e * k_stages * p.rows_per_expert + r0;
     const int64_t tsf_rows = shared ? p.tsf_rows_shared : p.tsf_rows_routed;
     const int32_t* tsf = (shared ? p.tsf_shared : p.tsf_routed) + (int64_t)tile.sf_chunk * kChunkRows;
@@ -453,6 +459,7 @@ __device__ __forceinline__ void sa_producer(const UmmaParams& p, const Cta& c, T
         tma_load_5d(a0 + stage * L::kABytes, wmap, k0, 0, group, 0, slice, bar);
       } else {
         tma_load_3d(a0 + stage * L::kABytes, wmap, k0, row, slice, bar);
+        if (halves) tma_load_3d(a0 + stage * L::kABytes + kTileRows * kTileK, wmap, k0, row2, slice2, bar);
         bulk_load(sf0 + stage * L::kSfBytes, sf, 1024, bar);       // two chunks already in tensor-memory order
       }
     };
@@ -1176,8 +1183,9 @@ bool set_weights(const Ctx& c, const MmoeWeights& w, bool has_shared, SaPlan* pl
   p2.wsf_shared = static_cast<const int32_t*>(w.shared_w2_sf);
   p1.routed_sliced = w.w13_slice_stride > 0 ? 1 : 0;
   p2.routed_sliced = w.w2_slice_stride > 0 ? 1 : 0;
+  p2.routed_halves = w.w2_slice_stride > 0 && (h / 2) % (2 * kTileRows) != 0 ? 1 : 0;
   int bad = make_w13_map(&p1.map_w_routed, true, w.w13, h, (uint64_t)el * 2 * inter, w.w13_slice_stride);
-  bad |= make_weight_map(&p2.map_w_routed, true, w.w2, inter, (uint64_t)el * h, w.w2_slice_stride, 2 * kTileRows);
+  bad |= make_weight_map(&p2.map_w_routed, true, w.w2, inter, (uint64_t)el * h, w.w2_slice_stride, (p2.routed_halves != 0 ? 1 : 2) * kTileRows);
   if (has_shared) {
     bad |= make_w13_map(&p1.map_w_shared, false, w.shared_w13, h, 2 * (uint64_t)inter, 0);
     bad |= make_weight_map(&p2.map_w_shared, false, w.shared_w2, inter, (uint64_t)h, 0, 2 * kTileRows);
