@@ -260,9 +260,10 @@ struct TaskWalk {
 // ------------------------------------------------------------------------------------------------ routing in the launch
 // Calls of at most kStagedTokens tokens: the epilogue warps of the first CTA to ask, idle until its first accumulator 15 us
 // later, order the routes and build the plan, which only epilogues and GEMM2 need.  All other CTAs wait for that one, so it has
-// to be one that runs: a CTA takes an SM to itself, and work on other streams may hold any of them back for as long as it likes.  A launch of its own took 8-20 us in front of GEMM1: little
-// work, but every instruction line comes from DRAM (each call streams its weights through the L2), so what counts is that
-// the code is short.  Pool blocks and tiles have 16 rows here, hence one tile per block.
+// to be one that runs: a CTA takes an SM to itself, and work on other streams may hold any of them back for as long as it
+// likes.  A launch of its own took 8-20 us in front of GEMM1: little work, but every instruction line comes from DRAM (each
+// call streams its weights through the L2), so what counts is that the code is short.  Pool blocks and tiles have 16 rows
+// here, hence one tile per block.
 constexpr int kRouteThreads = 128;
 constexpr int kMaxHereRoutes = kStagedTokens * 31, kMaxHereExperts = 512;
 struct alignas(16) RouteScratch {
