@@ -597,26 +597,35 @@ __device__ ExpertPlan build_plan(const PlanView& pv, int n, const PlanArgs& a, b
   return ExpertPlan{block_off, at.b, cut};
 }
 
-// Scale words of the call's own tokens in the chunks of the shared expert's tiles (chunk j = tile j), whole warps.
+// Scale words of the call's own tokens in the chunks of the shared expert's tiles (chunk j = tile j), whole warps: a warp takes
+// one word of all rows of a tile, so that its 128 words leave as one line (positions 4 (i % 32) + i / 32, see chunk_pos).  A warp
+// per token, which scattered the token's 40 words over as many lines, eight tokens one after the other, took 8-16 us of the
+// counting launch.
 struct SharedScales {
   const int32_t* x_sf;
   int32_t* out;          // nullptr: no shared expert
   int64_t rows;
   Cut cut;
 };
-__device__ void place_shared_scales(const SharedScales& s, int t, int words) {
-  const Cut cut = s.cut;
-  const int j = t / cut.step;
-  const int64_t pos = (int64_t)j * kChunkRows + chunk_pos(t - j * cut.step);
-  for (int w = threadIdx.x & 31; w < words; w += 32) s.out[w * s.rows + pos] = s.x_sf[(int64_t)t * words + w];
+__device__ void place_shared_scales(const SharedScales& s, int m, int words, int warp, int warps) {
+  const int lane = threadIdx.x & 31;
+  for (int task = warp; task < s.cut.parts * words; task += warps) {
+    const int j = task / words, w = task - j * words;
+    int32_t v[4];
+#pragma unroll
+    for (int a = 0; a < 4; ++a) {
+      const int i = lane + 32 * a, t = j * s.cut.step + i;
+      v[a] = i < s.cut.step && t < m ? s.x_sf[(int64_t)t * words + w] : 0;
+    }
+    *reinterpret_cast<int4*>(s.out + w * s.rows + (int64_t)j * kChunkRows + 4 * lane) = make_int4(v[0], v[1], v[2], v[3]);
+  }
 }
 
 // The shared expert's tiles depend only on the token count: with its scale chunks written it can run before the routed
 // experts' receive counts are known.
 __global__ void __launch_bounds__(256) shared_plan_kernel(int m, SharedScales scales, int words) {
   chain_begin();
-  const int warps = (gridDim.x * blockDim.x) >> 5;
-  for (int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < m; t += warps) place_shared_scales(scales, t, words);
+  place_shared_scales(scales, m, words, static_cast<int>((blockIdx.x * blockDim.x + threadIdx.x) >> 5), static_cast<int>((gridDim.x * blockDim.x) >> 5));
 }
 
 // General plan (any number of source ranks), one block: rows per expert from the receive counts, and for every (expert,
@@ -797,10 +806,17 @@ __global__ void __launch_bounds__(kRouteThreads) route_small_kernel(const RouteA
 }
 
 // Larger calls, first of two launches: one block per 128 tokens ranks its routes; the last block to finish sums the chunks
-// and builds the plan.
+// and builds the plan.  Further blocks place the shared expert's scales, which GEMM1 starts with while the next launch still places.
+__host__ __device__ inline int route_chunks(int m) { return m > kSortChunkTokens ? (m + kSortChunkTokens - 1) / kSortChunkTokens : 1; }
+
 __global__ void __launch_bounds__(kRouteThreads) route_count_kernel(const RouteArgs r) {
   chain_begin();
   extern __shared__ int32_t sm[];
+  const int chunks = route_chunks(r.a.m);
+  if ((int)blockIdx.x >= chunks) {
+    place_shared_scales(r.shared, r.a.m, r.h / kTileK, (blockIdx.x - chunks) * kRouteWarps + (threadIdx.x >> 5), (gridDim.x - chunks) * kRouteWarps);
+    return;
+  }
   const int E = r.a.e_local, r0 = blockIdx.x * kSortChunkTokens * r.k;
   const int n = max(0, min(kSortChunkTokens * r.k, r.a.m * r.k - r0)), n_even = (kSortChunkTokens * r.k + 1) & ~1;
   uint16_t* ids = reinterpret_cast<uint16_t*>(sm);
@@ -811,10 +827,6 @@ __global__ void __launch_bounds__(kRouteThreads) route_count_kernel(const RouteA
     if (id >= E) { report_bad_index(r.status); id = -1; }
     ids[i] = id < 0 ? 0xFFFF : static_cast<uint16_t>(id);
   }
-  // scale chunks of the shared expert's tiles: written here because GEMM1 starts with them while the next launch still places
-  if (r.shared.out != nullptr)
-    for (int t = blockIdx.x * kSortChunkTokens + (threadIdx.x >> 5); t < min(r.a.m, (blockIdx.x + 1) * kSortChunkTokens); t += kRouteWarps)
-      place_shared_scales(r.shared, t, r.h / kTileK);
   int total = block_rank_routes(ids, n, rank, warp_count, E);
   for (int i = threadIdx.x; i < n; i += kRouteThreads) r.route_pos[r0 + i] = ids[i] == 0xFFFF ? -1 : rank[i];
   const int e = threadIdx.x;
@@ -823,20 +835,20 @@ __global__ void __launch_bounds__(kRouteThreads) route_count_kernel(const RouteA
   __shared__ int last;
   __threadfence();
   __syncthreads();
-  if (threadIdx.x == 0) last = atomicAdd(&pv.hdr->ticket, 1) == (int)gridDim.x - 1;
+  if (threadIdx.x == 0) last = atomicAdd(&pv.hdr->ticket, 1) == chunks - 1;
   __syncthreads();
   if (!last) return;
   __threadfence();
   if (threadIdx.x == 0) pv.hdr->ticket = 0;
   total = 0;
   if (e < E)
-    for (int c0 = 0; c0 < (int)gridDim.x; c0 += 8) {         // eight independent loads in flight
+    for (int c0 = 0; c0 < chunks; c0 += 8) {         // eight independent loads in flight
       int v[8];
 #pragma unroll
-      for (int u = 0; u < 8; ++u) v[u] = c0 + u < (int)gridDim.x ? __ldcg(&r.chunk_count[(int64_t)(c0 + u) * E + e]) : 0;
+      for (int u = 0; u < 8; ++u) v[u] = c0 + u < chunks ? __ldcg(&r.chunk_count[(int64_t)(c0 + u) * E + e]) : 0;
 #pragma unroll
       for (int u = 0; u < 8; ++u) {
-        if (c0 + u < (int)gridDim.x) r.chunk_count[(int64_t)(c0 + u) * E + e] = total;
+        if (c0 + u < chunks) r.chunk_count[(int64_t)(c0 + u) * E + e] = total;
         total += v[u];
       }
     }
@@ -919,7 +931,7 @@ __global__ void __launch_bounds__(256) place_kernel(
   const int warp_in_block = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
   if (shared.out != nullptr) {
     const int m = pv.hdr->num_tokens;
-    for (int t = blockIdx.x * warps + warp_in_block; t < m; t += gridDim.x * warps) place_shared_scales(shared, t, words);
+    place_shared_scales(shared, m, words, blockIdx.x * warps + warp_in_block, gridDim.x * warps);
   }
   constexpr int kSlices = kPairTileRows / 32;
   for (int task = blockIdx.x; task < ntiles * kSlices; task += gridDim.x) {
@@ -1018,9 +1030,10 @@ cudaError_t launch_route_small(const Ctx& c, int m, int block_m, int32_t* stats,
 
 cudaError_t launch_route_large(const Ctx& c, int m, int block_m, int32_t* stats, cudaStream_t s) {
   const RouteArgs r = route_args(c, m, block_m, stats);
-  const int chunks = std::max(1, (m + kSortChunkTokens - 1) / kSortChunkTokens);
+  const int chunks = route_chunks(m);
+  const int scale_blocks = r.shared.out == nullptr ? 0 : std::min((r.shared.cut.parts * (r.h / kTileK) + kRouteWarps - 1) / kRouteWarps, 148);
   const size_t smem = (size_t)2 * ((kSortChunkTokens * r.k + 1) & ~1) * 2 + (size_t)kRouteWarps * r.a.e_local * 2;
-  launch_chained(route_count_kernel, dim3(chunks), dim3(kRouteThreads), smem, s, r);
+  launch_chained(route_count_kernel, dim3(chunks + scale_blocks), dim3(kRouteThreads), smem, s, r);
   if (m > 0) launch_chained(route_place_kernel, dim3(std::min((m + 7) / 8, 148 * 8)), dim3(256), 0, s, r);
   return cudaGetLastError();
 }
