@@ -237,11 +237,12 @@ int mmoe_combine_residual(const MmoeGeometry* geo, void* workspace, void* y_bf16
 /* EP1 convenience: count, place, experts, combine; same result as the separate calls.  One stream, one programmatic chain
  * of launches, so that each one's launch and set-up overlap its predecessor (MMOE_DISABLE_CHAINED_LAUNCH=1 in the
  * environment, read once per process: ordinary launches).  The first kernel of the chain reads nothing before everything in front
- * of the call has ended, whether or not the kernel in front triggers its successors early.  Up to 16 tokens (BLOCK_M 16) three launches: GEMM1 orders the
- * routes itself and takes the staged tokens as they are.  Up to 128 tokens four: one launch orders the routes, builds
- * the plan and places the rows in front of GEMM1, GEMM2 and combine.  Past that ordering and placement are two launches, and
- * past 192 tokens each GEMM is two: the experts with many rows on CTA pairs, the others on the weights-as-A kernels.  The
- * shared expert's tiles come first in GEMM1, which starts with them while the rows are still being placed. */
+ * of the call has ended, whether or not the kernel in front triggers its successors early.  Both GEMMs
+ * are one launch, in which each CTA claims its tasks.  Up to 16 tokens (BLOCK_M 16) it also orders the routes and takes
+ * the staged tokens as they are: two launches with the combine.  Up to 128 tokens three: one launch orders the routes,
+ * builds the plan and places the rows in front.  Past that ordering and placement are two launches, and past 192 tokens
+ * the experts with many rows run in two launches of their own, on CTA pairs.  The shared expert's tiles come first, while
+ * the rows are still being placed. */
 int mmoe_forward(const MmoeGeometry* geo, void* workspace, const MmoeWeights* weights, const MmoeOptions* opt,
                  void* y_bf16, int32_t num_tokens, int32_t block_m, int32_t* stats, void* stream);
 

@@ -579,3 +579,42 @@ def test_tile_cuts_at_their_edges(m, rows):
     read_status(buf)
     assert torch.equal(buf.l1_acts.view(torch.uint8), pool_one) and torch.equal(buf.l2_acts.view(torch.uint8), act_one)
     assert torch.equal(y, y_one)
+
+
+@pytest.mark.parametrize("hidden,inter,experts,shared", [(256, 128, 4, True), (256, 128, 512, False), (512, 256, 40, True), (2560, 1152, 6, True)])
+@pytest.mark.parametrize("m", [1, 16, 17, 129, 193])
+def test_both_gemms_in_one_launch(hidden, inter, experts, shared, m):
+    """Fewer tasks than CTAs and many times more, K loops of 1, 2 and 20 stages, with and without a shared expert, no expert hit at
+    all: bit for bit what a launch per GEMM leaves, call after call, with the counters of the launch back at zero."""
+    import ctypes
+    from vllm_plugin_b200 import api
+    from vllm_plugin_b200.backend import _native
+    from vllm_plugin_b200.backend.frontend import _weights_struct, check_mega_moe_arguments, read_status
+    layer = H.make_layer(hidden, inter, experts, min(6, experts), shared, seed=51)
+    dev = torch.device("cuda", 0)
+    weights = H.kernel_weights(layer, dev)
+    l1, l2, sl1, sl2 = weights
+    buf = None
+    for call in range(4):
+        hid = O.make_hidden(m, hidden, 7 + call)
+        ids, w = O.make_routing(m, experts, layer.num_topk, 8 + call, zipf_s=1.2, mask_frac=0.1)
+        if call == 2:
+            ids = torch.full_like(ids, -1)
+        y_one, buf = H.run_layer(layer, hid, ids, w, weights=weights, buf=buf)
+        assert buf.plan_words[9:14].cpu().tolist() == [0] * 5
+        y = torch.empty_like(y_one)
+        s13, s2 = check_mega_moe_arguments(y, l1, l2, buf, sl1, sl2, None, (1, 1, 32), "swiglu", 10.0, True, 1.0, 0.0)
+        ws = _weights_struct(l1, l2, sl1, sl2, s13, s2)
+        lib, geo, base = _native.load(), ctypes.byref(buf.geo), buf.base_ptr
+        sp = torch.cuda.current_stream(dev).cuda_stream
+        bm = api.stage_inputs_for_mega_moe(buf, hid.to(dev), ids.to(dev), w.to(dev))
+        _native.check(lib.mmoe_dispatch_count(geo, base, m, sp))
+        _native.check(lib.mmoe_dispatch_place(geo, base, m, bm, None, sp))
+        for mask in (1, 2):
+            opts = _native.MmoeOptions(10.0, 1, 0, 2000, mask)
+            _native.check(lib.mmoe_experts(geo, base, ctypes.byref(ws), ctypes.byref(opts), m, bm, sp))
+        _native.check(lib.mmoe_combine(geo, base, y.data_ptr(), m, sp))
+        read_status(buf)
+        assert torch.equal(y, y_one), call
+        if experts <= 40 and call < 2:
+            assert_parity(y_one, H.oracle_layer(layer, hid, ids, w), f"m {m} call {call}")

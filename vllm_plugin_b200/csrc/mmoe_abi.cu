@@ -421,7 +421,7 @@ namespace {
 // `peers` != NULL: EP > 1 with the write-back fused into GEMM2, followed by barrier 2
 int run_experts(const MmoeGeometry* geo, void* workspace, const void* const* peers, const MmoeWeights* weights,
                 const MmoeOptions* opt, int32_t num_tokens, int32_t block_m, void* stream, int tile_select = 0,
-                bool route_in_gemm = false, int32_t* stats = nullptr);
+                bool route_in_gemm = false, int32_t* stats = nullptr, bool both_layers = false);
 
 }  // namespace
 
@@ -463,7 +463,7 @@ int mmoe_experts_ep_return(const MmoeGeometry* geo, void* workspace, const void*
 namespace {
 int run_experts(const MmoeGeometry* geo, void* workspace, const void* const* peers, const MmoeWeights* weights,
                 const MmoeOptions* opt, int32_t num_tokens, int32_t block_m, void* stream, int tile_select, bool route_in_gemm,
-                int32_t* stats) {
+                int32_t* stats, bool both_layers) {
   mmoe::Ctx c;
   int rc = make_ctx(geo, workspace, &c);
   if (rc != MMOE_OK) return rc;
@@ -500,6 +500,7 @@ int run_experts(const MmoeGeometry* geo, void* workspace, const void* const* pee
     c.tile_select = tile_select;
     c.route_in_gemm = route_in_gemm;
     c.stats = stats;
+    c.both_layers = both_layers;
     e = mmoe::launch_experts_umma(c, *weights, o, num_tokens, block_m, st);
     if (e == cudaSuccess && peers != nullptr) e = mmoe::launch_ep_signal_return(c, peers, timeout_ns, st);
   } else {
@@ -509,6 +510,14 @@ int run_experts(const MmoeGeometry* geo, void* workspace, const void* const* pee
 }
 }  // namespace
 
+static int check_combine(const void* y_bf16, const void* residual_bf16, int32_t num_tokens) {
+  if (num_tokens > 0 && (y_bf16 == nullptr || (reinterpret_cast<uintptr_t>(y_bf16) & 15u) != 0))
+    return fail(MMOE_ERR_INVALID_ARGUMENT, "y must be a 16-byte aligned device pointer");
+  if ((reinterpret_cast<uintptr_t>(residual_bf16) & 15u) != 0)
+    return fail(MMOE_ERR_INVALID_ARGUMENT, "the residual must be a 16-byte aligned device pointer");
+  return MMOE_OK;
+}
+
 int mmoe_combine_residual(const MmoeGeometry* geo, void* workspace, void* y_bf16, const void* residual_bf16,
                           int32_t num_tokens, void* stream) {
   mmoe::Ctx c;
@@ -516,10 +525,8 @@ int mmoe_combine_residual(const MmoeGeometry* geo, void* workspace, void* y_bf16
   if (rc != MMOE_OK) return rc;
   rc = check_tokens(geo, num_tokens);
   if (rc != MMOE_OK) return rc;
-  if (num_tokens > 0 && (y_bf16 == nullptr || (reinterpret_cast<uintptr_t>(y_bf16) & 15u) != 0))
-    return fail(MMOE_ERR_INVALID_ARGUMENT, "y must be a 16-byte aligned device pointer");
-  if ((reinterpret_cast<uintptr_t>(residual_bf16) & 15u) != 0)
-    return fail(MMOE_ERR_INVALID_ARGUMENT, "the residual must be a 16-byte aligned device pointer");
+  rc = check_combine(y_bf16, residual_bf16, num_tokens);
+  if (rc != MMOE_OK) return rc;
   cudaError_t e = mmoe::launch_combine(c, y_bf16, residual_bf16, num_tokens, static_cast<cudaStream_t>(stream));
   return e == cudaSuccess ? MMOE_OK : cuda_fail(e, "combine launch");
 }
@@ -542,14 +549,17 @@ int mmoe_forward(const MmoeGeometry* geo, void* workspace, const MmoeWeights* we
   // route ordering, plan and placement: inside the GEMM launches up to kStagedTokens tokens, one launch up to 128, two beyond
   // (and where the pair kernels are forced on: those read the shared expert's scales from chunks that the larger form writes)
   const bool small_only = num_tokens > 0 && c.pair_above_for(num_tokens) == mmoe::kNeverPair;
-  const bool in_gemm = mmoe::staged_tokens(c, num_tokens, block_m) && opt != nullptr && opt->engine == 0 &&
-                       (opt->layer_mask == 0 || opt->layer_mask == 3);
+  const bool both_layers = num_tokens > 0 && opt != nullptr && opt->engine == 0 && (opt->layer_mask == 0 || opt->layer_mask == 3);
+  const bool in_gemm = both_layers && mmoe::staged_tokens(c, num_tokens, block_m);
+  // before any launch: the combine has to follow one of both GEMMs
+  rc = check_combine(y_bf16, opt != nullptr ? opt->residual : nullptr, num_tokens);
+  if (rc != MMOE_OK) return rc;
   if (!in_gemm) {
     const cudaError_t e = small_only && num_tokens <= 128 ? mmoe::launch_route_small(c, num_tokens, block_m, stats, st)
                                                           : mmoe::launch_route_large(c, num_tokens, block_m, stats, st);
     if (e != cudaSuccess) return cuda_fail(e, "route / plan / placement launch");
   }
-  rc = run_experts(geo, workspace, nullptr, weights, opt, num_tokens, block_m, stream, 0, in_gemm, stats);
+  rc = run_experts(geo, workspace, nullptr, weights, opt, num_tokens, block_m, stream, 0, in_gemm, stats, both_layers);
   if (rc == MMOE_OK) rc = mmoe_combine_residual(geo, workspace, y_bf16, opt != nullptr ? opt->residual : nullptr, num_tokens, stream);
   return rc;
 }

@@ -94,14 +94,16 @@ struct PlanHeader {
   int32_t small_cap;           // rows a weights-as-A tile of this call may have
   int32_t small_rows;          // rows of the largest one, rounded up to 16
   int32_t ticket;              // blocks of the route-counting launch that have finished; zero between launches
-  int32_t routed;              // 1 while a GEMM1 launch that orders the routes itself has the plan complete; GEMM2 clears it
-  uint32_t claims;             // CTAs of that GEMM1 launch that have asked to do it, modulo its grid: zero between launches
-  int32_t pad[4];
+  int32_t routed;              // 1 once a GEMM launch that orders the routes itself has the plan complete; zero between calls
+  uint32_t claims;             // CTAs of that launch that have asked to do it, modulo its grid: zero between launches
+  uint32_t next_task;          // tasks of a launch of both GEMMs that have been claimed: zero between calls
+  int32_t layer1_done;         // sum of `done` below: zero between calls
+  int32_t pad[2];
 };
 static_assert(sizeof(PlanHeader) == 64, "plan header is 64 bytes");
 
 // Plan region: header | expert_total[E_l] | expert_block_off[E_l+1] | expert_tile_off[E_l+1] | rank_off[R+1] |
-// seg_pool_start[E_l*R] | seg_recv_start[E_l*R] | tiles[max_tiles]
+// seg_pool_start[E_l*R] | seg_recv_start[E_l*R] | done[E_l+1] | tiles[max_tiles]
 struct PlanView {
   PlanHeader* hdr;
   int32_t* expert_total;
@@ -110,6 +112,7 @@ struct PlanView {
   int32_t* rank_off;
   int32_t* seg_pool_start;
   int32_t* seg_recv_start;
+  int32_t* done;               // launch of both GEMMs: finished parts of GEMM1 per expert, the shared one last; zero between calls
   Tile* tiles;
 };
 
@@ -131,7 +134,7 @@ __host__ __device__ inline int64_t shared_chunk_rows(int64_t max_tokens) { retur
 __host__ __device__ inline int64_t shared_tile_capacity(int64_t max_tokens) { return (max_tokens / 16 + 2) * 2; }
 
 __host__ __device__ inline int64_t plan_bytes(int e_local, int num_ranks, int64_t max_tiles) {
-  int64_t ints = e_local + 2 * (e_local + 1) + (num_ranks + 1) + 2 * (int64_t)e_local * num_ranks;
+  int64_t ints = e_local + 3 * (e_local + 1) + (num_ranks + 1) + 2 * (int64_t)e_local * num_ranks;
   return 64 + align_up(ints * 4, 32) + max_tiles * (int64_t)sizeof(Tile);
 }
 
@@ -146,6 +149,7 @@ __host__ __device__ inline PlanView plan_view(void* base, int e_local, int num_r
   v.rank_off = q;                q += num_ranks + 1;
   v.seg_pool_start = q;          q += (int64_t)e_local * num_ranks;
   v.seg_recv_start = q;          q += (int64_t)e_local * num_ranks;
+  v.done = q;                    q += e_local + 1;
   int64_t ints = q - reinterpret_cast<int32_t*>(p + 64);
   v.tiles = reinterpret_cast<Tile*>(p + 64 + align_up(ints * 4, 32));
   return v;
@@ -237,6 +241,7 @@ struct Ctx {             // resolved pointers of one call
   int kmax;              // min(k, E/R)
   int32_t* stats = nullptr;               // cumulative receive counts, for a GEMM1 launch that orders the routes itself ...
   bool route_in_gemm = false;             // ... which it does when this is set
+  bool both_layers = false;               // the combine that follows zeroes the counters which a launch of both GEMMs leaves
   const void* const* peer_ws = nullptr;   // set by the call that fuses the write-back into GEMM2 (EP > 1)
   int tile_select = 0;                    // 0: every tile of the plan, 1: routed tiles only, 2: the early shared tiles only
   int pair_above = kNeverPair;            // experts with more rows than this run on CTA pairs ...

@@ -1077,10 +1077,28 @@ __device__ __forceinline__ void add_bf16x8(float (&acc)[8], const uint4& v) {
 constexpr int kCombineSegVec = 64;
 __global__ void __launch_bounds__(256) combine_kernel(
     const uint4* __restrict__ rows, const int32_t* __restrict__ route_pos, const uint4* __restrict__ shared_out,
-    const uint4* __restrict__ residual, uint4* __restrict__ y, int m, int h, int k) {
-  chain_begin();
+    const uint4* __restrict__ residual, uint4* __restrict__ y, int m, int h, int k, char* plan_base, int e_local) {
+  chain_wait();
+  // The counters of a launch of both GEMMs, by a block more: in the call's last kernel nothing waits for that.  No block lets
+  // the next launch start before they are zero, so that the next such launch may claim its tasks at once.
+  const int blocks = plan_base != nullptr ? gridDim.x - 1 : gridDim.x;
+  if ((int)blockIdx.x != blocks) {
+    chain_release();
+  } else {
+    const PlanView pv = plan_view(plan_base, e_local, 1);
+    if (threadIdx.x == 0) {
+      pv.hdr->routed = 0;
+      pv.hdr->next_task = 0;
+      pv.hdr->layer1_done = 0;
+    }
+    for (int e = threadIdx.x; e <= e_local; e += blockDim.x) pv.done[e] = 0;
+    __threadfence();
+    __syncthreads();
+    chain_release();
+    return;
+  }
   const int vec = h / 8, segs = (vec + kCombineSegVec - 1) / kCombineSegVec, lane = threadIdx.x & 31;
-  const int64_t warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  const int64_t warps = ((int64_t)blocks * blockDim.x) >> 5;
   for (int64_t seg = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; seg < (int64_t)m * segs; seg += warps) {
     const int t = static_cast<int>(seg / segs);
     const int v0 = static_cast<int>(seg - (int64_t)t * segs) * kCombineSegVec + lane;
@@ -1145,10 +1163,11 @@ cudaError_t launch_combine(const Ctx& c, void* y, const void* residual, int m, c
   const int64_t segs = (int64_t)m * ((c.geo.hidden / 8 + kCombineSegVec - 1) / kCombineSegVec);      // one warp each
   const int blocks = static_cast<int>(std::min<int64_t>((segs + 7) / 8, 148 * 8));
   const uint4* rows = c.geo.num_ranks == 1 ? c.at<uint4>(c.lay.ret) : c.at<uint4>(c.lay.ret_recv);
-  launch_chained(combine_kernel, dim3(blocks), dim3(256), 0, s, rows, c.at<int32_t>(c.lay.route_pos),
+  char* plan = c.geo.num_ranks == 1 ? c.ws + c.lay.plan : nullptr;
+  launch_chained(combine_kernel, dim3(blocks + (plan != nullptr ? 1 : 0)), dim3(256), 0, s, rows, c.at<int32_t>(c.lay.route_pos),
                                         c.geo.num_shared_experts > 0 ? c.at<uint4>(c.lay.shared_out) : nullptr,
                                         static_cast<const uint4*>(residual), static_cast<uint4*>(y), m, c.geo.hidden,
-                                        c.geo.num_topk);
+                                        c.geo.num_topk, plan, c.e_local);
   return cudaGetLastError();
 }
 

@@ -16,11 +16,13 @@
 //              accumulator to the epilogue
 //   warps 2-5  epilogue: TMEM -> registers (thread = weight row, columns = tokens), fused math, global stores
 //   warp 7     layer 1: brings a stage's weight scales from stored into tensor-memory order ahead of the MMA warps
+//   warp 8     both layers in one launch: claims the CTA's next task (scheduler)
 //
-// Persistent CTAs (one per SM) walk a static task list (tile, 128-row weight block); TMEM accumulators are double
-// buffered so the epilogue of task i overlaps the loads and MMAs of task i+1.  Every wait is bounded: when the budget
-// expires the CTA records {kernel, role, block} in the status words, lets its in-flight copies land, frees its TMEM and
-// returns; nothing traps.
+// A call on one GPU runs both layers in one launch (moe_kernel) of persistent CTAs, one per SM, that claim their tasks (tile, 256
+// weight rows) from a counter; with several ranks, and where a caller asks for one layer, umma_kernel walks a list dealt out
+// beforehand.  TMEM accumulators are double buffered so the epilogue of task i overlaps the loads and MMAs of task i+1.  Every
+// wait is bounded: when the budget expires the CTA records {kernel, role, block} in the status words (kernel 1 and 2: the layer,
+// 4: both), lets its in-flight copies land, frees its TMEM and returns; nothing traps.
 //
 // Expert parallelism: layer 2 has a second form (kFused) whose epilogue stores every BF16 row straight into the buffer
 // of the rank the token came from (plain peer stores over NVLink, no TMA from or to peer memory), and `tile_select`
@@ -38,6 +40,7 @@ namespace mmoe {
 namespace {
 
 constexpr int kThreads = 256;   // producer, MMA 0, 4 epilogue warps, MMA 1, scale arranger (layer 1)
+constexpr int both_threads(bool staged) { return kThreads + (staged ? 64 : 32); }   // a scheduler, and a warp that places rows
 
 constexpr int kNumBoxes = kSmallTileRows / 16;
 
@@ -64,14 +67,14 @@ struct UmmaParams {
   SharedTiles shared_tiles;    // run first
   int with_routed;             // 0: only those
   int tile_rows;               // > 0: rows of the call's largest tile, known to the host; 0: in the plan
-  int early;                   // 1: the launch in front lets this one start when the staged tokens (layer 1) / the plan (layer 2) are complete
+  int early;                   // both layers: 1 when the launch in front lets this one start with the staged tokens complete, not the plan
   int skip_wait;               // 1: what this launch reads was complete before the launch in front of it let it start
   const int32_t* x_sf;         // layer 1: the staged tokens' scale words [T][K/128], gathered for tiles of staged tokens
-  // kernels of calls of at most kStagedTokens tokens: every routed tile of layer 1 is the staged tokens themselves (see TaskWalk)
+  // calls of at most kStagedTokens tokens: every routed tile of layer 1 is the staged tokens themselves (see TaskQueue)
   const int64_t* topk_idx;
   int32_t* sorted_route;
   int num_routes, topk;
-  // ... and with route_here the launch also orders the routes and builds the plan (layer 1) / places the rows (layer 2)
+  // ... and with route_here the launch also orders the routes, builds the plan and places the rows
   int route_here;
   const float* topk_weights;
   int32_t* route_pos;
@@ -104,6 +107,19 @@ struct UmmaParams {
   CUtensorMap map_tok_shared_box[kNumBoxes];
 };
 
+// A task as the scheduler hands it to the other roles of its CTA.
+struct QueueSlot {
+  Tile tile;
+  int32_t nb, layer;      // 256-row weight block; 0 in place of the layer: no more tasks
+  int32_t ready;          // layer 2: the token rows are complete
+};
+constexpr int kQueue = 4;
+
+// Both layers of a single-GPU call in one launch.
+struct MoeParams {
+  UmmaParams layer[2];
+};
+
 struct Control {          // lives at the start of shared memory
   uint64_t full[8];       // producer -> MMA warps: the stage's copies have landed
   uint64_t empty[8];      // MMA -> producer: the stage's shared memory may be overwritten
@@ -113,13 +129,21 @@ struct Control {          // lives at the start of shared memory
   uint64_t tmem_empty[2];
   uint32_t tmem_base;
   volatile int32_t abort_flag;
-  uint32_t hit[16];       // layer 1 with staged tokens: bit e = some token is routed to expert e
-  uint32_t routes_here;   // ... and this CTA orders the routes
-  // layer 2 with the write-back fused in: where output rows go.  slot s < 32: `ret_recv` of source rank s, slot 32: the
-  // shared expert's (local) output
-  __nv_bfloat16* out_base[33];
-  int32_t rank_off[33];   // fused write-back: first receive-order row of each source rank
-  int32_t home_base[32];  // ... and the send position on that rank of the first row it sent here
+  uint32_t routes_here;   // staged tokens: this CTA orders the routes
+  union {
+    struct {              // both layers in the launch
+      uint64_t q_full[kQueue];    // scheduler -> the other roles: a task
+      uint64_t q_empty[kQueue];   // ... which all of them have read
+      uint64_t q_want;            // producer -> scheduler: the next one, please
+      QueueSlot slots[kQueue];
+      uint32_t hit[16];   // staged tokens: bit e = some token is routed to expert e
+    };
+    struct {              // layer 2 with the write-back fused in: where output rows go
+      __nv_bfloat16* out_base[33];   // slot s < 32: `ret_recv` of source rank s, slot 32: the shared expert's (local) output
+      int32_t rank_off[33];          // first receive-order row of each source rank
+      int32_t home_base[32];         // ... and the send position on that rank of the first row it sent here
+    };
+  };
 };
 static_assert(sizeof(Control) <= 1024, "control block");
 
@@ -171,63 +195,47 @@ struct Cta {                       // where a role finds the CTA's resources
   uint32_t b_bytes;                // token slot of a stage
 };
 
-// The task list of one CTA as a role walks it.  First the shared expert's tasks, which need nothing but the staged tokens and
-// the host's count of them; then -- after what precedes this launch in the stream has completed -- the routed tiles of the
-// plan.  In the single-GPU decode call the shared expert's GEMM1 thus runs beside the route ordering.
-// Tile by tile, or for an expert with several tiles weight block by weight block, so that the tiles of a block read its
-// weights while they are in L2.  After the first round the CTAs take their tasks in the opposite order: the first ones,
-// whose shared tasks have twice the weight bytes, are not also the ones with a task more in the last round.
-//
-// GEMM1 of at most 16 tokens needs no placed rows either: an UMMA takes 16 token columns at least, so every expert that some
-// token is routed to multiplies all staged tokens, and the epilogue takes the columns of the tokens routed to it.  Which
-// experts those are every CTA reads from the route table itself; only the epilogue waits for the plan.
-template <bool kStaged>
+// Tile by tile, or for an expert with several tiles weight block by weight block, so that the tiles of a block read its weights
+// while they are in L2.
+__device__ __forceinline__ void locate_task(const Tile* tiles, int task, int n_blocks, Tile* tile, int* nb) {
+  const int i = task / n_blocks;
+  *tile = tiles[i];
+  *nb = task - i * n_blocks;
+  if (tile->parts > 1) {
+    const int first = i - tile->part, local = task - first * n_blocks;
+    *nb = local / tile->parts;
+    *tile = tiles[first + local - *nb * tile->parts];
+  }
+}
+
+// The task list of one CTA as a role walks it in a launch of one layer.  First the shared expert's tasks, which need nothing but
+// the staged tokens and the host's count of them; then -- after what precedes this launch in the stream has completed -- the
+// routed tiles of the plan.  After the first round the CTAs take their tasks in the opposite order: the first ones, whose shared
+// tasks have twice the weight bytes, are not also the ones with a task more in the last round.
+template <int kLaunchLayer>
 struct TaskWalk {
+  static constexpr bool kBoth = false;
+  static constexpr int kLayer = kLaunchLayer;
   const UmmaParams& p;
-  const uint32_t* hit;
-  int hit_experts;
-  int n_blocks, shared_tasks, routed_tasks, round;
+  int shared_tasks, routed_tasks, round;
   bool waited;
   const Tile* tiles;
   Tile tile;               // current task
   int nb;
   // `plan_ready`: the plan is complete, without a wait
-  __device__ __forceinline__ TaskWalk(const UmmaParams& params, const uint32_t* hit_words, bool plan_ready, int blocks_per_tile)
-      : p(params), hit(hit_words), hit_experts(0), n_blocks(blocks_per_tile), shared_tasks(params.shared_tiles.parts * blocks_per_tile),
-        routed_tasks(0), round(0),
-        waited(false), tiles(nullptr) {
-    if (kStaged) {
-      hit_experts = __reduce_add_sync(0xffffffffu, (threadIdx.x & 31) < 16 ? __popc(hit[threadIdx.x & 15]) : 0);
-      routed_tasks = p.with_routed ? hit_experts * n_blocks : 0;
-    } else if (plan_ready) {
-      load_plan(true);
-    }
-  }
-  // i-th expert (ascending) with a bit in `hit`; whole warp
-  __device__ __forceinline__ int hit_expert(int i) const {
-    const int lane = threadIdx.x & 31;
-    uint32_t word = lane < 16 ? hit[lane] : 0u;
-    const int mine = __popc(word);
-    int before = mine;
-#pragma unroll
-    for (int d = 1; d < 16; d <<= 1) {
-      const int t = __shfl_up_sync(0xffffffffu, before, d);
-      if (lane >= d) before += t;
-    }
-    before -= mine;
-    const int owner = __ffs(__ballot_sync(0xffffffffu, i >= before && i < before + mine)) - 1;
-    for (int drop = i - before; drop > 0 && lane == owner; --drop) word &= word - 1;
-    return __shfl_sync(0xffffffffu, 32 * lane + __ffs(word) - 1, owner);
+  __device__ __forceinline__ TaskWalk(const UmmaParams& params, bool plan_ready)
+      : p(params), shared_tasks(params.shared_tiles.parts * params.n_blocks), routed_tasks(0), round(0), waited(false), tiles(nullptr) {
+    if (plan_ready) load_plan(true);
   }
   __device__ __forceinline__ void load_plan(bool ready) {
     if (!ready) chain_wait();
     const PlanView pv = plan_view(const_cast<char*>(p.plan), p.e_local, p.num_ranks);
     tiles = pv.tiles;
-    routed_tasks = p.with_routed ? pv.hdr->num_small_tiles * n_blocks : 0;
+    routed_tasks = p.with_routed ? pv.hdr->num_small_tiles * p.n_blocks : 0;
     waited = true;
   }
   // true: tile and nb are the next task's
-  __device__ __forceinline__ bool next() {
+  __device__ __forceinline__ bool next(Waiter&) {
     int task = round == 0 ? blockIdx.x : (round + 1) * gridDim.x - 1 - blockIdx.x;
     ++round;
     if (task < shared_tasks) {
@@ -236,30 +244,55 @@ struct TaskWalk {
       return true;
     }
     task -= shared_tasks;
-    if (kStaged) {
-      if (task >= routed_tasks) return false;
-      const int u = task / n_blocks;
-      nb = task - u * n_blocks;
-      tile = Tile{hit_expert(u), 0, p.shared_tiles.m, 0, 0, 1, {0, 0}};
-      return true;
-    }
     if (!waited) load_plan(false);
     if (task >= routed_tasks) return false;
-    const int i = task / n_blocks;
-    tile = tiles[i];
-    nb = task - i * n_blocks;
-    if (tile.parts > 1) {
-      const int first = i - tile.part, local = task - first * n_blocks;
-      nb = local / tile.parts;
-      tile = tiles[first + local - nb * tile.parts];
-    }
+    locate_task(tiles, task, p.n_blocks, &tile, &nb);
     return true;
   }
 };
 
+// Both layers in one launch: the tasks as the scheduler hands them on.
+template <bool kOneLanePolls>
+struct TaskFeed {
+  static constexpr bool kBoth = true;
+  const MoeParams& f;
+  Control* ctl;
+  uint32_t taken;
+  Tile tile;               // current task
+  int nb, layer;
+  bool ready;
+  __device__ __forceinline__ TaskFeed(const MoeParams& params, Control* control) : f(params), ctl(control), taken(0) {}
+  __device__ __forceinline__ bool next(Waiter& waiter) {
+    const uint32_t slot = taken % kQueue, bar = smem_u32(&ctl->q_full[slot]), parity = (taken / kQueue) & 1u;
+    if (!(kOneLanePolls ? waiter.wait_warp(bar, parity) : waiter.wait_uniform(bar, parity))) return false;
+    const QueueSlot& s = ctl->slots[slot];
+    tile = s.tile;
+    nb = s.nb;
+    layer = s.layer;
+    ready = s.ready != 0;
+    __syncwarp();
+    if ((threadIdx.x & 31) == 0) mbar_arrive(smem_u32(&ctl->q_empty[slot]));
+    ++taken;
+    return layer != 0;
+  }
+};
+
+// body(layer as a type, parameters of that layer) for every task of a role
+template <typename Walk, typename Body>
+__device__ __forceinline__ void for_each_task(Walk& walk, Waiter& waiter, RoleState& st, Body&& body) {
+  while (st.ok && walk.next(waiter)) {
+    if constexpr (Walk::kBoth) {
+      if (walk.layer == 1) body(std::integral_constant<int, 1>{}, walk.f.layer[0]);
+      else body(std::integral_constant<int, 2>{}, walk.f.layer[1]);
+    } else {
+      body(std::integral_constant<int, Walk::kLayer>{}, walk.p);
+    }
+  }
+}
+
 // ------------------------------------------------------------------------------------------------ routing in the launch
 // Calls of at most kStagedTokens tokens: the epilogue warps of the first CTA to ask, idle until its first accumulator 15 us
-// later, order the routes and build the plan, which only epilogues and GEMM2 need.  All other CTAs wait for that one, so it has
+// later, order the routes and build the plan, which only epilogues and layer 2 need.  All other CTAs wait for that one, so it has
 // to be one that runs: a CTA takes an SM to itself, and work on other streams may hold any of them back for as long as it
 // likes.  A launch of its own took 8-20 us in front of GEMM1: little work, but every instruction line comes from DRAM (each
 // call streams its weights through the L2), so what counts is that the code is short.  Pool blocks and tiles have 16 rows
@@ -374,7 +407,7 @@ __device__ __noinline__ void sa_route(const UmmaParams& p, RouteScratch& s, int 
   if (t == 0) asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(&pv.hdr->routed), "r"(1) : "memory");
 }
 
-// Layer 2 of such a call: the placed rows and scales, which nothing in the call reads, by the warp that layer 1 uses for scales.
+// The placed rows and scales of such a call, which nothing in it reads, by a warp of their own.
 __device__ __noinline__ void sa_place(const UmmaParams& p) {
   const int lane = threadIdx.x & 31, vec = p.hidden / 16, words = p.hidden / kTileK;
   const PlanView pv = plan_view(const_cast<char*>(p.plan), p.e_local, 1);
@@ -411,99 +444,295 @@ __device__ __forceinline__ bool sa_wait_plan(const UmmaParams& p, Waiter& waiter
   }
 }
 
+// ------------------------------------------------------------------------------------------------ both layers in one launch
+// GEMM2 of an expert needs all of its GEMM1 tasks, wherever those ran.  A counter per expert (the last one: the shared expert)
+// counts the epilogue warps that have stored their part, and one for all experts spares a CTA the question once GEMM1 is over.
+// The rows are then read by bulk copies, hence the proxy fence between seeing the count and asking for them (one on this side too
+// takes 3 us behind a task's stores).
+__device__ __forceinline__ void sa_publish(const PlanView& pv, int slot) {
+  __syncwarp();
+  if ((threadIdx.x & 31) == 0) {
+    __threadfence();
+    asm volatile("red.release.gpu.global.add.s32 [%0], 1;" ::"l"(pv.done + slot) : "memory");
+    asm volatile("red.relaxed.gpu.global.add.s32 [%0], 1;" ::"l"(&pv.hdr->layer1_done) : "memory");
+  }
+}
+__device__ __forceinline__ bool sa_rows_ready(const int32_t* done, int need) {
+  int32_t v;
+  asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(done) : "memory");
+  if (!__all_sync(0xffffffffu, v >= need)) return false;
+  asm volatile("fence.proxy.async.global;" ::: "memory");
+  return true;
+}
+
+// The task list of such a launch: shared expert and routed tiles of layer 1, then of layer 2.  CTAs claim tasks from a counter when
+// the last stages of the one before are being requested, so that
+//   * the memory system never waits for the slowest CTA: claimed by whoever is free, GEMM2's tasks fill GEMM1's last round, and
+//     their weights are requested before the activations are complete.  Two launches with tasks dealt out beforehand: 4 tokens
+//     of 384 experts 94 -> 84 us, 7 tokens 147 -> 137, 128 tokens of 32 experts 150 -> 132, 64 of 384 762 -> 744, 256 of 384
+//     1166 -> 1138, 1021 of 384 skewed 483 -> 467;
+//   * what a CTA waits for was claimed earlier, by a CTA that runs: a call needs no particular CTA to be resident, whatever other
+//     streams do to the SMs.
+// A warp of its own claims and looks up (the scheduler): the latency of the counter and of the tables in the producer's loop
+// left stages empty, 10 % of GEMM2's time at HBM speed.
+// The shared expert's tasks of layer 1 need nothing but the staged tokens and the host's count of them, the routed ones the plan.
+//
+// GEMM1 of at most 16 tokens needs no placed rows either: an UMMA takes 16 token columns at least, so every expert that some
+// token is routed to multiplies all staged tokens, and the epilogue takes the columns of the tokens routed to it.  Which
+// experts those are every CTA reads from the route table itself; only the epilogue waits for the plan.
+// The 256 stored weight rows of a task.  Layer 1 reads W13 in its stored order [g0..7, u0..7, g8..15, ...] through a 5-D map (K, row
+// in group of 8, group of 16 rows, gate/up, slice): one box of 8 x 16 x 2 lands the 128 gate rows and then the 128 up rows of
+// 128 consecutive channels.  Layer 2 reads 256 consecutive rows; with slices of an odd number of 128-row blocks (`halves`) the
+// two blocks are loaded one by one, the second may be in the other slice.
+struct WeightRows {
+  const CUtensorMap* map;
+  int row, slice, row2, slice2;
+  bool halves;
+};
+template <int kLayer>
+__device__ __forceinline__ WeightRows sa_weight_rows(const UmmaParams& p, const Tile& tile, int nb) {
+  const bool shared = tile.expert == kSharedExpert, sliced = !shared && p.routed_sliced != 0;
+  const int e = shared ? 0 : tile.expert;
+  const int rows_slice = sliced ? p.rows_per_expert / 2 : p.rows_per_expert;   // rows of one expert in one slice
+  const int r0 = 2 * nb * kTileRows;                                           // first stored row of the task
+  const bool halves = kLayer == 2 && sliced && p.routed_halves != 0;
+  WeightRows w{shared ? &p.map_w_shared : &p.map_w_routed, e * rows_slice + r0 % rows_slice, sliced ? r0 / rows_slice : 0, 0, 0, halves};
+  if (halves) {
+    w.row2 = e * rows_slice + (r0 + kTileRows) % rows_slice;
+    w.slice2 = (r0 + kTileRows) / rows_slice;
+  }
+  return w;
+}
+
+// layer 2: the counter of a task's expert and what it has to reach
+__device__ __forceinline__ const int32_t* sa_done_of(const MoeParams& f, const PlanView& pv, const Tile& tile) {
+  return pv.done + (tile.expert == kSharedExpert ? f.layer[0].e_local : tile.expert);
+}
+template <bool kStaged>
+__device__ __forceinline__ int sa_need_of(const MoeParams& f, const Tile& tile) {
+  return 4 * f.layer[0].n_blocks * (kStaged && tile.expert != kSharedExpert ? 1 : tile.parts);
+}
+
+template <bool kStaged>
+struct TaskQueue {
+  const MoeParams& f;
+  Control* ctl;
+  PlanView pv;
+  bool plan_known, over;
+  int small_tiles, hit_experts;
+  uint32_t claimed;        // lane 0
+  uint32_t handed_on;
+  __device__ __forceinline__ TaskQueue(const MoeParams& params, Control* control)
+      : f(params), ctl(control), pv(plan_view(const_cast<char*>(params.layer[0].plan), params.layer[0].e_local, params.layer[0].num_ranks)),
+        plan_known(false), over(false), small_tiles(0), hit_experts(-1), claimed(0), handed_on(0) {}
+  __device__ __forceinline__ void load_plan() {
+    small_tiles = pv.hdr->num_small_tiles;
+    plan_known = true;
+  }
+  __device__ __forceinline__ bool wait_plan(Waiter& waiter) {
+    if (plan_known) return true;
+    if (kStaged) {
+      if (!sa_wait_plan(f.layer[0], waiter)) return false;
+    } else {
+      chain_wait();
+    }
+    load_plan();
+    return true;
+  }
+  // which experts are hit, from the route table
+  __device__ __forceinline__ void find_hits() {
+    const int lane = threadIdx.x & 31;
+    if (lane < 16) ctl->hit[lane] = 0u;
+    __syncwarp();
+    for (int i = lane; i < f.layer[0].num_routes; i += 32) {
+      const int64_t id = f.layer[0].topk_idx[i];
+      if (id >= 0 && id < f.layer[0].e_local) atomicOr(&ctl->hit[id >> 5], 1u << (id & 31));
+    }
+    __syncwarp();
+    hit_experts = __reduce_add_sync(0xffffffffu, lane < 16 ? __popc(ctl->hit[lane]) : 0);
+  }
+  // i-th expert (ascending) with a bit in `hit`; whole warp
+  __device__ __forceinline__ int hit_expert(int i) const {
+    const int lane = threadIdx.x & 31;
+    uint32_t word = lane < 16 ? ctl->hit[lane] : 0u;
+    const int mine = __popc(word);
+    int before = mine;
+#pragma unroll
+    for (int d = 1; d < 16; d <<= 1) {
+      const int t = __shfl_up_sync(0xffffffffu, before, d);
+      if (lane >= d) before += t;
+    }
+    before -= mine;
+    const int owner = __ffs(__ballot_sync(0xffffffffu, i >= before && i < before + mine)) - 1;
+    for (int drop = i - before; drop > 0 && lane == owner; --drop) word &= word - 1;
+    return __shfl_sync(0xffffffffu, 32 * lane + __ffs(word) - 1, owner);
+  }
+  __device__ __forceinline__ void claim() {
+    if ((threadIdx.x & 31) == 0) claimed = atomicAdd(&pv.hdr->next_task, 1u);
+  }
+  // what the claimed number stands for; false when the call is being abandoned
+  __device__ __forceinline__ bool decode(Waiter& waiter, QueueSlot* out) {
+    int i = static_cast<int>(__shfl_sync(0xffffffffu, claimed, 0));
+    const SharedTiles& shared = f.layer[0].shared_tiles;
+    for (int layer = 1; layer <= 2; ++layer) {
+      const int n_blocks = f.layer[layer - 1].n_blocks, shared_tasks = shared.parts * n_blocks;
+      out->layer = layer;
+      if (i < shared_tasks) {
+        out->nb = i / shared.parts;
+        out->tile = shared.at(i - out->nb * shared.parts);
+        return true;
+      }
+      i -= shared_tasks;
+      if (kStaged && layer == 1) {
+        if (hit_experts < 0) find_hits();
+        if (i < hit_experts * n_blocks) {
+          const int u = i / n_blocks;
+          out->nb = i - u * n_blocks;
+          out->tile = Tile{hit_expert(u), 0, shared.m, 0, 0, 1, {0, 0}};
+          return true;
+        }
+        i -= hit_experts * n_blocks;
+      } else {
+        if (!wait_plan(waiter)) return false;
+        if (i < small_tiles * n_blocks) {
+          locate_task(pv.tiles, i, n_blocks, &out->tile, &out->nb);
+          return true;
+        }
+        i -= small_tiles * n_blocks;
+      }
+    }
+    out->layer = 0;
+    return true;
+  }
+  // whether all of layer 1 is complete
+  __device__ __forceinline__ bool layer1_over() {
+    if (!over && plan_known) {
+      const int tiles = f.layer[0].shared_tiles.parts + (kStaged ? hit_experts : small_tiles);
+      over = sa_rows_ready(&pv.hdr->layer1_done, 4 * f.layer[0].n_blocks * tiles);
+    }
+    return over;
+  }
+  // to the other roles of the CTA
+  __device__ __forceinline__ bool hand_on(Waiter& waiter, QueueSlot& t) {
+    t.ready = t.layer == 2 && (layer1_over() || sa_rows_ready(sa_done_of(f, pv, t.tile), sa_need_of<kStaged>(f, t.tile))) ? 1 : 0;
+    const uint32_t slot = handed_on % kQueue;
+    if (!waiter.wait_uniform(smem_u32(&ctl->q_empty[slot]), ((handed_on / kQueue) & 1u) ^ 1u)) return false;
+    if ((threadIdx.x & 31) == 0) {
+      ctl->slots[slot] = t;
+      mbar_arrive(smem_u32(&ctl->q_full[slot]));
+    }
+    __syncwarp();
+    ++handed_on;
+    return true;
+  }
+};
+
 // ------------------------------------------------------------------------------------------------ producer
 // One warp in step, one elected lane issues.  Everything that does not change inside a task is computed once per task; the
 // K loop only bumps 32-bit coordinates and two pointers, because such a loop runs at instruction latency, not throughput.
+// `done` (layer 2 behind layer 1 in the same launch): the token tile is complete when this counter has reached `need`; until then
+// as many stages as there are get their weights.  `want`: a barrier that asks the scheduler for the next task.
 template <int kLayer, typename L, bool kStaged>
-__device__ __forceinline__ void sa_producer(const UmmaParams& p, const Cta& c, TaskWalk<kStaged && kLayer == 1> walk, bool early, int ready, Waiter& waiter,
-                                            RoleState& st) {
+__device__ __forceinline__ void sa_load_task(const UmmaParams& p, const Cta& c, const Tile& tile, int nb, Waiter& waiter, RoleState& st,
+                                             const int32_t* done, int need, uint32_t want) {
   const int k_stages = p.k_dim / kTileK;
   const uint32_t full0 = smem_u32(&c.ctl->full[0]), empty0 = smem_u32(&c.ctl->empty[0]);
   const uint32_t sf_full0 = smem_u32(&c.ctl->sf_full[0]);
   const uint32_t a0 = smem_u32(c.a_base), b0 = smem_u32(c.b_base), sf0 = smem_u32(c.sf_base);
-  // GEMM2 behind a GEMM1 that ordered the routes starts while that is still running: the weights of its first stages do not depend on that, so
-  // they are requested before the wait, the activations after it.
-  bool ahead = kStaged && kLayer == 2 && early;
-  // `ready`: stages of the first task whose weights have been requested already
-  while (st.ok && walk.next()) {
-    const Tile tile = walk.tile;
-    const int nb = walk.nb;
-    const bool shared = tile.expert == kSharedExpert;
-    const bool staged = kLayer == 1 && (shared || kStaged);     // the token tile is rows of the staged tokens
-    const int box_sel = (max(tile.n_valid, 1) - 1) >> 4;         // token box: n_valid rounded up to 16 rows
-    const uint32_t box_rows = 16u * (box_sel + 1);
-    const CUtensorMap* wmap = shared ? &p.map_w_shared : &p.map_w_routed;
-    const CUtensorMap* tmap = shared || staged ? &p.map_tok_shared_box[box_sel] : &p.map_tok_routed_box[box_sel];
-    const int e = shared ? 0 : tile.expert;
-    // The 256 stored weight rows of the task.  Layer 1 reads W13 in its stored order [g0..7, u0..7, g8..15, ...]
-    // through a 5-D map (K, row in group of 8, group of 16 rows, gate/up, slice): one box of 8 x 16 x 2 lands the
-    // 128 gate rows and then the 128 up rows of 128 consecutive channels.  Layer 2 reads 256 consecutive rows.
-    const bool sliced = !shared && p.routed_sliced != 0;
-    const int rows_slice = sliced ? p.rows_per_expert / 2 : p.rows_per_expert;   // rows of one expert in one slice
-    const int r0 = 2 * nb * kTileRows;                                           // first stored row of the task
-    const int slice = sliced ? r0 / rows_slice : 0;
-    const int row = e * rows_slice + r0 % rows_slice;
-    const int group = row / 16;
-    // Layer 2 with slices of an odd number of 128-row blocks: the task's two blocks are loaded one by one, the second may be in
-    // the other slice.
-    const bool halves = kLayer == 2 && sliced && p.routed_halves != 0;
-    const int slice2 = halves ? (r0 + kTileRows) / rows_slice : 0;
-    const int row2 = halves ? e * rows_slice + (r0 + kTileRows) % rows_slice : 0;
-    const int32_t* wsf = (shared ? p.wsf_shared : p.wsf_routed) + (int64_t)e * k_stages * p.rows_per_expert + r0;
-    const int64_t tsf_rows = shared ? p.tsf_rows_shared : p.tsf_rows_routed;
-    const int32_t* tsf = (shared ? p.tsf_shared : p.tsf_routed) + (int64_t)tile.sf_chunk * kChunkRows;
-    const uint32_t w_tx = (shared ? 2 * kTileRows * kTileK : kTileRows * kTileK) + (kLayer == 1 ? 0 : 1024);   // packed FP4 counts its global bytes
-    const uint32_t t_tx = box_rows * kTileK + (staged ? 0 : 512);     // scales of staged tokens come from the scale arranger
-    auto load_weights = [&](uint32_t stage, int k0, const int32_t* sf) {
-      const uint32_t bar = full0 + 8 * stage;
-      if (kLayer == 1) {
-        tma_load_5d(a0 + stage * L::kABytes, wmap, k0, 0, group, 0, slice, bar);
-      } else {
-        tma_load_3d(a0 + stage * L::kABytes, wmap, k0, row, slice, bar);
-        if (halves) tma_load_3d(a0 + stage * L::kABytes + kTileRows * kTileK, wmap, k0, row2, slice2, bar);
-        bulk_load(sf0 + stage * L::kSfBytes, sf, 1024, bar);       // two chunks already in tensor-memory order
-      }
-    };
-    if (kStaged && ahead) {
-      ready = min(static_cast<int>(c.num_stages), k_stages);
-      if (elect_one())
-        for (int kb = 0; kb < ready; ++kb) {
-          mbar_expect_tx_only(full0 + 8 * kb, w_tx);
-          load_weights(kb, kb * kTileK, wsf + (int64_t)kb * p.rows_per_expert);
-        }
-      __syncwarp();
-      chain_wait();
-      ahead = false;
+  const bool shared = tile.expert == kSharedExpert;
+  const bool staged = kLayer == 1 && (shared || kStaged);     // the token tile is rows of the staged tokens
+  const int box_sel = (max(tile.n_valid, 1) - 1) >> 4;         // token box: n_valid rounded up to 16 rows
+  const uint32_t box_rows = 16u * (box_sel + 1);
+  const CUtensorMap* tmap = shared || staged ? &p.map_tok_shared_box[box_sel] : &p.map_tok_routed_box[box_sel];
+  const int e = shared ? 0 : tile.expert;
+  const WeightRows w = sa_weight_rows<kLayer>(p, tile, nb);
+  const int32_t* wsf = (shared ? p.wsf_shared : p.wsf_routed) + (int64_t)e * k_stages * p.rows_per_expert + 2 * nb * kTileRows;
+  const int64_t tsf_rows = shared ? p.tsf_rows_shared : p.tsf_rows_routed;
+  const int32_t* tsf = (shared ? p.tsf_shared : p.tsf_routed) + (int64_t)tile.sf_chunk * kChunkRows;
+  const uint32_t w_tx = (shared ? 2 * kTileRows * kTileK : kTileRows * kTileK) + (kLayer == 1 ? 0 : 1024);   // packed FP4 counts its global bytes
+  const uint32_t t_tx = box_rows * kTileK + (staged ? 0 : 512);     // scales of staged tokens come from the scale arranger
+  auto load_weights = [&](uint32_t stage, int k0, const int32_t* sf) {
+    const uint32_t bar = full0 + 8 * stage;
+    if (kLayer == 1) {
+      tma_load_5d(a0 + stage * L::kABytes, w.map, k0, 0, w.row / 16, 0, w.slice, bar);
+    } else {
+      tma_load_3d(a0 + stage * L::kABytes, w.map, k0, w.row, w.slice, bar);
+      if (w.halves) tma_load_3d(a0 + stage * L::kABytes + kTileRows * kTileK, w.map, k0, w.row2, w.slice2, bar);
+      bulk_load(sf0 + stage * L::kSfBytes, sf, 1024, bar);       // two chunks already in tensor-memory order
     }
-    int k0 = 0;
-    for (int kb = 0; kb < k_stages; ++kb, k0 += kTileK, wsf += p.rows_per_expert, tsf += tsf_rows) {
-      if (!waiter.wait_uniform(empty0 + 8 * st.stage, st.phase ^ 1u)) { st.ok = false; break; }
-      const uint32_t bar = full0 + 8 * st.stage;
-      if (elect_one()) {
-        if (kLayer == 1 && (!kStaged || kb >= ready)) {
-          // scales of the 256 stored rows, rearranged by the scale arranger: their own barrier, first in the queue
-          mbar_expect_tx(sf_full0 + 8 * st.stage, 1024);
-          bulk_load(sf0 + st.stage * L::kSfBytes + 3 * 512, wsf, 1024, sf_full0 + 8 * st.stage);
+  };
+  int ahead = 0;                                                 // stages whose weights have been requested
+  if (kLayer == 2 && done != nullptr) {
+    if (!sa_rows_ready(done, need)) {
+      uint32_t stage = st.stage, phase = st.phase;
+      const int most = min(static_cast<int>(c.num_stages), k_stages);
+      for (; ahead < most; ++ahead) {
+        if (!waiter.wait_uniform(empty0 + 8 * stage, phase ^ 1u)) { st.ok = false; return; }
+        if (elect_one()) {
+          mbar_expect_tx_only(full0 + 8 * stage, w_tx);
+          load_weights(stage, ahead * kTileK, wsf + (int64_t)ahead * p.rows_per_expert);
         }
-        if (kStaged && kb < ready) {
-          mbar_expect_tx(bar, t_tx);
-        } else {
-          mbar_expect_tx(bar, w_tx + t_tx);
-          load_weights(st.stage, k0, wsf);
-        }
-        tma_load_2d(b0 + st.stage * c.b_bytes, tmap, k0, tile.row0, bar);
-        if (!staged) bulk_load(sf0 + st.stage * L::kSfBytes + 2 * 512, tsf, 512, bar);
+        __syncwarp();
+        if (++stage == c.num_stages) { stage = 0; phase ^= 1u; }
       }
-      __syncwarp();
-      if (++st.stage == c.num_stages) { st.stage = 0; st.phase ^= 1u; }
+      for (uint32_t spin = 0; !sa_rows_ready(done, need); ++spin) {
+        if ((spin & 63u) == 63u && __any_sync(0xffffffffu, waiter.abandoned())) { st.ok = false; return; }
+        __nanosleep(40);
+      }
     }
-    ready = 0;
   }
-  // A GEMM1 that orders the routes lets GEMM2 start once this CTA has nothing left to request and knows the plan to be complete,
-  // which is what GEMM2 counts on.
-  if (kStaged && kLayer == 1 && p.route_here) {
-    if (!sa_wait_plan(p, waiter)) st.ok = false;
-    chain_release();
+  const int want_at = max(k_stages - 8, 0);
+  int k0 = 0;
+  for (int kb = 0; kb < k_stages; ++kb, k0 += kTileK, wsf += p.rows_per_expert, tsf += tsf_rows) {
+    if ((kLayer == 1 || kb >= ahead) && !waiter.wait_uniform(empty0 + 8 * st.stage, st.phase ^ 1u)) { st.ok = false; return; }
+    const uint32_t bar = full0 + 8 * st.stage;
+    if (elect_one()) {
+      if (want != 0 && kb == want_at) mbar_arrive(want);
+      if (kLayer == 1) {
+        // scales of the 256 stored rows, rearranged by the scale arranger: their own barrier, first in the queue
+        mbar_expect_tx(sf_full0 + 8 * st.stage, 1024);
+        bulk_load(sf0 + st.stage * L::kSfBytes + 3 * 512, wsf, 1024, sf_full0 + 8 * st.stage);
+      }
+      if (kLayer == 2 && kb < ahead) {
+        mbar_expect_tx(bar, t_tx);
+      } else {
+        mbar_expect_tx(bar, w_tx + t_tx);
+        load_weights(st.stage, k0, wsf);
+      }
+      tma_load_2d(b0 + st.stage * c.b_bytes, tmap, k0, tile.row0, bar);
+      if (!staged) bulk_load(sf0 + st.stage * L::kSfBytes + 2 * 512, tsf, 512, bar);
+    }
+    __syncwarp();
+    if (++st.stage == c.num_stages) { st.stage = 0; st.phase ^= 1u; }
+  }
+}
+
+// One layer in the launch.
+template <int kLayer, typename L>
+__device__ __forceinline__ void sa_producer(const UmmaParams& p, const Cta& c, TaskWalk<kLayer> walk, Waiter& waiter, RoleState& st) {
+  while (st.ok && walk.next(waiter)) sa_load_task<kLayer, L, false>(p, c, walk.tile, walk.nb, waiter, st, nullptr, 0, 0u);
+}
+
+// Both layers.  The producer asks for the next task eight stages before the end of the one before, 3 us at HBM speed, and not
+// before it knows its own rows to be complete: a CTA that waits must not hold back another task.
+template <typename L, bool kStaged>
+__device__ __forceinline__ void sa_producer_both(const MoeParams& f, const Cta& c, TaskFeed<false> feed, Waiter& waiter, RoleState& st) {
+  const PlanView pv = plan_view(const_cast<char*>(f.layer[0].plan), f.layer[0].e_local, f.layer[0].num_ranks);
+  const uint32_t want = smem_u32(&c.ctl->q_want);
+  while (st.ok && feed.next(waiter)) {
+    if (feed.layer == 1) sa_load_task<1, L, kStaged>(f.layer[0], c, feed.tile, feed.nb, waiter, st, nullptr, 0, want);
+    else sa_load_task<2, L, false>(f.layer[1], c, feed.tile, feed.nb, waiter, st, feed.ready ? nullptr : sa_done_of(f, pv, feed.tile),
+                                   sa_need_of<kStaged>(f, feed.tile), want);
+  }
+}
+
+template <bool kStaged>
+__device__ __forceinline__ void sa_scheduler(const Cta& c, TaskQueue<kStaged>& queue, Waiter& waiter) {
+  for (uint32_t n = 0;; ++n) {
+    QueueSlot t;
+    if (!queue.decode(waiter, &t) || !queue.hand_on(waiter, t) || t.layer == 0) return;
+    if (!waiter.wait_uniform(smem_u32(&c.ctl->q_want), n & 1u)) return;
+    queue.claim();
   }
 }
 
@@ -513,11 +742,10 @@ __device__ __forceinline__ void sa_producer(const UmmaParams& p, const Cta& c, T
 // transpose inside each 128-row block); the accumulators want the scales of 128 gate (h = 0) and 128 up (h = 1) channels.
 // On the MMA warps' path this work was a third of a stage's issue time (about 230 of 700 clk, and a stage is 580 clk of
 // HBM time at the clock a power-capped B200 runs this kernel at).
-template <typename L, bool kStaged>
-__device__ __forceinline__ void sa_arrange_scales(const UmmaParams& p, const Cta& c, TaskWalk<kStaged> walk, Waiter& waiter,
-                                                  RoleState& st) {
+// (Layer 2's scales are stored in tensor-memory order; in a launch of both layers no task of layer 1 follows one of layer 2.)
+template <typename L, bool kStaged, typename Walk>
+__device__ __forceinline__ void sa_arrange_scales(const Cta& c, Walk walk, Waiter& waiter, RoleState& st) {
   const int lane = threadIdx.x & 31;
-  const int k_stages = p.k_dim / kTileK;
   const uint32_t sf_full0 = smem_u32(&c.ctl->sf_full[0]), sf_ready0 = smem_u32(&c.ctl->sf_ready[0]);
   int src[8];                                    // source word of the 8 destination words this lane writes
 #pragma unroll
@@ -528,7 +756,9 @@ __device__ __forceinline__ void sa_arrange_scales(const UmmaParams& p, const Cta
     const int r = 16 * ((m & 63) >> 3) + 8 * h + (m & 7);   // stored row inside its 128-row block
     src[t] = 128 * (m >> 6) + 4 * (r & 31) + (r >> 5);
   }
-  while (st.ok && walk.next()) {
+  for_each_task(walk, waiter, st, [&](auto layer, const UmmaParams& p) {
+    if constexpr (decltype(layer)::value == 1) {
+    const int k_stages = p.k_dim / kTileK;
     // The scales of staged tokens are gathered here, word kb of the staged scale rows (chunk position 4 (i % 32) + i / 32
     // for token i), two stages ahead: such tiles need no placement, only the staging.
     const bool staged = walk.tile.expert == kSharedExpert || kStaged;
@@ -562,16 +792,15 @@ __device__ __forceinline__ void sa_arrange_scales(const UmmaParams& p, const Cta
       __syncwarp();
       if (++st.stage == c.num_stages) { st.stage = 0; st.phase ^= 1u; }
     }
-  }
+    }
+  });
 }
 
 // Two warps, one per weight tile / accumulator (h = 0, 1).  The whole warp walks the loop so that loop state stays
 // warp-uniform; one elected lane issues.  Each warp copies the scales it needs into its own TMEM columns, so no
 // ordering between the two warps' tensor-core instructions is needed.
-template <int kLayer, typename L, bool kStaged>
-__device__ __forceinline__ void sa_mma(const UmmaParams& p, const Cta& c, TaskWalk<kStaged && kLayer == 1> walk, Waiter& waiter,
-                                       RoleState& st, int h) {
-  const int k_stages = p.k_dim / kTileK;
+template <typename L, typename Walk>
+__device__ __forceinline__ void sa_mma(const Cta& c, Walk walk, Waiter& waiter, RoleState& st, int h) {
   const uint32_t full0 = smem_u32(&c.ctl->full[0]), sf_ready0 = smem_u32(&c.ctl->sf_ready[0]);
   const uint32_t empty0 = smem_u32(&c.ctl->empty[0]);
   const uint64_t sw128_hi = desc_hi_sw128();
@@ -581,11 +810,13 @@ __device__ __forceinline__ void sa_mma(const UmmaParams& p, const Cta& c, TaskWa
   const uint32_t sf_lo0 = (smem_u32(c.sf_base) & 0x3FFFFu) >> 4;
   const uint32_t sfa_col = c.tmem_base + L::kSfCol + 4 * h;
   const uint32_t sfb_col = c.tmem_base + L::kSfCol + 8 + 4 * h;
-  for (; st.ok && walk.next(); ++st.it) {
+  for_each_task(walk, waiter, st, [&](auto layer, const UmmaParams& p) {
+    constexpr int kLayer = decltype(layer)::value;
+    const int k_stages = p.k_dim / kTileK;
     const Tile tile = walk.tile;
     const bool shared = tile.expert == kSharedExpert;
     const uint32_t acc_stage = st.it & 1u, acc_phase = (st.it >> 1) & 1u;
-    if (!waiter.wait_uniform(smem_u32(&c.ctl->tmem_empty[acc_stage]), acc_phase ^ 1u)) { st.ok = false; break; }
+    if (!waiter.wait_uniform(smem_u32(&c.ctl->tmem_empty[acc_stage]), acc_phase ^ 1u)) { st.ok = false; return; }
     tc_fence_after();
     const uint32_t n = static_cast<uint32_t>((tile.n_valid + 15) & ~15);
     const uint32_t idesc0 = make_idesc(shared ? 0u : 5u, 0u, n, 0);
@@ -611,7 +842,8 @@ __device__ __forceinline__ void sa_mma(const UmmaParams& p, const Cta& c, TaskWa
     }
     if (st.ok && elect_one()) tc_commit(smem_u32(&c.ctl->tmem_full[acc_stage]));
     __syncwarp();
-  }
+    ++st.it;
+  });
 }
 
 // ------------------------------------------------------------------------------------------------ epilogue
@@ -664,26 +896,33 @@ __device__ __forceinline__ bool sa_epilogue_staged(const UmmaParams& p, const Ct
   }
   tc_fence_before();
   mbar_arrive(smem_u32(&c.ctl->tmem_empty[acc_stage]));
+  sa_publish(pv, tile.expert);
   return true;
 }
 
-template <int kLayer, typename L, bool kFused, bool kStaged>
-__device__ __forceinline__ void sa_epilogue(const UmmaParams& p, const Cta& c, TaskWalk<kStaged && kLayer == 1> walk, Waiter& waiter,
-                                            RoleState& st) {
+template <typename L, bool kFused, bool kStaged, typename Walk>
+__device__ __forceinline__ void sa_epilogue(const Cta& c, Walk walk, bool plan_known, Waiter& waiter, RoleState& st) {
   Control* ctl = c.ctl;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int q = warp & 3;                     // TMEM lane quadrant this warp may read
   const uint32_t lane_sel = static_cast<uint32_t>(q * 32) << 16;
-  bool plan_known = false;
-  for (; st.ok && walk.next(); ++st.it) {
+  for_each_task(walk, waiter, st, [&](auto layer, const UmmaParams& p) {
+    constexpr int kLayer = decltype(layer)::value;
     const Tile tile = walk.tile;
     const int nb = walk.nb;
     const bool shared = tile.expert == kSharedExpert;
-    if (kStaged && kLayer == 1 && !shared) {
-      if (!plan_known && !sa_wait_plan(p, waiter)) { st.ok = false; break; }
+    if (!plan_known && !shared && !(kStaged && kLayer == 2)) {       // (the scheduler knew it before it handed on a task of layer 2)
+      if (kStaged) {
+        if (!sa_wait_plan(p, waiter)) { st.ok = false; return; }
+      } else {
+        chain_wait();
+      }
       plan_known = true;
-      if (!sa_epilogue_staged<L>(p, c, tile, nb, waiter, st)) { st.ok = false; break; }
-      continue;
+    }
+    if (kStaged && kLayer == 1 && !shared) {
+      if (!sa_epilogue_staged<L>(p, c, tile, nb, waiter, st)) { st.ok = false; return; }
+      ++st.it;
+      return;
     }
     const uint32_t acc_stage = st.it & 1u, acc_phase = (st.it >> 1) & 1u;
     // Per-token side data of the tile (top-k weight / destination row), one coalesced load per 32 tokens issued
@@ -695,7 +934,7 @@ __device__ __forceinline__ void sa_epilogue(const UmmaParams& p, const Cta& c, T
       const int i = 32 * cc + lane;
       if (i < tile.n_valid) {
         if (kLayer == 1) { if (!shared) wv[cc] = __ldg(p.pool_w + tile.row0 + i); }
-        else if (!kFused) dv[cc] = shared ? tile.row0 + i : __ldg(p.pool_dst + tile.row0 + i);
+        else if (!kFused) dv[cc] = shared ? tile.row0 + i : (kStaged ? p.pool_dst[tile.row0 + i] : __ldg(p.pool_dst + tile.row0 + i));
         else if (shared) dv[cc] = static_cast<int>((32u << kOutSlotShift) | static_cast<uint32_t>(tile.row0 + i));
         else {
           const int r = __ldg(p.pool_dst + tile.row0 + i);       // receive-order row
@@ -706,7 +945,7 @@ __device__ __forceinline__ void sa_epilogue(const UmmaParams& p, const Cta& c, T
         }
       }
     }
-    if (!waiter.wait_warp(smem_u32(&ctl->tmem_full[acc_stage]), acc_phase)) { st.ok = false; break; }
+    if (!waiter.wait_warp(smem_u32(&ctl->tmem_full[acc_stage]), acc_phase)) { st.ok = false; return; }
     tc_fence_after();
     const uint32_t d0 = c.tmem_base + lane_sel + acc_stage * L::kAccCols;
     const int n16 = (tile.n_valid + 15) & ~15;
@@ -805,7 +1044,10 @@ __device__ __forceinline__ void sa_epilogue(const UmmaParams& p, const Cta& c, T
     }
     tc_fence_before();
     mbar_arrive(smem_u32(&ctl->tmem_empty[acc_stage]));
-  }
+    if (Walk::kBoth && kLayer == 1)
+      sa_publish(plan_view(const_cast<char*>(p.plan), p.e_local, p.num_ranks), shared ? p.e_local : tile.expert);
+    ++st.it;
+  });
 }
 
 // ------------------------------------------------------------------------------------------------ set-up / teardown
@@ -829,8 +1071,13 @@ __device__ __forceinline__ Cta sa_carve(uint8_t* smem, int tile_rows, int max_st
   return c;
 }
 
+// rows of the largest tile of the call
+__device__ __forceinline__ int sa_tile_rows(const UmmaParams& p) {
+  return p.tile_rows > 0 ? p.tile_rows : max(16, min(kSmallTileRows, plan_view(const_cast<char*>(p.plan), p.e_local, p.num_ranks).hdr->small_rows));
+}
+
 // barriers and tensor memory: touches only this CTA's own shared / tensor memory
-template <typename L>
+template <typename L, bool kBoth>
 __device__ __forceinline__ void sa_setup(Control* ctl) {
   if (threadIdx.x == 0) {
     for (int i = 0; i < L::kMaxStages; ++i) {
@@ -843,8 +1090,13 @@ __device__ __forceinline__ void sa_setup(Control* ctl) {
       mbar_init(smem_u32(&ctl->tmem_full[i]), 2);      // both MMA warps finish an accumulator pair
       mbar_init(smem_u32(&ctl->tmem_empty[i]), 128);
     }
+    if (kBoth)
+      for (int i = 0; i < kQueue; ++i) {
+        mbar_init(smem_u32(&ctl->q_full[i]), 1);
+        mbar_init(smem_u32(&ctl->q_empty[i]), 8);      // producer, MMA, epilogue and scale warps
+      }
+    if (kBoth) mbar_init(smem_u32(&ctl->q_want), 1);
     ctl->abort_flag = 0;
-    for (int i = 0; i < 16; ++i) ctl->hit[i] = 0u;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if ((threadIdx.x >> 5) == 1) {
@@ -870,27 +1122,8 @@ __device__ __forceinline__ void sa_teardown(Control* ctl, uint32_t tmem_base) {
   }
 }
 
-// Layer 1, before the route table has been read: weights and scales of the first stages of a CTA's shared task, by the producer
-// warp (it has initialised the barriers itself).  Returns the number of stages.
-template <typename L>
-__device__ __forceinline__ int sa_request_shared(const UmmaParams& p, const Cta& c) {
-  const int nb = static_cast<int>(blockIdx.x) / p.shared_tiles.parts, stages = min(static_cast<int>(c.num_stages), p.k_dim / kTileK);
-  __syncwarp();
-  if (elect_one())
-#pragma unroll 1
-    for (int kb = 0; kb < stages; ++kb) {
-      const uint32_t bar = smem_u32(&c.ctl->full[kb]), sf_bar = smem_u32(&c.ctl->sf_full[kb]);
-      mbar_expect_tx(sf_bar, 1024);
-      bulk_load(smem_u32(c.sf_base) + kb * L::kSfBytes + 3 * 512, p.wsf_shared + (int64_t)kb * p.rows_per_expert + 2 * nb * kTileRows, 1024, sf_bar);
-      mbar_expect_tx_only(bar, 2 * kTileRows * kTileK);
-      tma_load_5d(smem_u32(c.a_base) + kb * L::kABytes, &p.map_w_shared, kb * kTileK, 0, 2 * nb * kTileRows / 16, 0, 0, bar);
-    }
-  __syncwarp();
-  return stages;
-}
-
 // One layer per launch.
-template <int kLayer, bool kFused, bool kStaged>
+template <int kLayer, bool kFused>
 __global__ void __launch_bounds__(kThreads, 1) umma_kernel(const __grid_constant__ UmmaParams p) {
   static_assert(!kFused || kLayer == 2, "only GEMM2 writes rows back");
   using L = Shape<kLayer>;
@@ -898,30 +1131,15 @@ __global__ void __launch_bounds__(kThreads, 1) umma_kernel(const __grid_constant
   uint8_t* smem = sa_align(smem_raw);
   Control* ctl = reinterpret_cast<Control*>(smem);
   const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);   // warp-uniform for the compiler too
-  if (kLayer == 2 || !kStaged || !p.route_here) chain_release();
-  sa_setup<L>(ctl);
+  chain_release();
+  sa_setup<L, false>(ctl);
   // Everything above touches only this CTA's own shared and tensor memory, so it may run while the kernel before this
-  // one in the stream is still running.  GEMM1 of a call without pair tiles goes on with the shared expert: its launch is let
-  // start by the route ordering's blocks once they have seen the staging complete.  GEMM2 behind a GEMM1 that orders the routes
-  // itself starts when all CTAs of that have seen the plan complete.
-  const bool early = p.early != 0;
+  // one in the stream is still running.
   if (warp == 0 && elect_one()) {
     prefetch_map(&p.map_w_routed);
     prefetch_map(&p.map_w_shared);
   }
-  if ((!early || (kStaged && kLayer == 1 && p.route_here)) && !p.skip_wait) chain_wait();
-  // GEMM1 that orders the routes follows the staging itself, whose predecessors may be anything: not even weights are read
-  // ahead of the wait, but the shared expert's ahead of the route table.
-  int ready = 0;
-  if (kStaged && kLayer == 1 && p.route_here && warp == 0 && static_cast<int>(blockIdx.x) < p.shared_tiles.parts * p.n_blocks)
-    ready = sa_request_shared<L>(p, sa_carve<L>(smem, p.tile_rows, p.max_stages));
-  if (kStaged && kLayer == 1) {
-    __syncthreads();                         // the words are zero
-    for (int i = threadIdx.x; i < p.num_routes; i += kThreads) {
-      const int64_t id = p.topk_idx[i];
-      if (id >= 0 && id < p.e_local) atomicOr(&ctl->hit[id >> 5], 1u << (id & 31));
-    }
-  }
+  if (!p.skip_wait) chain_wait();
   if (kFused) {
     if (threadIdx.x == 0) ctl->out_base[32] = p.shared_out;
     const int t = threadIdx.x - 32;
@@ -940,29 +1158,78 @@ __global__ void __launch_bounds__(kThreads, 1) umma_kernel(const __grid_constant
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const int tile_rows = p.tile_rows > 0 ? p.tile_rows
-                                       : max(16, min(kSmallTileRows, plan_view(const_cast<char*>(p.plan), p.e_local, p.num_ranks).hdr->small_rows));
-  Cta c = sa_carve<L>(smem, tile_rows, p.max_stages);
+  Cta c = sa_carve<L>(smem, sa_tile_rows(p), p.max_stages);
   c.tmem_base = __shfl_sync(0xffffffffu, ctl->tmem_base, 0);
-  const TaskWalk<kStaged && kLayer == 1> walk(p, ctl->hit, kLayer == 2 || !early, p.n_blocks);
+  const TaskWalk<kLayer> walk(p, true);
   Waiter waiter{&ctl->abort_flag, p.status, global_timer() + static_cast<uint64_t>(p.timeout_ns), kLayer, warp};
   RoleState st;
   if (warp == 0) {
-    sa_producer<kLayer, L, kStaged>(p, c, walk, early, ready, waiter, st);
+    sa_producer<kLayer, L>(p, c, walk, waiter, st);
   } else if (warp == 1 || warp == 6) {
-    sa_mma<kLayer, L, kStaged>(p, c, walk, waiter, st, warp == 1 ? 0 : 1);
+    sa_mma<L>(c, walk, waiter, st, warp == 1 ? 0 : 1);
   } else if (warp == 7) {
-    if constexpr (kLayer == 1) sa_arrange_scales<L, kStaged>(p, c, walk, waiter, st);
-    else if (kStaged && p.route_here) sa_place(p);
+    if constexpr (kLayer == 1) sa_arrange_scales<L, false>(c, walk, waiter, st);
   } else {
-    const int t = static_cast<int>(threadIdx.x) - 64;
-    if (kStaged && kLayer == 1 && p.route_here && sa_claim_route(p, ctl, t))
-      sa_route(p, *reinterpret_cast<RouteScratch*>(c.sf_base + c.num_stages * L::kSfBytes), t);
-    sa_epilogue<kLayer, L, kFused, kStaged>(p, c, walk, waiter, st);
+    sa_epilogue<L, kFused, false>(c, walk, true, waiter, st);
   }
   chain_wait();       // a CTA that has not waited yet must not end before what precedes the launch
-  if (kStaged && kLayer == 2 && p.route_here && blockIdx.x == 0 && threadIdx.x == 0)      // GEMM1 has completed: nobody looks at the flag any more
-    plan_view(const_cast<char*>(p.plan), p.e_local, p.num_ranks).hdr->routed = 0;
+  sa_teardown(ctl, c.tmem_base);
+}
+
+// Both layers of a single-GPU call, for the experts that do not run on CTA pairs.  kStaged: calls of at most kStagedTokens tokens.
+template <bool kStaged>
+__global__ void __launch_bounds__(both_threads(kStaged), 1) moe_kernel(const __grid_constant__ MoeParams f) {
+  using L = Shape<1>;
+  const UmmaParams& p = f.layer[0];
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = sa_align(smem_raw);
+  Control* ctl = reinterpret_cast<Control*>(smem);
+  const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);
+  const PlanView pv = plan_view(const_cast<char*>(p.plan), p.e_local, p.num_ranks);
+  chain_release();
+  if (p.skip_wait && p.shared_tiles.parts == 0 && pv.hdr->num_small_tiles == 0) {      // every expert ran on the pairs in front
+    chain_wait();
+    return;
+  }
+  // The first claim may come this early: the counters were zero before the last call's combine let anything start.
+  TaskQueue<kStaged> queue(f, ctl);
+  if (warp == 8) queue.claim();
+  sa_setup<L, true>(ctl);
+  // Everything above touches only this CTA's own shared and tensor memory, and a plan that is complete.  The launch of a call
+  // without pair tiles goes on with the shared expert: it is let start by the route ordering's blocks once they have seen the
+  // staging complete.  One that orders the routes itself follows the staging, whose predecessors may be anything: not even
+  // weights are read ahead of the wait.
+  if (warp == 0 && elect_one()) {
+    prefetch_map(&p.map_w_routed);
+    prefetch_map(&p.map_w_shared);
+  }
+  const bool route_here = kStaged && p.route_here, plan_ready = !p.early && !route_here;
+  if ((!p.early || route_here) && !p.skip_wait) chain_wait();
+  if (plan_ready) queue.load_plan();
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  Cta c = sa_carve<L>(smem, sa_tile_rows(p), p.max_stages);
+  c.tmem_base = __shfl_sync(0xffffffffu, ctl->tmem_base, 0);
+  Waiter waiter{&ctl->abort_flag, p.status, global_timer() + static_cast<uint64_t>(p.timeout_ns), 4, warp};
+  RoleState st;
+  if (warp == 0) {
+    sa_producer_both<L, kStaged>(f, c, TaskFeed<false>(f, ctl), waiter, st);
+  } else if (warp == 1 || warp == 6) {
+    sa_mma<L>(c, TaskFeed<false>(f, ctl), waiter, st, warp == 1 ? 0 : 1);
+  } else if (warp == 7) {
+    sa_arrange_scales<L, kStaged>(c, TaskFeed<false>(f, ctl), waiter, st);
+  } else if (warp == 8) {
+    sa_scheduler<kStaged>(c, queue, waiter);
+  } else if (warp == 9) {
+    if (route_here && sa_wait_plan(p, waiter)) sa_place(p);
+  } else {
+    const int t = static_cast<int>(threadIdx.x) - 64;
+    if (route_here && sa_claim_route(p, ctl, t))
+      sa_route(p, *reinterpret_cast<RouteScratch*>(c.sf_base + c.num_stages * L::kSfBytes), t);
+    sa_epilogue<L, false, kStaged>(c, TaskFeed<true>(f, ctl), plan_ready, waiter, st);
+  }
+  chain_wait();       // a CTA that has not waited yet must not end before what precedes the launch
   sa_teardown(ctl, c.tmem_base);
 }
 
@@ -1002,15 +1269,22 @@ int make_w13_map(CUtensorMap* map, bool fp4, const void* base, uint64_t k_elems,
   return r == CUDA_SUCCESS ? 0 : static_cast<int>(r);
 }
 
-template <int kLayer, bool kFused, bool kStaged>
-cudaError_t prepare_one() {
-  return cudaFuncSetAttribute(umma_kernel<kLayer, kFused, kStaged>, cudaFuncAttributeMaxDynamicSharedMemorySize, Shape<kLayer>::kSmemBytes);
+template <typename Kernel>
+cudaError_t prepare_one(Kernel* kernel, int smem_bytes) {
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
 }
 
-template <int kLayer, bool kFused, bool kStaged>
+template <int kLayer, bool kFused>
 cudaError_t launch_layer(UmmaParams& p, cudaStream_t s) {
   p.max_stages = g_tune_stages;
-  launch_chained(umma_kernel<kLayer, kFused, kStaged>, dim3(tc_num_sms()), dim3(kThreads), Shape<kLayer>::kSmemBytes, s, p);
+  launch_chained(umma_kernel<kLayer, kFused>, dim3(tc_num_sms()), dim3(kThreads), Shape<kLayer>::kSmemBytes, s, p);
+  return cudaGetLastError();
+}
+
+template <bool kStaged>
+cudaError_t launch_both(MoeParams& p, cudaStream_t s) {
+  p.layer[0].max_stages = g_tune_stages;
+  launch_chained(moe_kernel<kStaged>, dim3(tc_num_sms()), dim3(both_threads(kStaged)), Shape<1>::kSmemBytes, s, p);
   return cudaGetLastError();
 }
 
@@ -1036,7 +1310,7 @@ struct PlanKey {
   }
 };
 constexpr int kPlanCacheSize = 256;
-struct SaPlan { UmmaParams layer[2]; };
+using SaPlan = MoeParams;
 struct TmPlan { TmParams layer[2]; };
 PlanCache<PlanKey, SaPlan, kPlanCacheSize> g_sa_plans;
 PlanCache<PlanKey, TmPlan, kPlanCacheSize> g_tm_plans;
@@ -1281,11 +1555,11 @@ int prepare_umma(const MmoeGeometry& geo) {
   int sms = 0;
   if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return MMOE_ERR_CUDA;
   cudaError_t e = cudaSuccess;
-  if (e == cudaSuccess) e = prepare_one<1, false, false>();
-  if (e == cudaSuccess) e = prepare_one<1, false, true>();
-  if (e == cudaSuccess) e = prepare_one<2, false, false>();
-  if (e == cudaSuccess) e = prepare_one<2, true, false>();
-  if (e == cudaSuccess) e = prepare_one<2, false, true>();
+  if (e == cudaSuccess) e = prepare_one(umma_kernel<1, false>, Shape<1>::kSmemBytes);
+  if (e == cudaSuccess) e = prepare_one(umma_kernel<2, false>, Shape<2>::kSmemBytes);
+  if (e == cudaSuccess) e = prepare_one(umma_kernel<2, true>, Shape<2>::kSmemBytes);
+  if (e == cudaSuccess) e = prepare_one(moe_kernel<false>, Shape<1>::kSmemBytes);
+  if (e == cudaSuccess) e = prepare_one(moe_kernel<true>, Shape<1>::kSmemBytes);
   if (e == cudaSuccess) e = tm_prepare();
   if (e != cudaSuccess) return MMOE_ERR_CUDA;
   g_num_sms[dev] = sms;
@@ -1321,13 +1595,24 @@ cudaError_t launch_experts_umma(const Ctx& c, const MmoeWeights& w, const MmoeOp
   const Cut cut = shared_cut(with_shared ? m : 0, pair_above);
   const SharedTiles shared{cut.parts, cut.step, m}, none{0, 16, 0};
   const bool shared_pairs = m > pair_above;
-  const auto [pairs, small] = gemm_forms(c, m, with_shared);
-  const bool staged = staged_tokens(c, m, block_m);
+  const GemmForms forms = gemm_forms(c, m, with_shared);
+  const bool pairs = forms.pairs, small = forms.small;
+  const bool staged = staged_tokens(c, m, block_m);      // only in a launch of both layers
   const PlanKey key = make_key(c, w, has_shared);
   std::shared_ptr<const TmPlan> tm_plan;
   std::shared_ptr<const SaPlan> sa_plan;
   if (pairs && (tm_plan = kept_plan<TmPlan>(g_tm_plans, key, c, w, has_shared)) == nullptr) return cudaErrorInvalidValue;
   if (small && (sa_plan = kept_plan<SaPlan>(g_sa_plans, key, c, w, has_shared)) == nullptr) return cudaErrorInvalidValue;
+  auto small_params = [&](UmmaParams& p, int layer) {
+    patch(p, layer == 2);
+    p.shared_tiles = shared_pairs ? none : shared;
+    p.tile_rows = c.tile_select == 2 ? cut.step : (pairs || c.geo.num_ranks > 1 ? 0 : small_only_cap(m, block_m));
+    // The pair launch in front reads and writes nothing that this one does, and lets it start only after its own wait.
+    p.skip_wait = pairs ? 1 : 0;
+  };
+  // The whole of one GPU's call: the pairs' two launches, then one for all other experts.  It needs nothing of the pairs'
+  // launches, so its CTAs start as theirs run out of tasks.
+  const bool both = c.both_layers && small;
   for (int layer = 1; layer <= 2; ++layer) {
     if ((mask & layer) == 0) continue;
     if (e == cudaSuccess && pairs) {
@@ -1336,22 +1621,21 @@ cudaError_t launch_experts_umma(const Ctx& c, const MmoeWeights& w, const MmoeOp
       p.shared_tiles = shared_pairs ? shared : none;
       e = tm_launch(layer, layer == 2 && fused, p, s);
     }
-    if (e == cudaSuccess && small) {
+    if (e == cudaSuccess && small && !both) {
       UmmaParams p = sa_plan->layer[layer - 1];
-      patch(p, layer == 2);
-      p.shared_tiles = shared_pairs ? none : shared;
-      p.tile_rows = c.tile_select == 2 ? cut.step : (pairs || c.geo.num_ranks > 1 ? 0 : small_only_cap(m, block_m));
-      // The pair launch in front reads and writes nothing that this one does, and lets it start only after its own wait.
-      p.skip_wait = pairs ? 1 : 0;
-      p.early = c.geo.num_ranks == 1 && !pairs && c.tile_select == 0 && (layer == 1 || c.route_in_gemm) ? 1 : 0;
-      p.num_routes = m * c.geo.num_topk;
-      p.route_here = c.route_in_gemm ? 1 : 0;
-      p.stats = c.stats;
-      // (instances of their own for the calls that route in the launch: the others keep the shorter code)
-      if (layer == 1) e = staged ? launch_layer<1, false, true>(p, s) : launch_layer<1, false, false>(p, s);
-      else if (fused) e = launch_layer<2, true, false>(p, s);
-      else e = staged ? launch_layer<2, false, true>(p, s) : launch_layer<2, false, false>(p, s);
+      small_params(p, layer);
+      e = layer == 1 ? launch_layer<1, false>(p, s) : (fused ? launch_layer<2, true>(p, s) : launch_layer<2, false>(p, s));
     }
+  }
+  if (e == cudaSuccess && both) {
+    MoeParams p = *sa_plan;
+    for (int layer = 1; layer <= 2; ++layer) small_params(p.layer[layer - 1], layer);
+    UmmaParams& p1 = p.layer[0];
+    p1.early = pairs ? 0 : 1;
+    p1.num_routes = m * c.geo.num_topk;
+    p1.route_here = p.layer[1].route_here = c.route_in_gemm ? 1 : 0;
+    p1.stats = c.stats;
+    e = staged ? launch_both<true>(p, s) : launch_both<false>(p, s);
   }
   return e;
 }
