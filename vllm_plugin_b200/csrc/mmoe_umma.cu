@@ -153,14 +153,14 @@ static_assert(sizeof(Control) <= 1024, "control block");
 // accumulator each.
 //
 // The token slot of a stage is as large as the largest tile of the call (rounded up to 16 rows), which the plan records, so
-// one kernel serves every call: 6 stages at 16 rows, 5 at 32-80, 4 at 96 and 112.
+// one kernel serves every call: 6 stages up to 32 rows, 5 up to 80, 4 at 96 and 112.
 template <int kLayer>
 struct Shape {
   static constexpr int kABytes = 2 * kTileRows * kTileK;           // byte containers in shared memory
-  // scale area of a stage: [weight scales of the two tiles, 2 x 512][token scales 512][layer 1: stored-order scales
-  // 1024].  Layer 2 receives the two 512-byte chunks in tensor-memory order.  Layer 1 receives them in stored (gate/up
-  // interleaved) order and the scale arranger rewrites them into the first 1024 bytes.
-  static constexpr int kSfBytes = 3 * 512 + (kLayer == 1 ? 1024 : 0);
+  // scale area of a stage: weight scales of the two tiles, 2 x 512, and token scales, 512.  Layer 1 receives the weight scales in
+  // stored (gate/up interleaved) order, and the scale arranger rewrites them in place: with 1 KB more for the stored order, token
+  // slots of 32 rows had five stages instead of six (24 tokens of 384 experts 370 -> 360 us, 1000 tokens 1284 -> 1249).
+  static constexpr int kSfBytes = 3 * 512;
   static constexpr int kMaxStages = 8;
   static constexpr int kRingBytes = kSmemBudget - 1024;
   static constexpr int kSmemBytes = 1024 + kRingBytes + 1024;      // control block + stages + alignment slack
@@ -691,7 +691,7 @@ __device__ __forceinline__ void sa_load_task(const UmmaParams& p, const Cta& c, 
       if (kLayer == 1) {
         // scales of the 256 stored rows, rearranged by the scale arranger: their own barrier, first in the queue
         mbar_expect_tx(sf_full0 + 8 * st.stage, 1024);
-        bulk_load(sf0 + st.stage * L::kSfBytes + 3 * 512, wsf, 1024, sf_full0 + 8 * st.stage);
+        bulk_load(sf0 + st.stage * L::kSfBytes, wsf, 1024, sf_full0 + 8 * st.stage);
       }
       if (kLayer == 2 && kb < ahead) {
         mbar_expect_tx(bar, t_tx);
@@ -777,7 +777,8 @@ __device__ __forceinline__ void sa_arrange_scales(const Cta& c, Walk walk, Waite
       uint32_t* area = reinterpret_cast<uint32_t*>(c.sf_base + st.stage * L::kSfBytes);
       uint32_t v[8];
 #pragma unroll
-      for (int t = 0; t < 8; ++t) v[t] = area[3 * 128 + src[t]];
+      for (int t = 0; t < 8; ++t) v[t] = area[src[t]];
+      __syncwarp();
 #pragma unroll
       for (int t = 0; t < 8; ++t) area[lane + 32 * t] = v[t];
       if (staged) {
