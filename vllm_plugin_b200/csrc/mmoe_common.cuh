@@ -52,18 +52,22 @@ __host__ __device__ inline Cut cut_rows(int n, bool pairs, int small_cap) {
   const int parts = (n + small_cap - 1) / small_cap;
   return Cut{parts, ((n + parts - 1) / parts + 15) & ~15};
 }
-// The cut of the shared expert's m tokens: known to the host, so that its tiles need no plan.
-__host__ __device__ inline Cut shared_cut(int m, int pair_above) { return cut_rows(m, m > pair_above, kDeepTileRows); }
 // GEMM1 of a call of at most this many tokens on one GPU multiplies every expert that is hit with all staged tokens and orders
 // the routes itself (an UMMA takes 16 token columns at least); see staged_tokens().
 constexpr int kStagedTokens = 16;
-// Cap of a call without pair tiles (also known to the host: the largest tile of such a call fixes its stage layout): no expert
-// has more rows than there are tokens unless a token names it twice, which then costs another tile.  An expert of any size has
-// to fit the scale chunks of its pool blocks, see chunks_per_block().
+// Cap of a call without pair tiles, known to the host: the largest tile of such a call fixes its stage layout.  Tiles of up to 32
+// rows leave room for six stages, which is worth more than fewer tiles: BLOCK_M says how many rows an expert is to be expected to
+// have, one with more of them takes several.  With tiles as large as the call has tokens (up to 80): 64 tokens of 384 experts
+// 728 -> 709 us, 100 tokens 894 -> 870, 160 tokens 1058 -> 1029, 192 tokens of 97 experts 325 -> 321; with tiles of 16 rows 710, 874,
+// 1036 and 321.  An expert of any size has to fit the scale chunks of its pool blocks, see chunks_per_block().
+constexpr int kSixStageRows = 32;
 __host__ __device__ inline int small_only_cap(int m, int block_m) {
-  const int rows = (m + 15) & ~15, least = block_m <= 64 ? block_m : (block_m <= 128 ? 64 : kDeepTileRows);
-  return rows >= kDeepTileRows ? kDeepTileRows : (rows > least ? rows : least);
+  const int least = block_m <= 64 ? block_m : (block_m <= 128 ? 64 : kDeepTileRows);
+  return m <= least || least >= kSixStageRows ? least : kSixStageRows;
 }
+// The cut of the shared expert's m tokens, known to the host as well, so that its tiles need no plan.  `cap`: rows of its tiles if
+// it is not on pairs.
+__host__ __device__ inline Cut shared_cut(int m, int pair_above, int cap) { return cut_rows(m, m > pair_above, cap); }
 
 // Scale-factor chunks (128 token rows each) reserved per pool block of a BLOCK_M variant: at least as many as the non-empty
 // tiles an expert's rows are cut into (small_cap >= 16 for BLOCK_M 16, >= 32 for 32, >= 64 for 64, >= 80 for 192 and 240).
@@ -258,6 +262,10 @@ struct Ctx {             // resolved pointers of one call
     if (geo.num_ranks == 1) return m <= pair_above ? kNeverPair : pair_above;
     const int64_t routes = (int64_t)m * geo.num_topk;
     return pair_above > 0 && m > 0 && routes <= kFewRoutes && routes <= (int64_t)kFewRows * e_local ? kNeverPair : pair_above;
+  }
+  // rows of the shared expert's tiles in such a call, where it does not run on pairs
+  int shared_cap_for(int m, int block_m) const {
+    return geo.num_ranks == 1 && tile_select != 2 && pair_above_for(m) == kNeverPair ? small_only_cap(m, block_m) : kDeepTileRows;
   }
   template <typename T> T* at(int64_t off) const { return reinterpret_cast<T*>(ws + off); }
   bool fused() const { return peer_ws != nullptr && geo.num_ranks > 1 && tile_select != 2; }

@@ -484,7 +484,7 @@ cudaError_t launch_pack(const Ctx& c, int m, cudaStream_t s) {
 // order (token, slot) -- a fixed order where the reference's is arrival order.
 // =====================================================================================================================
 struct PlanArgs {
-  int e_local, num_ranks, block_m, pair_above, m, has_shared;
+  int e_local, num_ranks, block_m, pair_above, m, has_shared, shared_cap;
 };
 
 // Exclusive prefix of one value pair per thread over the block (a multiple of 32 threads, at most 1024), with the totals.
@@ -556,7 +556,7 @@ __device__ ExpertPlan build_plan(const PlanView& pv, int n, const PlanArgs& a, b
   const int cap = a.pair_above == kNeverPair && a.num_ranks == 1 ? small_only_cap(a.m, a.block_m) : (num_wide * 8 > num_small ? kSmallTileRows : kDeepTileRows);
   const bool small = n > 0 && !on_pairs(n, a.pair_above, cap);
   const Cut cut = cut_rows(n, n > 0 && !small, cap);
-  const Cut sh_cut = shared_cut(a.has_shared ? a.m : 0, a.pair_above);
+  const Cut sh_cut = shared_cut(a.has_shared ? a.m : 0, a.pair_above, a.shared_cap);
   const bool shared_small = a.m <= a.pair_above;
   const int blocks = (n + a.block_m - 1) / a.block_m;
   ScanPair total;
@@ -983,13 +983,15 @@ __global__ void __launch_bounds__(256) place_kernel(
 
 namespace {
 PlanArgs plan_args(const Ctx& c, int m, int block_m) {
-  return PlanArgs{c.e_local, c.geo.num_ranks, block_m, c.pair_above_for(m), m, c.geo.num_shared_experts > 0 && m > 0 ? 1 : 0};
+  return PlanArgs{c.e_local, c.geo.num_ranks, block_m, c.pair_above_for(m), m, c.geo.num_shared_experts > 0 && m > 0 ? 1 : 0,
+                  c.shared_cap_for(m, block_m)};
 }
 
+// (on the weights-as-A kernels GEMM1 gathers them itself)
 SharedScales shared_scales(const Ctx& c, int m, int pair_above) {
-  const bool on = c.geo.num_shared_experts > 0 && m > 0;
+  const bool on = c.geo.num_shared_experts > 0 && m > pair_above;
   return SharedScales{c.at<int32_t>(c.lay.x_sf), on ? c.at<int32_t>(c.lay.shared_tile_sf) : nullptr, shared_chunk_rows(c.geo.num_max_tokens),
-                      shared_cut(m, pair_above)};
+                      shared_cut(m, pair_above, kDeepTileRows)};
 }
 
 RouteArgs route_args(const Ctx& c, int m, int block_m, int32_t* stats) {
@@ -1039,7 +1041,7 @@ cudaError_t launch_route_large(const Ctx& c, int m, int block_m, int32_t* stats,
 }
 
 cudaError_t launch_shared_plan(const Ctx& c, int m, cudaStream_t s) {
-  if (m == 0 || c.geo.num_shared_experts == 0) return cudaSuccess;
+  if (m <= c.pair_above || c.geo.num_shared_experts == 0) return cudaSuccess;
   launch_chained(shared_plan_kernel, dim3(std::max(1, std::min((m + 7) / 8, 148 * 2))), dim3(256), 0, s, m, shared_scales(c, m, c.pair_above),
                  c.geo.hidden / kTileK);
   return cudaGetLastError();
