@@ -297,14 +297,14 @@ def run_ours(args):
     barrier()
     step_ms = reduce_ranks(ev0.elapsed_time(ev1) / args.steps)
     value = world * m / (step_ms * 1e-3)
-    # EP1: quantiser, route counting + plan, placement, two GEMM launches on CTA pairs, one for all other experts, combine = 7; no
-    # pairs up to 192 tokens, one routing launch up to 128, none up to 16 (in pool blocks of 16 rows).  The peer
+    # EP1: quantiser, route counting + plan, placement, two GEMM launches on CTA pairs, one for all other experts, combine = 7; one
+    # routing launch up to 256 tokens, no pairs up to 192, no routing launch up to 16 (in pool blocks of 16 rows).  The peer
     # exchange: quantiser, 3 route-ordering passes, publish, push, 2 flag waits, a flag kernel, shared-expert plan and 2 GEMMs,
     # plan, place, 4 GEMM launches (2 for few routes), combine = 19; its unfused form has the shared expert in the same
     # launches and a return copy (16); NCCL: the pack kernel instead of the exchange (12)
     if world == 1:
         in_gemm = m <= 16 and api.get_block_m_for_mega_moe(1, E, t_cap, m, K) == 16
-        launches_per_step = 7 if m > 192 else 5 if m > 128 else 3 if in_gemm else 4
+        launches_per_step = 7 if m > 256 else 6 if m > 192 else 3 if in_gemm else 4
     else:
         launches_per_step = {"nccl": 12, "peer-unfused": 16, "peer": 19}[args.ep_transport] - (2 if m * K <= min(3072, 96 * e_local) else 0)
 

@@ -546,16 +546,16 @@ int mmoe_forward(const MmoeGeometry* geo, void* workspace, const MmoeWeights* we
   if (rc != MMOE_OK) return rc;
   if (!valid_block_m(block_m)) return fail(MMOE_ERR_INVALID_ARGUMENT, "block_m=%d is not a BLOCK_M value", block_m);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  // route ordering, plan and placement: inside the GEMM launches up to kStagedTokens tokens, one launch up to 128, two beyond
-  // (and where the pair kernels are forced on: those read the shared expert's scales from chunks that the larger form writes)
-  const bool small_only = num_tokens > 0 && c.pair_above_for(num_tokens) == mmoe::kNeverPair;
+  // route ordering, plan and placement: inside the GEMM launch up to kStagedTokens tokens, one launch up to kSmallRoutes routes, two
+  // beyond (and where the shared expert runs on CTA pairs: those read its scales from chunks that the larger form writes)
+  const bool one_launch = num_tokens > 0 && num_tokens <= c.shared_above_for(num_tokens) && num_tokens * geo->num_topk <= mmoe::kSmallRoutes;
   const bool both_layers = num_tokens > 0 && opt != nullptr && opt->engine == 0 && (opt->layer_mask == 0 || opt->layer_mask == 3);
   const bool in_gemm = both_layers && mmoe::staged_tokens(c, num_tokens, block_m);
   // before any launch: the combine has to follow one of both GEMMs
   rc = check_combine(y_bf16, opt != nullptr ? opt->residual : nullptr, num_tokens);
   if (rc != MMOE_OK) return rc;
   if (!in_gemm) {
-    const cudaError_t e = small_only && num_tokens <= 128 ? mmoe::launch_route_small(c, num_tokens, block_m, stats, st)
+    const cudaError_t e = one_launch ? mmoe::launch_route_small(c, num_tokens, block_m, stats, st)
                                                           : mmoe::launch_route_large(c, num_tokens, block_m, stats, st);
     if (e != cudaSuccess) return cuda_fail(e, "route / plan / placement launch");
   }

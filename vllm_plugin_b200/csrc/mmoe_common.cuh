@@ -20,6 +20,10 @@ constexpr int kChunkRows = 128;    // token rows per scale-factor chunk (one 512
 constexpr int kSmallTileRows = 112;      // largest token tile of the weights-as-A kernels (UMMA N): four accumulators of 112 TMEM columns
 constexpr int kPairTileRows = 128;       // largest token tile of the tokens-as-A kernels (half of a CTA pair's 256 rows)
 constexpr int kNeverPair = 0x7fffffff;
+// The shared expert of a call on one GPU that may have pair tiles: on the pairs past this many tokens, else in tiles of the
+// weights-as-A kernels, which need no scale chunks, so that one launch orders and places the routes.  200 tokens of 48 experts 204 ->
+// 196 us, 256 of 384 1135 -> 1134; 384 tokens 1158 -> 1166, 512 1179 -> 1202.
+constexpr int kSharedPairsAbove = 256;
 
 // Rows of a weights-as-A tile: five stages of up to 80 rows fit the shared memory, four of 112.
 constexpr int kDeepTileRows = 80;
@@ -73,6 +77,9 @@ __host__ __device__ inline Cut shared_cut(int m, int pair_above, int cap) { retu
 // tiles an expert's rows are cut into (small_cap >= 16 for BLOCK_M 16, >= 32 for 32, >= 64 for 64, >= 80 for 192 and 240).
 __host__ __device__ inline int chunks_per_block(int block_m) { return block_m <= 64 ? 1 : (block_m <= 128 ? 2 : 3); }
 constexpr int kSortChunkTokens = 128;
+// Routes that one block orders by itself (see route_small_kernel).  Against two launches: 160 tokens of 32 experts 140.5 -> 134.0
+// us, 130 of 384 978 -> 970, 192 of 384 1074 -> 1068.
+constexpr int kSmallRoutes = 4096;
 constexpr int kSharedExpert = -2;  // MmoeTile::expert of a shared-expert tile
 
 // One unit of token rows handed to the grouped GEMMs: `n_valid` rows starting at `row0` of the token matrix (pool rows for
@@ -263,9 +270,14 @@ struct Ctx {             // resolved pointers of one call
     const int64_t routes = (int64_t)m * geo.num_topk;
     return pair_above > 0 && m > 0 && routes <= kFewRoutes && routes <= (int64_t)kFewRows * e_local ? kNeverPair : pair_above;
   }
-  // rows of the shared expert's tiles in such a call, where it does not run on pairs
+  // The shared expert of such a call runs on CTA pairs past this many tokens ...
+  int shared_above_for(int m) const {
+    const int above = tile_select == 2 ? pair_above : pair_above_for(m);
+    return geo.num_ranks == 1 && tile_select != 2 && above > 0 && above < kSharedPairsAbove ? kSharedPairsAbove : above;
+  }
+  // ... and up to it in tiles of so many rows.
   int shared_cap_for(int m, int block_m) const {
-    return geo.num_ranks == 1 && tile_select != 2 && pair_above_for(m) == kNeverPair ? small_only_cap(m, block_m) : kDeepTileRows;
+    return geo.num_ranks == 1 && tile_select != 2 ? small_only_cap(m, block_m) : kDeepTileRows;
   }
   template <typename T> T* at(int64_t off) const { return reinterpret_cast<T*>(ws + off); }
   bool fused() const { return peer_ws != nullptr && geo.num_ranks > 1 && tile_select != 2; }

@@ -484,7 +484,7 @@ cudaError_t launch_pack(const Ctx& c, int m, cudaStream_t s) {
 // order (token, slot) -- a fixed order where the reference's is arrival order.
 // =====================================================================================================================
 struct PlanArgs {
-  int e_local, num_ranks, block_m, pair_above, m, has_shared, shared_cap;
+  int e_local, num_ranks, block_m, pair_above, m, has_shared, shared_above, shared_cap;
 };
 
 // Exclusive prefix of one value pair per thread over the block (a multiple of 32 threads, at most 1024), with the totals.
@@ -556,8 +556,8 @@ __device__ ExpertPlan build_plan(const PlanView& pv, int n, const PlanArgs& a, b
   const int cap = a.pair_above == kNeverPair && a.num_ranks == 1 ? small_only_cap(a.m, a.block_m) : (num_wide * 8 > num_small ? kSmallTileRows : kDeepTileRows);
   const bool small = n > 0 && !on_pairs(n, a.pair_above, cap);
   const Cut cut = cut_rows(n, n > 0 && !small, cap);
-  const Cut sh_cut = shared_cut(a.has_shared ? a.m : 0, a.pair_above, a.shared_cap);
-  const bool shared_small = a.m <= a.pair_above;
+  const Cut sh_cut = shared_cut(a.has_shared ? a.m : 0, a.shared_above, a.shared_cap);
+  const bool shared_small = a.m <= a.shared_above;
   const int blocks = (n + a.block_m - 1) / a.block_m;
   ScanPair total;
   const ScanPair at = block_scan_pair(
@@ -664,7 +664,7 @@ __global__ void __launch_bounds__(kPlanThreads) plan_kernel(char* __restrict__ p
 constexpr int kRouteThreads = 512;     // one thread per expert in the plan, 16 warps that rank routes
 constexpr int kRouteWarps = kRouteThreads / 32;
 
-// Stable rank of up to kSortChunkTokens * k routes among the routes of the same expert, by the whole block: every warp ranks
+// Stable rank of up to kSmallRoutes routes (or kSortChunkTokens * k) among the routes of the same expert, by the whole block: every warp ranks
 // a run of its own against its own counters (lanes with the same expert find each other with match.any), then each
 // expert's counters are summed over the warps.  ids[i] (0xFFFF = masked) -> rank[i]; returns thread e's expert total.
 // (One warp walking all routes took 10 us for 768; 16 warps take 2.)
@@ -744,7 +744,7 @@ __device__ void write_single_rank_plan(const RouteArgs& r, const PlanView& pv, i
   }
 }
 
-// Calls of at most 128 tokens: ONE launch.  Every block ranks the routes and builds the plan for itself in shared memory
+// Calls of at most kSmallRoutes routes: ONE launch.  Every block ranks the routes and builds the plan for itself in shared memory
 // (2-3 us, less than a second launch behind a grid-wide hand-over), block 0 writes it out, and each block places its share
 // of the routes, one warp per route.  The shared expert's scales are not placed: its GEMM1 gathers them itself.
 __global__ void __launch_bounds__(kRouteThreads) route_small_kernel(const RouteArgs r) {
@@ -805,7 +805,7 @@ __global__ void __launch_bounds__(kRouteThreads) route_small_kernel(const RouteA
   }
 }
 
-// Larger calls, first of two launches: one block per 128 tokens ranks its routes; the last block to finish sums the chunks
+// Larger calls, and those whose shared expert runs on CTA pairs, first of two launches: one block per 128 tokens ranks its routes; the last block to finish sums the chunks
 // and builds the plan.  Further blocks place the shared expert's scales, which GEMM1 starts with while the next launch still places.
 __host__ __device__ inline int route_chunks(int m) { return m > kSortChunkTokens ? (m + kSortChunkTokens - 1) / kSortChunkTokens : 1; }
 
@@ -984,7 +984,7 @@ __global__ void __launch_bounds__(256) place_kernel(
 namespace {
 PlanArgs plan_args(const Ctx& c, int m, int block_m) {
   return PlanArgs{c.e_local, c.geo.num_ranks, block_m, c.pair_above_for(m), m, c.geo.num_shared_experts > 0 && m > 0 ? 1 : 0,
-                  c.shared_cap_for(m, block_m)};
+                  c.shared_above_for(m), c.shared_cap_for(m, block_m)};
 }
 
 // (on the weights-as-A kernels GEMM1 gathers them itself)
@@ -1014,7 +1014,7 @@ RouteArgs route_args(const Ctx& c, int m, int block_m, int32_t* stats) {
   r.pool_w = c.at<float>(c.lay.pool_w);
   r.pool_dst = c.at<int32_t>(c.lay.pool_dst);
   r.pool_sf_rows = c.lay.pool_sf_rows;
-  r.shared = shared_scales(c, m, c.pair_above_for(m));
+  r.shared = shared_scales(c, m, c.shared_above_for(m));
   r.h = c.geo.hidden;
   r.k = c.geo.num_topk;
   r.a = plan_args(c, m, block_m);
@@ -1056,7 +1056,7 @@ cudaError_t launch_plan_place(const Ctx& c, int m, int block_m, int32_t* stats, 
       direct ? c.at<int32_t>(c.lay.x_sf) : c.at<int32_t>(c.lay.recv_sf),
       direct ? c.at<float>(c.lay.topk_weights) : c.at<float>(c.lay.recv_w), c.at<int32_t>(c.lay.sorted_route),
       c.at<uint4>(c.lay.pool_x), c.at<int32_t>(c.lay.pool_sf), c.at<float>(c.lay.pool_w), c.at<int32_t>(c.lay.pool_dst),
-      c.lay.pool_sf_rows, c.e_local, R, c.geo.hidden, c.geo.num_topk, direct ? 1 : 0, shared_scales(c, m, c.pair_above_for(m)));
+      c.lay.pool_sf_rows, c.e_local, R, c.geo.hidden, c.geo.num_topk, direct ? 1 : 0, shared_scales(c, m, c.shared_above_for(m)));
   return cudaGetLastError();
 }
 

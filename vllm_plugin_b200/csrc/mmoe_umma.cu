@@ -1591,11 +1591,11 @@ cudaError_t launch_experts_umma(const Ctx& c, const MmoeWeights& w, const MmoeOp
   };
   // Experts with many rows run on CTA pairs, the others on the weights-as-A kernels: which ones is in the plan.  The shared
   // expert is one or the other by the call's token count.
-  const int pair_above = c.tile_select == 2 ? c.pair_above : c.pair_above_for(m);
+  const int shared_above = c.shared_above_for(m);
   const bool with_shared = has_shared && c.tile_select != 1;
-  const Cut cut = shared_cut(with_shared ? m : 0, pair_above, c.shared_cap_for(m, block_m));
+  const Cut cut = shared_cut(with_shared ? m : 0, shared_above, c.shared_cap_for(m, block_m));
   const SharedTiles shared{cut.parts, cut.step, m}, none{0, 16, 0};
-  const bool shared_pairs = m > pair_above;
+  const bool shared_pairs = m > shared_above;
   const GemmForms forms = gemm_forms(c, m, with_shared);
   const bool pairs = forms.pairs, small = forms.small;
   const bool staged = staged_tokens(c, m, block_m);      // only in a launch of both layers

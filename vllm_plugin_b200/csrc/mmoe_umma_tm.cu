@@ -223,6 +223,11 @@ __global__ void __launch_bounds__(tm_threads(kLayer), 1) tm_kernel(const __grid_
   const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   const uint32_t cta = cluster_ctarank();                         // 0 = leader
 
+  if (p.shared_tiles.parts == 0) {        // routed tiles only, of which the call may have none
+    chain_wait();
+    const PlanHeader* hdr = plan_view(const_cast<char*>(p.plan), p.e_local, p.num_ranks).hdr;
+    if (p.with_routed == 0 || hdr->num_routed_tiles == hdr->num_small_tiles) return;
+  }
   if (threadIdx.x == 0) {
     for (int i = 0; i < kTmStages; ++i) {
       mbar_init(smem_u32(&ctl->full[i]), 1);
