@@ -771,11 +771,14 @@ __global__ void __launch_bounds__(kRouteThreads) route_small_kernel(const RouteA
     s_off[threadIdx.x] = ep.row_off;
     s_step[threadIdx.x] = ep.cut.step;
   }
-  if (blockIdx.x == 0) write_single_rank_plan(r, pv, total, ep);
+  if (blockIdx.x == 0) {
+    write_single_rank_plan(r, pv, total, ep);
+    return;
+  }
   __syncthreads();
-  const int lane = threadIdx.x & 31, warps = gridDim.x * kRouteWarps;
+  const int lane = threadIdx.x & 31, warps = (gridDim.x - 1) * kRouteWarps;
   const int vec = r.h / 16, words = r.h / kTileK, cpb = chunks_per_block(r.a.block_m);
-  for (int i = blockIdx.x * kRouteWarps + (threadIdx.x >> 5); i < n; i += warps) {
+  for (int i = (blockIdx.x - 1) * kRouteWarps + (threadIdx.x >> 5); i < n; i += warps) {
     const int e = ids[i];
     if (e == 0xFFFF) {
       if (lane == 0) r.route_pos[i] = -1;
@@ -1025,7 +1028,7 @@ RouteArgs route_args(const Ctx& c, int m, int block_m, int32_t* stats) {
 cudaError_t launch_route_small(const Ctx& c, int m, int block_m, int32_t* stats, cudaStream_t s) {
   const int n = m * c.geo.num_topk, e = c.geo.num_experts;
   const size_t smem = (size_t)3 * e * 4 + (size_t)2 * ((n + 1) & ~1) * 2 + (size_t)kRouteWarps * e * 2;
-  launch_chained(route_small_kernel, dim3(std::min((n + kRouteWarps - 1) / kRouteWarps, 148)), dim3(kRouteThreads), smem, s,
+  launch_chained(route_small_kernel, dim3(1 + std::min((n + kRouteWarps - 1) / kRouteWarps, 147)), dim3(kRouteThreads), smem, s,
                  route_args(c, m, block_m, stats));
   return cudaGetLastError();
 }
