@@ -20,32 +20,39 @@ __device__ __forceinline__ int interleave_src_row(int r, int rows) {
   return ((r >> 3) & 1) * (rows >> 1) + channel;
 }
 
-// One warp per output row; four 16-byte loads in flight per lane.
-__global__ void __launch_bounds__(256) interleave_rows_kernel(const uint4* __restrict__ src, uint4* __restrict__ dst,
-                                                              int64_t total_rows, int rows, int vec) {
-  const int lane = threadIdx.x & 31;
-  const int64_t warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  for (int64_t row = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; row < total_rows; row += warps) {
-    const int64_t g = row / rows;
-    const int r = static_cast<int>(row - g * rows);
-    const uint4* s = src + (g * rows + interleave_src_row(r, rows)) * vec;
-    uint4* d = dst + row * vec;
-    for (int v0 = lane; v0 < vec; v0 += 128) {
-      uint4 q[4];
+// Copies run in pieces of 20 KB, contiguous on both sides: five 16-byte loads in flight per thread, and a block per piece.  Blocks that
+// walked pieces 148 x 8 apart instead read and wrote too many DRAM pages at a time: 48 experts, rows and both halves 494 -> 446 us
+// (transform 210 -> 195, two-slice copy 292 -> 254 us, 6.7 TB/s); with ten loads of 128 threads 450, four of 512 462.
+// kAgain: the result is read again soon (the two-slice copy of what the transform has written).
+constexpr int kCopyThreads = 256, kCopyLoads = 5;
+template <bool kAgain>
+__device__ __forceinline__ void copy_run(const uint4* __restrict__ src, uint4* __restrict__ dst, int64_t n) {
+  for (int64_t v0 = threadIdx.x; v0 < n; v0 += kCopyLoads * kCopyThreads) {
+    uint4 q[kCopyLoads];
 #pragma unroll
-      for (int u = 0; u < 4; ++u)
-        if (v0 + 32 * u < vec) q[u] = __ldcs(s + v0 + 32 * u);
+    for (int u = 0; u < kCopyLoads; ++u)
+      if (v0 + kCopyThreads * u < n) q[u] = __ldcs(src + v0 + kCopyThreads * u);
 #pragma unroll
-      for (int u = 0; u < 4; ++u)
-        if (v0 + 32 * u < vec) d[v0 + 32 * u] = q[u];
-    }
+    for (int u = 0; u < kCopyLoads; ++u)
+      if (v0 + kCopyThreads * u < n) {
+        if (kAgain) dst[v0 + kCopyThreads * u] = q[u];
+        else __stcs(dst + v0 + kCopyThreads * u, q[u]);
+      }
   }
+}
+
+// A block per eight output rows, which are neighbours in the input too.
+__global__ void __launch_bounds__(kCopyThreads) interleave_rows_kernel(const uint4* __restrict__ src, uint4* __restrict__ dst, int rows, int vec) {
+  const int64_t row = 8 * (int64_t)blockIdx.x, g = row / rows;
+  const int r = static_cast<int>(row - g * rows);
+  copy_run<true>(src + (g * rows + interleave_src_row(r, rows)) * vec, dst + row * vec, 8 * (int64_t)vec);
 }
 
 // One warp per 128-word block of a K column: stored position 4c + a holds row 32a + c of the block (after the optional
 // gate/up interleave), so lane c gathers rows c, 32 + c, 64 + c, 96 + c -- four coalesced loads per warp (runs of eight
 // words when rows are interleaved) -- and stores them as one 16-byte vector.  Two blocks in flight per warp.  HBM-bound;
-// 48 experts (35 + 18 MB each way, in two launches): 45 us with one thread per word, 24 us in this form.
+// 48 experts (35 + 18 MB each way, in two launches): 45 us with one thread per word, 24 us in this form, 22.5 with
+// a grid that is not cut off at 148 x 8 blocks.
 __global__ void __launch_bounds__(256) scale_layout_kernel(const int32_t* __restrict__ src, int32_t* __restrict__ dst,
                                                            int64_t total_blocks, int rows, int row_stride, int interleave) {
   const int lane = threadIdx.x & 31;
@@ -76,39 +83,24 @@ __global__ void __launch_bounds__(256) scale_layout_kernel(const int32_t* __rest
   }
 }
 
-// Two-slice form of row-major matrices: half h of matrix g goes to dst + h * slice_stride + g * half_vec, contiguous both
-// ways, so the copy is cut into pieces of 1024 vectors (16 KB) of one half each; a block takes a piece at a time with four
-// 16-byte loads in flight per thread.  Pure HBM traffic: 48 experts (2 x 849 MB) take 284 us, 6.0 TB/s; as two strided
-// byte-tensor copies per matrix they took 1790 us.
-constexpr int kSplitPieceVec = 1024;
-__global__ void __launch_bounds__(256) split_halves_kernel(const uint4* __restrict__ src, uint4* __restrict__ dst,
-                                                           int num_halves, int64_t half_vec, int64_t slice_vec) {
-  const int64_t pieces_per_half = (half_vec + kSplitPieceVec - 1) / kSplitPieceVec;
-  const int64_t pieces = num_halves * pieces_per_half;
-  for (int64_t i = blockIdx.x; i < pieces; i += gridDim.x) {
-    const int64_t piece = pieces - 1 - i;                // from the end: what a transform in front has written last is still in L2
-    const int64_t half = piece / pieces_per_half;        // 2 g + h, in source order
-    const int64_t v0 = (piece - half * pieces_per_half) * kSplitPieceVec + threadIdx.x;
-    const uint4* s = src + half * half_vec;
-    uint4* d = dst + (half & 1) * slice_vec + (half >> 1) * half_vec;
-    uint4 q[4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u)
-      if (v0 + 256 * u < half_vec) q[u] = __ldcs(s + v0 + 256 * u);
-#pragma unroll
-    for (int u = 0; u < 4; ++u)
-      if (v0 + 256 * u < half_vec) __stcs(d + v0 + 256 * u, q[u]);
-  }
+// Two-slice form of row-major matrices: half h of matrix g goes to dst + h * slice_stride + g * half_vec, contiguous both ways, so
+// the copy is cut into pieces of one half each.  (As two strided byte-tensor copies per matrix 48 experts took 1790 us.)
+constexpr int kSplitPieceVec = kCopyThreads * kCopyLoads;
+__global__ void __launch_bounds__(kCopyThreads) split_halves_kernel(const uint4* __restrict__ src, uint4* __restrict__ dst,
+                                                                    int64_t pieces_per_half, int64_t half_vec, int64_t slice_vec) {
+  const int64_t piece = (int64_t)gridDim.x - 1 - blockIdx.x;   // from the end: what a transform in front has written last is still in L2
+  const int64_t half = piece / pieces_per_half;                // 2 g + h, in source order
+  const int64_t v0 = (piece - half * pieces_per_half) * kSplitPieceVec, left = half_vec - v0;
+  copy_run<false>(src + half * half_vec + v0, dst + (half & 1) * slice_vec + (half >> 1) * half_vec + v0, left < kSplitPieceVec ? left : kSplitPieceVec);
 }
 
 }  // namespace
 
 cudaError_t launch_interleave_rows(const void* src, void* dst, int groups, int rows, int row_bytes, cudaStream_t s) {
-  const int64_t total = (int64_t)groups * rows;
-  if (total == 0) return cudaSuccess;
-  const int blocks = static_cast<int>(total / 8 + 1 < 148 * 16 ? total / 8 + 1 : 148 * 16);
-  interleave_rows_kernel<<<blocks, 256, 0, s>>>(static_cast<const uint4*>(src), static_cast<uint4*>(dst), total, rows,
-                                               row_bytes / 16);
+  const int64_t eights = (int64_t)groups * rows / 8;             // rows % 16 == 0: checked by the entry point
+  if (eights == 0) return cudaSuccess;
+  if (eights > INT32_MAX) return cudaErrorInvalidValue;
+  interleave_rows_kernel<<<static_cast<int>(eights), kCopyThreads, 0, s>>>(static_cast<const uint4*>(src), static_cast<uint4*>(dst), rows, row_bytes / 16);
   return cudaGetLastError();
 }
 
@@ -116,16 +108,17 @@ cudaError_t launch_scale_layout(const int32_t* src, int32_t* dst, int groups, in
                                 int interleave, cudaStream_t s) {
   const int64_t blocks128 = (int64_t)groups * kwords * (rows / 128);     // rows % 128 == 0: checked by the entry point
   if (blocks128 == 0) return cudaSuccess;
-  const int blocks = static_cast<int>(blocks128 / 16 + 1 < 148 * 8 ? blocks128 / 16 + 1 : 148 * 8);
-  scale_layout_kernel<<<blocks, 256, 0, s>>>(src, dst, blocks128, rows, row_stride, interleave);
+  if (blocks128 / 16 >= INT32_MAX) return cudaErrorInvalidValue;
+  scale_layout_kernel<<<static_cast<int>(blocks128 / 16 + 1), 256, 0, s>>>(src, dst, blocks128, rows, row_stride, interleave);
   return cudaGetLastError();
 }
 
 cudaError_t launch_split_halves(const void* src, void* dst, int groups, int64_t half_bytes, int64_t slice_stride, cudaStream_t s) {
-  const int64_t half_vec = half_bytes / 16, pieces = 2 * (int64_t)groups * ((half_vec + kSplitPieceVec - 1) / kSplitPieceVec);
+  const int64_t half_vec = half_bytes / 16, per_half = (half_vec + kSplitPieceVec - 1) / kSplitPieceVec, pieces = 2 * (int64_t)groups * per_half;
   if (pieces == 0) return cudaSuccess;
-  split_halves_kernel<<<static_cast<int>(pieces < 148 * 8 ? pieces : 148 * 8), 256, 0, s>>>(
-      static_cast<const uint4*>(src), static_cast<uint4*>(dst), 2 * groups, half_vec, slice_stride / 16);
+  if (pieces > INT32_MAX) return cudaErrorInvalidValue;
+  split_halves_kernel<<<static_cast<int>(pieces), kCopyThreads, 0, s>>>(static_cast<const uint4*>(src), static_cast<uint4*>(dst), per_half, half_vec,
+                                                                        slice_stride / 16);
   return cudaGetLastError();
 }
 
