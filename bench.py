@@ -307,6 +307,7 @@ def run_ours(args):
         launches_per_step = 7 if m > 256 else 6 if m > 192 else 3 if in_gemm else 4
     else:
         launches_per_step = {"nccl": 12, "peer-unfused": 16, "peer": 19}[args.ep_transport] - (2 if m * K <= min(3072, 96 * e_local) else 0)
+        launches_per_step -= 1 if args.ep_transport == "peer" and m <= 192 else 0     # no shared-expert plan: nothing on CTA pairs
 
     # ---- eager host cost of one call (staging + layer), microseconds of CPU time per call with nothing to wait for
     torch.cuda.synchronize(dev)
@@ -491,7 +492,8 @@ def run_ours(args):
         "kernel_family": family,
         "phase_note": "phases timed back to back on one stream through the C ABI (past 128 tokens: shared_ms = the shared "
                       "expert's two GEMM launches, gemm1_ms / gemm2_ms = the routed experts' launches); the product call at "
-                      "one GPU orders, plans and places in one or two launches and runs shared and routed tiles together; "
+                      "one GPU orders, plans and places in one or two launches and runs shared and routed tiles, and both GEMMs of the experts "
+                      "that are not on CTA pairs, in one launch; "
                       "at more GPUs it overlaps the exchange with the shared expert",
         "layer_tflops_per_gpu": flops_mean / (step_ms * 1e-3) / 1e12,
         "layer_tensor_frac": flops_mean / (step_ms * 1e-3) / 1e12 / tensor_peak,

@@ -294,7 +294,7 @@ inline GemmForms gemm_forms(const Ctx& c, int m, bool with_shared) {
   return GemmForms{pair_above != kNeverPair, pair_above > 0};
 }
 
-// Whether GEMM1 of such a call takes the staged tokens as they are instead of the rows of the pool.  With more than one rank the
+// Whether GEMM1 of such a call, in one launch with GEMM2, takes the staged tokens as they are instead of the rows of the pool.  With more than one rank the
 // rows come from other ranks and the route table names experts of all of them: only one GPU's call may.
 inline bool staged_tokens(const Ctx& c, int m, int block_m) {
   return c.geo.num_ranks == 1 && c.tile_select != 2 && c.pair_above_for(m) == kNeverPair && m > 0 && m <= kStagedTokens &&

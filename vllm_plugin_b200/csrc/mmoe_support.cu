@@ -745,8 +745,8 @@ __device__ void write_single_rank_plan(const RouteArgs& r, const PlanView& pv, i
 }
 
 // Calls of at most kSmallRoutes routes: ONE launch.  Every block ranks the routes and builds the plan for itself in shared memory
-// (2-3 us, less than a second launch behind a grid-wide hand-over), block 0 writes it out, and each block places its share
-// of the routes, one warp per route.  The shared expert's scales are not placed: its GEMM1 gathers them itself.
+// (2-3 us, less than a second launch behind a grid-wide hand-over), block 0 writes it out, and the others place the
+// routes, one warp per route (block 0 with its share of them came in 0.5-1 us late).  The shared expert's scales are not placed: its GEMM1 gathers them itself.
 __global__ void __launch_bounds__(kRouteThreads) route_small_kernel(const RouteArgs r) {
   chain_wait();
   chain_release();       // in this order: the GEMM1 launch starts knowing that the staging has completed
