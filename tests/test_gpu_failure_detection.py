@@ -108,3 +108,31 @@ def test_host_side_argument_errors_map_to_the_reference_exception_classes():
         api.fp8_fp4_mega_moe(y, l1, l2, buf, sl1, sl2, activation_alpha=1.702)
     with pytest.raises(AssertionError):
         api.fp8_fp4_mega_moe(y, (l1[0], l1[1].contiguous()), l2, buf, sl1, sl2)   # scales must be MN-major
+
+
+@pytest.mark.parametrize("m", [8, 100, 300])
+def test_an_error_left_by_an_earlier_call_is_not_taken_for_a_failed_launch(m):
+    """Reading the status on a capturing stream is an error of the host, which the CUDA runtime remembers.  The layer call behind it
+    neither reports that error as its own nor stops halfway, and so is the call behind that one right as well."""
+    from vllm_plugin_b200 import api
+    from vllm_plugin_b200.backend import _native
+    import helpers as H
+    from helpers import O
+    layer = H.make_layer(512, 256, 8, 2, True, seed=4)
+    l1, l2, sl1, sl2 = weights = H.kernel_weights(layer, "cuda")
+    hid = O.make_hidden(m, 512, 1).cuda()
+    ids, w = O.make_routing(m, 8, 2, 2)
+    want, buf = H.run_layer(layer, hid, ids, w, weights=weights)
+    assert O.parity_metrics(want.cpu(), H.oracle_layer(layer, hid.cpu(), ids, w))["rel_l2"] <= 1e-3
+    lib, rt = _native.load(), ctypes.CDLL("libcudart.so.12")
+    side, graph, words = torch.cuda.Stream(), ctypes.c_void_p(), (ctypes.c_int32 * 8)()
+    api.stage_inputs_for_mega_moe(buf, hid, ids.cuda(), w.cuda())
+    assert rt.cudaStreamBeginCapture(ctypes.c_void_p(side.cuda_stream), 2) == 0                # 2: relaxed
+    assert lib.mmoe_read_status(ctypes.byref(buf.geo), buf.base_ptr, words, side.cuda_stream) == _native.MMOE_ERR_CUDA
+    rt.cudaStreamEndCapture(ctypes.c_void_p(side.cuda_stream), ctypes.byref(graph))
+    rt.cudaGetLastError()                                                                      # this copy of the runtime, not the library's
+    for _ in range(2):
+        y = torch.zeros_like(want)
+        api.fp8_fp4_mega_moe(y, l1, l2, buf, sl1, sl2, activation_clamp=10.0)
+        api.read_status(buf)
+        assert torch.equal(y, want)

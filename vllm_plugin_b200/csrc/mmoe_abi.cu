@@ -596,8 +596,10 @@ int mmoe_forward_ep(const MmoeGeometry* geo, void* workspace, const void* const*
   // ... while the shared expert, which needs only this rank's own tokens, runs both of its GEMMs here
   mmoe::Ctx c;
   rc = make_ctx(geo, workspace, &c);
-  if (rc == MMOE_OK && mmoe::launch_shared_plan(c, num_tokens, main_stream) != cudaSuccess)
-    rc = cuda_fail(cudaGetLastError(), "shared plan launch");
+  if (rc == MMOE_OK) {
+    const cudaError_t planned = mmoe::launch_shared_plan(c, num_tokens, main_stream);
+    if (planned != cudaSuccess) rc = cuda_fail(planned, "shared plan launch");
+  }
   if (rc == MMOE_OK) rc = run_experts(geo, workspace, nullptr, weights, opt, num_tokens, block_m, stream, 2);
   // join (always, so that a capture is never left forked)
   if (e == cudaSuccess) e = cudaStreamWaitEvent(main_stream, lane->join, 0);

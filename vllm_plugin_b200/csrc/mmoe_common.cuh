@@ -333,6 +333,19 @@ struct ChainScope {
 };
 bool chained();   // true: launch with the attribute
 
+// The three forms of a launch.  Each returns the status of this launch alone: cudaGetLastError() behind one also returns what an
+// earlier call left on the thread, and a kernel that does run would be taken for one that does not.
+template <typename... KArgs, typename... Args>
+cudaError_t launch_plain(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(std::forward<Args>(args))...);
+}
+
+// as part of the chain
 template <typename... KArgs, typename... Args>
 cudaError_t launch_chained(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args&&... args) {
   cudaLaunchConfig_t cfg = {};
@@ -348,7 +361,7 @@ cudaError_t launch_chained(void (*kernel)(KArgs...), dim3 grid, dim3 block, size
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(std::forward<Args>(args))...);
 }
 
-// the same for a kernel of CTA clusters
+// ... and a kernel of CTA clusters
 template <typename... KArgs, typename... Args>
 cudaError_t launch_clustered(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, int cluster, cudaStream_t s, Args&&... args) {
   cudaLaunchConfig_t cfg = {};

@@ -239,25 +239,26 @@ static_assert(kMaxRanks == 32, "the GEMM2 kernel indexes the totals table as [32
 cudaError_t launch_ep_dispatch(const Ctx& c, const void* const* peer_ws, int m, int64_t timeout_ns, cudaStream_t s) {
   (void)m;
   const Peers peers = make_peers(peer_ws, c.geo.num_ranks);
-  ep_publish_kernel<<<1, 1024, 0, s>>>(peers, c.lay, c.geo.num_ranks, c.geo.rank, c.e_local);
-  ep_push_kernel<<<148 * 2, 256, 0, s>>>(peers, c.lay, c.geo.num_ranks, c.geo.rank, c.e_local, c.geo.hidden, c.geo.num_topk,
-                                         timeout_ns);
-  ep_wait_kernel<<<1, 32, 0, s>>>(peers, c.lay, c.geo.num_ranks, c.geo.rank, 1, timeout_ns);
-  return cudaGetLastError();
+  cudaError_t e = launch_plain(ep_publish_kernel, dim3(1), dim3(1024), 0, s, peers, c.lay, c.geo.num_ranks, c.geo.rank, c.e_local);
+  if (e == cudaSuccess)
+    e = launch_plain(ep_push_kernel, dim3(148 * 2), dim3(256), 0, s, peers, c.lay, c.geo.num_ranks, c.geo.rank, c.e_local, c.geo.hidden,
+                     c.geo.num_topk, timeout_ns);
+  if (e == cudaSuccess) e = launch_plain(ep_wait_kernel, dim3(1), dim3(32), 0, s, peers, c.lay, c.geo.num_ranks, c.geo.rank, 1, timeout_ns);
+  return e;
 }
 
 cudaError_t launch_ep_return(const Ctx& c, const void* const* peer_ws, int64_t timeout_ns, cudaStream_t s) {
   const Peers peers = make_peers(peer_ws, c.geo.num_ranks);
-  ep_return_kernel<<<148 * 2, 256, 0, s>>>(peers, c.lay, c.geo.num_ranks, c.geo.rank, c.geo.hidden);
-  ep_wait_kernel<<<1, 32, 0, s>>>(peers, c.lay, c.geo.num_ranks, c.geo.rank, 2, timeout_ns);
-  return cudaGetLastError();
+  cudaError_t e = launch_plain(ep_return_kernel, dim3(148 * 2), dim3(256), 0, s, peers, c.lay, c.geo.num_ranks, c.geo.rank, c.geo.hidden);
+  if (e == cudaSuccess) e = launch_plain(ep_wait_kernel, dim3(1), dim3(32), 0, s, peers, c.lay, c.geo.num_ranks, c.geo.rank, 2, timeout_ns);
+  return e;
 }
 
 cudaError_t launch_ep_signal_return(const Ctx& c, const void* const* peer_ws, int64_t timeout_ns, cudaStream_t s) {
   const Peers peers = make_peers(peer_ws, c.geo.num_ranks);
-  ep_signal_kernel<<<1, 32, 0, s>>>(peers, c.lay, c.geo.num_ranks, c.geo.rank);
-  ep_wait_kernel<<<1, 32, 0, s>>>(peers, c.lay, c.geo.num_ranks, c.geo.rank, 2, timeout_ns);
-  return cudaGetLastError();
+  cudaError_t e = launch_plain(ep_signal_kernel, dim3(1), dim3(32), 0, s, peers, c.lay, c.geo.num_ranks, c.geo.rank);
+  if (e == cudaSuccess) e = launch_plain(ep_wait_kernel, dim3(1), dim3(32), 0, s, peers, c.lay, c.geo.num_ranks, c.geo.rank, 2, timeout_ns);
+  return e;
 }
 
 }  // namespace mmoe

@@ -186,10 +186,9 @@ cudaError_t launch_route_stage(const Ctx& c, const void* hidden, const void* ids
   int blocks = static_cast<int>(std::min<int64_t>((segs + 7) / 8, 148 * 8));
   if (blocks < 1) blocks = 1;
   const RouterArgs router{logits, num_logical, replica_count, replica_slots, max_copies};
-  launch_chained(stage_kernel, dim3(blocks), dim3(256), 0, s, static_cast<const uint4*>(hidden), c.at<uint2>(c.lay.x), c.at<int32_t>(c.lay.x_sf),
+  return launch_chained(stage_kernel, dim3(blocks), dim3(256), 0, s, static_cast<const uint4*>(hidden), c.at<uint2>(c.lay.x), c.at<int32_t>(c.lay.x_sf),
       c.at<int32_t>(c.lay.shared_x_sf), c.lay.shared_sf_rows, c.geo.num_shared_experts > 0 ? shared_bm : 0, ids, ids64, w,
       pad, c.at<int64_t>(c.lay.topk_idx), c.at<float>(c.lay.topk_weights), m, h, c.geo.num_topk, router);
-  return cudaGetLastError();
 }
 
 // =====================================================================================================================
@@ -238,9 +237,8 @@ cudaError_t launch_stage_nvfp4(const void* hidden, void* q_out, void* sf_out, fl
   const int64_t blocks16 = num_tokens * hidden_size / 16;
   if (blocks16 == 0) return cudaSuccess;
   const int grid = static_cast<int>(std::min<int64_t>((blocks16 + 255) / 256, 148 * 16));
-  stage_nvfp4_kernel<<<grid, 256, 0, s>>>(static_cast<const uint4*>(hidden), static_cast<uint2*>(q_out),
-                                          static_cast<uint8_t*>(sf_out), global_scale, blocks16);
-  return cudaGetLastError();
+  return launch_plain(stage_nvfp4_kernel, dim3(grid), dim3(256), 0, s, static_cast<const uint4*>(hidden), static_cast<uint2*>(q_out),
+                      static_cast<uint8_t*>(sf_out), global_scale, blocks16);
 }
 
 // =====================================================================================================================
@@ -382,17 +380,17 @@ cudaError_t launch_count_sort(const Ctx& c, int m, cudaStream_t s) {
   const int chunks = max(1, (m + kSortChunkTokens - 1) / kSortChunkTokens);
   int32_t* chunk_count = c.at<int32_t>(c.lay.sort_scratch);
   const size_t smem = (size_t)(kSortChunkTokens * k + e) * sizeof(int32_t);
-  launch_chained(sort_local_kernel, dim3(chunks), dim3(kSortThreads), smem, s, c.at<int64_t>(c.lay.topk_idx), c.at<int32_t>(c.lay.route_pos),
-                                                       chunk_count, c.at<int32_t>(c.lay.status), m, k, e);
-  launch_chained(sort_scan_kernel, dim3(1), dim3(1024), 0, s, chunk_count, c.at<int32_t>(c.lay.send_count), c.at<int32_t>(c.lay.send_offset),
-                                      c.geo.num_ranks == 1 ? c.at<int32_t>(c.lay.recv_count) : nullptr, chunks, e);
-  if (m > 0) {
+  cudaError_t err = launch_chained(sort_local_kernel, dim3(chunks), dim3(kSortThreads), smem, s, c.at<int64_t>(c.lay.topk_idx),
+                                   c.at<int32_t>(c.lay.route_pos), chunk_count, c.at<int32_t>(c.lay.status), m, k, e);
+  if (err == cudaSuccess)
+    err = launch_chained(sort_scan_kernel, dim3(1), dim3(1024), 0, s, chunk_count, c.at<int32_t>(c.lay.send_count), c.at<int32_t>(c.lay.send_offset),
+                         c.geo.num_ranks == 1 ? c.at<int32_t>(c.lay.recv_count) : nullptr, chunks, e);
+  if (err == cudaSuccess && m > 0) {
     const int blocks = static_cast<int>(std::min<int64_t>(((int64_t)m * k + kSortThreads - 1) / kSortThreads, 148 * 8));
-    launch_chained(sort_place_kernel, dim3(blocks), dim3(kSortThreads), 0, s, c.at<int64_t>(c.lay.topk_idx), chunk_count,
-                                                      c.at<int32_t>(c.lay.send_offset), c.at<int32_t>(c.lay.route_pos),
-                                                      c.at<int32_t>(c.lay.sorted_route), m, k, e);
+    err = launch_chained(sort_place_kernel, dim3(blocks), dim3(kSortThreads), 0, s, c.at<int64_t>(c.lay.topk_idx), chunk_count,
+                         c.at<int32_t>(c.lay.send_offset), c.at<int32_t>(c.lay.route_pos), c.at<int32_t>(c.lay.sorted_route), m, k, e);
   }
-  return cudaGetLastError();
+  return err;
 }
 
 // ---------------------------------------------------------------------------------------------------------------------
@@ -435,14 +433,14 @@ cudaError_t route_order_static(const int64_t* topk_idx, int m, int k, int num_ex
   // nothing in the scratch has to start at zero: pass A overwrites every (chunk, expert) cell that passes B and C read
   const int chunks = std::max(1, (m + kSortChunkTokens - 1) / kSortChunkTokens);
   const size_t smem = (size_t)(kSortChunkTokens * k + num_experts) * sizeof(int32_t);
-  sort_local_kernel<<<chunks, kSortThreads, smem, s>>>(topk_idx, route_pos, chunk_count, nullptr, m, k, num_experts);
-  sort_scan_kernel<<<1, 1024, 0, s>>>(chunk_count, send_count, send_offset, nullptr, chunks, num_experts);
-  if (m > 0) {
+  e = launch_plain(sort_local_kernel, dim3(chunks), dim3(kSortThreads), smem, s, topk_idx, route_pos, chunk_count, nullptr, m, k, num_experts);
+  if (e == cudaSuccess) e = launch_plain(sort_scan_kernel, dim3(1), dim3(1024), 0, s, chunk_count, send_count, send_offset, nullptr, chunks, num_experts);
+  if (e == cudaSuccess && m > 0) {
     const int blocks = static_cast<int>(std::min<int64_t>(((int64_t)m * k + kSortThreads - 1) / kSortThreads, 148 * 8));
-    sort_place_kernel<<<blocks, kSortThreads, 0, s>>>(topk_idx, chunk_count, send_offset, route_pos, sorted_route, m, k,
-                                                      num_experts);
+    e = launch_plain(sort_place_kernel, dim3(blocks), dim3(kSortThreads), 0, s, topk_idx, chunk_count, send_offset, route_pos, sorted_route, m, k,
+                     num_experts);
   }
-  return cudaGetLastError();
+  return e;
 }
 
 int route_order_static_max_tokens() { return kStaticMaxTokens; }
@@ -471,11 +469,9 @@ __global__ void __launch_bounds__(256) pack_kernel(
 
 cudaError_t launch_pack(const Ctx& c, int m, cudaStream_t s) {
   if (m == 0) return cudaSuccess;
-  pack_kernel<<<148 * 4, 256, 0, s>>>(c.at<uint4>(c.lay.x), c.at<int32_t>(c.lay.x_sf), c.at<float>(c.lay.topk_weights),
-                                      c.at<int32_t>(c.lay.sorted_route), c.at<int32_t>(c.lay.send_offset),
-                                      c.at<uint4>(c.lay.send_x), c.at<int32_t>(c.lay.send_sf), c.at<float>(c.lay.send_w),
-                                      c.geo.hidden, c.geo.num_topk, c.geo.num_experts);
-  return cudaGetLastError();
+  return launch_plain(pack_kernel, dim3(148 * 4), dim3(256), 0, s, c.at<uint4>(c.lay.x), c.at<int32_t>(c.lay.x_sf), c.at<float>(c.lay.topk_weights),
+                      c.at<int32_t>(c.lay.sorted_route), c.at<int32_t>(c.lay.send_offset), c.at<uint4>(c.lay.send_x),
+                      c.at<int32_t>(c.lay.send_sf), c.at<float>(c.lay.send_w), c.geo.hidden, c.geo.num_topk, c.geo.num_experts);
 }
 
 // =====================================================================================================================
@@ -1028,9 +1024,8 @@ RouteArgs route_args(const Ctx& c, int m, int block_m, int32_t* stats) {
 cudaError_t launch_route_small(const Ctx& c, int m, int block_m, int32_t* stats, cudaStream_t s) {
   const int n = m * c.geo.num_topk, e = c.geo.num_experts;
   const size_t smem = (size_t)3 * e * 4 + (size_t)2 * ((n + 1) & ~1) * 2 + (size_t)kRouteWarps * e * 2;
-  launch_chained(route_small_kernel, dim3(1 + std::min((n + kRouteWarps - 1) / kRouteWarps, 147)), dim3(kRouteThreads), smem, s,
-                 route_args(c, m, block_m, stats));
-  return cudaGetLastError();
+  return launch_chained(route_small_kernel, dim3(1 + std::min((n + kRouteWarps - 1) / kRouteWarps, 147)), dim3(kRouteThreads), smem, s,
+                        route_args(c, m, block_m, stats));
 }
 
 cudaError_t launch_route_large(const Ctx& c, int m, int block_m, int32_t* stats, cudaStream_t s) {
@@ -1038,29 +1033,28 @@ cudaError_t launch_route_large(const Ctx& c, int m, int block_m, int32_t* stats,
   const int chunks = route_chunks(m);
   const int scale_blocks = r.shared.out == nullptr ? 0 : std::min((r.shared.cut.parts * (r.h / kTileK) + kRouteWarps - 1) / kRouteWarps, 148);
   const size_t smem = (size_t)2 * ((kSortChunkTokens * r.k + 1) & ~1) * 2 + (size_t)kRouteWarps * r.a.e_local * 2;
-  launch_chained(route_count_kernel, dim3(chunks + scale_blocks), dim3(kRouteThreads), smem, s, r);
-  if (m > 0) launch_chained(route_place_kernel, dim3(std::min((m + 7) / 8, 148 * 8)), dim3(256), 0, s, r);
-  return cudaGetLastError();
+  cudaError_t e = launch_chained(route_count_kernel, dim3(chunks + scale_blocks), dim3(kRouteThreads), smem, s, r);
+  if (e == cudaSuccess && m > 0) e = launch_chained(route_place_kernel, dim3(std::min((m + 7) / 8, 148 * 8)), dim3(256), 0, s, r);
+  return e;
 }
 
 cudaError_t launch_shared_plan(const Ctx& c, int m, cudaStream_t s) {
   if (m <= c.pair_above || c.geo.num_shared_experts == 0) return cudaSuccess;
-  launch_chained(shared_plan_kernel, dim3(std::max(1, std::min((m + 7) / 8, 148 * 2))), dim3(256), 0, s, m, shared_scales(c, m, c.pair_above),
-                 c.geo.hidden / kTileK);
-  return cudaGetLastError();
+  return launch_chained(shared_plan_kernel, dim3(std::max(1, std::min((m + 7) / 8, 148 * 2))), dim3(256), 0, s, m, shared_scales(c, m, c.pair_above),
+                        c.geo.hidden / kTileK);
 }
 
 cudaError_t launch_plan_place(const Ctx& c, int m, int block_m, int32_t* stats, cudaStream_t s) {
   const int R = c.geo.num_ranks;
-  launch_chained(plan_kernel, dim3(1), dim3(kPlanThreads), 0, s, c.ws + c.lay.plan, c.at<int32_t>(c.lay.recv_count), stats,
-                 plan_args(c, m, block_m));
+  cudaError_t e = launch_chained(plan_kernel, dim3(1), dim3(kPlanThreads), 0, s, c.ws + c.lay.plan, c.at<int32_t>(c.lay.recv_count), stats,
+                                 plan_args(c, m, block_m));
+  if (e != cudaSuccess) return e;
   const bool direct = R == 1;
-  launch_chained(place_kernel, dim3(148 * 8), dim3(256), 0, s, c.ws + c.lay.plan, direct ? c.at<uint4>(c.lay.x) : c.at<uint4>(c.lay.recv_x),
+  return launch_chained(place_kernel, dim3(148 * 8), dim3(256), 0, s, c.ws + c.lay.plan, direct ? c.at<uint4>(c.lay.x) : c.at<uint4>(c.lay.recv_x),
       direct ? c.at<int32_t>(c.lay.x_sf) : c.at<int32_t>(c.lay.recv_sf),
       direct ? c.at<float>(c.lay.topk_weights) : c.at<float>(c.lay.recv_w), c.at<int32_t>(c.lay.sorted_route),
       c.at<uint4>(c.lay.pool_x), c.at<int32_t>(c.lay.pool_sf), c.at<float>(c.lay.pool_w), c.at<int32_t>(c.lay.pool_dst),
       c.lay.pool_sf_rows, c.e_local, R, c.geo.hidden, c.geo.num_topk, direct ? 1 : 0, shared_scales(c, m, c.shared_above_for(m)));
-  return cudaGetLastError();
 }
 
 // =====================================================================================================================
@@ -1169,11 +1163,9 @@ cudaError_t launch_combine(const Ctx& c, void* y, const void* residual, int m, c
   const int blocks = static_cast<int>(std::min<int64_t>((segs + 7) / 8, 148 * 8));
   const uint4* rows = c.geo.num_ranks == 1 ? c.at<uint4>(c.lay.ret) : c.at<uint4>(c.lay.ret_recv);
   char* plan = c.geo.num_ranks == 1 ? c.ws + c.lay.plan : nullptr;
-  launch_chained(combine_kernel, dim3(blocks + (plan != nullptr ? 1 : 0)), dim3(256), 0, s, rows, c.at<int32_t>(c.lay.route_pos),
-                                        c.geo.num_shared_experts > 0 ? c.at<uint4>(c.lay.shared_out) : nullptr,
-                                        static_cast<const uint4*>(residual), static_cast<uint4*>(y), m, c.geo.hidden,
-                                        c.geo.num_topk, plan, c.e_local);
-  return cudaGetLastError();
+  return launch_chained(combine_kernel, dim3(blocks + (plan != nullptr ? 1 : 0)), dim3(256), 0, s, rows, c.at<int32_t>(c.lay.route_pos),
+                        c.geo.num_shared_experts > 0 ? c.at<uint4>(c.lay.shared_out) : nullptr, static_cast<const uint4*>(residual),
+                        static_cast<uint4*>(y), m, c.geo.hidden, c.geo.num_topk, plan, c.e_local);
 }
 
 // =====================================================================================================================
@@ -1321,30 +1313,29 @@ cudaError_t launch_experts_simt(const Ctx& c, const MmoeWeights& w, const MmoeOp
   const int h = c.geo.hidden, inter = c.geo.intermediate;
   const int blocks = 148 * 8;
   char* plan = c.ws + c.lay.plan;
-  simt_l1_kernel<<<blocks, 128, 0, s>>>(plan, c.e_local, c.geo.num_ranks, 0, 0, c.at<uint8_t>(c.lay.pool_x),
-                                        c.at<int32_t>(c.lay.pool_sf), c.lay.pool_sf_rows, c.at<float>(c.lay.pool_w),
-                                        static_cast<const uint8_t*>(w.w13), static_cast<const int32_t*>(w.w13_sf),
-                                        c.at<uint8_t>(c.lay.act_x), c.at<uint8_t>(c.lay.act_sf), c.lay.pool_sf_rows, h,
-                                        inter, o.activation_clamp, o.fast_math, 0, w.w13_slice_stride);
-  simt_l2_kernel<<<blocks, 128, 0, s>>>(plan, c.e_local, c.geo.num_ranks, 0, c.at<uint8_t>(c.lay.act_x),
-                                        c.at<int32_t>(c.lay.act_sf), c.lay.pool_sf_rows,
-                                        static_cast<const uint8_t*>(w.w2), static_cast<const int32_t*>(w.w2_sf),
-                                        c.at<int32_t>(c.lay.pool_dst), c.at<__nv_bfloat16>(c.lay.ret), h, inter, 0,
-                                        w.w2_slice_stride);
+  const dim3 g(blocks), b(128);
+  cudaError_t e = launch_plain(simt_l1_kernel, g, b, 0, s, plan, c.e_local, c.geo.num_ranks, 0, 0, c.at<uint8_t>(c.lay.pool_x),
+                               c.at<int32_t>(c.lay.pool_sf), c.lay.pool_sf_rows, c.at<float>(c.lay.pool_w),
+                               static_cast<const uint8_t*>(w.w13), static_cast<const int32_t*>(w.w13_sf),
+                               c.at<uint8_t>(c.lay.act_x), c.at<uint8_t>(c.lay.act_sf), c.lay.pool_sf_rows, h,
+                               inter, o.activation_clamp, o.fast_math, 0, w.w13_slice_stride);
+  if (e == cudaSuccess)
+    e = launch_plain(simt_l2_kernel, g, b, 0, s, plan, c.e_local, c.geo.num_ranks, 0, c.at<uint8_t>(c.lay.act_x),
+                     c.at<int32_t>(c.lay.act_sf), c.lay.pool_sf_rows, static_cast<const uint8_t*>(w.w2),
+                     static_cast<const int32_t*>(w.w2_sf), c.at<int32_t>(c.lay.pool_dst), c.at<__nv_bfloat16>(c.lay.ret), h, inter, 0,
+                     w.w2_slice_stride);
   if (c.geo.num_shared_experts > 0 && m > 0) {
-    simt_l1_kernel<<<blocks, 128, 0, s>>>(plan, c.e_local, c.geo.num_ranks, 0, 1, c.at<uint8_t>(c.lay.x),
-                                          c.at<int32_t>(c.lay.x_sf), 0, nullptr,
-                                          static_cast<const uint8_t*>(w.shared_w13),
-                                          static_cast<const int32_t*>(w.shared_w13_sf),
-                                          c.at<uint8_t>(c.lay.shared_act_x), c.at<uint8_t>(c.lay.shared_act_sf),
-                                          c.lay.shared_sf_rows, h, inter, o.activation_clamp, o.fast_math, 1, 0);
-    simt_l2_kernel<<<blocks, 128, 0, s>>>(plan, c.e_local, c.geo.num_ranks, 1, c.at<uint8_t>(c.lay.shared_act_x),
-                                          c.at<int32_t>(c.lay.shared_act_sf), c.lay.shared_sf_rows,
-                                          static_cast<const uint8_t*>(w.shared_w2),
-                                          static_cast<const int32_t*>(w.shared_w2_sf), nullptr,
-                                          c.at<__nv_bfloat16>(c.lay.shared_out), h, inter, 1, 0);
+    if (e == cudaSuccess)
+      e = launch_plain(simt_l1_kernel, g, b, 0, s, plan, c.e_local, c.geo.num_ranks, 0, 1, c.at<uint8_t>(c.lay.x),
+                       c.at<int32_t>(c.lay.x_sf), 0, nullptr, static_cast<const uint8_t*>(w.shared_w13),
+                       static_cast<const int32_t*>(w.shared_w13_sf), c.at<uint8_t>(c.lay.shared_act_x),
+                       c.at<uint8_t>(c.lay.shared_act_sf), c.lay.shared_sf_rows, h, inter, o.activation_clamp, o.fast_math, 1, 0);
+    if (e == cudaSuccess)
+      e = launch_plain(simt_l2_kernel, g, b, 0, s, plan, c.e_local, c.geo.num_ranks, 1, c.at<uint8_t>(c.lay.shared_act_x),
+                       c.at<int32_t>(c.lay.shared_act_sf), c.lay.shared_sf_rows, static_cast<const uint8_t*>(w.shared_w2),
+                       static_cast<const int32_t*>(w.shared_w2_sf), nullptr, c.at<__nv_bfloat16>(c.lay.shared_out), h, inter, 1, 0);
   }
-  return cudaGetLastError();
+  return e;
 }
 
 }  // namespace mmoe

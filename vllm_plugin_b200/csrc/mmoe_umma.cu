@@ -1278,15 +1278,13 @@ cudaError_t prepare_one(Kernel* kernel, int smem_bytes) {
 template <int kLayer, bool kFused>
 cudaError_t launch_layer(UmmaParams& p, cudaStream_t s) {
   p.max_stages = g_tune_stages;
-  launch_chained(umma_kernel<kLayer, kFused>, dim3(tc_num_sms()), dim3(kThreads), Shape<kLayer>::kSmemBytes, s, p);
-  return cudaGetLastError();
+  return launch_chained(umma_kernel<kLayer, kFused>, dim3(tc_num_sms()), dim3(kThreads), Shape<kLayer>::kSmemBytes, s, p);
 }
 
 template <bool kStaged>
 cudaError_t launch_both(MoeParams& p, cudaStream_t s) {
   p.layer[0].max_stages = g_tune_stages;
-  launch_chained(moe_kernel<kStaged>, dim3(tc_num_sms()), dim3(both_threads(kStaged)), Shape<1>::kSmemBytes, s, p);
-  return cudaGetLastError();
+  return launch_chained(moe_kernel<kStaged>, dim3(tc_num_sms()), dim3(both_threads(kStaged)), Shape<1>::kSmemBytes, s, p);
 }
 
 // ---------------------------------------------------------------------------------------------------------------

@@ -100,8 +100,8 @@ cudaError_t launch_interleave_rows(const void* src, void* dst, int groups, int r
   const int64_t eights = (int64_t)groups * rows / 8;             // rows % 16 == 0: checked by the entry point
   if (eights == 0) return cudaSuccess;
   if (eights > INT32_MAX) return cudaErrorInvalidValue;
-  interleave_rows_kernel<<<static_cast<int>(eights), kCopyThreads, 0, s>>>(static_cast<const uint4*>(src), static_cast<uint4*>(dst), rows, row_bytes / 16);
-  return cudaGetLastError();
+  return launch_plain(interleave_rows_kernel, dim3(static_cast<unsigned>(eights)), dim3(kCopyThreads), 0, s, static_cast<const uint4*>(src),
+                      static_cast<uint4*>(dst), rows, row_bytes / 16);
 }
 
 cudaError_t launch_scale_layout(const int32_t* src, int32_t* dst, int groups, int rows, int row_stride, int kwords,
@@ -109,17 +109,15 @@ cudaError_t launch_scale_layout(const int32_t* src, int32_t* dst, int groups, in
   const int64_t blocks128 = (int64_t)groups * kwords * (rows / 128);     // rows % 128 == 0: checked by the entry point
   if (blocks128 == 0) return cudaSuccess;
   if (blocks128 / 16 >= INT32_MAX) return cudaErrorInvalidValue;
-  scale_layout_kernel<<<static_cast<int>(blocks128 / 16 + 1), 256, 0, s>>>(src, dst, blocks128, rows, row_stride, interleave);
-  return cudaGetLastError();
+  return launch_plain(scale_layout_kernel, dim3(static_cast<unsigned>(blocks128 / 16 + 1)), dim3(256), 0, s, src, dst, blocks128, rows, row_stride, interleave);
 }
 
 cudaError_t launch_split_halves(const void* src, void* dst, int groups, int64_t half_bytes, int64_t slice_stride, cudaStream_t s) {
   const int64_t half_vec = half_bytes / 16, per_half = (half_vec + kSplitPieceVec - 1) / kSplitPieceVec, pieces = 2 * (int64_t)groups * per_half;
   if (pieces == 0) return cudaSuccess;
   if (pieces > INT32_MAX) return cudaErrorInvalidValue;
-  split_halves_kernel<<<static_cast<int>(pieces), kCopyThreads, 0, s>>>(static_cast<const uint4*>(src), static_cast<uint4*>(dst), per_half, half_vec,
-                                                                        slice_stride / 16);
-  return cudaGetLastError();
+  return launch_plain(split_halves_kernel, dim3(static_cast<unsigned>(pieces)), dim3(kCopyThreads), 0, s, static_cast<const uint4*>(src),
+                      static_cast<uint4*>(dst), per_half, half_vec, slice_stride / 16);
 }
 
 }  // namespace mmoe
