@@ -560,7 +560,10 @@ int mmoe_forward(const MmoeGeometry* geo, void* workspace, const MmoeWeights* we
     if (e != cudaSuccess) return cuda_fail(e, "route / plan / placement launch");
   }
   rc = run_experts(geo, workspace, nullptr, weights, opt, num_tokens, block_m, stream, 0, in_gemm, stats, both_layers);
-  if (rc == MMOE_OK) rc = mmoe_combine_residual(geo, workspace, y_bf16, opt != nullptr ? opt->residual : nullptr, num_tokens, stream);
+  if (rc != MMOE_OK) return rc;                  // the launch of both GEMMs is the last of these: it did not run
+  rc = mmoe_combine_residual(geo, workspace, y_bf16, opt->residual, num_tokens, stream);
+  // It did run, and the next one has to find its counters at zero, or it takes every task for claimed and computes nothing.
+  if (rc != MMOE_OK && both_layers) mmoe::zero_counters(c, st);
   return rc;
 }
 

@@ -1,6 +1,7 @@
 // HBM-bound support kernels of the MegaMoE layer for sm_100a: input quantiser, route ordering, pool plan and
 // placement, top-k combine.  All integer work here is deterministic (no order-dependent atomics), so the dispatch
 // layout is reproducible run to run.
+#include <stddef.h>
 #include <stdlib.h>
 
 #include <algorithm>
@@ -1166,6 +1167,14 @@ cudaError_t launch_combine(const Ctx& c, void* y, const void* residual, int m, c
   return launch_chained(combine_kernel, dim3(blocks + (plan != nullptr ? 1 : 0)), dim3(256), 0, s, rows, c.at<int32_t>(c.lay.route_pos),
                         c.geo.num_shared_experts > 0 ? c.at<uint4>(c.lay.shared_out) : nullptr, static_cast<const uint4*>(residual),
                         static_cast<uint4*>(y), m, c.geo.hidden, c.geo.num_topk, plan, c.e_local);
+}
+
+cudaError_t zero_counters(const Ctx& c, cudaStream_t s) {
+  const PlanView pv = plan_view(c.ws + c.lay.plan, c.e_local, c.geo.num_ranks);
+  const size_t first = offsetof(PlanHeader, routed), end = offsetof(PlanHeader, layer1_done) + sizeof pv.hdr->layer1_done;
+  cudaError_t e = cudaMemsetAsync(reinterpret_cast<char*>(pv.hdr) + first, 0, end - first, s);      // `claims` lies between, zero already
+  if (e == cudaSuccess) e = cudaMemsetAsync(pv.done, 0, (c.e_local + 1) * sizeof *pv.done, s);
+  return e;
 }
 
 // =====================================================================================================================
