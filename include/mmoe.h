@@ -46,7 +46,8 @@ typedef struct MmoeGeometry {
   int32_t num_max_tokens;      /* per-rank token capacity T, a multiple of 1920 */
 } MmoeGeometry;
 
-/* Byte offsets of every region of the per-rank workspace (one allocation owned by the caller).  The first five are the
+/* Byte offsets of every region of the per-rank workspace (one allocation owned by the caller, 1024-byte aligned, all zero before
+ * its first use: the status words and the counters in the plan region are taken as they are).  The first five are the
  * views the serving engine writes or reads (`SymmBuffer.x / x_sf / topk_idx / topk_weights / shared_l1_acts_sf`,
  * backend/workspace.py:72-76,147-161); the rest are private to the kernels.  Replaces `build_symm_buffer_layout`
  * (backend/heuristics.py:504-674). */
@@ -79,7 +80,7 @@ typedef struct MmoeLayout {
   int64_t ret_recv;         /* EP>1 only: bf16 [T*kmax, H] outputs returned to this rank, in send order */
   int64_t shared_out;       /* bf16 [T, H] */
   int64_t ep_sync;          /* EP>1 only: epoch, per-barrier arrival flags and the [R][R] route-total table of the peer exchange */
-  int64_t status;           /* int32 [8] device status words, zero = healthy */
+  int64_t status;           /* int32 [8] device status words, zero = healthy; see mmoe_read_status */
   int64_t pool_rows;        /* row capacity of pool_x / act_x */
   int64_t pool_sf_rows;     /* row capacity (multiple of 128) of the pool SF chunk matrices */
   int64_t max_routes;       /* T * min(k, E/R): rows one rank can send */
@@ -274,7 +275,10 @@ int mmoe_split_halves(const void* src, void* dst, int32_t num_groups, int64_t ha
  * MMOE_OK, MMOE_ERR_DEVICE_TIMEOUT (a bounded wait expired: the outputs of that call are not valid) or
  * MMOE_ERR_INVALID_ARGUMENT (expert ids >= num_experts were seen and treated as masked).  The words are sticky until
  * read, so one read after any number of calls reports whether any of them failed; after the read a healthy call
- * reports MMOE_OK again.  Replaces the reference's device `trap` after a 300 s spin (backend/kernel/comm.py:229-250). */
+ * reports MMOE_OK again.  `words8` (may be NULL): [0] 1 after a timeout, then [1] the kernel, [2] its role and [3] its block that gave
+ * up first; [4] the number of bad expert ids.  Kernels: 1 and 2 GEMM1 / GEMM2 on the weights-as-A kernels, 4 both in one launch, 21
+ * and 22 GEMM1 / GEMM2 on CTA pairs (role: the warp), 10 + b barrier b of the peer exchange (role: the rank that did not arrive).
+ * A call that gave up leaves the workspace fit for the next one.  Replaces the reference's device `trap` after a 300 s spin (backend/kernel/comm.py:229-250). */
 int mmoe_read_status(const MmoeGeometry* geo, void* workspace, int32_t* words8, void* stream);
 
 /* Process-wide tuning of the tensor-core kernels (the reference keeps such knobs in `KernelOptions`,

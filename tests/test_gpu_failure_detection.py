@@ -136,3 +136,79 @@ def test_an_error_left_by_an_earlier_call_is_not_taken_for_a_failed_launch(m):
         api.fp8_fp4_mega_moe(y, l1, l2, buf, sl1, sl2, activation_clamp=10.0)
         api.read_status(buf)
         assert torch.equal(y, want)
+
+
+@pytest.mark.parametrize("hidden,inter,m,missing", [(512, 256, 8, "routed"), (512, 256, 8, "shared"), (512, 256, 100, "routed"),
+                                                    (2560, 1152, 16, "shared"), (2560, 1152, 150, "routed"), (2560, 1152, 300, "routed")])
+def test_rows_that_never_become_complete_and_the_call_behind(hidden, inter, m, missing):
+    """GEMM2 waits for a count of GEMM1's finished parts.  Here the count of one expert starts far below zero, as if parts of it were
+    lost: its GEMM2 tasks give up, every other task of the call is done, and the next call on the buffer is right."""
+    import time
+    from vllm_plugin_b200 import api
+    import helpers as H
+    from helpers import O
+    e, k = 8, 2
+    layer = H.make_layer(hidden, inter, e, k, True, seed=5)
+    weights = H.kernel_weights(layer, "cuda")
+    hid = O.make_hidden(m, hidden, 1)
+    ids, w = O.make_routing(m, e, k, 2)
+    want, buf = H.run_layer(layer, hid, ids, w, weights=weights)
+    rows = buf.ret[:m * k].clone()
+    assert O.parity_metrics(want.cpu(), H.oracle_layer(layer, hid, ids, w))["rel_l2"] <= 1e-3
+    lost = int(ids[0, 0]) if missing == "routed" else e
+    done = buf._view(buf.layout.plan, (16 + 5 * e + 4 + e + 1,), torch.int32)[16 + 5 * e + 4:]
+    api.set_kernel_options(timeout_ms=200)
+    try:
+        for _ in range(2):
+            buf.ret.zero_()
+            done[lost] = buf.plan_words[13] = -2 ** 30                    # 13: all experts' parts
+            torch.cuda.synchronize()
+            t0 = time.perf_counter()
+            with pytest.raises(RuntimeError, match="device wait expired: kernel 4"):
+                H.run_layer(layer, hid, ids, w, weights=weights, buf=buf)
+            assert 0.15 < time.perf_counter() - t0 < 2.0
+            assert buf.plan_words[9:14].cpu().tolist() == [0] * 5 and not done.any()
+            pos = buf.route_pos[:m].cpu().long()
+            for x in range(e):
+                if x != lost and bool((ids == x).any()):
+                    assert torch.equal(buf.ret[pos[ids == x].cuda()], rows[pos[ids == x].cuda()]), x
+            for _ in range(2):
+                y, _ = H.run_layer(layer, hid, ids, w, weights=weights, buf=buf)
+                assert torch.equal(y, want)
+    finally:
+        api.set_kernel_options(timeout_ms=2000)
+
+
+@pytest.fixture(scope="module")
+def run_wait(tmp_path_factory):
+    import os
+    import shutil
+    import subprocess
+    nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
+    if not os.path.exists(nvcc):
+        pytest.skip("nvcc is not installed")
+    so = str(tmp_path_factory.mktemp("waits") / "waits.so")
+    subprocess.run([nvcc, "-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-std=c++17", "-shared", "-Xcompiler", "-fPIC", "-o", so,
+                    os.path.join(os.path.dirname(__file__), "waits.cu")], check=True, capture_output=True)
+    fn = ctypes.CDLL(so).run_wait
+    fn.argtypes = [ctypes.c_int, ctypes.c_void_p, ctypes.c_int, ctypes.c_void_p, ctypes.c_int64, ctypes.c_void_p, ctypes.c_void_p]
+    return fn
+
+
+@pytest.mark.parametrize("which,name", list(enumerate(["the plan", "a task, whole warp", "a task, one lane polls", "a free slot for a task"])))
+def test_every_other_wait_of_the_launch_of_both_gemms_gives_up(run_wait, which, name):
+    """The waits that a call cannot be made to lose from outside, each in a kernel of one warp: for the plan of a launch that orders the
+    routes itself, for the scheduler's next task, and the scheduler's own for a free slot."""
+    plan, status, out = (torch.zeros(n, dtype=torch.int32, device="cuda") for n in (4096, 8, 1))
+    stream = torch.cuda.current_stream().cuda_stream
+    start, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    start.record()
+    assert run_wait(which, plan.data_ptr(), 8, status.data_ptr(), 100_000_000, out.data_ptr(), stream) == 0
+    end.record()
+    torch.cuda.synchronize()
+    assert out.item() == 1 and status.tolist()[:4] == [1, 4, 10 + which, 0]
+    assert 90 < start.elapsed_time(end) < 1000
+    if which == 0:                                 # ... and ends at once where the flag is set
+        plan[10] = 1
+        assert run_wait(which, plan.data_ptr(), 8, status.data_ptr(), 100_000_000, out.data_ptr(), stream) == 0
+        assert out.item() == 2

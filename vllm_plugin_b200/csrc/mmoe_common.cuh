@@ -172,6 +172,9 @@ __host__ __device__ inline int chunk_pos(int i) { return (i & 31) * 4 + ((i >> 5
 
 // Device status words (int32[8]): [0] != 0 means a bounded wait expired; [1] kernel id, [2] role, [3] block,
 // [4] bad-argument counter (e.g. an expert id out of range seen by the dispatch).
+// Kernel ids: 1, 2 weights-as-A, one layer (role: warp); 4 weights-as-A, both layers; 10 + b barrier b of the exchange (role: the rank
+// that did not come); 21, 22 CTA pairs, one layer.
+constexpr int kStatusBothLayers = 4, kStatusPairs = 20;
 enum { kStatusTimeout = 0, kStatusKernel = 1, kStatusRole = 2, kStatusBlock = 3, kStatusBadIndex = 4 };
 
 #ifdef __CUDACC__

@@ -21,8 +21,8 @@
 // A call on one GPU runs both layers in one launch (moe_kernel) of persistent CTAs, one per SM, that claim their tasks (tile, 256
 // weight rows) from a counter; with several ranks, and where a caller asks for one layer, umma_kernel walks a list dealt out
 // beforehand.  TMEM accumulators are double buffered so the epilogue of task i overlaps the loads and MMAs of task i+1.  Every
-// wait is bounded: when the budget expires the CTA records {kernel, role, block} in the status words (kernel 1 and 2: the layer,
-// 4: both), lets its in-flight copies land, frees its TMEM and returns; nothing traps.
+// wait is bounded: when the budget expires the CTA records {kernel, role, block} in the status words, lets its in-flight copies
+// land, frees its TMEM and returns; nothing traps.
 //
 // Expert parallelism: layer 2 has a second form (kFused) whose epilogue stores every BF16 row straight into the buffer
 // of the rank the token came from (plain peer stores over NVLink, no TMA from or to peer memory), and `tile_select`
@@ -1212,7 +1212,7 @@ __global__ void __launch_bounds__(both_threads(kStaged), 1) moe_kernel(const __g
   tc_fence_after();
   Cta c = sa_carve<L>(smem, sa_tile_rows(p), p.max_stages);
   c.tmem_base = __shfl_sync(0xffffffffu, ctl->tmem_base, 0);
-  Waiter waiter{&ctl->abort_flag, p.status, global_timer() + static_cast<uint64_t>(p.timeout_ns), 4, warp};
+  Waiter waiter{&ctl->abort_flag, p.status, global_timer() + static_cast<uint64_t>(p.timeout_ns), kStatusBothLayers, warp};
   RoleState st;
   if (warp == 0) {
     sa_producer_both<L, kStaged>(f, c, TaskFeed<false>(f, ctl), waiter, st);

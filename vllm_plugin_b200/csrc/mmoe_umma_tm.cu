@@ -269,7 +269,7 @@ __global__ void __launch_bounds__(tm_threads(kLayer), 1) tm_kernel(const __grid_
   PairWalk walk(p, cta, kLayer == 2);
   const int k_stages = p.k_dim / kTileK;
 
-  Waiter waiter{&ctl->abort_flag, p.status, global_timer() + static_cast<uint64_t>(p.timeout_ns), 20 + kLayer, warp};
+  Waiter waiter{&ctl->abort_flag, p.status, global_timer() + static_cast<uint64_t>(p.timeout_ns), kStatusPairs + kLayer, warp};
   const uint32_t full0 = smem_u32(&ctl->full[0]), empty0 = smem_u32(&ctl->empty[0]);
 
   // Every role walks the same task list; its loop runs at instruction latency, so everything that does not change inside a
