@@ -61,7 +61,8 @@ static void cache() {
 static void cuts() {
   for (int block_m : kBlockMs) {
     bool caps[kSmallTileRows + 1] = {};
-    for (int m = 0; m <= 300; ++m) caps[small_only_cap(m, block_m)] = true;
+    for (int m = 0; m <= 300; ++m)
+      for (int experts : {1, 63, 64, 512}) caps[small_only_cap(m, block_m, experts)] = true;
     caps[kDeepTileRows] = caps[kSmallTileRows] = true;                 // calls with pair tiles
     for (int cap = 0; cap <= kSmallTileRows; ++cap)
       for (int n = 1; caps[cap] && n <= 1100; ++n)

@@ -618,3 +618,73 @@ def test_both_gemms_in_one_launch(hidden, inter, experts, shared, m):
         assert torch.equal(y, y_one), call
         if experts <= 40 and call < 2:
             assert_parity(y_one, H.oracle_layer(layer, hid, ids, w), f"m {m} call {call}")
+
+
+@pytest.mark.parametrize("hidden,inter,shared", [(512, 256, True), (512, 256, False), (2560, 1152, True)])
+@pytest.mark.parametrize("bm,hot,cold", [(16, (160, 160, 128), 1), (16, (160, 128, 128), 1), (16, (160, 160, 128), 49), (16, (160, 160, 128), 50),
+                                         (16, (192, 192, 192), 0), (16, (64,), 7), (32, (64, 33), 5), (32, (65, 33), 5), (64, (100, 65, 33), 12)])
+def test_tile_rows_that_a_call_without_pairs_finds_in_its_plan(hidden, inter, shared, bm, hot, cold):
+    """The launch of both GEMMs starts with the shared expert in stages of 32 token rows; where tiles of 80 rows would be fewer by eight, and by
+    one in eight, its roles start over with larger ones.  Bit for bit what a launch per GEMM leaves, call after call, on either side of
+    the lines (160, 160 and 128 rows: eight tiles fewer of 14 and one per cold expert)."""
+    import ctypes
+    from vllm_plugin_b200 import api
+    from vllm_plugin_b200.backend import _native
+    from vllm_plugin_b200.backend.frontend import _weights_struct, check_mega_moe_arguments, read_status
+    if cold > 12 and hidden > 512:
+        pytest.skip("as many experts as the narrow layer has are checked there")
+    e, k, m = 72 if hidden == 512 else 24, 4, max(hot)
+    layer = H.make_layer(hidden, inter, e, k, shared, seed=81)
+    ids = torch.full((m, k), -1, dtype=torch.int64)
+    for slot, n in enumerate(hot):
+        ids[m - n:, slot] = 3 * slot + 1
+    for t in range(cold):
+        ids[t, 3] = 8 + t
+    counts = torch.bincount(ids[ids >= 0], minlength=e).tolist()
+    narrow, wide = (sum(-(-n // rows) for n in counts) for rows in (32, 80))
+    fewer = narrow - wide
+    cap = 80 if bm == 64 or (bm == 32 and m > 64 and e < 64) or (fewer >= 8 and 8 * fewer > narrow) else 32
+    w = torch.rand((m, k), generator=torch.Generator().manual_seed(2))
+    dev = torch.device("cuda", 0)
+    weights = H.kernel_weights(layer, dev)
+    l1, l2, sl1, sl2 = weights
+    lib, sp, buf = _native.load(), torch.cuda.current_stream(dev).cuda_stream, None
+    api.set_kernel_options(block_m=bm)
+    try:
+        for call in range(3):
+            hid = O.make_hidden(m, hidden, 5 + call)
+            y_one, buf = H.run_layer(layer, hid, ids, w, weights=weights, buf=buf)
+            words = buf.plan_words.cpu().tolist()
+            assert words[6] == (wide if cap == 80 else narrow) and words[7] == cap and words[9:14] == [0] * 5
+            y = torch.empty_like(y_one)
+            s13, s2 = check_mega_moe_arguments(y, l1, l2, buf, sl1, sl2, None, (1, 1, 32), "swiglu", 10.0, True, 1.0, 0.0)
+            ws, geo, base = _weights_struct(l1, l2, sl1, sl2, s13, s2), ctypes.byref(buf.geo), buf.base_ptr
+            api.stage_inputs_for_mega_moe(buf, hid.to(dev), ids.to(dev), w.to(dev))
+            _native.check(lib.mmoe_dispatch_count(geo, base, m, sp))
+            _native.check(lib.mmoe_dispatch_place(geo, base, m, bm, None, sp))
+            for mask in (1, 2):
+                opts = _native.MmoeOptions(10.0, 1, 0, 2000, mask)
+                _native.check(lib.mmoe_experts(geo, base, ctypes.byref(ws), ctypes.byref(opts), m, bm, sp))
+            _native.check(lib.mmoe_combine(geo, base, y.data_ptr(), m, sp))
+            read_status(buf)
+            assert torch.equal(y, y_one), call
+            if call == 0:
+                assert_parity(y_one, H.oracle_layer(layer, hid, ids, w), f"block_m {bm} hot {hot}")
+    finally:
+        api.set_kernel_options(block_m=0)
+
+
+@pytest.mark.parametrize("rows,cap", [((200, 30), 32), ((200, 33), 80), ((40, 17), 80)])
+def test_shared_expert_cut_as_the_routed_tiles_behind_pair_launches(rows, cap):
+    """193 to 256 tokens: the shared expert's tiles have 32 rows, 80 where some routed tile has more than 32 anyway."""
+    layer = H.make_layer(512, 256, 64, 6, True, seed=82)
+    m = 210
+    ids = torch.full((m, 6), -1, dtype=torch.int64)
+    for slot, n in enumerate(rows):
+        ids[m - n:, slot] = 9 * slot + 2
+    w = torch.rand((m, 6), generator=torch.Generator().manual_seed(3))
+    hid = O.make_hidden(m, layer.hidden, 6)
+    y, buf = H.run_layer(layer, hid, ids, w)
+    words = buf.plan_words.cpu().tolist()
+    assert words[4] <= 32 and words[1] == -(-m // cap) and words[14] == -(-(-(-m // words[1])) // 16) * 16
+    assert_parity(y, H.oracle_layer(layer, hid, ids, w), f"rows {rows}")

@@ -59,15 +59,30 @@ __host__ __device__ inline Cut cut_rows(int n, bool pairs, int small_cap) {
 // GEMM1 of a call of at most this many tokens on one GPU multiplies every expert that is hit with all staged tokens and orders
 // the routes itself (an UMMA takes 16 token columns at least); see staged_tokens().
 constexpr int kStagedTokens = 16;
-// Cap of a call without pair tiles, known to the host: the largest tile of such a call fixes its stage layout.  Tiles of up to 32
-// rows leave room for six stages, which is worth more than fewer tiles: BLOCK_M says how many rows an expert is to be expected to
-// have, one with more of them takes several.  With tiles as large as the call has tokens (up to 80): 64 tokens of 384 experts
-// 728 -> 709 us, 100 tokens 894 -> 870, 160 tokens 1058 -> 1029, 192 tokens of 97 experts 325 -> 321; with tiles of 16 rows 710, 874,
-// 1036 and 321.  An expert of any size has to fit the scale chunks of its pool blocks, see chunks_per_block().
+// Token slots with which a call without pair tiles starts, known to the host because its launch starts before the plan is complete;
+// also the cut of its shared expert.  Slots of up to 32 rows leave room for six stages, of up to 80 for five.  Six are worth 3 % where
+// a call reads many experts for a few rows each, and a tile more per 32 rows of the others costs its CTA a task:
+//   BLOCK_M 16, slots of 80 -> 32: 64 tokens of 384 experts 696 -> 674 us, 192 tokens 1044 -> 1012, 192 of 128 (top-3) 383 -> 375; with
+//     Zipf(1.2) popularity and two hot experts, 64 tokens of 384 127 -> 128, but 128 tokens 154 -> 165 and 192 tokens 185 -> 206.  Those
+//     start with 32, and the plan decides whether they stay there (wide_tiles()).
+//   BLOCK_M 32, 10 to 24 rows expected: 192 tokens of 97 experts 319 -> 312, skewed 189 -> 210, like the above.  Few experts: up to 64
+//     tokens of 32 and 16 121 -> 119 and 66 -> 64; past that there is little to gain, 192 tokens of 48, 128 of 32 and 96 of 16 (top-3)
+//     181 -> 182, 129 -> 129, 76.8 -> 75.7, and skewed 170 -> 193, 123 -> 134, 75 -> 76: those keep slots of 80.
+// An expert of any size fits the scale chunks of its pool blocks either way, see chunks_per_block().
 constexpr int kSixStageRows = 32;
-__host__ __device__ inline int small_only_cap(int m, int block_m) {
-  const int least = block_m <= 64 ? block_m : (block_m <= 128 ? 64 : kDeepTileRows);
-  return m <= least || least >= kSixStageRows ? least : kSixStageRows;
+constexpr int kFewExperts = 64, kFewExpertsTokens = 64;
+__host__ __device__ inline int small_only_cap(int m, int block_m, int e_local) {
+  if (block_m == 16 && m <= 16) return 16;
+  return block_m == 16 || (block_m == 32 && (m <= kFewExpertsTokens || e_local >= kFewExperts)) ? kSixStageRows : kDeepTileRows;
+}
+// Whether the experts of a call that starts with slots of 32 rows are cut at 80, from the number of tiles that either makes.  The CTAs
+// then drain their pipeline and start over (see sa_scheduler), which has to be earned back.  Zipf(1.2) and two hot experts: 18 tiles
+// fewer of 70, 192 tokens of 384 and of 97 experts 206 -> 194 and 212 -> 202 us; ten of 57 and of 37, 128 of 384 165 -> 161, 192 of 128
+// (top-3) 120 -> 118; eight of 46, 96 of 384 140.7 -> 140.5; five of 23, 96 of 128 89 -> 92.  One in eight: a call that only waits for HBM
+// has 3 % to gain from the sixth stage however many tiles it has.
+__host__ __device__ inline bool wide_tiles(int tiles32, int tiles80) {
+  const int fewer = tiles32 - tiles80;
+  return fewer >= 8 && 8 * fewer > tiles32;
 }
 // The cut of the shared expert's m tokens, known to the host as well, so that its tiles need no plan.  `cap`: rows of its tiles if
 // it is not on pairs.
@@ -109,7 +124,8 @@ struct PlanHeader {
   uint32_t claims;             // CTAs of that launch that have asked to do it, modulo its grid: zero between launches
   uint32_t next_task;          // tasks of a launch of both GEMMs that have been claimed: zero between calls
   int32_t layer1_done;         // sum of `done` below: zero between calls
-  int32_t pad[2];
+  int32_t shared_step;         // rows of the shared expert's tiles ...
+  int32_t shared_pairs;        // ... and 1 if they run on CTA pairs (neither is written where the launch orders the routes itself)
 };
 static_assert(sizeof(PlanHeader) == 64, "plan header is 64 bytes");
 
@@ -278,9 +294,10 @@ struct Ctx {             // resolved pointers of one call
     const int above = tile_select == 2 ? pair_above : pair_above_for(m);
     return geo.num_ranks == 1 && tile_select != 2 && above > 0 && above < kSharedPairsAbove ? kSharedPairsAbove : above;
   }
-  // ... and up to it in tiles of so many rows.
+  // ... and up to it in tiles of so many rows, which the plan of a call that may have pair tiles raises to kDeepTileRows.
   int shared_cap_for(int m, int block_m) const {
-    return geo.num_ranks == 1 && tile_select != 2 ? small_only_cap(m, block_m) : kDeepTileRows;
+    if (geo.num_ranks > 1 || tile_select == 2) return kDeepTileRows;
+    return pair_above_for(m) == kNeverPair ? small_only_cap(m, block_m, e_local) : kSixStageRows;
   }
   template <typename T> T* at(int64_t off) const { return reinterpret_cast<T*>(ws + off); }
   bool fused() const { return peer_ws != nullptr && geo.num_ranks > 1 && tile_select != 2; }

@@ -543,18 +543,26 @@ struct ExpertPlan {
 // table, offsets and header, written by the blocks that pass `write`.  The whole block takes part.
 __device__ ExpertPlan build_plan(const PlanView& pv, int n, const PlanArgs& a, bool write) {
   const int e = threadIdx.x;
-  __shared__ int s_rows;
-  if (threadIdx.x == 0) s_rows = 16;
+  __shared__ int s_rows, s_tiles;
+  if (threadIdx.x == 0) {
+    s_rows = 16;
+    s_tiles = 0;
+  }
   // With pair tiles in the call or rows from other ranks, weights-as-A tiles of 112 rows (four stages fit the shared memory) only
   // when enough experts gain a tile by it, else of 80 (five stages).
   const bool may_be_small = n > 0 && !on_pairs(n, a.pair_above, kSmallTileRows);
   const bool wide = may_be_small && ((n > kDeepTileRows && n <= kSmallTileRows) || n > 2 * kDeepTileRows);
   const int num_small = __syncthreads_count(may_be_small), num_wide = __syncthreads_count(wide);
-  const int cap = a.pair_above == kNeverPair && a.num_ranks == 1 ? small_only_cap(a.m, a.block_m) : (num_wide * 8 > num_small ? kSmallTileRows : kDeepTileRows);
+  const bool no_pairs = a.pair_above == kNeverPair && a.num_ranks == 1;
+  int cap = no_pairs ? small_only_cap(a.m, a.block_m, a.e_local) : (num_wide * 8 > num_small ? kSmallTileRows : kDeepTileRows);
+  if (no_pairs && cap == kSixStageRows) {
+    const int tiles = __reduce_add_sync(0xffffffffu, cut_rows(n, false, kSixStageRows).parts << 16 | cut_rows(n, false, kDeepTileRows).parts);
+    if ((threadIdx.x & 31) == 0 && tiles != 0) atomicAdd(&s_tiles, tiles);
+    __syncthreads();
+    if (wide_tiles(s_tiles >> 16, s_tiles & 0xFFFF)) cap = kDeepTileRows;
+  }
   const bool small = n > 0 && !on_pairs(n, a.pair_above, cap);
   const Cut cut = cut_rows(n, n > 0 && !small, cap);
-  const Cut sh_cut = shared_cut(a.has_shared ? a.m : 0, a.shared_above, a.shared_cap);
-  const bool shared_small = a.m <= a.shared_above;
   const int blocks = (n + a.block_m - 1) / a.block_m;
   ScanPair total;
   const ScanPair at = block_scan_pair(
@@ -574,6 +582,11 @@ __device__ ExpertPlan build_plan(const PlanView& pv, int n, const PlanArgs& a, b
       emit_tiles(pv.tiles + first_tile, e, block_off * a.block_m, n, cut, block_off * chunks_per_block(a.block_m));
     }
     __syncthreads();
+    // Behind pair launches the shared expert's cut is taken from the plan: where the routed tiles have larger slots anyway, its
+    // tiles are as large (256 tokens of 384 experts, skewed, 234 -> 228 us; even 1077, 1104 with tiles of 80 rows in any case).
+    const bool shared_small = a.m <= a.shared_above;
+    const int shared_cap = !no_pairs && a.num_ranks == 1 && s_rows > a.shared_cap ? kDeepTileRows : a.shared_cap;
+    const Cut sh_cut = shared_cut(a.has_shared ? a.m : 0, a.shared_above, shared_cap);
     if (threadIdx.x == 0) {
       PlanHeader& h = *pv.hdr;
       h.num_routed_tiles = small_total + pair_total;
@@ -585,6 +598,8 @@ __device__ ExpertPlan build_plan(const PlanView& pv, int n, const PlanArgs& a, b
       h.num_small_tiles = small_total;
       h.small_cap = cap;
       h.small_rows = max(s_rows, shared_small && a.has_shared ? sh_cut.step : 16);
+      h.shared_step = sh_cut.step;
+      h.shared_pairs = a.has_shared && !shared_small ? 1 : 0;
       pv.expert_block_off[a.e_local] = h.num_pool_blocks;
       pv.expert_tile_off[a.e_local] = h.num_routed_tiles;
     }

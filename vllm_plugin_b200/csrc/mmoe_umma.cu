@@ -65,8 +65,9 @@ struct UmmaParams {
   __nv_bfloat16* shared_out;
   int32_t* pool_dst;
   SharedTiles shared_tiles;    // run first
+  int shared_in_plan;          // 1: their cut is the plan's, which is complete when the launch starts
   int with_routed;             // 0: only those
-  int tile_rows;               // > 0: rows of the call's largest tile, known to the host; 0: in the plan
+  int tile_rows;               // > 0: rows of the token slots that the launch starts with; 0: those of the call's largest tile, in the plan
   int early;                   // both layers: 1 when the launch in front lets this one start with the staged tokens complete, not the plan
   int skip_wait;               // 1: what this launch reads was complete before the launch in front of it let it start
   const int32_t* x_sf;         // layer 1: the staged tokens' scale words [T][K/128], gathered for tiles of staged tokens
@@ -130,6 +131,7 @@ struct Control {          // lives at the start of shared memory
   uint32_t tmem_base;
   volatile int32_t abort_flag;
   uint32_t routes_here;   // staged tokens: this CTA orders the routes
+  int32_t next_rows;      // both layers: > 0 when the roles are to start over with token slots of so many rows
   union {
     struct {              // both layers in the launch
       uint64_t q_full[kQueue];    // scheduler -> the other roles: a task
@@ -208,6 +210,12 @@ __device__ __forceinline__ void locate_task(const Tile* tiles, int task, int n_b
   }
 }
 
+__device__ __forceinline__ SharedTiles sa_shared_tiles(const UmmaParams& p) {
+  if (!p.shared_in_plan || p.shared_tiles.parts == 0) return p.shared_tiles;
+  const PlanHeader* hdr = plan_view(const_cast<char*>(p.plan), p.e_local, p.num_ranks).hdr;
+  return SharedTiles{hdr->num_shared_tiles, hdr->shared_step, p.shared_tiles.m};
+}
+
 // The task list of one CTA as a role walks it in a launch of one layer.  First the shared expert's tasks, which need nothing but
 // the staged tokens and the host's count of them; then -- after what precedes this launch in the stream has completed -- the
 // routed tiles of the plan.  After the first round the CTAs take their tasks in the opposite order: the first ones, whose shared
@@ -217,6 +225,7 @@ struct TaskWalk {
   static constexpr bool kBoth = false;
   static constexpr int kLayer = kLaunchLayer;
   const UmmaParams& p;
+  const SharedTiles shared;
   int shared_tasks, routed_tasks, round;
   bool waited;
   const Tile* tiles;
@@ -224,7 +233,7 @@ struct TaskWalk {
   int nb;
   // `plan_ready`: the plan is complete, without a wait
   __device__ __forceinline__ TaskWalk(const UmmaParams& params, bool plan_ready)
-      : p(params), shared_tasks(params.shared_tiles.parts * params.n_blocks), routed_tasks(0), round(0), waited(false), tiles(nullptr) {
+      : p(params), shared(sa_shared_tiles(params)), shared_tasks(shared.parts * params.n_blocks), routed_tasks(0), round(0), waited(false), tiles(nullptr) {
     if (plan_ready) load_plan(true);
   }
   __device__ __forceinline__ void load_plan(bool ready) {
@@ -239,8 +248,8 @@ struct TaskWalk {
     int task = round == 0 ? blockIdx.x : (round + 1) * gridDim.x - 1 - blockIdx.x;
     ++round;
     if (task < shared_tasks) {
-      nb = task / p.shared_tiles.parts;
-      tile = p.shared_tiles.at(task - nb * p.shared_tiles.parts);
+      nb = task / shared.parts;
+      tile = shared.at(task - nb * shared.parts);
       return true;
     }
     task -= shared_tasks;
@@ -518,15 +527,19 @@ struct TaskQueue {
   const MoeParams& f;
   Control* ctl;
   PlanView pv;
+  SharedTiles shared;
   bool plan_known, over;
-  int small_tiles, hit_experts;
+  int small_tiles, small_rows, hit_experts;
   uint32_t claimed;        // lane 0
   uint32_t handed_on;
   __device__ __forceinline__ TaskQueue(const MoeParams& params, Control* control)
       : f(params), ctl(control), pv(plan_view(const_cast<char*>(params.layer[0].plan), params.layer[0].e_local, params.layer[0].num_ranks)),
-        plan_known(false), over(false), small_tiles(0), hit_experts(-1), claimed(0), handed_on(0) {}
+        shared(params.layer[0].shared_tiles), plan_known(false), over(false), small_tiles(0), small_rows(0), hit_experts(-1), claimed(0),
+        handed_on(0) {}
   __device__ __forceinline__ void load_plan() {
     small_tiles = pv.hdr->num_small_tiles;
+    small_rows = pv.hdr->small_rows;
+    shared = sa_shared_tiles(f.layer[0]);
     plan_known = true;
   }
   __device__ __forceinline__ bool wait_plan(Waiter& waiter) {
@@ -573,7 +586,6 @@ struct TaskQueue {
   // what the claimed number stands for; false when the call is being abandoned
   __device__ __forceinline__ bool decode(Waiter& waiter, QueueSlot* out) {
     int i = static_cast<int>(__shfl_sync(0xffffffffu, claimed, 0));
-    const SharedTiles& shared = f.layer[0].shared_tiles;
     for (int layer = 1; layer <= 2; ++layer) {
       const int n_blocks = f.layer[layer - 1].n_blocks, shared_tasks = shared.parts * n_blocks;
       out->layer = layer;
@@ -607,7 +619,7 @@ struct TaskQueue {
   // whether all of layer 1 is complete
   __device__ __forceinline__ bool layer1_over() {
     if (!over && plan_known) {
-      const int tiles = f.layer[0].shared_tiles.parts + (kStaged ? hit_experts : small_tiles);
+      const int tiles = shared.parts + (kStaged ? hit_experts : small_tiles);
       over = sa_rows_ready(&pv.hdr->layer1_done, 4 * f.layer[0].n_blocks * tiles);
     }
     return over;
@@ -724,13 +736,27 @@ __device__ __forceinline__ void sa_producer_both(const MoeParams& f, const Cta& 
     else sa_load_task<2, L, false>(f.layer[1], c, feed.tile, feed.nb, waiter, st, feed.ready ? nullptr : sa_done_of(f, pv, feed.tile),
                                    sa_need_of<kStaged>(f, feed.tile), want);
   }
+  if (kStaged || !st.ok || c.ctl->next_rows == 0) return;
+  // before another stage layout: every stage has been read, and the barriers have seen all that will arrive on them
+  for (uint32_t i = 0; i < c.num_stages; ++i) {
+    if (!waiter.wait_uniform(smem_u32(&c.ctl->empty[st.stage]), st.phase ^ 1u)) return;
+    if (++st.stage == c.num_stages) { st.stage = 0; st.phase ^= 1u; }
+  }
 }
 
+// `rows`: the token slots.  A launch that started before the plan was complete, with the shared expert's tasks, may find larger tiles in it.
+// The roles then leave as if there were no more tasks, and start over with slots of that size and with the task just claimed.
 template <bool kStaged>
-__device__ __forceinline__ void sa_scheduler(const Cta& c, TaskQueue<kStaged>& queue, Waiter& waiter) {
+__device__ __forceinline__ void sa_scheduler(const Cta& c, TaskQueue<kStaged>& queue, int rows, Waiter& waiter) {
+  queue.handed_on = 0;
   for (uint32_t n = 0;; ++n) {
     QueueSlot t;
-    if (!queue.decode(waiter, &t) || !queue.hand_on(waiter, t) || t.layer == 0) return;
+    if (!queue.decode(waiter, &t)) return;
+    if (!kStaged && t.layer != 0 && queue.small_rows > rows) {
+      if ((threadIdx.x & 31) == 0) c.ctl->next_rows = queue.small_rows;
+      t.layer = 0;
+    }
+    if (!queue.hand_on(waiter, t) || t.layer == 0) return;
     if (!waiter.wait_uniform(smem_u32(&c.ctl->q_want), n & 1u)) return;
     queue.claim();
   }
@@ -1077,28 +1103,39 @@ __device__ __forceinline__ int sa_tile_rows(const UmmaParams& p) {
   return p.tile_rows > 0 ? p.tile_rows : max(16, min(kSmallTileRows, plan_view(const_cast<char*>(p.plan), p.e_local, p.num_ranks).hdr->small_rows));
 }
 
+// one thread; kAgain: the barriers have been in use, and nothing will arrive on them any more
+template <typename L, bool kBoth, bool kAgain>
+__device__ __forceinline__ void sa_barriers(Control* ctl) {
+  auto init = [](uint64_t& bar, uint32_t count) {
+    if (kAgain) mbar_inval(smem_u32(&bar));
+    mbar_init(smem_u32(&bar), count);
+  };
+  for (int i = 0; i < L::kMaxStages; ++i) {
+    init(ctl->full[i], 1);
+    init(ctl->empty[i], 2);          // both MMA warps release a stage
+    init(ctl->sf_full[i], 1);
+    init(ctl->sf_ready[i], 1);
+  }
+  for (int i = 0; i < 2; ++i) {
+    init(ctl->tmem_full[i], 2);      // both MMA warps finish an accumulator pair
+    init(ctl->tmem_empty[i], 128);
+  }
+  if (kBoth)
+    for (int i = 0; i < kQueue; ++i) {
+      init(ctl->q_full[i], 1);
+      init(ctl->q_empty[i], 8);      // producer, MMA, epilogue and scale warps
+    }
+  if (kBoth) init(ctl->q_want, 1);
+  ctl->next_rows = 0;
+  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+}
+
 // barriers and tensor memory: touches only this CTA's own shared / tensor memory
 template <typename L, bool kBoth>
 __device__ __forceinline__ void sa_setup(Control* ctl) {
   if (threadIdx.x == 0) {
-    for (int i = 0; i < L::kMaxStages; ++i) {
-      mbar_init(smem_u32(&ctl->full[i]), 1);
-      mbar_init(smem_u32(&ctl->empty[i]), 2);          // both MMA warps release a stage
-      mbar_init(smem_u32(&ctl->sf_full[i]), 1);
-      mbar_init(smem_u32(&ctl->sf_ready[i]), 1);
-    }
-    for (int i = 0; i < 2; ++i) {
-      mbar_init(smem_u32(&ctl->tmem_full[i]), 2);      // both MMA warps finish an accumulator pair
-      mbar_init(smem_u32(&ctl->tmem_empty[i]), 128);
-    }
-    if (kBoth)
-      for (int i = 0; i < kQueue; ++i) {
-        mbar_init(smem_u32(&ctl->q_full[i]), 1);
-        mbar_init(smem_u32(&ctl->q_empty[i]), 8);      // producer, MMA, epilogue and scale warps
-      }
-    if (kBoth) mbar_init(smem_u32(&ctl->q_want), 1);
     ctl->abort_flag = 0;
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    sa_barriers<L, kBoth, false>(ctl);
   }
   if ((threadIdx.x >> 5) == 1) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&ctl->tmem_base)),
@@ -1207,31 +1244,46 @@ __global__ void __launch_bounds__(both_threads(kStaged), 1) moe_kernel(const __g
   const bool route_here = kStaged && p.route_here, plan_ready = !p.early && !route_here;
   if ((!p.early || route_here) && !p.skip_wait) chain_wait();
   if (plan_ready) queue.load_plan();
+  int rows = sa_tile_rows(p);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  Cta c = sa_carve<L>(smem, sa_tile_rows(p), p.max_stages);
-  c.tmem_base = __shfl_sync(0xffffffffu, ctl->tmem_base, 0);
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, ctl->tmem_base, 0);
   Waiter waiter{&ctl->abort_flag, p.status, global_timer() + static_cast<uint64_t>(p.timeout_ns), kStatusBothLayers, warp};
-  RoleState st;
-  if (warp == 0) {
-    sa_producer_both<L, kStaged>(f, c, TaskFeed<false>(f, ctl), waiter, st);
-  } else if (warp == 1 || warp == 6) {
-    sa_mma<L>(c, TaskFeed<false>(f, ctl), waiter, st, warp == 1 ? 0 : 1);
-  } else if (warp == 7) {
-    sa_arrange_scales<L, kStaged>(c, TaskFeed<false>(f, ctl), waiter, st);
-  } else if (warp == 8) {
-    sa_scheduler<kStaged>(c, queue, waiter);
-  } else if (warp == 9) {
-    if (route_here && sa_wait_plan(p, waiter)) sa_place(p);
-  } else {
-    const int t = static_cast<int>(threadIdx.x) - 64;
-    if (route_here && sa_claim_route(p, ctl, t))
-      sa_route(p, *reinterpret_cast<RouteScratch*>(c.sf_base + c.num_stages * L::kSfBytes), t);
-    sa_epilogue<L, false, kStaged>(c, TaskFeed<true>(f, ctl), plan_ready, waiter, st);
+  for (;;) {
+    Cta c = sa_carve<L>(smem, rows, p.max_stages);
+    c.tmem_base = tmem_base;
+    RoleState st;
+    if (warp == 0) {
+      sa_producer_both<L, kStaged>(f, c, TaskFeed<false>(f, ctl), waiter, st);
+    } else if (warp == 1 || warp == 6) {
+      sa_mma<L>(c, TaskFeed<false>(f, ctl), waiter, st, warp == 1 ? 0 : 1);
+    } else if (warp == 7) {
+      sa_arrange_scales<L, kStaged>(c, TaskFeed<false>(f, ctl), waiter, st);
+    } else if (warp == 8) {
+      sa_scheduler<kStaged>(c, queue, rows, waiter);
+    } else if (warp == 9) {
+      if (route_here && sa_wait_plan(p, waiter)) sa_place(p);
+    } else {
+      const int t = static_cast<int>(threadIdx.x) - 64;
+      if (route_here && sa_claim_route(p, ctl, t))
+        sa_route(p, *reinterpret_cast<RouteScratch*>(c.sf_base + c.num_stages * L::kSfBytes), t);
+      sa_epilogue<L, false, kStaged>(c, TaskFeed<true>(f, ctl), plan_ready, waiter, st);
+    }
+    if (kStaged) break;
+    // Another stage layout, once: behind this barrier no role waits, copies or multiplies, and the accumulators have been read.
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const int next = ctl->abort_flag != 0 ? 0 : ctl->next_rows;
+    if (next == 0) break;
+    rows = next;
+    __syncthreads();                                   // everyone has read it
+    if (threadIdx.x == 0) sa_barriers<L, true, true>(ctl);
+    __syncthreads();
   }
   chain_wait();       // a CTA that has not waited yet must not end before what precedes the launch
-  sa_teardown(ctl, c.tmem_base);
+  sa_teardown(ctl, tmem_base);
 }
 
 // ---------------------------------------------------------------------------------------------------------------
@@ -1605,7 +1657,8 @@ cudaError_t launch_experts_umma(const Ctx& c, const MmoeWeights& w, const MmoeOp
   auto small_params = [&](UmmaParams& p, int layer) {
     patch(p, layer == 2);
     p.shared_tiles = shared_pairs ? none : shared;
-    p.tile_rows = c.tile_select == 2 ? cut.step : (pairs || c.geo.num_ranks > 1 ? 0 : small_only_cap(m, block_m));
+    p.tile_rows = c.tile_select == 2 ? cut.step : 0;
+    p.shared_in_plan = pairs && c.geo.num_ranks == 1 && c.tile_select != 2 ? 1 : 0;
     // The pair launch in front reads and writes nothing that this one does, and lets it start only after its own wait.
     p.skip_wait = pairs ? 1 : 0;
   };
@@ -1631,6 +1684,7 @@ cudaError_t launch_experts_umma(const Ctx& c, const MmoeWeights& w, const MmoeOp
     for (int layer = 1; layer <= 2; ++layer) small_params(p.layer[layer - 1], layer);
     UmmaParams& p1 = p.layer[0];
     p1.early = pairs ? 0 : 1;
+    if (!pairs) p1.tile_rows = small_only_cap(m, block_m, c.e_local);
     p1.num_routes = m * c.geo.num_topk;
     p1.route_here = p.layer[1].route_here = c.route_in_gemm ? 1 : 0;
     p1.stats = c.stats;
