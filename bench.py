@@ -35,11 +35,12 @@ sys.path.insert(0, ROOT)
 H, I, E, K = 5120, 2304, 384, 6
 M_HEADLINE = 3840
 SWEEP = (1, 8, 64, 256, 1024, 2048, 3840)
-# DRAM read + write of the grouped-GEMM1 launches over what they must move (weights and weight scales of the experts
-# hit, FP8 token rows and scales in, FP8 activations and scales out), from ncu captures of small cases: weights-as-A
-# kernels at E=64 / M=640 (867.5 MB measured / 860.8 MB), tokens-as-A kernels at E=8 / M=640 (157.5 / 158.9 MB, the
-# last activation rows still in L2 when the kernel ends).  Both parts grow in proportion to the experts and tokens.
-NCU_TRAFFIC_RATIO_GEMM1 = {"weights-as-A": 1.008, "tokens-as-A": 0.991}
+# DRAM read + write of a launch over what it must move (weights and weight scales of the experts hit, token rows and scales
+# in, rows and scales out), from ncu captures of small cases: both GEMMs in one launch at E=64 / M=640 (1280.9 MB
+# measured / 1272.0 MB), GEMM1 alone on the weights-as-A kernels at E=64 / M=640 (867.5 / 860.8 MB, an earlier form of them) and on
+# CTA pairs at E=8 / M=640 (157.5 / 158.9 MB, the last rows still in L2 when the kernel ends).  Both parts grow in
+# proportion to the experts and tokens.
+NCU_TRAFFIC_RATIO = {"moe": 1.007, "weights-as-A": 1.008, "tokens-as-A": 0.991}
 # tensor pipe rate of `tcgen05.mma.kind::mxf8f6f4.block_scale` measured with back-to-back instructions (M=128, N>=160):
 # 8190 MAC per clock and SM, i.e. the nominal 8192
 TENSOR_MAC_PER_CLK_SM = 8192
@@ -221,6 +222,59 @@ def graph_latency(layer_call, sets, out, dev, reps):
     return lat[len(lat) // 2], lat[int(len(lat) * 0.9)]
 
 
+def captured_kernels(call, keep=None):
+    """``call`` captured into a CUDA graph: ``(graph, [names of its kernels])``, with ``keep`` = i reduced to its i-th kernel."""
+    from cuda.bindings import driver
+
+    def ok(result):
+        assert result[0] == driver.CUresult.CUDA_SUCCESS, result[0]
+        return result[1] if len(result) == 2 else result[1:]
+
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph):
+        call()
+    raw = driver.CUgraph(graph.raw_cuda_graph())
+    nodes = ok(driver.cuGraphGetNodes(raw, ok(driver.cuGraphGetNodes(raw))[1]))[0]
+    kernels = []
+    for node in nodes:
+        if ok(driver.cuGraphNodeGetType(node)) == driver.CUgraphNodeType.CU_GRAPH_NODE_TYPE_KERNEL:
+            params = ok(driver.cuGraphKernelNodeGetParams(node))
+            name = ok(driver.cuFuncGetName(params.func)) if int(params.func) else ok(driver.cuKernelGetName(params.kern))
+            kernels.append((name.decode(), node))
+    if keep is not None:
+        for node in nodes:
+            if int(node) != int(kernels[keep][1]):
+                ok(driver.cuGraphDestroyNode(node))
+    graph.instantiate()
+    return graph, [name for name, _ in kernels]
+
+
+# kernels of a call on one GPU, by a part of their (mangled) names
+KERNEL_PHASES = (("stage_kernel", "stage"), ("route_small_kernel", "route"), ("route_count_kernel", "route_count"),
+                 ("route_place_kernel", "route_place"), ("tm_kernelILi1", "pairs_gemm1"), ("tm_kernelILi2", "pairs_gemm2"),
+                 ("moe_kernel", "moe"), ("combine_kernel", "combine"))
+
+
+def time_kernels(call, dev, reps):
+    """Mean device time (ms) of every kernel that ``call`` launches, by name, each replayed as a graph of its own in the call's
+    order: ``(times, number of kernels)``.  Without the overlap that the call's chain of launches has."""
+    stream = torch.cuda.current_stream(dev)
+    names = captured_kernels(call)[1]
+    graphs = [captured_kernels(call, keep=i)[0] for i in range(len(names))]
+    evs = [torch.cuda.Event(enable_timing=True) for _ in range(len(names) + 1)]
+    acc = {}
+    for it in range(3 + reps):
+        evs[0].record(stream)
+        for graph, ev in zip(graphs, evs[1:]):
+            graph.replay()
+            ev.record(stream)
+        torch.cuda.synchronize(dev)
+        for i, name in enumerate(names if it >= 3 else ()):
+            phase = next(p for part, p in KERNEL_PHASES if part in name)
+            acc.setdefault(phase, []).append(evs[i].elapsed_time(evs[i + 1]))
+    return {phase + "_ms": statistics.mean(v) for phase, v in acc.items()}, len(names)
+
+
 def run_ours(args):
     import ctypes
 
@@ -297,15 +351,11 @@ def run_ours(args):
     barrier()
     step_ms = reduce_ranks(ev0.elapsed_time(ev1) / args.steps)
     value = world * m / (step_ms * 1e-3)
-    # EP1: quantiser, route counting + plan, placement, two GEMM launches on CTA pairs, one for all other experts, combine = 7; one
-    # routing launch up to 256 tokens, no pairs up to 192, no routing launch up to 16 (in pool blocks of 16 rows).  The peer
-    # exchange: quantiser, 3 route-ordering passes, publish, push, 2 flag waits, a flag kernel, shared-expert plan and 2 GEMMs,
-    # plan, place, 4 GEMM launches (2 for few routes), combine = 19; its unfused form has the shared expert in the same
-    # launches and a return copy (16); NCCL: the pack kernel instead of the exchange (12)
-    if world == 1:
-        in_gemm = m <= 16 and api.get_block_m_for_mega_moe(1, E, t_cap, m, K) == 16
-        launches_per_step = 7 if m > 256 else 6 if m > 192 else 3 if in_gemm else 4
-    else:
+    # One GPU: counted in the captured call, below.  The peer exchange: quantiser, 3 route-ordering passes, publish, push, 2 flag
+    # waits, a flag kernel, shared-expert plan and 2 GEMMs, plan, place, 4 GEMM launches (2 for few routes), combine = 19; its unfused
+    # form has the shared expert in the same launches and a return copy (16); NCCL: the pack kernel instead of the exchange (12)
+    launches_per_step = None
+    if world > 1:
         launches_per_step = {"nccl": 12, "peer-unfused": 16, "peer": 19}[args.ep_transport] - (2 if m * K <= min(3072, 96 * e_local) else 0)
         launches_per_step -= 1 if args.ep_transport == "peer" and m <= 192 else 0     # no shared-expert plan: nothing on CTA pairs
 
@@ -375,9 +425,9 @@ def run_ours(args):
     h2d_bytes = hid_h.numel() * 2 + ids_h.numel() * 8 + w_h.numel() * 4
     d2h_bytes = y_h[0].numel() * 2
 
-    # ---- the phases of one call timed back to back on one stream through the C ABI (the product call overlaps the
-    # exchange / ordering with the shared expert on a second stream; these are the costs of the parts).  Every rank runs
-    # the same sequence, the exchange kernels wait for their peers.
+    # ---- one GPU: every kernel that the timed call launches.  Several: the phases of a call timed back to back on one stream
+    # through the C ABI (the product call overlaps the exchange / ordering with the shared expert on a second stream; these are the
+    # costs of the parts).  Every rank runs the same sequence, the exchange kernels wait for their peers.
     geo = ctypes.byref(buf.geo)
     wst = _weights_struct(syn)
     bm = api.get_block_m_for_mega_moe(world, E, t_cap, m, K)
@@ -392,15 +442,14 @@ def run_ours(args):
     names = ["stage", "order", "exchange", "place", "shared", "gemm1", "gemm2", "return", "combine"]
     evs = [torch.cuda.Event(enable_timing=True) for _ in range(len(names) + 1)]
     acc = {n: [] for n in names}
-    can_time_phases = world == 1 or peers is not None
+    can_time_phases = world > 1 and peers is not None
     for it in range((3 + min(args.steps, 10)) if can_time_phases else 0):
         evs[0].record(stream)
         api.stage_inputs_for_mega_moe(buf, hid, ids, w)
         evs[1].record(stream)
         _native.check(lib.mmoe_dispatch_count(geo, ws, m, sp))
         evs[2].record(stream)
-        if world > 1:
-            _native.check(lib.mmoe_ep_dispatch(geo, ws, peers, m, ctypes.byref(opts1), sp))
+        _native.check(lib.mmoe_ep_dispatch(geo, ws, peers, m, ctypes.byref(opts1), sp))
         evs[3].record(stream)
         _native.check(lib.mmoe_dispatch_place(geo, ws, m, bm, None, sp))
         evs[4].record(stream)
@@ -418,8 +467,7 @@ def run_ours(args):
         else:
             _native.check(lib.mmoe_experts(geo, ws, ctypes.byref(wst), ctypes.byref(opts2), m, bm, sp))
         evs[7].record(stream)
-        if world > 1:
-            _native.check(lib.mmoe_ep_return(geo, ws, peers, ctypes.byref(opts1), sp))
+        _native.check(lib.mmoe_ep_return(geo, ws, peers, ctypes.byref(opts1), sp))
         evs[8].record(stream)
         _native.check(lib.mmoe_combine(geo, ws, y.data_ptr(), m, sp))
         evs[9].record(stream)
@@ -429,6 +477,8 @@ def run_ours(args):
                 acc[n].append(evs[j].elapsed_time(evs[j + 1]))
     barrier()
     phases = {n + "_ms": reduce_ranks(statistics.mean(v)) for n, v in acc.items() if v} if can_time_phases else {}
+    if world == 1:
+        phases, launches_per_step = time_kernels(lambda: layer_call(hid, ids, w, y), dev, min(args.steps, 10))
 
     # ---- algorithmic work of this rank's share of the step
     all_ids = ids
@@ -448,53 +498,67 @@ def run_ours(args):
     # experts with more than 192 rows run on CTA pairs; with the benchmark's uniform routing nearly all are on one side
     family = {0: "tokens-as-A" if expected_rows > 192 else "weights-as-A", 1: "weights-as-A",
               2: "tokens-as-A", 3: "tokens-as-A"}[args.orientation]
-    kernel_name = ("tm_kernel<1> (grouped GEMM1 + SwiGLU/requant, tokens-as-A on CTA pairs)" if family == "tokens-as-A"
-                   else "umma_kernel<1> (grouped GEMM1 + SwiGLU/requant, weights-as-A)")
-    kernel_name += ", the launches over the routed experts' tiles" if m > 128 else ", one launch over routed and shared tiles"
     sm_mhz = float((clocks or {}).get("sm_mhz") or 0.0)
     sm_mhz = reduce_ranks(sm_mhz, "max") or 1965.0                               # rank 0 samples its GPU
     tensor_peak = 2 * TENSOR_MAC_PER_CLK_SM * NUM_SMS * sm_mhz * 1e6 / 1e12      # TFLOP/s at the sampled SM clock
     tensor_peak_max = 2 * TENSOR_MAC_PER_CLK_SM * NUM_SMS * 1965.0 * 1e6 / 1e12
     roofline = None
     kernels = dict(phases)
-    if "gemm1_ms" in phases:
-        g1_ms, g2_ms = phases["gemm1_ms"], phases["gemm2_ms"]
-        # rows and weights of the timed launches: the routed experts alone when the shared expert has its own launches
-        shared_rows = 0 if split else m
-        rows = pairs_mean - m + shared_rows
-        pairs_mean = rows
-        g1_flops, g2_flops = rows * 4 * I * H, rows * 2 * I * H
-        w13_bytes = distinct_mean * (I * H + 2 * I * H // 32) + (0 if split else 2 * I * H + 2 * I * H // 32)
-        w2_bytes = distinct_mean * (H * I // 2 + H * I // 32) + (0 if split else H * I + H * I // 32)
-        g1_tflops, g1_gbs = g1_flops / (g1_ms * 1e-3) / 1e12, w13_bytes / (g1_ms * 1e-3) / 1e9
-        tensor_bound = g1_flops / (tensor_peak * 1e12) > w13_bytes / (peak_hbm * 1e9)
-        token_side_bytes = pairs_mean * (H + H // 32 + I + I // 32)     # FP8 rows + scales in, activations + scales out
-        common = {"kernel": kernel_name, "traffic": (w13_bytes + token_side_bytes) * NCU_TRAFFIC_RATIO_GEMM1[family],
-                  "traffic_source": "DRAM read+write over (weight bytes + token rows in + activations out) from the ncu capture "
-                                    "of a small case of this kernel, scaled by the experts hit and the rows processed",
+    # The call's longest GEMM launch, and the rows and experts of its tiles
+    w13_expert, w2_expert = I * H + 2 * I * H // 32, H * I // 2 + H * I // 32     # bytes of a routed expert; the shared one has twice the weights
+    work = None
+    if world == 1:
+        on_moe, on_pairs, shared_on_pairs = tiles_of(buf)
+        if phases.get("moe_ms", 0.0) >= phases.get("pairs_gemm1_ms", 0.0):
+            rows, experts = on_moe
+            shared = 0 if shared_on_pairs else 1
+            work = ("moe", "moe_kernel (both grouped GEMMs + SwiGLU/requant of every expert that is not on CTA pairs)", phases["moe_ms"],
+                    (rows + shared * m) * 6 * I * H, experts * (w13_expert + w2_expert) + shared * (3 * I * H + 3 * I * H // 32),
+                    (rows + shared * m) * (H + H // 32 + I + I // 32 + 2 * H))
+        else:
+            rows, experts = on_pairs
+            shared = 1 if shared_on_pairs else 0
+            work = ("tokens-as-A", "tm_kernel<1> (grouped GEMM1 + SwiGLU/requant, tokens-as-A on CTA pairs)", phases["pairs_gemm1_ms"],
+                    (rows + shared * m) * 4 * I * H, experts * w13_expert + shared * (2 * I * H + 2 * I * H // 32),
+                    (rows + shared * m) * (H + H // 32 + I + I // 32))
+    elif "gemm1_ms" in phases:
+        # the routed experts alone when the shared expert has its own launches
+        rows = pairs_mean - m + (0 if split else m)
+        work = (family, ("tm_kernel<1> (grouped GEMM1 + SwiGLU/requant, tokens-as-A on CTA pairs)" if family == "tokens-as-A"
+                         else "umma_kernel<1> (grouped GEMM1 + SwiGLU/requant, weights-as-A)")
+                + (", the launches over the routed experts' tiles" if split else ", one launch over routed and shared tiles"),
+                phases["gemm1_ms"], rows * 4 * I * H, distinct_mean * w13_expert + (0 if split else 2 * I * H + 2 * I * H // 32),
+                rows * (H + H // 32 + I + I // 32))
+        g2_s, g2_flops = phases["gemm2_ms"] * 1e-3, rows * 2 * I * H
+        kernels.update({
+            "gemm1_tflops": work[3] / (work[2] * 1e-3) / 1e12, "gemm2_tflops": g2_flops / g2_s / 1e12,
+            "gemm1_gbs": work[4] / (work[2] * 1e-3) / 1e9,
+            "gemm2_gbs": (distinct_mean * w2_expert + (0 if split else H * I + H * I // 32)) / g2_s / 1e9,
+            "gemm1_tensor_frac": work[3] / (work[2] * 1e-3) / 1e12 / tensor_peak, "gemm2_tensor_frac": g2_flops / g2_s / 1e12 / tensor_peak})
+    if work is not None:
+        capture, kernel_name, ms, w_flops, w_bytes, token_side_bytes = work
+        tflops, gbs = w_flops / (ms * 1e-3) / 1e12, w_bytes / (ms * 1e-3) / 1e9
+        common = {"kernel": kernel_name, "traffic": (w_bytes + token_side_bytes) * NCU_TRAFFIC_RATIO[capture],
+                  "traffic_source": "DRAM read+write over (weight bytes + token rows in and out) from the ncu capture of a small "
+                                    "case of this kernel, scaled by the experts hit and the rows processed",
                   "token_side_bytes_per_launch": token_side_bytes,
-                  "algorithmic_bytes_per_launch": w13_bytes, "algorithmic_flops_per_launch": g1_flops, "ms_per_launch": g1_ms}
-        if tensor_bound:
-            roofline = {"bound": "tensor", "achieved": g1_tflops, "peak": tensor_peak, "unit": "TFLOP/s",
-                        "frac": g1_tflops / tensor_peak,
+                  "algorithmic_bytes_per_launch": w_bytes, "algorithmic_flops_per_launch": w_flops, "ms_per_launch": ms}
+        if w_flops / (tensor_peak * 1e12) > w_bytes / (peak_hbm * 1e9):
+            roofline = {"bound": "tensor", "achieved": tflops, "peak": tensor_peak, "unit": "TFLOP/s",
+                        "frac": tflops / tensor_peak,
                         "peak_kind": "of measured: 8192 MAC/clk/SM (back-to-back tcgen05.mma kind::mxf8f6f4.block_scale "
                                      f"micro-benchmark) x 148 SMs at the SM clock sampled during the run ({sm_mhz:.0f} MHz)",
-                        "peak_at_max_clock": tensor_peak_max, "frac_of_peak_at_max_clock": g1_tflops / tensor_peak_max,
+                        "peak_at_max_clock": tensor_peak_max, "frac_of_peak_at_max_clock": tflops / tensor_peak_max,
                         **common}
         else:
-            roofline = {"bound": "hbm", "achieved": g1_gbs, "peak": peak_hbm, "unit": "GB/s", "frac": g1_gbs / peak_hbm,
+            roofline = {"bound": "hbm", "achieved": gbs, "peak": peak_hbm, "unit": "GB/s", "frac": gbs / peak_hbm,
                         "peak_kind": f"of {peak_kind}", **common}
-        kernels.update({
-            "gemm1_tflops": g1_tflops, "gemm2_tflops": g2_flops / (g2_ms * 1e-3) / 1e12,
-            "gemm1_gbs": g1_gbs, "gemm2_gbs": w2_bytes / (g2_ms * 1e-3) / 1e9,
-            "gemm1_tensor_frac": g1_tflops / tensor_peak, "gemm2_tensor_frac": g2_flops / (g2_ms * 1e-3) / 1e12 / tensor_peak})
     kernels.update({
         "kernel_family": family,
-        "phase_note": "phases timed back to back on one stream through the C ABI (past 128 tokens: shared_ms = the shared "
-                      "expert's two GEMM launches, gemm1_ms / gemm2_ms = the routed experts' launches); the product call at "
-                      "one GPU orders, plans and places in one or two launches and runs shared and routed tiles, and both GEMMs of the experts "
-                      "that are not on CTA pairs, in one launch; "
-                      "at more GPUs it overlaps the exchange with the shared expert",
+        "phase_note": "one GPU: every kernel of the timed call, replayed as a CUDA graph of its own in the call's order, launch "
+                      "latency included and without the overlap of the call's chain; more GPUs: phases timed back to back on one stream through the "
+                      "C ABI (past 128 tokens: shared_ms = the shared expert's two GEMM launches, gemm1_ms / gemm2_ms = the routed "
+                      "experts' launches), while the product call overlaps the exchange with the shared expert",
         "layer_tflops_per_gpu": flops_mean / (step_ms * 1e-3) / 1e12,
         "layer_tensor_frac": flops_mean / (step_ms * 1e-3) / 1e12 / tensor_peak,
         "layer_algorithmic_gbs_per_gpu": bytes_mean / (step_ms * 1e-3) / 1e9,
@@ -569,6 +633,15 @@ def run_ours(args):
     if dist is not None:
         dist.barrier()
         dist.destroy_process_group()
+
+
+def tiles_of(buf):
+    """Of the last call on one GPU, from its plan: ``(rows, experts)`` in tiles of the weights-as-A kernels, the same on CTA pairs, and
+    whether the shared expert is on pairs."""
+    words = buf.plan_words.cpu().tolist()
+    tiles = buf.plan_tiles()
+    small, pairs = tiles[:words[6]], tiles[words[6]:words[0]]
+    return (*((int(t[:, 2].sum()), int(torch.unique(t[t[:, 2] > 0, 0]).numel())) for t in (small, pairs)), words[15] != 0)
 
 
 def self_check(syn, buf, hid, ids, w, y, all_ids, rank, world, e_local, dev, reduce_ranks):

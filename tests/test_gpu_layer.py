@@ -656,6 +656,9 @@ def test_tile_rows_that_a_call_without_pairs_finds_in_its_plan(hidden, inter, sh
             y_one, buf = H.run_layer(layer, hid, ids, w, weights=weights, buf=buf)
             words = buf.plan_words.cpu().tolist()
             assert words[6] == (wide if cap == 80 else narrow) and words[7] == cap and words[9:14] == [0] * 5
+            tiles = buf.plan_tiles()
+            assert torch.bincount(tiles[:words[0], 0].long(), tiles[:words[0], 2].double(), minlength=e).long().tolist() == counts
+            assert tiles[words[0]:, 2].sum() == (m if shared else 0) and bool((tiles[words[0]:, 0] == -2).all())
             y = torch.empty_like(y_one)
             s13, s2 = check_mega_moe_arguments(y, l1, l2, buf, sl1, sl2, None, (1, 1, 32), "swiglu", 10.0, True, 1.0, 0.0)
             ws, geo, base = _weights_struct(l1, l2, sl1, sl2, s13, s2), ctypes.byref(buf.geo), buf.base_ptr
