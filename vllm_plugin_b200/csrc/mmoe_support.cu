@@ -563,6 +563,8 @@ __device__ ExpertPlan build_plan(const PlanView& pv, int n, const PlanArgs& a, b
   }
   const bool small = n > 0 && !on_pairs(n, a.pair_above, cap);
   const Cut cut = cut_rows(n, n > 0 && !small, cap);
+  Cut sh_cut = shared_cut(a.has_shared ? a.m : 0, a.shared_above, a.shared_cap);
+  const bool shared_small = a.m <= a.shared_above;
   const int blocks = (n + a.block_m - 1) / a.block_m;
   ScanPair total;
   const ScanPair at = block_scan_pair(
@@ -584,9 +586,7 @@ __device__ ExpertPlan build_plan(const PlanView& pv, int n, const PlanArgs& a, b
     __syncthreads();
     // Behind pair launches the shared expert's cut is taken from the plan: where the routed tiles have larger slots anyway, its
     // tiles are as large (256 tokens of 384 experts, skewed, 234 -> 228 us; even 1077, 1104 with tiles of 80 rows in any case).
-    const bool shared_small = a.m <= a.shared_above;
-    const int shared_cap = !no_pairs && a.num_ranks == 1 && s_rows > a.shared_cap ? kDeepTileRows : a.shared_cap;
-    const Cut sh_cut = shared_cut(a.has_shared ? a.m : 0, a.shared_above, shared_cap);
+    if (shared_small && !no_pairs && a.num_ranks == 1 && s_rows > a.shared_cap) sh_cut = shared_cut(a.has_shared ? a.m : 0, a.shared_above, kDeepTileRows);
     if (threadIdx.x == 0) {
       PlanHeader& h = *pv.hdr;
       h.num_routed_tiles = small_total + pair_total;
@@ -824,7 +824,8 @@ __global__ void __launch_bounds__(kRouteThreads) route_small_kernel(const RouteA
 // and builds the plan.  Further blocks place the shared expert's scales, which GEMM1 starts with while the next launch still places.
 __host__ __device__ inline int route_chunks(int m) { return m > kSortChunkTokens ? (m + kSortChunkTokens - 1) / kSortChunkTokens : 1; }
 
-__global__ void __launch_bounds__(kRouteThreads) route_count_kernel(const RouteArgs r) {
+// Three blocks per SM, for 40 registers: its blocks start beside the staging's last ones (with 64, 3840 tokens of 48 experts 956 -> 960 us).
+__global__ void __launch_bounds__(kRouteThreads, 3) route_count_kernel(const RouteArgs r) {
   chain_begin();
   extern __shared__ int32_t sm[];
   const int chunks = route_chunks(r.a.m);
