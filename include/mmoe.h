@@ -240,10 +240,10 @@ int mmoe_combine_residual(const MmoeGeometry* geo, void* workspace, void* y_bf16
  * environment, read once per process: ordinary launches).  The first kernel of the chain reads nothing before everything in front
  * of the call has ended, whether or not the kernel in front triggers its successors early.  Both GEMMs
  * are one launch, in which each CTA claims its tasks.  Up to 16 tokens (BLOCK_M 16) it also orders the routes and takes
- * the staged tokens as they are: two launches with the combine.  Up to 256 tokens one launch more orders the routes,
- * builds the plan and places the rows in front; past that these are two.  Past 192 tokens the experts with many rows run in two
- * launches of their own, on CTA pairs.  The shared expert's tiles come first, while
- * the rows are still being placed. */
+ * the staged tokens as they are: two launches with the combine.  Up to 256 tokens and 4096 routes one launch more orders the
+ * routes, builds the plan and places the rows in front; past either these are two.  Past 192 tokens the experts with many rows run
+ * in two launches of their own, on CTA pairs.  The shared expert's tiles come first, up to 192 and past 256 tokens while the rows are
+ * still being placed.  A call that stops because a launch failed leaves the workspace fit for the next one. */
 int mmoe_forward(const MmoeGeometry* geo, void* workspace, const MmoeWeights* weights, const MmoeOptions* opt,
                  void* y_bf16, int32_t num_tokens, int32_t block_m, int32_t* stats, void* stream);
 

@@ -620,9 +620,13 @@ def test_both_gemms_in_one_launch(hidden, inter, experts, shared, m):
             assert_parity(y_one, H.oracle_layer(layer, hid, ids, w), f"m {m} call {call}")
 
 
-@pytest.mark.parametrize("hidden,inter,shared", [(512, 256, True), (512, 256, False), (2560, 1152, True)])
-@pytest.mark.parametrize("bm,hot,cold", [(16, (160, 160, 128), 1), (16, (160, 128, 128), 1), (16, (160, 160, 128), 49), (16, (160, 160, 128), 50),
-                                         (16, (192, 192, 192), 0), (16, (64,), 7), (32, (64, 33), 5), (32, (65, 33), 5), (64, (100, 65, 33), 12)])
+TILE_ROWS = [(16, (160, 160, 128), 1), (16, (160, 128, 128), 1), (16, (192, 192, 192), 0), (16, (64,), 7), (32, (64, 33), 5), (32, (65, 33), 5),
+             (64, (100, 65, 33), 12)]
+MANY_COLD = [(16, (160, 160, 128), 49), (16, (160, 160, 128), 50)]
+
+
+@pytest.mark.parametrize("hidden,inter,shared,bm,hot,cold", [(512, 256, shared, *case) for shared in (True, False) for case in TILE_ROWS + MANY_COLD] +
+                         [(2560, 1152, True, *case) for case in TILE_ROWS])
 def test_tile_rows_that_a_call_without_pairs_finds_in_its_plan(hidden, inter, shared, bm, hot, cold):
     """The launch of both GEMMs starts with the shared expert in stages of 32 token rows; where tiles of 80 rows would be fewer by eight, and by
     one in eight, its roles start over with larger ones.  Bit for bit what a launch per GEMM leaves, call after call, on either side of
@@ -631,8 +635,6 @@ def test_tile_rows_that_a_call_without_pairs_finds_in_its_plan(hidden, inter, sh
     from vllm_plugin_b200 import api
     from vllm_plugin_b200.backend import _native
     from vllm_plugin_b200.backend.frontend import _weights_struct, check_mega_moe_arguments, read_status
-    if cold > 12 and hidden > 512:
-        pytest.skip("as many experts as the narrow layer has are checked there")
     e, k, m = 72 if hidden == 512 else 24, 4, max(hot)
     layer = H.make_layer(hidden, inter, e, k, shared, seed=81)
     ids = torch.full((m, k), -1, dtype=torch.int64)

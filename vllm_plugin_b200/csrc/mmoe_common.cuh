@@ -21,8 +21,10 @@ constexpr int kSmallTileRows = 112;      // largest token tile of the weights-as
 constexpr int kPairTileRows = 128;       // largest token tile of the tokens-as-A kernels (half of a CTA pair's 256 rows)
 constexpr int kNeverPair = 0x7fffffff;
 // The shared expert of a call on one GPU that may have pair tiles: on the pairs past this many tokens, else in tiles of the
-// weights-as-A kernels, which need no scale chunks, so that one launch orders and places the routes.  200 tokens of 48 experts 204 ->
-// 196 us, 256 of 384 1135 -> 1134; 384 tokens 1158 -> 1166, 512 1179 -> 1202.
+// weights-as-A kernels, which need no scale chunks, so that one launch orders and places the routes (up to kSmallRoutes of them).  On
+// pairs -> in tiles: 200 tokens of 48 experts 204 -> 195 us, of 16 (top-3) 105 -> 94, 256 of 384 1081 -> 1078, of 128 (top-3) 407 -> 400,
+// of 48 206 -> 198, of 32 163 -> 155, of 16 110 -> 100; skewed popularity, 200 of 384 203 -> 194, 256 of 384 224 -> 228, of 128 144 ->
+// 146, of 97 217 -> 217, of 48 199 -> 199, of 16 114 -> 108.  384 tokens 1158 -> 1166, 512 1179 -> 1202.
 constexpr int kSharedPairsAbove = 256;
 
 // Rows of a weights-as-A tile: five stages of up to 80 rows fit the shared memory, four of 112.

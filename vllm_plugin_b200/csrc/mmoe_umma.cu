@@ -736,11 +736,13 @@ __device__ __forceinline__ void sa_producer_both(const MoeParams& f, const Cta& 
     else sa_load_task<2, L, false>(f.layer[1], c, feed.tile, feed.nb, waiter, st, feed.ready ? nullptr : sa_done_of(f, pv, feed.tile),
                                    sa_need_of<kStaged>(f, feed.tile), want);
   }
-  if (kStaged || !st.ok || c.ctl->next_rows == 0) return;
-  // before another stage layout: every stage has been read, and the barriers have seen all that will arrive on them
-  for (uint32_t i = 0; i < c.num_stages; ++i) {
-    if (!waiter.wait_uniform(smem_u32(&c.ctl->empty[st.stage]), st.phase ^ 1u)) return;
-    if (++st.stage == c.num_stages) { st.stage = 0; st.phase ^= 1u; }
+  if constexpr (!kStaged) {
+    if (!st.ok || c.ctl->next_rows == 0) return;
+    // before another stage layout: every stage has been read, and the barriers have seen all that will arrive on them
+    for (uint32_t i = 0; i < c.num_stages; ++i) {
+      if (!waiter.wait_uniform(smem_u32(&c.ctl->empty[st.stage]), st.phase ^ 1u)) return;
+      if (++st.stage == c.num_stages) { st.stage = 0; st.phase ^= 1u; }
+    }
   }
 }
 

@@ -20,7 +20,9 @@ __device__ __forceinline__ int interleave_src_row(int r, int rows) {
   return ((r >> 3) & 1) * (rows >> 1) + channel;
 }
 
-// Copies run in pieces of 20 KB, contiguous on both sides: five 16-byte loads in flight per thread, and a block per piece.  Blocks that
+// Copies run in pieces that are contiguous on both sides, with a block per piece and five 16-byte loads in flight per thread: 20 KB for
+// the two-slice copy, eight rows for the row order, which is 20 KB at hidden 5120 (other widths leave part of the loads idle in the
+// last pass).  Blocks that
 // walked pieces 148 x 8 apart instead read and wrote too many DRAM pages at a time: 48 experts, rows and both halves 494 -> 446 us
 // (transform 210 -> 195, two-slice copy 292 -> 254 us, 6.7 TB/s); with ten loads of 128 threads 450, four of 512 462.
 // kAgain: the result is read again soon (the two-slice copy of what the transform has written).
