@@ -139,23 +139,29 @@ def test_an_error_left_by_an_earlier_call_is_not_taken_for_a_failed_launch(m):
 
 
 @pytest.mark.parametrize("hidden,inter,m,missing", [(512, 256, 8, "routed"), (512, 256, 8, "shared"), (512, 256, 100, "routed"),
-                                                    (2560, 1152, 16, "shared"), (2560, 1152, 150, "routed"), (2560, 1152, 300, "routed")])
+                                                    (2560, 1152, 16, "shared"), (2560, 1152, 150, "routed"), (2560, 1152, 300, "routed"),
+                                                    (512, 256, 160, "restarted"), (2560, 1152, 160, "restarted")])
 def test_rows_that_never_become_complete_and_the_call_behind(hidden, inter, m, missing):
     """GEMM2 waits for a count of GEMM1's finished parts.  Here the count of one expert starts far below zero, as if parts of it were
-    lost: its GEMM2 tasks give up, every other task of the call is done, and the next call on the buffer is right."""
+    lost: its GEMM2 tasks give up, every other task of the call is done, and the next call on the buffer is right.  "restarted": a skewed call,
+    whose CTAs have started over with larger token slots."""
     import time
     from vllm_plugin_b200 import api
     import helpers as H
     from helpers import O
-    e, k = 8, 2
+    e, k = 8, 3
     layer = H.make_layer(hidden, inter, e, k, True, seed=5)
     weights = H.kernel_weights(layer, "cuda")
     hid = O.make_hidden(m, hidden, 1)
     ids, w = O.make_routing(m, e, k, 2)
+    if missing == "restarted":
+        ids[:] = torch.tensor([6, 1, 4])
+        api.set_kernel_options(block_m=16)
     want, buf = H.run_layer(layer, hid, ids, w, weights=weights)
     rows = buf.ret[:m * k].clone()
     assert O.parity_metrics(want.cpu(), H.oracle_layer(layer, hid, ids, w))["rel_l2"] <= 1e-3
-    lost = int(ids[0, 0]) if missing == "routed" else e
+    assert buf.plan_words[7] == 80 or missing != "restarted"
+    lost = e if missing == "shared" else int(ids[0, 0])
     done = buf._view(buf.layout.plan, (16 + 5 * e + 4 + e + 1,), torch.int32)[16 + 5 * e + 4:]
     api.set_kernel_options(timeout_ms=200)
     try:
@@ -176,7 +182,7 @@ def test_rows_that_never_become_complete_and_the_call_behind(hidden, inter, m, m
                 y, _ = H.run_layer(layer, hid, ids, w, weights=weights, buf=buf)
                 assert torch.equal(y, want)
     finally:
-        api.set_kernel_options(timeout_ms=2000)
+        api.set_kernel_options(timeout_ms=2000, block_m=0)
 
 
 @pytest.fixture(scope="module")

@@ -329,11 +329,13 @@ def test_cuda_graph_replay_of_every_variant():
         assert_parity(y, H.oracle_layer(layer, hid_b, ids, w), f"graph replay m={m}")
 
 
-@pytest.mark.parametrize("m", [1, 16, 17, 200])
-def test_calls_in_flight_together_on_two_streams(m):
+@pytest.mark.parametrize("m,bm", [(1, 0), (16, 0), (17, 0), (200, 0), (160, 16)])
+def test_calls_in_flight_together_on_two_streams(request, m, bm):
     """Two buffers, two streams, and a third stream whose matrix products take SMs away from both: the CTAs of a call may start
-    one by one, and every call leaves bit for bit what it leaves alone."""
+    one by one, and every call leaves bit for bit what it leaves alone.  (160, 16): with CTAs that start over with larger token slots."""
     from vllm_plugin_b200 import api
+    request.addfinalizer(lambda: api.set_kernel_options(block_m=0))
+    api.set_kernel_options(block_m=bm)
     layer = H.make_layer(512, 256, 32, 6, True, seed=41)
     weights = H.kernel_weights(layer, "cuda")
     lanes = []
@@ -341,6 +343,7 @@ def test_calls_in_flight_together_on_two_streams(m):
         hid = O.make_hidden(m, layer.hidden, 50 + lane)
         ids, w = O.make_routing(m, 32, 6, 60 + lane, zipf_s=1.2, mask_frac=0.05)
         want, buf = H.run_layer(layer, hid, ids, w, weights=weights)
+        assert buf.plan_words[7] == 80 or bm == 0
         x, ids, w = hid.cuda(), ids.cuda(), w.cuda()
         ys = [torch.empty_like(want) for _ in range(20)]
         torch.cuda.synchronize()
