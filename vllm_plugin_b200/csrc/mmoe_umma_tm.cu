@@ -94,8 +94,12 @@ __device__ __forceinline__ uint32_t map_to_cta(uint32_t addr, uint32_t rank) {
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
   return r;
 }
-__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+// Arrival on a barrier of either CTA of the pair.  What it hands over are columns of tensor memory, ordered by the tcgen05 fences on
+// either side; no memory access rides on it.  So the default release, of CTA scope, is enough: one of cluster scope first waits for
+// this warp's outstanding stores to global memory, which stood between every two tasks of the issuer (3840 tokens of 48 experts 970 ->
+// 942 us, 2560 of 16 387 -> 381; GEMM2, whose epilogue stores most, 294 -> 275).
+__device__ __forceinline__ void mbar_arrive_pair(uint32_t cluster_addr) {
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
 __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
@@ -412,7 +416,7 @@ __global__ void __launch_bounds__(tm_threads(kLayer), 1) tm_kernel(const __grid_
       // None of this warp's rows is a token: nothing to do (350 rows per expert, fast_math off: 1035 -> 913 us).
       if (q * 32 >= tile.n_valid) {
         tc_fence_before();
-        if (lane == 0) mbar_arrive_cluster(overlap_free_leader);
+        if (lane == 0) mbar_arrive_pair(overlap_free_leader);
         continue;
       }
       const uint32_t d0 = tmem_base + lane_sel + acc * kTmAccStride;
@@ -430,7 +434,7 @@ __global__ void __launch_bounds__(tm_threads(kLayer), 1) tm_kernel(const __grid_
         if (step == 0) {
           tc_fence_before();
           __syncwarp();
-          if (lane == 0) mbar_arrive_cluster(overlap_free_leader);
+          if (lane == 0) mbar_arrive_pair(overlap_free_leader);
         }
         if (kLayer == 1) {
           uint32_t w[8];
