@@ -457,12 +457,13 @@ __device__ __forceinline__ bool sa_wait_plan(const UmmaParams& p, Waiter& waiter
 // GEMM2 of an expert needs all of its GEMM1 tasks, wherever those ran.  A counter per expert (the last one: the shared expert)
 // counts the epilogue warps that have stored their part, and one for all experts spares a CTA the question once GEMM1 is over.
 // The rows are then read by bulk copies, hence the proxy fence between seeing the count and asking for them (one on this side too
-// takes 3 us behind a task's stores).
+// takes 3 us behind a task's stores).  One fence releases both additions; with a sequentially consistent one and a release of its
+// own on the first addition, each of which waits for the stores, one token took 39.45 us instead of 38.95, seven 134.2 instead of 133.1.
 __device__ __forceinline__ void sa_publish(const PlanView& pv, int slot) {
   __syncwarp();
   if ((threadIdx.x & 31) == 0) {
-    __threadfence();
-    asm volatile("red.release.gpu.global.add.s32 [%0], 1;" ::"l"(pv.done + slot) : "memory");
+    asm volatile("fence.acq_rel.gpu;" ::: "memory");
+    asm volatile("red.relaxed.gpu.global.add.s32 [%0], 1;" ::"l"(pv.done + slot) : "memory");
     asm volatile("red.relaxed.gpu.global.add.s32 [%0], 1;" ::"l"(&pv.hdr->layer1_done) : "memory");
   }
 }
