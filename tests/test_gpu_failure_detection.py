@@ -185,6 +185,35 @@ def test_rows_that_never_become_complete_and_the_call_behind(hidden, inter, m, m
         api.set_kernel_options(timeout_ms=2000, block_m=0)
 
 
+@pytest.mark.parametrize("missing", ["routed", "shared"])
+def test_pairs_that_wait_for_lost_rows_and_the_call_behind(missing):
+    """The same where the experts run on CTA pairs, whose GEMM2 starts behind GEMM1's finished parts as SMs come free."""
+    from vllm_plugin_b200 import api
+    import helpers as H
+    from helpers import O
+    e, k, m, hidden, inter = 4, 2, 1000, 512, 256
+    layer = H.make_layer(hidden, inter, e, k, True, seed=6)
+    weights = H.kernel_weights(layer, "cuda")
+    hid = O.make_hidden(m, hidden, 1)
+    ids, w = O.make_routing(m, e, k, 2)
+    want, buf = H.run_layer(layer, hid, ids, w, weights=weights)
+    assert O.parity_metrics(want.cpu(), H.oracle_layer(layer, hid, ids, w))["rel_l2"] <= 1e-3
+    assert buf.plan_words[6] == 0                                         # every expert on pairs
+    done = buf._view(buf.layout.plan, (16 + 5 * e + 4 + e + 3,), torch.int32)[16 + 5 * e + 4:]      # and the claimed tasks behind it
+    api.set_kernel_options(timeout_ms=200)
+    try:
+        for _ in range(2):
+            done[e if missing == "shared" else 1] = -2 ** 30
+            with pytest.raises(RuntimeError, match="device wait expired: kernel 22"):
+                H.run_layer(layer, hid, ids, w, weights=weights, buf=buf)
+            assert not done.any()
+            for _ in range(2):
+                y, _ = H.run_layer(layer, hid, ids, w, weights=weights, buf=buf)
+                assert torch.equal(y, want)
+    finally:
+        api.set_kernel_options(timeout_ms=2000)
+
+
 @pytest.fixture(scope="module")
 def run_wait(tmp_path_factory):
     import os

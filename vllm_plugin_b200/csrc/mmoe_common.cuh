@@ -132,7 +132,7 @@ struct PlanHeader {
 static_assert(sizeof(PlanHeader) == 64, "plan header is 64 bytes");
 
 // Plan region: header | expert_total[E_l] | expert_block_off[E_l+1] | expert_tile_off[E_l+1] | rank_off[R+1] |
-// seg_pool_start[E_l*R] | seg_recv_start[E_l*R] | done[E_l+1] | tiles[max_tiles]
+// seg_pool_start[E_l*R] | seg_recv_start[E_l*R] | done[E_l+1] | pair_tasks[2] | tiles[max_tiles]
 struct PlanView {
   PlanHeader* hdr;
   int32_t* expert_total;
@@ -141,7 +141,8 @@ struct PlanView {
   int32_t* rank_off;
   int32_t* seg_pool_start;
   int32_t* seg_recv_start;
-  int32_t* done;               // launch of both GEMMs: finished parts of GEMM1 per expert, the shared one last; zero between calls
+  int32_t* done;               // one GPU, both GEMMs: finished parts of GEMM1 per expert, the shared one last; zero between calls
+  int32_t* pair_tasks;         // ... and the tasks of either layer that CTA pairs have claimed, likewise
   Tile* tiles;
 };
 
@@ -163,7 +164,7 @@ __host__ __device__ inline int64_t shared_chunk_rows(int64_t max_tokens) { retur
 __host__ __device__ inline int64_t shared_tile_capacity(int64_t max_tokens) { return (max_tokens / 16 + 2) * 2; }
 
 __host__ __device__ inline int64_t plan_bytes(int e_local, int num_ranks, int64_t max_tiles) {
-  int64_t ints = e_local + 3 * (e_local + 1) + (num_ranks + 1) + 2 * (int64_t)e_local * num_ranks;
+  int64_t ints = e_local + 3 * (e_local + 1) + (num_ranks + 1) + 2 * (int64_t)e_local * num_ranks + 2;
   return 64 + align_up(ints * 4, 32) + max_tiles * (int64_t)sizeof(Tile);
 }
 
@@ -179,6 +180,7 @@ __host__ __device__ inline PlanView plan_view(void* base, int e_local, int num_r
   v.seg_pool_start = q;          q += (int64_t)e_local * num_ranks;
   v.seg_recv_start = q;          q += (int64_t)e_local * num_ranks;
   v.done = q;                    q += e_local + 1;
+  v.pair_tasks = q;              q += 2;
   int64_t ints = q - reinterpret_cast<int32_t*>(p + 64);
   v.tiles = reinterpret_cast<Tile*>(p + 64 + align_up(ints * 4, 32));
   return v;

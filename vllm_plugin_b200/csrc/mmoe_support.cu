@@ -1107,7 +1107,7 @@ __global__ void __launch_bounds__(256) combine_kernel(
       pv.hdr->next_task = 0;
       pv.hdr->layer1_done = 0;
     }
-    for (int e = threadIdx.x; e <= e_local; e += blockDim.x) pv.done[e] = 0;
+    for (int e = threadIdx.x; e < e_local + 3; e += blockDim.x) pv.done[e] = 0;      // and `pair_tasks` behind it
     __threadfence();
     __syncthreads();
     chain_release();
@@ -1189,7 +1189,7 @@ cudaError_t zero_counters(const Ctx& c, cudaStream_t s) {
   const PlanView pv = plan_view(c.ws + c.lay.plan, c.e_local, c.geo.num_ranks);
   const size_t first = offsetof(PlanHeader, routed), end = offsetof(PlanHeader, layer1_done) + sizeof pv.hdr->layer1_done;
   cudaError_t e = cudaMemsetAsync(reinterpret_cast<char*>(pv.hdr) + first, 0, end - first, s);      // `claims` lies between, zero already
-  if (e == cudaSuccess) e = cudaMemsetAsync(pv.done, 0, (c.e_local + 1) * sizeof *pv.done, s);
+  if (e == cudaSuccess) e = cudaMemsetAsync(pv.done, 0, (c.e_local + 3) * sizeof *pv.done, s);
   return e;
 }
 

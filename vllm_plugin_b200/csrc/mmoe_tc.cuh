@@ -212,6 +212,22 @@ struct Waiter {
     }
   }
 };
+
+// GEMM2 of an expert needs all of its GEMM1 tasks, wherever those ran.  A counter per expert (PlanView::done) counts the epilogue
+// warps that have stored their part; one lane of each, behind a __syncwarp().
+__device__ __forceinline__ void part_release() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
+__device__ __forceinline__ void part_count(int32_t* counter) {
+  asm volatile("red.relaxed.gpu.global.add.s32 [%0], 1;" ::"l"(counter) : "memory");
+}
+// Whether the counter has come to `need`, whole warp.  The rows are then read by bulk copies, hence the proxy fence (one on the
+// writing side too takes 3 us behind a task's stores).
+__device__ __forceinline__ bool rows_ready(const int32_t* done, int need) {
+  int32_t v;
+  asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(done) : "memory");
+  if (!__all_sync(0xffffffffu, v >= need)) return false;
+  asm volatile("fence.proxy.async.global;" ::: "memory");
+  return true;
+}
 #endif  // __CUDACC__
 
 // ---------------------------------------------------------------------------------------------------------------
@@ -263,6 +279,8 @@ struct TmParams {
   int hidden, inter;
   float clamp;
   int fast_math;
+  int32_t* tasks;                  // both layers of a single-GPU call: counter of the claimed tasks of this layer ...
+  int32_t* done;                   // ... and PlanView::done; else null
 };
 cudaError_t tm_prepare();
 cudaError_t tm_launch(int layer, bool fused, const TmParams& p, cudaStream_t s);

@@ -454,25 +454,16 @@ __device__ __forceinline__ bool sa_wait_plan(const UmmaParams& p, Waiter& waiter
 }
 
 // ------------------------------------------------------------------------------------------------ both layers in one launch
-// GEMM2 of an expert needs all of its GEMM1 tasks, wherever those ran.  A counter per expert (the last one: the shared expert)
-// counts the epilogue warps that have stored their part, and one for all experts spares a CTA the question once GEMM1 is over.
-// The rows are then read by bulk copies, hence the proxy fence between seeing the count and asking for them (one on this side too
-// takes 3 us behind a task's stores).  One fence releases both additions; with a sequentially consistent one and a release of its
-// own on the first addition, each of which waits for the stores, one token took 39.45 us instead of 38.95, seven 134.2 instead of 133.1.
+// Counts a part of GEMM1 (see part_release), for its expert and in one counter for all, which spares a CTA the question once GEMM1 is
+// over.  One fence releases both additions; with a sequentially consistent one and a release of its own on the first addition, each of
+// which waits for the stores, one token took 39.45 us instead of 38.95, seven 134.2 instead of 133.1.
 __device__ __forceinline__ void sa_publish(const PlanView& pv, int slot) {
   __syncwarp();
   if ((threadIdx.x & 31) == 0) {
-    asm volatile("fence.acq_rel.gpu;" ::: "memory");
-    asm volatile("red.relaxed.gpu.global.add.s32 [%0], 1;" ::"l"(pv.done + slot) : "memory");
-    asm volatile("red.relaxed.gpu.global.add.s32 [%0], 1;" ::"l"(&pv.hdr->layer1_done) : "memory");
+    part_release();
+    part_count(pv.done + slot);
+    part_count(&pv.hdr->layer1_done);
   }
-}
-__device__ __forceinline__ bool sa_rows_ready(const int32_t* done, int need) {
-  int32_t v;
-  asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(done) : "memory");
-  if (!__all_sync(0xffffffffu, v >= need)) return false;
-  asm volatile("fence.proxy.async.global;" ::: "memory");
-  return true;
 }
 
 // The task list of such a launch: shared expert and routed tiles of layer 1, then of layer 2.  CTAs claim tasks from a counter when
@@ -621,13 +612,13 @@ struct TaskQueue {
   __device__ __forceinline__ bool layer1_over() {
     if (!over && plan_known) {
       const int tiles = shared.parts + (kStaged ? hit_experts : small_tiles);
-      over = sa_rows_ready(&pv.hdr->layer1_done, 4 * f.layer[0].n_blocks * tiles);
+      over = rows_ready(&pv.hdr->layer1_done, 4 * f.layer[0].n_blocks * tiles);
     }
     return over;
   }
   // to the other roles of the CTA
   __device__ __forceinline__ bool hand_on(Waiter& waiter, QueueSlot& t) {
-    t.ready = t.layer == 2 && (layer1_over() || sa_rows_ready(sa_done_of(f, pv, t.tile), sa_need_of<kStaged>(f, t.tile))) ? 1 : 0;
+    t.ready = t.layer == 2 && (layer1_over() || rows_ready(sa_done_of(f, pv, t.tile), sa_need_of<kStaged>(f, t.tile))) ? 1 : 0;
     const uint32_t slot = handed_on % kQueue;
     if (!waiter.wait_uniform(smem_u32(&ctl->q_empty[slot]), ((handed_on / kQueue) & 1u) ^ 1u)) return false;
     if ((threadIdx.x & 31) == 0) {
@@ -676,7 +667,7 @@ __device__ __forceinline__ void sa_load_task(const UmmaParams& p, const Cta& c, 
   };
   int ahead = 0;                                                 // stages whose weights have been requested
   if (kLayer == 2 && done != nullptr) {
-    if (!sa_rows_ready(done, need)) {
+    if (!rows_ready(done, need)) {
       uint32_t stage = st.stage, phase = st.phase;
       const int most = min(static_cast<int>(c.num_stages), k_stages);
       for (; ahead < most; ++ahead) {
@@ -688,7 +679,7 @@ __device__ __forceinline__ void sa_load_task(const UmmaParams& p, const Cta& c, 
         __syncwarp();
         if (++stage == c.num_stages) { stage = 0; phase ^= 1u; }
       }
-      for (uint32_t spin = 0; !sa_rows_ready(done, need); ++spin) {
+      for (uint32_t spin = 0; !rows_ready(done, need); ++spin) {
         if ((spin & 63u) == 63u && __any_sync(0xffffffffu, waiter.abandoned())) { st.ok = false; return; }
         __nanosleep(40);
       }
@@ -1662,18 +1653,22 @@ cudaError_t launch_experts_umma(const Ctx& c, const MmoeWeights& w, const MmoeOp
     p.shared_tiles = shared_pairs ? none : shared;
     p.tile_rows = c.tile_select == 2 ? cut.step : 0;
     p.shared_in_plan = pairs && c.geo.num_ranks == 1 && c.tile_select != 2 ? 1 : 0;
-    // The pair launch in front reads and writes nothing that this one does, and lets it start only after its own wait.
+    // The pair launches in front read and write nothing that this one does, and the first lets the others start only after its own wait.
     p.skip_wait = pairs ? 1 : 0;
   };
   // The whole of one GPU's call: the pairs' two launches, then one for all other experts.  It needs nothing of the pairs'
   // launches, so its CTAs start as theirs run out of tasks.
   const bool both = c.both_layers && small;
+  const PlanView pv = plan_view(c.ws + c.lay.plan, c.e_local, c.geo.num_ranks);
+  const bool claims = c.both_layers && pairs;
   for (int layer = 1; layer <= 2; ++layer) {
     if ((mask & layer) == 0) continue;
     if (e == cudaSuccess && pairs) {
       TmParams p = tm_plan->layer[layer - 1];
       patch(p, layer == 2);
       p.shared_tiles = shared_pairs ? shared : none;
+      p.tasks = claims ? pv.pair_tasks + (layer - 1) : nullptr;
+      p.done = claims ? pv.done : nullptr;
       e = tm_launch(layer, layer == 2 && fused, p, s);
     }
     if (e == cudaSuccess && small && !both) {
@@ -1693,6 +1688,8 @@ cudaError_t launch_experts_umma(const Ctx& c, const MmoeWeights& w, const MmoeOp
     p1.stats = c.stats;
     e = staged ? launch_both<true>(p, s) : launch_both<false>(p, s);
   }
+  // a pair launch may have run, and no combine follows, which would zero its counters
+  if (e != cudaSuccess && claims) cudaMemsetAsync(pv.done, 0, (c.e_local + 3) * sizeof *pv.done, s);
   return e;
 }
 

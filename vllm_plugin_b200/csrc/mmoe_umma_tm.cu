@@ -32,6 +32,7 @@
 //              (.cta_group::2), and none uses cluster multicast
 //   warp 1     issuer (leader): scale copies into TMEM, UMMAs, one commit that frees the stage in both CTAs
 //   warps 2-9  epilogue (both CTAs; layer 2: warps 2-5)
+//   last warp  scheduler (leader), where the pairs claim their tasks
 //
 // Copies and tensor-core instructions are issued by one elected lane of a warp that walks its loop in step (all lanes wait,
 // elect.sync around the issue): operands then stay in uniform registers.  From a lane that alone runs the loop a stage took
@@ -52,7 +53,7 @@ namespace {
 // instructions, and with the IEEE sigmoid (fast_math off) that is longer than the 22 thousand clk of a task's UMMAs (2800
 // tokens, 48 experts: 1304 us with one, 1024 with two).  Layer 2 only converts and stores, and has no shared memory left for more staging blocks.
 __host__ __device__ constexpr int tm_epilogue_warps(int layer) { return layer == 1 ? 8 : 4; }
-constexpr int tm_threads(int layer) { return 64 + 32 * tm_epilogue_warps(layer); }
+constexpr int tm_threads(int layer) { return 64 + 32 * tm_epilogue_warps(layer) + 32; }
 constexpr int kTmN = 256;                          // weight rows of a task (UMMA N)
 constexpr int kTmRows = 128;                       // token rows of a tile (UMMA M per CTA)
 constexpr int kTmABytes = kTmRows * kTileK;        // 16 KB
@@ -66,11 +67,17 @@ constexpr uint32_t kTmSfCol = 480;                 // scale columns: two sets of
 constexpr int tm_smem_bytes(int layer) { return 1024 + kTmStages * kTmStageBytes + (layer == 2 ? kTmStagingBytes : 0) + 1024; }
 static_assert(tm_smem_bytes(2) <= 227 * 1024, "shared memory budget");
 
+constexpr int kPairQueue = 4;   // tasks that the scheduler may be ahead of the epilogue
+
 struct TmControl {        // lives at the start of shared memory (same layout in both CTAs of a pair)
   uint64_t full[8];       // leader only: every copy of the stage, in both CTAs, has landed
   uint64_t empty[8];      // issuer -> producers of both CTAs: the stage may be overwritten
   uint64_t tmem_full[2];  // issuer -> epilogue of both CTAs
   uint64_t overlap_free;  // leader only: epilogue warps of both CTAs -> issuer: the overlapped columns have been read
+  uint64_t q_full[kPairQueue];    // scheduler -> the roles of this CTA: a task ...
+  uint64_t q_empty[kPairQueue];   // leader only: ... which all roles of both CTAs have read
+  uint64_t q_want;                // leader only: producer -> scheduler: the next one, please
+  volatile int32_t q_task[kPairQueue];
   uint32_t tmem_base;
   volatile int32_t abort_flag;
   // layer 2 with the write-back fused in: slot s < 32 is `ret_recv` of source rank s
@@ -136,35 +143,45 @@ __device__ __forceinline__ void pair_load_3d(uint32_t dst, const CUtensorMap* ma
       : "memory");
 }
 
-// The task list of one unit as a role walks it: first the shared expert's tasks, which need nothing but the staged tokens
+// The scheduler's word to CTA `rank` of the pair: `task` in its queue slot, and the slot's barrier completed with it.
+__device__ __forceinline__ void pair_send_task(uint32_t task_addr, uint32_t bar_addr, uint32_t rank, int task) {
+  const uint32_t dst = map_to_cta(task_addr, rank), bar = map_to_cta(bar_addr, rank);
+  asm volatile("mbarrier.arrive.expect_tx.shared::cluster.b64 _, [%0], 4;" ::"r"(bar) : "memory");
+  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(dst), "r"(task), "r"(bar) : "memory");
+}
+
+// The task list as a role of a pair walks it: first the shared expert's tasks, which need nothing but the staged tokens
 // and are on the host's count of tokens, then -- once everything before this launch in the stream has completed -- the pair
 // tiles of the plan.  In GEMM1 of the single-GPU call the placement of the routed rows, and the launch itself, hide behind
 // the shared expert this way.
+// Either dealt out beforehand, or (both layers of a single-GPU call) claimed from a counter by the leader's scheduler: SMs come free
+// one by one, over 25 us behind the placement and 50 behind GEMM1, and a pair that starts late takes fewer tasks.  GEMM2 then starts
+// where GEMM1 has ended and waits expert by expert for its counted parts, not for its last CTA.  3840 tokens of 48 experts, 30 calls in
+// a row: GEMM1's CTAs end over 52 -> 18 us, the call 966 -> 920; at the power limit 965 -> 959, 2560 of 16 381 -> 379.
 struct PairWalk {
   const TmParams& p;
+  TmControl* ctl;
   uint32_t cta;
   int n_blocks, task, stride;
+  uint32_t taken, q_empty_leader;
   bool waited;
   int routed_tiles;
   const Tile* tiles;
   Tile tile;              // this CTA's half of the current task
   int peer_valid, nb;     // rows of the other half; weight block
-  __device__ __forceinline__ PairWalk(const TmParams& params, uint32_t cta_rank, bool has_waited)
-      : p(params), cta(cta_rank), n_blocks(params.rows_per_expert / kTmN), task(blockIdx.x / 2), stride(gridDim.x / 2),
-        waited(false), routed_tiles(0), tiles(nullptr) {
-    if (has_waited) load_plan();
+  __device__ __forceinline__ PairWalk(const TmParams& params, TmControl* control, uint32_t cta_rank, bool plan_ready)
+      : p(params), ctl(control), cta(cta_rank), n_blocks(params.rows_per_expert / kTmN), task(blockIdx.x / 2), stride(gridDim.x / 2),
+        taken(0), q_empty_leader(map_to_cta(smem_u32(&control->q_empty[0]), 0)), waited(false), routed_tiles(0), tiles(nullptr) {
+    if (plan_ready) load_plan();
   }
   __device__ __forceinline__ void load_plan() {
-    chain_wait();
     const PlanView pv = plan_view(const_cast<char*>(p.plan), p.e_local, p.num_ranks);
     tiles = pv.tiles + pv.hdr->num_small_tiles;
     routed_tiles = p.with_routed ? pv.hdr->num_routed_tiles - pv.hdr->num_small_tiles : 0;
     waited = true;
   }
-  // true: tile, peer_valid and nb are the next task's
-  __device__ __forceinline__ bool next() {
-    const int t = task;
-    task += stride;
+  // true: tile, peer_valid and nb are those of task t; false behind the last one
+  __device__ __forceinline__ bool locate(int t) {
     const int pair = t / n_blocks, first = p.shared_tiles.parts / 2;
     nb = t - pair * n_blocks;
     if (pair < first) {
@@ -172,12 +189,30 @@ struct PairWalk {
       peer_valid = p.shared_tiles.at(2 * pair + static_cast<int>(cta ^ 1u)).n_valid;
       return true;
     }
-    if (!waited) load_plan();
+    if (!waited) {
+      chain_wait();
+      load_plan();
+    }
     const int i = 2 * (pair - first);
     if (i >= routed_tiles) return false;
     tile = tiles[i + cta];
     peer_valid = tiles[i + (cta ^ 1u)].n_valid;
     return true;
+  }
+  // true: ... of this role's next task; false when there is none or the call is being abandoned
+  template <bool kOneLanePolls>
+  __device__ __forceinline__ bool next(Waiter& waiter) {
+    int t = task;
+    task += stride;
+    if (p.tasks != nullptr) {
+      const uint32_t slot = taken % kPairQueue, bar = smem_u32(&ctl->q_full[slot]), parity = (taken / kPairQueue) & 1u;
+      if (!(kOneLanePolls ? waiter.wait_warp(bar, parity) : waiter.wait_uniform(bar, parity))) return false;
+      t = ctl->q_task[slot];
+      __syncwarp();
+      if ((threadIdx.x & 31) == 0) mbar_arrive_pair(q_empty_leader + 8 * slot);
+      ++taken;
+    }
+    return locate(t);
   }
 };
 
@@ -227,10 +262,16 @@ __global__ void __launch_bounds__(tm_threads(kLayer), 1) tm_kernel(const __grid_
   const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   const uint32_t cta = cluster_ctarank();                         // 0 = leader
 
+  // GEMM2 behind GEMM1 of the same call: GEMM1 lets it start after its own wait, so all that comes before GEMM1 is complete, and
+  // GEMM1 itself counts its finished parts.
+  const bool behind_layer1 = kLayer == 2 && p.done != nullptr;
   if (p.shared_tiles.parts == 0) {        // routed tiles only, of which the call may have none
-    chain_wait();
+    if (!behind_layer1) chain_wait();
     const PlanHeader* hdr = plan_view(const_cast<char*>(p.plan), p.e_local, p.num_ranks).hdr;
-    if (p.with_routed == 0 || hdr->num_routed_tiles == hdr->num_small_tiles) return;
+    if (p.with_routed == 0 || hdr->num_routed_tiles == hdr->num_small_tiles) {
+      chain_wait();
+      return;
+    }
   }
   if (threadIdx.x == 0) {
     for (int i = 0; i < kTmStages; ++i) {
@@ -239,6 +280,11 @@ __global__ void __launch_bounds__(tm_threads(kLayer), 1) tm_kernel(const __grid_
     }
     for (int i = 0; i < 2; ++i) mbar_init(smem_u32(&ctl->tmem_full[i]), 1);
     mbar_init(smem_u32(&ctl->overlap_free), 2 * tm_epilogue_warps(kLayer));   // one arrival per epilogue warp of the pair
+    for (int i = 0; i < kPairQueue; ++i) {
+      mbar_init(smem_u32(&ctl->q_full[i]), 1);
+      mbar_init(smem_u32(&ctl->q_empty[i]), 2 * tm_epilogue_warps(kLayer) + 3);   // ... and both producers and the issuer
+    }
+    mbar_init(smem_u32(&ctl->q_want), 1);
     ctl->abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -246,11 +292,11 @@ __global__ void __launch_bounds__(tm_threads(kLayer), 1) tm_kernel(const __grid_
     asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&ctl->tmem_base)), "r"(kTmemCols) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
   }
-  // Everything above touches only this CTA's own shared and tensor memory.  GEMM2, and GEMM1 behind an ordinary launch, wait
-  // here for everything before them; GEMM1 in a programmatic chain starts when the blocks of the placement have all started,
+  // Everything above touches only this CTA's own shared and tensor memory.  GEMM2 that does not count GEMM1's parts waits
+  // here for everything before it; GEMM1 in a programmatic chain starts when the blocks of the placement have all started,
   // i.e. after the launches before it (staging, counting) have completed, and waits when it comes to the routed tiles.
   // Only then does it let the next launch start.
-  if (kLayer == 2) chain_wait();
+  if (kLayer == 2 && !behind_layer1) chain_wait();
   if (kFused) {
     const int t = threadIdx.x - 32;
     if (t >= 0 && t < p.num_ranks) {
@@ -270,7 +316,7 @@ __global__ void __launch_bounds__(tm_threads(kLayer), 1) tm_kernel(const __grid_
   cluster_sync_all();                       // the peer's barriers are initialised before anything arrives on them
   tc_fence_after();
   const uint32_t tmem_base = __shfl_sync(0xffffffffu, ctl->tmem_base, 0);
-  PairWalk walk(p, cta, kLayer == 2);
+  PairWalk walk(p, ctl, cta, kLayer == 2);
   const int k_stages = p.k_dim / kTileK;
 
   Waiter waiter{&ctl->abort_flag, p.status, global_timer() + static_cast<uint64_t>(p.timeout_ns), kStatusPairs + kLayer, warp};
@@ -284,8 +330,10 @@ __global__ void __launch_bounds__(tm_threads(kLayer), 1) tm_kernel(const __grid_
     const uint32_t a0 = smem_u32(a_base), b0 = smem_u32(b_base), sf0 = smem_u32(sf_base);
     const uint32_t leader_full0 = map_to_cta(full0, 0);
     const int half = p.rows_per_expert / 2;
+    const uint32_t want = p.tasks != nullptr && cta == 0 ? smem_u32(&ctl->q_want) : 0u;
+    const int want_at = max(k_stages - 8, 0);            // a claim in time, and not earlier: that would hoard tasks
     bool ok = true, released = false;
-    while (ok && walk.next()) {
+    while (ok && walk.next<false>(waiter)) {
       const Tile tile = walk.tile;
       const int nb = walk.nb;
       if (!released && walk.waited) {
@@ -309,10 +357,20 @@ __global__ void __launch_bounds__(tm_threads(kLayer), 1) tm_kernel(const __grid_
       const int wsf_col = nb * kTmN, tsf_col = tile.sf_chunk * kChunkRows;
       int wsf_row = e * k_stages;
       int k0 = 0;
+      if (behind_layer1) {
+        const int32_t* done = p.done + (shared ? p.e_local : e);
+        const int need = tile.parts * tm_epilogue_warps(1) * (2 * p.inter / kTmN);
+        for (uint32_t spin = 0; ok && !rows_ready(done, need); ++spin) {
+          if ((spin & 63u) == 63u && __any_sync(0xffffffffu, waiter.abandoned())) ok = false;
+          __nanosleep(40);
+        }
+        if (!ok) break;
+      }
       for (int kb = 0; kb < k_stages; ++kb, k0 += kTileK, ++wsf_row) {
         if (!waiter.wait_uniform(empty0 + 8 * stage, phase ^ 1u)) { ok = false; break; }
         const uint32_t bar = leader_full0 + 8 * stage;
         if (elect_one()) {
+          if (want != 0 && kb == want_at) mbar_arrive(want);
           if (cta == 0) mbar_expect_tx(full0 + 8 * stage, tx);
           pair_load_3d(b0 + stage * kTmBBytes, wmap, k0, row, slice, bar);
           pair_load_2d(a0 + stage * kTmABytes, tmap, k0, tile.row0, bar);
@@ -332,7 +390,7 @@ __global__ void __launch_bounds__(tm_threads(kLayer), 1) tm_kernel(const __grid_
       const uint32_t a_lo0 = (smem_u32(a_base) & 0x3FFFFu) >> 4;
       const uint32_t b_lo0 = (smem_u32(b_base) & 0x3FFFFu) >> 4;
       const uint32_t sf_lo0 = (smem_u32(sf_base) & 0x3FFFFu) >> 4;
-      for (; ok && walk.next(); ++it) {
+      for (; ok && walk.next<false>(waiter); ++it) {
         const bool shared = walk.tile.expert == kSharedExpert;
         // M = 256 over the pair; idesc field [24,29) = M >> 4
         const uint32_t idesc0 = make_idesc(0u, shared ? 0u : 5u, static_cast<uint32_t>(kTmN), 0) + ((128u >> 4) << 24);
@@ -368,6 +426,21 @@ __global__ void __launch_bounds__(tm_threads(kLayer), 1) tm_kernel(const __grid_
         __syncwarp();
       }
     }
+  } else if (warp == 2 + tm_epilogue_warps(kLayer)) {
+    // --------------------------------------------------------------------------------------------- scheduler
+    if (cta == 0 && p.tasks != nullptr) {
+      for (uint32_t n = 0;; ++n) {
+        int t = 0;
+        if (lane == 0) t = atomicAdd(p.tasks, 1);
+        t = __shfl_sync(0xffffffffu, t, 0);
+        const uint32_t slot = n % kPairQueue;
+        if (!waiter.wait_uniform(smem_u32(&ctl->q_empty[slot]), ((n / kPairQueue) & 1u) ^ 1u)) break;
+        if (lane < 2) pair_send_task(smem_u32(const_cast<int32_t*>(&ctl->q_task[slot])), smem_u32(&ctl->q_full[slot]), lane, t);
+        __syncwarp();
+        if (!walk.locate(t)) break;
+        if (!waiter.wait_uniform(smem_u32(&ctl->q_want), n & 1u)) break;
+      }
+    }
   } else {
     // --------------------------------------------------------------------------------------------- epilogue
     const int q = warp & 3;                       // TMEM lane quadrant this warp may read
@@ -376,7 +449,16 @@ __global__ void __launch_bounds__(tm_threads(kLayer), 1) tm_kernel(const __grid_
     const uint32_t overlap_free_leader = map_to_cta(smem_u32(&ctl->overlap_free), 0);
     uint32_t it = 0;
     bool ok = true;
-    for (; ok && walk.next(); ++it) {
+    // layer 1: this warp's part of a task is stored
+    auto publish = [&](const Tile& tile) {
+      if (kLayer == 2 || p.done == nullptr) return;
+      __syncwarp();
+      if (lane == 0) {
+        part_release();
+        part_count(p.done + (tile.expert == kSharedExpert ? p.e_local : tile.expert));
+      }
+    };
+    for (; ok && walk.next<true>(waiter); ++it) {
       const Tile tile = walk.tile;
       const int nb = walk.nb;
       const bool shared = tile.expert == kSharedExpert;
@@ -417,6 +499,7 @@ __global__ void __launch_bounds__(tm_threads(kLayer), 1) tm_kernel(const __grid_
       if (q * 32 >= tile.n_valid) {
         tc_fence_before();
         if (lane == 0) mbar_arrive_pair(overlap_free_leader);
+        publish(tile);
         continue;
       }
       const uint32_t d0 = tmem_base + lane_sel + acc * kTmAccStride;
@@ -477,6 +560,7 @@ __global__ void __launch_bounds__(tm_threads(kLayer), 1) tm_kernel(const __grid_
         const int64_t sf_rows = shared ? p.act_sf_rows_shared : p.act_sf_rows_routed;
         reinterpret_cast<uint16_t*>(act_sf + nb * sf_rows + (int64_t)tile.sf_chunk * kChunkRows + chunk_pos(i))[side] = static_cast<uint16_t>(sf_word);
       }
+      publish(tile);
     }
   }
 
