@@ -623,6 +623,30 @@ def test_both_gemms_in_one_launch(hidden, inter, experts, shared, m):
             assert_parity(y_one, H.oracle_layer(layer, hid, ids, w), f"m {m} call {call}")
 
 
+@pytest.mark.parametrize("hidden,k,shared", [(512, 6, True), (2560, 10, True), (256, 3, False)])
+@pytest.mark.parametrize("few", [16, 64])
+def test_small_kernels_of_few_tokens_against_those_of_more(hidden, k, shared, few):
+    """Staging and combine have forms of their own for few tokens: what they leave for a token is bit for bit what a call with one token
+    more leaves, with a residual, masked routes and more slots than are in flight at once."""
+    from vllm_plugin_b200 import api
+    layer = H.make_layer(hidden, 256, 12, k, shared, seed=61)
+    l1, l2, sl1, sl2 = weights = H.kernel_weights(layer, "cuda")
+    hid = O.make_hidden(few + 1, hidden, 3)
+    ids, w = O.make_routing(few + 1, 12, k, 4, mask_frac=0.2)
+    res = torch.randn(few + 1, hidden, generator=torch.Generator().manual_seed(5)).to(torch.bfloat16).cuda()
+    got = []
+    for m in (few, few + 1):
+        y, buf = H.run_layer(layer, hid[:m], ids[:m], w[:m], weights=weights)
+        plain = y.clone()
+        api.fp8_fp4_mega_moe(y, l1, l2, buf, sl1, sl2, activation_clamp=10.0, residual=res[:m])
+        assert torch.equal(y, plain + res[:m])
+        got.append((plain[:few], y[:few].clone(), buf.x[:few].view(torch.uint8).clone(), buf.x_sf[:few].clone(), buf.topk_idx[:few].clone()))
+    for a, b in zip(*got):
+        assert torch.equal(a, b)
+    met = O.parity_metrics(got[0][0].cpu(), H.oracle_layer(layer, hid[:few], ids[:few], w[:few]))
+    assert met["rel_l2"] <= 1e-3, met
+
+
 TILE_ROWS = [(16, (160, 160, 128), 1), (16, (160, 128, 128), 1), (16, (192, 192, 192), 0), (16, (64,), 7), (32, (64, 33), 5), (32, (65, 33), 5),
              (64, (100, 65, 33), 12)]
 MANY_COLD = [(16, (160, 160, 128), 49), (16, (160, 160, 128), 50)]

@@ -6,6 +6,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <type_traits>
 
 #include <cuda_fp4.h>
 
@@ -41,6 +42,10 @@ bool chained() { return g_chain_scope; }
 // scale word.  HBM-bound: 3840 x 5120 (60 MB) took 30 us with one division per vector and single-value conversions.
 // =====================================================================================================================
 constexpr int kStageSegVec = 128;
+// Calls of at most so many tokens wait for the code (see opaque()) as much as for memory: theirs is rolled, in 32-bit arithmetic, a third
+// of the length.  With the narrow combine, which is the other half of it: one token 39.05 -> 38.8 us, seven 133.1 -> 131.8.  In the registers
+// of the rolled form (44) the staging of 1021 tokens lets the placement's blocks start so early that they crowd some SMs: 463 -> 471.
+constexpr int kFewTokens = 64;
 
 __device__ __forceinline__ void stage_vector(const uint4& raw, uint2* __restrict__ q_out, uint32_t* word_out) {
   const __nv_bfloat162* p = reinterpret_cast<const __nv_bfloat162*>(&raw);
@@ -122,19 +127,20 @@ __device__ void route_token(const RouterArgs& r, int64_t t, int k, bool is_pad, 
   }
 }
 
-__global__ void __launch_bounds__(256) stage_kernel(
+template <bool kFew>
+__global__ void __launch_bounds__(256, kFew ? 1 : 3) stage_kernel(
     const uint4* __restrict__ hidden, uint2* __restrict__ x_q, int32_t* __restrict__ x_sf,
     int32_t* __restrict__ shared_sf, int64_t shared_rows, int shared_bm,
     const void* __restrict__ ids_in, int ids64, const float* __restrict__ w_in, const uint8_t* __restrict__ pad,
     int64_t* __restrict__ ids_out, float* __restrict__ w_out, int m, int h, int k, RouterArgs router) {
   chain_begin();
-  const int vec_per_row = h / 8, segs = (vec_per_row + kStageSegVec - 1) / kStageSegVec, words = h / kTileK;
+  const int vec_per_row = h / 8, words = h / kTileK;
+  const uint32_t segs = (vec_per_row + kStageSegVec - 1) / kStageSegVec, total = m * segs;
   const int lane = threadIdx.x & 31;
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  for (int64_t seg = tid >> 5; seg < (int64_t)m * segs; seg += stride >> 5) {
+  const uint32_t stride = gridDim.x * blockDim.x, tid = blockIdx.x * blockDim.x + threadIdx.x;
+  for (uint32_t seg = tid >> 5; seg < total; seg += stride >> 5) {
     const int t = static_cast<int>(seg / segs);
-    const int v0 = static_cast<int>(seg - (int64_t)t * segs) * kStageSegVec + lane;
+    const int v0 = static_cast<int>(seg - t * segs) * kStageSegVec + lane;
     const uint4* row = hidden + (int64_t)t * vec_per_row;
     uint4 raw[4];
 #pragma unroll
@@ -142,13 +148,13 @@ __global__ void __launch_bounds__(256) stage_kernel(
     // row of token t in the BLOCK_M-dependent shared-expert scale layout (backend/staging.py:85-95)
     const int mm = shared_bm > 0 ? t % shared_bm : 0;
     const int64_t shared_row = shared_bm > 0 ? (int64_t)(t / shared_bm) * ((shared_bm + 127) / 128 * 128) + (mm / 128) * 128 + (mm % 32) * 4 + (mm % 128) / 32 : 0;
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int v = v0 + 32 * u;                     // rows are whole multiples of 32 vectors: a warp is in or out together
-      if (v >= vec_per_row) break;
+#pragma unroll (kFew ? 1 : 4)
+    for (int v = v0; v < v0 + 128 && v < vec_per_row; v += 32) {      // rows are whole multiples of 32 vectors: a warp is in or out together
       uint2 q;
       uint32_t word;
-      stage_vector(raw[u], &q, &word);
+      stage_vector(raw[0], &q, &word);
+#pragma unroll
+      for (int u = 0; u < 3; ++u) raw[u] = raw[u + 1];
       x_q[(int64_t)t * vec_per_row + v] = q;
       if ((lane & 15) == 0) {
         x_sf[(int64_t)t * words + v / 16] = static_cast<int32_t>(word);
@@ -157,15 +163,13 @@ __global__ void __launch_bounds__(256) stage_kernel(
     }
   }
   if (router.logits != nullptr) {
-    const int64_t warp = tid >> 5, warps = stride >> 5;
-    for (int64_t t = warp; t < m; t += warps) route_token(router, t, k, pad != nullptr && pad[t] != 0, ids_out, w_out);
+    for (int t = tid >> 5; t < m; t += stride >> 5) route_token(router, t, k, pad != nullptr && pad[t] != 0, ids_out, w_out);
     return;
   }
   // routing repack (backend/staging.py:244-251)
-  const int64_t routes = (int64_t)m * k;
-  for (int64_t r = tid; r < routes; r += stride) {
-    const int64_t t = r / k;
-    const bool is_pad = pad != nullptr && pad[t] != 0;
+  const uint32_t routes = m * k;
+  for (uint32_t r = tid; r < routes; r += stride) {
+    const bool is_pad = pad != nullptr && pad[r / k] != 0;
     const int64_t id = ids64 ? static_cast<const int64_t*>(ids_in)[r] : static_cast<const int32_t*>(ids_in)[r];
     ids_out[r] = is_pad ? -1 : id;
     w_out[r] = is_pad ? 0.f : w_in[r];
@@ -187,8 +191,8 @@ cudaError_t launch_route_stage(const Ctx& c, const void* hidden, const void* ids
   int blocks = static_cast<int>(std::min<int64_t>((segs + 7) / 8, 148 * 8));
   if (blocks < 1) blocks = 1;
   const RouterArgs router{logits, num_logical, replica_count, replica_slots, max_copies};
-  return launch_chained(stage_kernel, dim3(blocks), dim3(256), 0, s, static_cast<const uint4*>(hidden), c.at<uint2>(c.lay.x), c.at<int32_t>(c.lay.x_sf),
-      c.at<int32_t>(c.lay.shared_x_sf), c.lay.shared_sf_rows, c.geo.num_shared_experts > 0 ? shared_bm : 0, ids, ids64, w,
+  return launch_chained(m <= kFewTokens ? stage_kernel<true> : stage_kernel<false>, dim3(blocks), dim3(256), 0, s, static_cast<const uint4*>(hidden),
+      c.at<uint2>(c.lay.x), c.at<int32_t>(c.lay.x_sf), c.at<int32_t>(c.lay.shared_x_sf), c.lay.shared_sf_rows, c.geo.num_shared_experts > 0 ? shared_bm : 0, ids, ids64, w,
       pad, c.at<int64_t>(c.lay.topk_idx), c.at<float>(c.lay.topk_weights), m, h, c.geo.num_topk, router);
 }
 
@@ -1104,6 +1108,69 @@ __device__ __forceinline__ void add_bf16x8(float (&acc)[8], const uint4& v) {
   }
 }
 
+// The counters of a launch of both GEMMs, by a block more: in the call's last kernel nothing waits for that.  No block lets
+// the next launch start before they are zero, so that the next such launch may claim its tasks at once.  True for that block.
+__device__ __forceinline__ bool combine_zeroes(char* plan_base, int e_local) {
+  if (plan_base == nullptr || blockIdx.x != gridDim.x - 1) {
+    chain_release();
+    return false;
+  }
+  const PlanView pv = plan_view(plan_base, e_local, 1);
+  if (threadIdx.x == 0) {
+    pv.hdr->routed = 0;
+    pv.hdr->next_task = 0;
+    pv.hdr->layer1_done = 0;
+  }
+  for (int e = threadIdx.x; e < e_local + 3; e += blockDim.x) pv.done[e] = 0;      // and `pair_tasks` behind it
+  __threadfence();
+  __syncthreads();
+  chain_release();
+  return true;
+}
+
+// What the serving engine's separate BF16 addition leaves: the layer output rounded to BF16 first, then the sum of the two BF16 values
+// rounded once more.
+__device__ __forceinline__ __nv_bfloat162 add_residual(__nv_bfloat162 o, __nv_bfloat162 r) {
+  const float2 a = __bfloat1622float2(o), b = __bfloat1622float2(r);
+  return __floats2bfloat162_rn(__fadd_rn(a.x, b.x), __fadd_rn(a.y, b.y));
+}
+
+// Calls of at most kNarrowTokens tokens, where latency and code on its way from DRAM are all there is to wait for (see kFewTokens): two
+// outputs per thread, a quarter of the instructions.  Past that the rows are enough to be worth 16 bytes a load.
+constexpr int kNarrowTokens = 16;
+__global__ void __launch_bounds__(256) combine_narrow_kernel(
+    const uint32_t* __restrict__ rows, const int32_t* __restrict__ route_pos, const uint32_t* __restrict__ shared_out,
+    const uint32_t* __restrict__ residual, uint32_t* __restrict__ y, int m, int h, int k, char* plan_base, int e_local) {
+  chain_wait();
+  if (combine_zeroes(plan_base, e_local)) return;
+  const uint32_t pairs = h / 2, i = blockIdx.x * blockDim.x + threadIdx.x, t = i / pairs;
+  if (t >= static_cast<uint32_t>(m)) return;
+  const uint32_t sh = shared_out != nullptr ? shared_out[i] : 0u, res = residual != nullptr ? residual[i] : 0u;
+  const int32_t* pos = route_pos + t * k;
+  const uint32_t* col = rows + (i - t * pairs);
+  float lo = 0.f, hi = 0.f;
+  auto add = [&](uint32_t v) {
+    lo = __fadd_rn(lo, __uint_as_float(v << 16));
+    hi = __fadd_rn(hi, __uint_as_float(v & 0xFFFF0000u));
+  };
+#pragma unroll 1
+  for (int s0 = 0; s0 < k; s0 += 8) {
+    int p[8];
+    uint32_t q[8];
+#pragma unroll
+    for (int s = 0; s < 8; ++s) p[s] = s0 + s < k ? pos[s0 + s] : -1;
+#pragma unroll
+    for (int s = 0; s < 8; ++s) q[s] = p[s] >= 0 ? col[(int64_t)p[s] * pairs] : 0u;
+#pragma unroll
+    for (int s = 0; s < 8; ++s)
+      if (p[s] >= 0) add(q[s]);
+  }
+  if (shared_out != nullptr) add(sh);
+  __nv_bfloat162 out = __floats2bfloat162_rn(lo, hi);
+  if (residual != nullptr) out = add_residual(out, *reinterpret_cast<const __nv_bfloat162*>(&res));
+  y[i] = *reinterpret_cast<const uint32_t*>(&out);
+}
+
 // A warp takes 64 vectors of 8 outputs of one token; a lane has the rows of up to eight slots of its two vectors in flight at
 // once (with one dependent load after the other 3840 x 5120 top-6, 315 MB, took 63 us).
 constexpr int kCombineSegVec = 64;
@@ -1111,29 +1178,13 @@ __global__ void __launch_bounds__(256) combine_kernel(
     const uint4* __restrict__ rows, const int32_t* __restrict__ route_pos, const uint4* __restrict__ shared_out,
     const uint4* __restrict__ residual, uint4* __restrict__ y, int m, int h, int k, char* plan_base, int e_local) {
   chain_wait();
-  // The counters of a launch of both GEMMs, by a block more: in the call's last kernel nothing waits for that.  No block lets
-  // the next launch start before they are zero, so that the next such launch may claim its tasks at once.
+  if (combine_zeroes(plan_base, e_local)) return;
   const int blocks = plan_base != nullptr ? gridDim.x - 1 : gridDim.x;
-  if ((int)blockIdx.x != blocks) {
-    chain_release();
-  } else {
-    const PlanView pv = plan_view(plan_base, e_local, 1);
-    if (threadIdx.x == 0) {
-      pv.hdr->routed = 0;
-      pv.hdr->next_task = 0;
-      pv.hdr->layer1_done = 0;
-    }
-    for (int e = threadIdx.x; e < e_local + 3; e += blockDim.x) pv.done[e] = 0;      // and `pair_tasks` behind it
-    __threadfence();
-    __syncthreads();
-    chain_release();
-    return;
-  }
-  const int vec = h / 8, segs = (vec + kCombineSegVec - 1) / kCombineSegVec, lane = threadIdx.x & 31;
-  const int64_t warps = ((int64_t)blocks * blockDim.x) >> 5;
-  for (int64_t seg = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; seg < (int64_t)m * segs; seg += warps) {
+  const int vec = h / 8, lane = threadIdx.x & 31;
+  const uint32_t segs = (vec + kCombineSegVec - 1) / kCombineSegVec, total = m * segs, warps = (blocks * blockDim.x) >> 5;
+  for (uint32_t seg = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; seg < total; seg += warps) {
     const int t = static_cast<int>(seg / segs);
-    const int v0 = static_cast<int>(seg - (int64_t)t * segs) * kCombineSegVec + lane;
+    const int v0 = static_cast<int>(seg - t * segs) * kCombineSegVec + lane;
     const bool both = v0 + 32 < vec;                 // rows are whole multiples of 32 vectors
     const int my_pos = lane < k ? route_pos[(int64_t)t * k + lane] : -1;
     const int64_t i = (int64_t)t * vec + v0;
@@ -1176,14 +1227,9 @@ __global__ void __launch_bounds__(256) combine_kernel(
 #pragma unroll
       for (int j = 0; j < 4; ++j) o[j] = __floats2bfloat162_rn(acc[u][2 * j], acc[u][2 * j + 1]);
       if (residual != nullptr) {
-        // what the serving engine's separate BF16 addition leaves: the layer output rounded to BF16 first, then the sum
-        // of the two BF16 values rounded once more
         const __nv_bfloat162* r = reinterpret_cast<const __nv_bfloat162*>(&res[u]);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const float2 a = __bfloat1622float2(o[j]), b = __bfloat1622float2(r[j]);
-          o[j] = __floats2bfloat162_rn(__fadd_rn(a.x, b.x), __fadd_rn(a.y, b.y));
-        }
+        for (int j = 0; j < 4; ++j) o[j] = add_residual(o[j], r[j]);
       }
       y[i + 32 * u] = out;
     }
@@ -1192,13 +1238,20 @@ __global__ void __launch_bounds__(256) combine_kernel(
 
 cudaError_t launch_combine(const Ctx& c, void* y, const void* residual, int m, cudaStream_t s) {
   if (m == 0) return cudaSuccess;
-  const int64_t segs = (int64_t)m * ((c.geo.hidden / 8 + kCombineSegVec - 1) / kCombineSegVec);      // one warp each
-  const int blocks = static_cast<int>(std::min<int64_t>((segs + 7) / 8, 148 * 8));
-  const uint4* rows = c.geo.num_ranks == 1 ? c.at<uint4>(c.lay.ret) : c.at<uint4>(c.lay.ret_recv);
-  char* plan = c.geo.num_ranks == 1 ? c.ws + c.lay.plan : nullptr;
-  return launch_chained(combine_kernel, dim3(blocks + (plan != nullptr ? 1 : 0)), dim3(256), 0, s, rows, c.at<int32_t>(c.lay.route_pos),
-                        c.geo.num_shared_experts > 0 ? c.at<uint4>(c.lay.shared_out) : nullptr, static_cast<const uint4*>(residual),
-                        static_cast<uint4*>(y), m, c.geo.hidden, c.geo.num_topk, plan, c.e_local);
+  const int h = c.geo.hidden;
+  const bool one_rank = c.geo.num_ranks == 1;
+  const void* rows = c.ws + (one_rank ? c.lay.ret : c.lay.ret_recv);
+  const void* shared = c.geo.num_shared_experts > 0 ? c.ws + c.lay.shared_out : nullptr;
+  char* plan = one_rank ? c.ws + c.lay.plan : nullptr;
+  auto launch = [&](auto kernel, auto* out, int64_t blocks) {
+    using T = std::remove_pointer_t<decltype(out)>;
+    return launch_chained(kernel, dim3(static_cast<unsigned>(blocks) + (one_rank ? 1 : 0)), dim3(256), 0, s, static_cast<const T*>(rows),
+                          c.at<int32_t>(c.lay.route_pos), static_cast<const T*>(shared), static_cast<const T*>(residual), out, m, h, c.geo.num_topk,
+                          plan, c.e_local);
+  };
+  if (m <= kNarrowTokens) return launch(combine_narrow_kernel, static_cast<uint32_t*>(y), ((int64_t)m * (h / 2) + 255) / 256);
+  const int64_t segs = (int64_t)m * ((h / 8 + kCombineSegVec - 1) / kCombineSegVec);      // one warp each
+  return launch(combine_kernel, static_cast<uint4*>(y), std::min<int64_t>((segs + 7) / 8, 148 * 8));
 }
 
 cudaError_t zero_counters(const Ctx& c, cudaStream_t s) {
