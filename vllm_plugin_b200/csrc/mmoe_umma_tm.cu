@@ -39,7 +39,7 @@
 // 563-703 clk.
 //
 // The same roles exist in the reference's kernel (backend/kernel/tma_warps.py, mma_warp.py, epilogue.py).  Persistent
-// pairs walk the static task list tile-major, so that the pairs working at the same time share token tiles and the tiles
+// pairs take the tasks tile-major, so that the pairs working at the same time share token tiles and the tiles
 // of one expert share its weights in L2.  Every wait is bounded (see Waiter).
 #include <cuda_fp8.h>
 
