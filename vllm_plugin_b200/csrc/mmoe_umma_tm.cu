@@ -32,7 +32,7 @@
 //              (.cta_group::2), and none uses cluster multicast
 //   warp 1     issuer (leader): scale copies into TMEM, UMMAs, one commit that frees the stage in both CTAs
 //   warps 2-9  epilogue (both CTAs; layer 2: warps 2-5)
-//   last warp  scheduler (leader), where the pairs claim their tasks
+//   last warp  where the pairs claim their tasks: scheduler (leader), forwarder of the queue (peer)
 //
 // Copies and tensor-core instructions are issued by one elected lane of a warp that walks its loop in step (all lanes wait,
 // elect.sync around the issue): operands then stay in uniform registers.  From a lane that alone runs the loop a stage took
@@ -43,6 +43,7 @@
 // of one expert share its weights in L2.  Every wait is bounded (see Waiter).
 #include <cuda_fp8.h>
 
+#include "mmoe_pair_queue.h"
 #include "mmoe_tc.cuh"
 
 namespace mmoe {
@@ -67,15 +68,13 @@ constexpr uint32_t kTmSfCol = 480;                 // scale columns: two sets of
 constexpr int tm_smem_bytes(int layer) { return 1024 + kTmStages * kTmStageBytes + (layer == 2 ? kTmStagingBytes : 0) + 1024; }
 static_assert(tm_smem_bytes(2) <= 227 * 1024, "shared memory budget");
 
-constexpr int kPairQueue = 4;   // tasks that the scheduler may be ahead of the epilogue
-
 struct TmControl {        // lives at the start of shared memory (same layout in both CTAs of a pair)
   uint64_t full[8];       // leader only: every copy of the stage, in both CTAs, has landed
   uint64_t empty[8];      // issuer -> producers of both CTAs: the stage may be overwritten
   uint64_t tmem_full[2];  // issuer -> epilogue of both CTAs
   uint64_t overlap_free;  // leader only: epilogue warps of both CTAs -> issuer: the overlapped columns have been read
   uint64_t q_full[kPairQueue];    // scheduler -> the roles of this CTA: a task ...
-  uint64_t q_empty[kPairQueue];   // leader only: ... which all roles of both CTAs have read
+  uint64_t q_empty[kPairQueue];   // ... which all roles of this CTA have read; in the leader also those of the peer
   uint64_t q_want;                // leader only: producer -> scheduler: the next one, please
   volatile int32_t q_task[kPairQueue];
   uint32_t tmem_base;
@@ -101,8 +100,8 @@ __device__ __forceinline__ uint32_t map_to_cta(uint32_t addr, uint32_t rank) {
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
   return r;
 }
-// Arrival on a barrier of either CTA of the pair.  What it hands over are columns of tensor memory, ordered by the tcgen05 fences on
-// either side; no memory access rides on it.  So the default release, of CTA scope, is enough: one of cluster scope first waits for
+// Arrival on the barrier that hands columns of tensor memory back, in either CTA of the pair: ordered by the tcgen05 fences on
+// either side, and no memory access rides on it (the queue of tasks has arrivals of its own).  So the default release, of CTA scope, is enough: one of cluster scope first waits for
 // this warp's outstanding stores to global memory, which stood between every two tasks of the issuer (3840 tokens of 48 experts 970 ->
 // 942 us, 2560 of 16 387 -> 381; GEMM2, whose epilogue stores most, 294 -> 275).
 __device__ __forceinline__ void mbar_arrive_pair(uint32_t cluster_addr) {
@@ -143,12 +142,47 @@ __device__ __forceinline__ void pair_load_3d(uint32_t dst, const CUtensorMap* ma
       : "memory");
 }
 
-// The scheduler's word to CTA `rank` of the pair: `task` in its queue slot, and the slot's barrier completed with it.
-__device__ __forceinline__ void pair_send_task(uint32_t task_addr, uint32_t bar_addr, uint32_t rank, int task) {
-  const uint32_t dst = map_to_cta(task_addr, rank), bar = map_to_cta(bar_addr, rank);
-  asm volatile("mbarrier.arrive.expect_tx.shared::cluster.b64 _, [%0], 4;" ::"r"(bar) : "memory");
-  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(dst), "r"(task), "r"(bar) : "memory");
-}
+// What the queue of claimed tasks is made of (mmoe_pair_queue.h); every function by the whole warp.
+template <bool kOneLanePolls>
+struct PairPort {
+  TmControl* ctl;
+  Waiter& waiter;
+  __device__ __forceinline__ uint32_t bar(PairBarrier which, uint32_t slot) const {
+    return smem_u32(which == kPairFull ? &ctl->q_full[slot] : &ctl->q_empty[slot]);
+  }
+  __device__ __forceinline__ bool wait_own(PairBarrier which, uint32_t slot, uint32_t parity) {
+    if (!(kOneLanePolls ? waiter.wait_warp(bar(which, slot), parity) : waiter.wait_uniform(bar(which, slot), parity))) return false;
+    __syncwarp();
+    return true;
+  }
+  // ... and what the other CTA did before completing the phase is visible to every lane.  The phase is over and the next one needs this role.
+  __device__ __forceinline__ bool wait_pair(PairBarrier which, uint32_t slot, uint32_t parity) {
+    if (!wait_own(which, slot, parity)) return false;
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%0], %1;\n\t}"
+                 ::"r"(bar(which, slot)), "r"(parity) : "memory");
+    return true;
+  }
+  __device__ __forceinline__ int read(uint32_t slot) const { return ctl->q_task[slot]; }
+  __device__ __forceinline__ void arrive_own(PairBarrier which, uint32_t slot) {
+    __syncwarp();
+    if ((threadIdx.x & 31) == 0) mbar_arrive(bar(which, slot));
+  }
+  __device__ __forceinline__ void arrive_leader(PairBarrier which, uint32_t slot) {
+    __syncwarp();
+    if ((threadIdx.x & 31) == 0)
+      asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(map_to_cta(bar(which, slot), 0)) : "memory");
+  }
+  // lane r: to CTA r, the slot's barrier completed with it
+  __device__ __forceinline__ void send(uint32_t slot, int task) {
+    const uint32_t lane = threadIdx.x & 31;
+    if (lane < 2) {
+      const uint32_t dst = map_to_cta(smem_u32(const_cast<int32_t*>(&ctl->q_task[slot])), lane), full = map_to_cta(bar(kPairFull, slot), lane);
+      asm volatile("mbarrier.arrive.expect_tx.release.cluster.shared::cluster.b64 _, [%0], 4;" ::"r"(full) : "memory");
+      asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(dst), "r"(task), "r"(full) : "memory");
+    }
+    __syncwarp();
+  }
+};
 
 // The task list as a role of a pair walks it: first the shared expert's tasks, which need nothing but the staged tokens
 // and are on the host's count of tokens, then -- once everything before this launch in the stream has completed -- the pair
@@ -163,7 +197,7 @@ struct PairWalk {
   TmControl* ctl;
   uint32_t cta;
   int n_blocks, task, stride;
-  uint32_t taken, q_empty_leader;
+  uint32_t taken;
   bool waited;
   int routed_tiles;
   const Tile* tiles;
@@ -171,7 +205,7 @@ struct PairWalk {
   int peer_valid, nb;     // rows of the other half; weight block
   __device__ __forceinline__ PairWalk(const TmParams& params, TmControl* control, uint32_t cta_rank, bool plan_ready)
       : p(params), ctl(control), cta(cta_rank), n_blocks(params.rows_per_expert / kTmN), task(blockIdx.x / 2), stride(gridDim.x / 2),
-        taken(0), q_empty_leader(map_to_cta(smem_u32(&control->q_empty[0]), 0)), waited(false), routed_tiles(0), tiles(nullptr) {
+        taken(0), waited(false), routed_tiles(0), tiles(nullptr) {
     if (plan_ready) load_plan();
   }
   __device__ __forceinline__ void load_plan() {
@@ -205,12 +239,8 @@ struct PairWalk {
     int t = task;
     task += stride;
     if (p.tasks != nullptr) {
-      const uint32_t slot = taken % kPairQueue, bar = smem_u32(&ctl->q_full[slot]), parity = (taken / kPairQueue) & 1u;
-      if (!(kOneLanePolls ? waiter.wait_warp(bar, parity) : waiter.wait_uniform(bar, parity))) return false;
-      t = ctl->q_task[slot];
-      __syncwarp();
-      if ((threadIdx.x & 31) == 0) mbar_arrive_pair(q_empty_leader + 8 * slot);
-      ++taken;
+      PairPort<kOneLanePolls> port{ctl, waiter};
+      if (!pair_take(port, taken++, &t)) return false;
     }
     return locate(t);
   }
@@ -280,9 +310,9 @@ __global__ void __launch_bounds__(tm_threads(kLayer), 1) tm_kernel(const __grid_
     }
     for (int i = 0; i < 2; ++i) mbar_init(smem_u32(&ctl->tmem_full[i]), 1);
     mbar_init(smem_u32(&ctl->overlap_free), 2 * tm_epilogue_warps(kLayer));   // one arrival per epilogue warp of the pair
-    for (int i = 0; i < kPairQueue; ++i) {
-      mbar_init(smem_u32(&ctl->q_full[i]), 1);
-      mbar_init(smem_u32(&ctl->q_empty[i]), 2 * tm_epilogue_warps(kLayer) + 3);   // ... and both producers and the issuer
+    for (uint32_t i = 0; i < kPairQueue; ++i) {
+      mbar_init(smem_u32(&ctl->q_full[i]), pair_full_count());
+      mbar_init(smem_u32(&ctl->q_empty[i]), pair_empty_count(cta == 0, tm_epilogue_warps(kLayer) + (cta == 0 ? 2 : 1)));   // ... producer and issuer
     }
     mbar_init(smem_u32(&ctl->q_want), 1);
     ctl->abort_flag = 0;
@@ -427,19 +457,20 @@ __global__ void __launch_bounds__(tm_threads(kLayer), 1) tm_kernel(const __grid_
       }
     }
   } else if (warp == 2 + tm_epilogue_warps(kLayer)) {
-    // --------------------------------------------------------------------------------------------- scheduler
-    if (cta == 0 && p.tasks != nullptr) {
+    // --------------------------------------------------------------------------------------------- scheduler, forwarder
+    PairPort<false> port{ctl, waiter};
+    if (p.tasks == nullptr) {
+    } else if (cta == 0) {
       for (uint32_t n = 0;; ++n) {
         int t = 0;
         if (lane == 0) t = atomicAdd(p.tasks, 1);
         t = __shfl_sync(0xffffffffu, t, 0);
-        const uint32_t slot = n % kPairQueue;
-        if (!waiter.wait_uniform(smem_u32(&ctl->q_empty[slot]), ((n / kPairQueue) & 1u) ^ 1u)) break;
-        if (lane < 2) pair_send_task(smem_u32(const_cast<int32_t*>(&ctl->q_task[slot])), smem_u32(&ctl->q_full[slot]), lane, t);
-        __syncwarp();
-        if (!walk.locate(t)) break;
+        if (!pair_put(port, n, t) || !walk.locate(t)) break;
         if (!waiter.wait_uniform(smem_u32(&ctl->q_want), n & 1u)) break;
       }
+    } else {
+      int t;
+      for (uint32_t n = 0; pair_peek(port, n, &t) && walk.locate(t) && pair_forward(port, n);) ++n;
     }
   } else {
     // --------------------------------------------------------------------------------------------- epilogue
