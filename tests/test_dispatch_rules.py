@@ -99,3 +99,10 @@ def test_experts_just_past_one_pair_task(rules):
             assert not on_pairs and tiles <= (4 if cap == 80 else 3), case
         else:
             assert on_pairs, case
+
+
+def test_what_a_call_rewrites_is_not_read_as_constant():
+    """The GEMM launches run beside the launches that write their inputs: nothing in them goes through the read-only path."""
+    for name in ("mmoe_umma.cu", "mmoe_umma_tm.cu", "mmoe_tc.cuh", "mmoe_common.cuh"):
+        with open(os.path.join(ROOT, "vllm_plugin_b200", "csrc", name)) as f:
+            assert "__ldg(p." not in f.read().replace("__ldg(x_sf", "__ldg(p."), name

@@ -647,6 +647,33 @@ def test_small_kernels_of_few_tokens_against_those_of_more(hidden, k, shared, fe
     assert met["rel_l2"] <= 1e-3, met
 
 
+@pytest.mark.parametrize("shared,m,skewed", [(True, 700, False), (False, 700, False), (True, 700, True), (False, 700, True), (True, 230, False)])
+def test_launches_behind_the_pairs_wait_where_they_are_not_told(shared, m, skewed):
+    """GEMM1 on CTA pairs counts in memory that what precedes it is complete, and what follows it waits for all of GEMM1 where it does not
+    find that: here a count far below zero.  Pair tiles only, beside others, and none at all behind the shared expert's; the count
+    is back at zero behind every call."""
+    from vllm_plugin_b200 import api
+    e, k = 16, 2
+    layer = H.make_layer(512, 256, e, k, shared, seed=71)
+    weights = H.kernel_weights(layer, "cuda")
+    hid = O.make_hidden(m, 512, 3)
+    ids, w = O.make_routing(m, e, k, 4)
+    ids[:, 0] = 5
+    ids[:, 1] = 7 if not skewed else torch.arange(m) % 4
+    if m == 230:
+        ids[:] = torch.arange(2 * m).view(m, 2) % e
+    want, buf = H.run_layer(layer, hid, ids, w, weights=weights)
+    assert_parity(want, H.oracle_layer(layer, hid, ids, w), f"m {m} shared {shared} skewed {skewed}")
+    small, routed = int(buf.plan_words[6]), int(buf.plan_words[0])
+    assert (small > 0) == (skewed or m == 230) and (small < routed) == (m == 700)
+    told = buf._view(buf.layout.plan, (16 + 6 * e + 8,), torch.int32)[-1:]
+    assert not told.any()
+    for call in range(4):
+        told.fill_(-2 ** 30 if call % 2 == 0 else 0)
+        y, _ = H.run_layer(layer, hid, ids, w, weights=weights, buf=buf)
+        assert torch.equal(y, want) and not told.any(), call
+
+
 TILE_ROWS = [(16, (160, 160, 128), 1), (16, (160, 128, 128), 1), (16, (192, 192, 192), 0), (16, (64,), 7), (32, (64, 33), 5), (32, (65, 33), 5),
              (64, (100, 65, 33), 12)]
 MANY_COLD = [(16, (160, 160, 128), 49), (16, (160, 160, 128), 50)]

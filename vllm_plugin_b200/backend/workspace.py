@@ -176,7 +176,7 @@ class SymmBuffer:
         scale chunk, which tile of how many of its expert.  Tiles of the weights-as-A kernels come first, then those of the CTA
         pairs, then the shared expert's."""
         e_l, r = self.num_experts // self.num_ranks, self.num_ranks
-        ints = e_l + 3 * (e_l + 1) + (r + 1) + 2 * e_l * r + 2
+        ints = e_l + 3 * (e_l + 1) + (r + 1) + 2 * e_l * r + 3
         first = 16 + (ints + 7) // 8 * 8
         words = self.plan_words.cpu()
         return self._view(self.layout.plan, (first + 8 * int(words[0] + words[1]),), torch.int32)[first:].cpu().view(-1, 8)

@@ -132,7 +132,7 @@ struct PlanHeader {
 static_assert(sizeof(PlanHeader) == 64, "plan header is 64 bytes");
 
 // Plan region: header | expert_total[E_l] | expert_block_off[E_l+1] | expert_tile_off[E_l+1] | rank_off[R+1] |
-// seg_pool_start[E_l*R] | seg_recv_start[E_l*R] | done[E_l+1] | pair_tasks[2] | tiles[max_tiles]
+// seg_pool_start[E_l*R] | seg_recv_start[E_l*R] | done[E_l+1] | pair_tasks[2] | pairs_open | tiles[max_tiles]
 struct PlanView {
   PlanHeader* hdr;
   int32_t* expert_total;
@@ -142,7 +142,8 @@ struct PlanView {
   int32_t* seg_pool_start;
   int32_t* seg_recv_start;
   int32_t* done;               // one GPU, both GEMMs: finished parts of GEMM1 per expert, the shared one last; zero between calls
-  int32_t* pair_tasks;         // ... and the tasks of either layer that CTA pairs have claimed, likewise
+  int32_t* pair_tasks;         // ... the tasks of either layer that CTA pairs have claimed, likewise
+  int32_t* pairs_open;         // ... and the CTA pairs of GEMM1 that have seen everything in front of them complete (see open_chain), likewise
   Tile* tiles;
 };
 
@@ -164,7 +165,7 @@ __host__ __device__ inline int64_t shared_chunk_rows(int64_t max_tokens) { retur
 __host__ __device__ inline int64_t shared_tile_capacity(int64_t max_tokens) { return (max_tokens / 16 + 2) * 2; }
 
 __host__ __device__ inline int64_t plan_bytes(int e_local, int num_ranks, int64_t max_tiles) {
-  int64_t ints = e_local + 3 * (e_local + 1) + (num_ranks + 1) + 2 * (int64_t)e_local * num_ranks + 2;
+  int64_t ints = e_local + 3 * (e_local + 1) + (num_ranks + 1) + 2 * (int64_t)e_local * num_ranks + 3;
   return 64 + align_up(ints * 4, 32) + max_tiles * (int64_t)sizeof(Tile);
 }
 
@@ -181,6 +182,7 @@ __host__ __device__ inline PlanView plan_view(void* base, int e_local, int num_r
   v.seg_recv_start = q;          q += (int64_t)e_local * num_ranks;
   v.done = q;                    q += e_local + 1;
   v.pair_tasks = q;              q += 2;
+  v.pairs_open = q;              q += 1;
   int64_t ints = q - reinterpret_cast<int32_t*>(p + 64);
   v.tiles = reinterpret_cast<Tile*>(p + 64 + align_up(ints * 4, 32));
   return v;
@@ -332,13 +334,30 @@ inline bool staged_tokens(const Ctx& c, int m, int block_m) {
 // set-up -- barrier initialisation, tensor-memory allocation -- overlap this kernel's run); chain_wait() waits until
 // everything BEFORE this kernel in the stream has completed and its memory is visible.  Most kernels begin with both, in this
 // order (chain_begin()), and touch no global memory before.  The wait is transitive: the next kernel's wait ends only when
-// this grid has completed, and this grid completes only after its own wait has.  A kernel of this library that waits first
-// and releases then tells its successor more: what precedes IT has completed when the successor starts, which may use that
-// without a wait.  Nothing is taken to be complete about a kernel from elsewhere, which may release as early as it likes.  Both
-// instructions do nothing in a kernel that was launched without the attribute below.
+// this grid has completed, and this grid completes only after its own wait has.  Nothing is taken to be complete about a kernel from
+// elsewhere, which may release as early as it likes.  Both instructions do nothing in a kernel that was launched without the
+// attribute below.
+//
+// A kernel of this library that waits first and releases then tells its successor more: what precedes IT has completed when the
+// successor starts, which may use that without waiting for IT.  But visibility is promised to a grid that waits, and to no other.  So
+//   * what follows the pairs' GEMM1 (their GEMM2, and the launch of both GEMMs) is told in memory: GEMM1 counts a release (open_chain)
+//     between its wait and its chain_release(), and every thread of the launches behind acquires it or, where it finds nothing, waits
+//     for all of GEMM1 after all (chain_opened);
+//   * a GEMM launch behind the route ordering starts with the staged tokens alone.  Nobody counts for it: it relies on the ordering's
+//     wait having brought the staged rows and scales to the L2, and reads them there (bulk copies, __ldcg), never through an L1.
+// What one launch of a call writes for another (pool_w, pool_dst, scales) is never read through the read-only path (__ldg), which is for
+// memory that nobody writes while the kernel runs.
 // ---------------------------------------------------------------------------------------------------------------------
 __device__ __forceinline__ void chain_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void open_chain(int32_t* word) {
+  asm volatile("red.release.gpu.global.add.s32 [%0], 1;" ::"l"(word) : "memory");
+}
+__device__ __forceinline__ bool chain_opened(const int32_t* word) {
+  int32_t v;
+  asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(word) : "memory");
+  return v > 0;
+}
 __device__ __forceinline__ void chain_begin() {
   chain_release();
   chain_wait();

@@ -1121,7 +1121,7 @@ __device__ __forceinline__ bool combine_zeroes(char* plan_base, int e_local) {
     pv.hdr->next_task = 0;
     pv.hdr->layer1_done = 0;
   }
-  for (int e = threadIdx.x; e < e_local + 3; e += blockDim.x) pv.done[e] = 0;      // and `pair_tasks` behind it
+  for (int e = threadIdx.x; e < e_local + 4; e += blockDim.x) pv.done[e] = 0;      // and `pair_tasks`, `pairs_open` behind it
   __threadfence();
   __syncthreads();
   chain_release();
@@ -1258,7 +1258,7 @@ cudaError_t zero_counters(const Ctx& c, cudaStream_t s) {
   const PlanView pv = plan_view(c.ws + c.lay.plan, c.e_local, c.geo.num_ranks);
   const size_t first = offsetof(PlanHeader, routed), end = offsetof(PlanHeader, layer1_done) + sizeof pv.hdr->layer1_done;
   cudaError_t e = cudaMemsetAsync(reinterpret_cast<char*>(pv.hdr) + first, 0, end - first, s);      // `claims` lies between, zero already
-  if (e == cudaSuccess) e = cudaMemsetAsync(pv.done, 0, (c.e_local + 3) * sizeof *pv.done, s);
+  if (e == cudaSuccess) e = cudaMemsetAsync(pv.done, 0, (c.e_local + 4) * sizeof *pv.done, s);
   return e;
 }
 

@@ -69,7 +69,7 @@ struct UmmaParams {
   int with_routed;             // 0: only those
   int tile_rows;               // > 0: rows of the token slots that the launch starts with; 0: those of the call's largest tile, in the plan
   int early;                   // both layers: 1 when the launch in front lets this one start with the staged tokens complete, not the plan
-  int skip_wait;               // 1: what this launch reads was complete before the launch in front of it let it start
+  int behind_pairs;            // both layers: 1 when the launches in front are the pairs', of which this one needs nothing (see chain_opened)
   const int32_t* x_sf;         // layer 1: the staged tokens' scale words [T][K/128], gathered for tiles of staged tokens
   // calls of at most kStagedTokens tokens: every routed tile of layer 1 is the staged tokens themselves (see TaskQueue)
   const int64_t* topk_idx;
@@ -787,7 +787,7 @@ __device__ __forceinline__ void sa_arrange_scales(const Cta& c, Walk walk, Waite
     auto gather = [&](uint32_t (&w)[4], int kb) {
 #pragma unroll
       for (int a = 0; a < 4; ++a)
-        w[a] = staged && kb < k_stages && lane + 32 * a < walk.tile.n_valid ? __ldg(x_sf + 32 * a * k_stages + kb) : 0u;
+        w[a] = staged && kb < k_stages && lane + 32 * a < walk.tile.n_valid ? __ldcg(x_sf + 32 * a * k_stages + kb) : 0u;
     };
     gather(ahead[0], 0);
     gather(ahead[1], 1);
@@ -954,11 +954,11 @@ __device__ __forceinline__ void sa_epilogue(const Cta& c, Walk walk, bool plan_k
     for (int cc = 0; cc < 4; ++cc) {
       const int i = 32 * cc + lane;
       if (i < tile.n_valid) {
-        if (kLayer == 1) { if (!shared) wv[cc] = __ldg(p.pool_w + tile.row0 + i); }
-        else if (!kFused) dv[cc] = shared ? tile.row0 + i : (kStaged ? p.pool_dst[tile.row0 + i] : __ldg(p.pool_dst + tile.row0 + i));
+        if (kLayer == 1) { if (!shared) wv[cc] = __ldcg(p.pool_w + tile.row0 + i); }
+        else if (!kFused) dv[cc] = shared ? tile.row0 + i : __ldcg(p.pool_dst + tile.row0 + i);
         else if (shared) dv[cc] = static_cast<int>((32u << kOutSlotShift) | static_cast<uint32_t>(tile.row0 + i));
         else {
-          const int r = __ldg(p.pool_dst + tile.row0 + i);       // receive-order row
+          const int r = __ldcg(p.pool_dst + tile.row0 + i);      // receive-order row
           int sr = 0;
           while (sr + 1 < p.num_ranks && r >= ctl->rank_off[sr + 1]) ++sr;
           dv[cc] = static_cast<int>((static_cast<uint32_t>(sr) << kOutSlotShift) |
@@ -1171,7 +1171,7 @@ __global__ void __launch_bounds__(kThreads, 1) umma_kernel(const __grid_constant
     prefetch_map(&p.map_w_routed);
     prefetch_map(&p.map_w_shared);
   }
-  if (!p.skip_wait) chain_wait();
+  chain_wait();
   if (kFused) {
     if (threadIdx.x == 0) ctl->out_base[32] = p.shared_out;
     const int t = threadIdx.x - 32;
@@ -1204,7 +1204,6 @@ __global__ void __launch_bounds__(kThreads, 1) umma_kernel(const __grid_constant
   } else {
     sa_epilogue<L, kFused, false>(c, walk, true, waiter, st);
   }
-  chain_wait();       // a CTA that has not waited yet must not end before what precedes the launch
   sa_teardown(ctl, c.tmem_base);
 }
 
@@ -1219,7 +1218,8 @@ __global__ void __launch_bounds__(both_threads(kStaged), 1) moe_kernel(const __g
   const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);
   const PlanView pv = plan_view(const_cast<char*>(p.plan), p.e_local, p.num_ranks);
   chain_release();
-  if (p.skip_wait && p.shared_tiles.parts == 0 && pv.hdr->num_small_tiles == 0) {      // every expert ran on the pairs in front
+  if (p.behind_pairs && !chain_opened(pv.pairs_open)) chain_wait();
+  if (p.behind_pairs && p.shared_tiles.parts == 0 && pv.hdr->num_small_tiles == 0) {      // every expert ran on the pairs in front
     chain_wait();
     return;
   }
@@ -1236,7 +1236,7 @@ __global__ void __launch_bounds__(both_threads(kStaged), 1) moe_kernel(const __g
     prefetch_map(&p.map_w_shared);
   }
   const bool route_here = kStaged && p.route_here, plan_ready = !p.early && !route_here;
-  if ((!p.early || route_here) && !p.skip_wait) chain_wait();
+  if ((!p.early || route_here) && !p.behind_pairs) chain_wait();
   if (plan_ready) queue.load_plan();
   int rows = sa_tile_rows(p);
   tc_fence_before();
@@ -1648,17 +1648,16 @@ cudaError_t launch_experts_umma(const Ctx& c, const MmoeWeights& w, const MmoeOp
   std::shared_ptr<const SaPlan> sa_plan;
   if (pairs && (tm_plan = kept_plan<TmPlan>(g_tm_plans, key, c, w, has_shared)) == nullptr) return cudaErrorInvalidValue;
   if (small && (sa_plan = kept_plan<SaPlan>(g_sa_plans, key, c, w, has_shared)) == nullptr) return cudaErrorInvalidValue;
+  // The whole of one GPU's call: the pairs' two launches, then one for all other experts.  It needs nothing of the pairs'
+  // launches, so its CTAs start as theirs run out of tasks.
+  const bool both = c.both_layers && small;
   auto small_params = [&](UmmaParams& p, int layer) {
     patch(p, layer == 2);
     p.shared_tiles = shared_pairs ? none : shared;
     p.tile_rows = c.tile_select == 2 ? cut.step : 0;
     p.shared_in_plan = pairs && c.geo.num_ranks == 1 && c.tile_select != 2 ? 1 : 0;
-    // The pair launches in front read and write nothing that this one does, and the first lets the others start only after its own wait.
-    p.skip_wait = pairs ? 1 : 0;
+    p.behind_pairs = pairs && both ? 1 : 0;
   };
-  // The whole of one GPU's call: the pairs' two launches, then one for all other experts.  It needs nothing of the pairs'
-  // launches, so its CTAs start as theirs run out of tasks.
-  const bool both = c.both_layers && small;
   const PlanView pv = plan_view(c.ws + c.lay.plan, c.e_local, c.geo.num_ranks);
   const bool claims = c.both_layers && pairs;
   for (int layer = 1; layer <= 2; ++layer) {
@@ -1689,7 +1688,7 @@ cudaError_t launch_experts_umma(const Ctx& c, const MmoeWeights& w, const MmoeOp
     e = staged ? launch_both<true>(p, s) : launch_both<false>(p, s);
   }
   // a pair launch may have run, and no combine follows, which would zero its counters
-  if (e != cudaSuccess && claims) cudaMemsetAsync(pv.done, 0, (c.e_local + 3) * sizeof *pv.done, s);
+  if (e != cudaSuccess && claims) cudaMemsetAsync(pv.done, 0, (c.e_local + 4) * sizeof *pv.done, s);
   return e;
 }
 

@@ -292,13 +292,17 @@ __global__ void __launch_bounds__(tm_threads(kLayer), 1) tm_kernel(const __grid_
   const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   const uint32_t cta = cluster_ctarank();                         // 0 = leader
 
-  // GEMM2 behind GEMM1 of the same call: GEMM1 lets it start after its own wait, so all that comes before GEMM1 is complete, and
+  // GEMM2 behind GEMM1 of the same call: GEMM1 opens the chain after its own wait, so all that comes before GEMM1 is complete, and
   // GEMM1 itself counts its finished parts.
-  const bool behind_layer1 = kLayer == 2 && p.done != nullptr;
+  const PlanView pv = plan_view(const_cast<char*>(p.plan), p.e_local, p.num_ranks);
+  const bool behind_layer1 = kLayer == 2 && p.done != nullptr, opens = kLayer == 1 && p.done != nullptr;
+  auto wait_front = [&] {
+    if (!behind_layer1 || !chain_opened(pv.pairs_open)) chain_wait();
+  };
   if (p.shared_tiles.parts == 0) {        // routed tiles only, of which the call may have none
-    if (!behind_layer1) chain_wait();
-    const PlanHeader* hdr = plan_view(const_cast<char*>(p.plan), p.e_local, p.num_ranks).hdr;
-    if (p.with_routed == 0 || hdr->num_routed_tiles == hdr->num_small_tiles) {
+    wait_front();
+    if (p.with_routed == 0 || pv.hdr->num_routed_tiles == pv.hdr->num_small_tiles) {
+      if (opens && threadIdx.x == 0) open_chain(pv.pairs_open);
       chain_wait();
       return;
     }
@@ -326,7 +330,7 @@ __global__ void __launch_bounds__(tm_threads(kLayer), 1) tm_kernel(const __grid_
   // here for everything before it; GEMM1 in a programmatic chain starts when the blocks of the placement have all started,
   // i.e. after the launches before it (staging, counting) have completed, and waits when it comes to the routed tiles.
   // Only then does it let the next launch start.
-  if (kLayer == 2 && !behind_layer1) chain_wait();
+  if (kLayer == 2 && p.shared_tiles.parts != 0) wait_front();
   if (kFused) {
     const int t = threadIdx.x - 32;
     if (t >= 0 && t < p.num_ranks) {
@@ -363,13 +367,18 @@ __global__ void __launch_bounds__(tm_threads(kLayer), 1) tm_kernel(const __grid_
     const uint32_t want = p.tasks != nullptr && cta == 0 ? smem_u32(&ctl->q_want) : 0u;
     const int want_at = max(k_stages - 8, 0);            // a claim in time, and not earlier: that would hoard tasks
     bool ok = true, released = false;
+    auto release = [&] {                                 // once everything in front of the launch is complete
+      if (released || !walk.waited) return;
+      __syncwarp();
+      if (opens && cta == 0 && lane == 0) open_chain(pv.pairs_open);
+      __syncwarp();
+      chain_release();
+      released = true;
+    };
     while (ok && walk.next<false>(waiter)) {
+      release();
       const Tile tile = walk.tile;
       const int nb = walk.nb;
-      if (!released && walk.waited) {
-        chain_release();
-        released = true;
-      }
       const bool shared = tile.expert == kSharedExpert;
       const int e = shared ? 0 : tile.expert;
       const int r0 = nb * kTmN + static_cast<int>(cta) * (kTmN / 2);     // this CTA's 128 stored weight rows: inside one slice
@@ -411,6 +420,7 @@ __global__ void __launch_bounds__(tm_threads(kLayer), 1) tm_kernel(const __grid_
         if (++stage == kTmStages) { stage = 0; phase ^= 1u; }
       }
     }
+    release();
   } else if (warp == 1) {
     // --------------------------------------------------------------------------------------------- issuer
     if (cta == 0) {
@@ -500,14 +510,14 @@ __global__ void __launch_bounds__(tm_threads(kLayer), 1) tm_kernel(const __grid_
       float wt = 1.0f;
       __nv_bfloat16* out = nullptr;
       if (kLayer == 1) {
-        if (!shared && live) wt = __ldg(p.pool_w + row);
+        if (!shared && live) wt = __ldcg(p.pool_w + row);
       } else if (live) {
         if (shared) {
           out = p.shared_out + row * p.hidden;
         } else if (!kFused) {
-          out = p.ret + (int64_t)__ldg(p.pool_dst + row) * p.hidden;
+          out = p.ret + (int64_t)__ldcg(p.pool_dst + row) * p.hidden;
         } else {
-          const int r = __ldg(p.pool_dst + row);          // receive-order row -> source rank and its send position
+          const int r = __ldcg(p.pool_dst + row);         // receive-order row -> source rank and its send position
           int sr = 0;
           while (sr + 1 < p.num_ranks && r >= ctl->rank_off[sr + 1]) ++sr;
           out = ctl->out_base[sr] + (int64_t)(ctl->home_base[sr] + r - ctl->rank_off[sr]) * p.hidden;
