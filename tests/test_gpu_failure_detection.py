@@ -214,6 +214,54 @@ def test_pairs_that_wait_for_lost_rows_and_the_call_behind(missing):
         api.set_kernel_options(timeout_ms=2000)
 
 
+@pytest.mark.parametrize("missing", ["routed", "shared"])
+def test_pairs_with_several_tasks_each_and_lost_rows(missing):
+    """Five and more tasks per pair and layer, so that every slot of a pair's queue is used again, with roles that stop at different places
+    of it.  Only what was lost is missing, the wait ends near its limit, and the calls behind are right."""
+    import time
+    from vllm_plugin_b200 import api
+    import helpers as H
+    from helpers import O
+    e, k, m, hidden, inter = 12, 6, 1500, 2560, 1152
+    layer = H.make_layer(hidden, inter, e, k, True, seed=8)
+    weights = H.kernel_weights(layer, "cuda")
+    hid = O.make_hidden(m, hidden, 1)
+    ids, w = O.make_routing(m, e, k, 2)
+    want, buf = H.run_layer(layer, hid, ids, w, weights=weights)
+    shared_out = buf._view(buf.layout.shared_out, (m, hidden), torch.bfloat16)
+    rows, shared_rows = buf.ret[:m * k].clone(), shared_out.clone()
+    sample = torch.arange(0, m, 25)
+    assert O.parity_metrics(want.cpu()[sample], H.oracle_layer(layer, hid[sample], ids[sample], w[sample]))["rel_l2"] <= 1e-3
+    assert buf.plan_words[6] == 0                                         # every expert on pairs
+    pairs = torch.cuda.get_device_properties(0).multi_processor_count // 2
+    tiles = (int(buf.plan_words[0]) + int(buf.plan_words[1])) // 2
+    assert tiles * (2 * inter // 256) >= 5 * pairs and tiles * (hidden // 256) >= 5 * pairs
+    lost = e if missing == "shared" else int(ids[0, 0])
+    done = buf._view(buf.layout.plan, (16 + 6 * e + 8,), torch.int32)[16 + 5 * e + 4:]              # and what lies behind it
+    api.set_kernel_options(timeout_ms=200)
+    try:
+        for _ in range(2):
+            buf.ret.zero_()
+            shared_out.zero_()
+            done[lost] = -2 ** 30
+            torch.cuda.synchronize()
+            t0 = time.perf_counter()
+            with pytest.raises(RuntimeError, match="device wait expired: kernel 22"):
+                H.run_layer(layer, hid, ids, w, weights=weights, buf=buf)
+            assert 0.15 < time.perf_counter() - t0 < 2.0
+            assert not done.any()
+            pos = buf.route_pos[:m].cpu().long()
+            for x in range(e):
+                if x != lost:
+                    assert torch.equal(buf.ret[pos[ids == x].cuda()], rows[pos[ids == x].cuda()]), x
+            assert torch.equal(shared_out, shared_rows) == (missing != "shared")
+            for _ in range(2):
+                y, _ = H.run_layer(layer, hid, ids, w, weights=weights, buf=buf)
+                assert torch.equal(y, want)
+    finally:
+        api.set_kernel_options(timeout_ms=2000)
+
+
 @pytest.fixture(scope="module")
 def run_wait(tmp_path_factory):
     import os
