@@ -363,15 +363,6 @@ __device__ __forceinline__ void chain_begin() {
   chain_wait();
 }
 
-// A call streams its weights through the L2, so the small kernels around the GEMMs find their code in DRAM: 1-2 us per stretch that is not
-// there.  One that has to wait for the launch in front may walk its own code first, without touching memory that is not its
-// own: `for (int go = opaque(0);; go = opaque(1)) { if (go) chain_wait(); ... if (go) break; }`.  The compiler is not to know which round
-// it is in, or it makes a copy of the code for the first.
-__device__ __forceinline__ int opaque(int v) {
-  asm volatile("" : "+r"(v));
-  return v;
-}
-
 // The entry points of single-GPU calls open a ChainScope; every launch outside one is an ordinary one.  A GEMM CTA holds an SM
 // to itself, so what starts early there is the next launch's CTA on an SM that has run out of tasks.  Chain plus shared
 // expert first, measured together: 7 tokens 163 -> 141 us, 128 tokens / 32 experts 155 -> 144, 3840 / 384 1784 -> 1683.

@@ -739,7 +739,6 @@ struct RouteArgs {
   int64_t pool_sf_rows;
   SharedScales shared;
   int h, k;
-  int walk;                  // 1: walk the code while the launch in front runs
   PlanArgs a;
 };
 
@@ -764,11 +763,12 @@ __device__ void write_single_rank_plan(const RouteArgs& r, const PlanView& pv, i
 // Calls of at most kSmallRoutes routes: ONE launch.  Every block ranks the routes and builds the plan for itself in shared memory
 // (2-3 us, less than a second launch behind a grid-wide hand-over), block 0 writes it out, and the others place the
 // routes, one warp per route (block 0 with its share of them came in 0.5-1 us late).  The shared expert's scales are not placed: its GEMM1 gathers them itself.
-// The ranking and the plan are a chain of barriers in code that lies in DRAM (see opaque()): walking them once on masked routes while the
-// staging runs, 128 tokens of 32 experts are placed 8.3 us behind the staging instead of 12, and the call takes 130.4 us instead of 132.5.
-// Not in a captured call: where the staging comes first in a graph nothing is left to walk in, and the walk takes what it
-// saves (64 tokens of 384 experts 709 -> 711).  The same did nothing for the route counting and the combine.
+// The ranking and the plan are a chain of barriers in code that lies in DRAM.  Walking it once on masked routes in front of the wait saved 0.6 us of
+// calls in a row (128 tokens of 32 experts 131.2 -> 130.6) and cost 2.1 where the staging had ended already, as it has in every call
+// that finds the GPU idle (141.9 -> 144.0 from event to event; 32 tokens 129.6 -> 134.2).
 __global__ void __launch_bounds__(kRouteThreads) route_small_kernel(const RouteArgs r) {
+  chain_wait();
+  chain_release();       // in this order: the GEMM1 launch starts knowing that the staging has completed
   extern __shared__ int32_t sm[];
   const int E = r.a.e_local, n = r.a.m * r.k, n_even = (n + 1) & ~1;
   int32_t* s_block = sm;                             // [E] first pool block
@@ -777,25 +777,14 @@ __global__ void __launch_bounds__(kRouteThreads) route_small_kernel(const RouteA
   uint16_t* ids = reinterpret_cast<uint16_t*>(s_step + E);
   uint16_t* rank = ids + n_even;
   uint16_t* warp_count = rank + n_even;              // [16][E]
-  const PlanView pv = plan_view(r.plan, E, 1);
-  int total;
-  ExpertPlan ep;
-#pragma unroll 1
-  for (int go = opaque(r.walk ? 0 : 1);; go = opaque(1)) {
-    if (go) {
-      chain_wait();
-      chain_release();   // in this order: the GEMM1 launch starts knowing that the staging has completed
-    }
-    const int routes = go ? n : min(n, 32);
-    for (int i = threadIdx.x; i < routes; i += kRouteThreads) {
-      int64_t id = go ? r.topk_idx[i] : -1;
-      if (id >= E) { if (blockIdx.x == 0) report_bad_index(r.status); id = -1; }
-      ids[i] = id < 0 ? 0xFFFF : static_cast<uint16_t>(id);
-    }
-    total = block_rank_routes(ids, routes, rank, warp_count, E);
-    ep = build_plan(pv, total, r.a, go && blockIdx.x == 0);
-    if (go) break;
+  for (int i = threadIdx.x; i < n; i += kRouteThreads) {
+    int64_t id = r.topk_idx[i];
+    if (id >= E) { if (blockIdx.x == 0) report_bad_index(r.status); id = -1; }
+    ids[i] = id < 0 ? 0xFFFF : static_cast<uint16_t>(id);
   }
+  const int total = block_rank_routes(ids, n, rank, warp_count, E);
+  const PlanView pv = plan_view(r.plan, E, 1);
+  const ExpertPlan ep = build_plan(pv, total, r.a, blockIdx.x == 0);
   if ((int)threadIdx.x < E) {
     s_block[threadIdx.x] = ep.block_off;
     s_off[threadIdx.x] = ep.row_off;
@@ -1059,10 +1048,8 @@ RouteArgs route_args(const Ctx& c, int m, int block_m, int32_t* stats) {
 cudaError_t launch_route_small(const Ctx& c, int m, int block_m, int32_t* stats, cudaStream_t s) {
   const int n = m * c.geo.num_topk, e = c.geo.num_experts;
   const size_t smem = (size_t)3 * e * 4 + (size_t)2 * ((n + 1) & ~1) * 2 + (size_t)kRouteWarps * e * 2;
-  RouteArgs r = route_args(c, m, block_m, stats);
-  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-  r.walk = chained() && cudaStreamIsCapturing(s, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone ? 1 : 0;
-  return launch_chained(route_small_kernel, dim3(1 + std::min((n + kRouteWarps - 1) / kRouteWarps, 147)), dim3(kRouteThreads), smem, s, r);
+  return launch_chained(route_small_kernel, dim3(1 + std::min((n + kRouteWarps - 1) / kRouteWarps, 147)), dim3(kRouteThreads), smem, s,
+                        route_args(c, m, block_m, stats));
 }
 
 cudaError_t launch_route_large(const Ctx& c, int m, int block_m, int32_t* stats, cudaStream_t s) {
