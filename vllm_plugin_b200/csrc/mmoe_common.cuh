@@ -344,7 +344,8 @@ inline bool staged_tokens(const Ctx& c, int m, int block_m) {
 //     between its wait and its chain_release(), and every thread of the launches behind acquires it or, where it finds nothing, waits
 //     for all of GEMM1 after all (chain_opened);
 //   * a GEMM launch behind the route ordering starts with the staged tokens alone.  Nobody counts for it: it relies on the ordering's
-//     wait having brought the staged rows and scales to the L2, and reads them there (bulk copies, __ldcg), never through an L1.
+//     wait having brought the staged rows and scales to the L2, and reads them there: by bulk copies, and the scales behind a fence that
+//     leaves nothing older in the L1.
 // What one launch of a call writes for another (pool_w, pool_dst, scales) is never read through the read-only path (__ldg), which is for
 // memory that nobody writes while the kernel runs.
 // ---------------------------------------------------------------------------------------------------------------------

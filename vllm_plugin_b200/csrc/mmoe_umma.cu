@@ -776,18 +776,20 @@ __device__ __forceinline__ void sa_arrange_scales(const Cta& c, Walk walk, Waite
     const int r = 16 * ((m & 63) >> 3) + 8 * h + (m & 7);   // stored row inside its 128-row block
     src[t] = 128 * (m >> 6) + 4 * (r & 31) + (r >> 5);
   }
+  if (!kStaged) asm volatile("fence.acq_rel.gpu;" ::: "memory");      // nothing of the rows staged before is left in the L1
   for_each_task(walk, waiter, st, [&](auto layer, const UmmaParams& p) {
     if constexpr (decltype(layer)::value == 1) {
     const int k_stages = p.k_dim / kTileK;
     // The scales of staged tokens are gathered here, word kb of the staged scale rows (chunk position 4 (i % 32) + i / 32
-    // for token i), two stages ahead: such tiles need no placement, only the staging.
+    // for token i), two stages ahead: such tiles need no placement, only the staging.  Through the L1, which has a row's next 31 words then
+    // (from the L2 each: 7 tokens 131 -> 136 us).
     const bool staged = walk.tile.expert == kSharedExpert || kStaged;
     const int32_t* x_sf = p.x_sf + (int64_t)(walk.tile.row0 + lane) * k_stages;
     uint32_t ahead[2][4] = {};
     auto gather = [&](uint32_t (&w)[4], int kb) {
 #pragma unroll
       for (int a = 0; a < 4; ++a)
-        w[a] = staged && kb < k_stages && lane + 32 * a < walk.tile.n_valid ? __ldcg(x_sf + 32 * a * k_stages + kb) : 0u;
+        w[a] = staged && kb < k_stages && lane + 32 * a < walk.tile.n_valid ? __ldca(x_sf + 32 * a * k_stages + kb) : 0u;
     };
     gather(ahead[0], 0);
     gather(ahead[1], 1);
@@ -955,7 +957,7 @@ __device__ __forceinline__ void sa_epilogue(const Cta& c, Walk walk, bool plan_k
       const int i = 32 * cc + lane;
       if (i < tile.n_valid) {
         if (kLayer == 1) { if (!shared) wv[cc] = __ldcg(p.pool_w + tile.row0 + i); }
-        else if (!kFused) dv[cc] = shared ? tile.row0 + i : __ldcg(p.pool_dst + tile.row0 + i);
+        else if (!kFused) dv[cc] = shared ? tile.row0 + i : (kStaged ? p.pool_dst[tile.row0 + i] : __ldcg(p.pool_dst + tile.row0 + i));
         else if (shared) dv[cc] = static_cast<int>((32u << kOutSlotShift) | static_cast<uint32_t>(tile.row0 + i));
         else {
           const int r = __ldcg(p.pool_dst + tile.row0 + i);      // receive-order row
@@ -1218,8 +1220,9 @@ __global__ void __launch_bounds__(both_threads(kStaged), 1) moe_kernel(const __g
   const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);
   const PlanView pv = plan_view(const_cast<char*>(p.plan), p.e_local, p.num_ranks);
   chain_release();
-  if (p.behind_pairs && !chain_opened(pv.pairs_open)) chain_wait();
-  if (p.behind_pairs && p.shared_tiles.parts == 0 && pv.hdr->num_small_tiles == 0) {      // every expert ran on the pairs in front
+  const bool behind_pairs = !kStaged && p.behind_pairs != 0;
+  if (behind_pairs && !chain_opened(pv.pairs_open)) chain_wait();
+  if (behind_pairs && p.shared_tiles.parts == 0 && pv.hdr->num_small_tiles == 0) {      // every expert ran on the pairs in front
     chain_wait();
     return;
   }
@@ -1236,7 +1239,7 @@ __global__ void __launch_bounds__(both_threads(kStaged), 1) moe_kernel(const __g
     prefetch_map(&p.map_w_shared);
   }
   const bool route_here = kStaged && p.route_here, plan_ready = !p.early && !route_here;
-  if ((!p.early || route_here) && !p.behind_pairs) chain_wait();
+  if ((!p.early || route_here) && !behind_pairs) chain_wait();
   if (plan_ready) queue.load_plan();
   int rows = sa_tile_rows(p);
   tc_fence_before();
