@@ -42,10 +42,6 @@ bool chained() { return g_chain_scope; }
 // scale word.  HBM-bound: 3840 x 5120 (60 MB) took 30 us with one division per vector and single-value conversions.
 // =====================================================================================================================
 constexpr int kStageSegVec = 128;
-// Calls of at most so many tokens wait for the code (see opaque()) as much as for memory: theirs is rolled, in 32-bit arithmetic, a third
-// of the length.  With the narrow combine, which is the other half of it: one token 39.05 -> 38.8 us, seven 133.1 -> 131.8.  In the registers
-// of the rolled form (44) the staging of 1021 tokens lets the placement's blocks start so early that they crowd some SMs: 463 -> 471.
-constexpr int kFewTokens = 64;
 
 __device__ __forceinline__ void stage_vector(const uint4& raw, uint2* __restrict__ q_out, uint32_t* word_out) {
   const __nv_bfloat162* p = reinterpret_cast<const __nv_bfloat162*>(&raw);
@@ -127,8 +123,9 @@ __device__ void route_token(const RouterArgs& r, int64_t t, int k, bool is_pad, 
   }
 }
 
-template <bool kFew>
-__global__ void __launch_bounds__(256, kFew ? 1 : 3) stage_kernel(
+// Four blocks to an SM (53 registers): with five (48) the blocks of the placement behind it start so early that they crowd some SMs, 1021 tokens
+// skewed 481 -> 488 us.
+__global__ void __launch_bounds__(256, 1) stage_kernel(
     const uint4* __restrict__ hidden, uint2* __restrict__ x_q, int32_t* __restrict__ x_sf,
     int32_t* __restrict__ shared_sf, int64_t shared_rows, int shared_bm,
     const void* __restrict__ ids_in, int ids64, const float* __restrict__ w_in, const uint8_t* __restrict__ pad,
@@ -148,7 +145,7 @@ __global__ void __launch_bounds__(256, kFew ? 1 : 3) stage_kernel(
     // row of token t in the BLOCK_M-dependent shared-expert scale layout (backend/staging.py:85-95)
     const int mm = shared_bm > 0 ? t % shared_bm : 0;
     const int64_t shared_row = shared_bm > 0 ? (int64_t)(t / shared_bm) * ((shared_bm + 127) / 128 * 128) + (mm / 128) * 128 + (mm % 32) * 4 + (mm % 128) / 32 : 0;
-#pragma unroll (kFew ? 1 : 4)
+#pragma unroll 1          // a third of the code, which lies in DRAM when a call begins: one token 38.7 -> 38.4 us, 2 to 3840 tokens the same
     for (int v = v0; v < v0 + 128 && v < vec_per_row; v += 32) {      // rows are whole multiples of 32 vectors: a warp is in or out together
       uint2 q;
       uint32_t word;
@@ -191,7 +188,7 @@ cudaError_t launch_route_stage(const Ctx& c, const void* hidden, const void* ids
   int blocks = static_cast<int>(std::min<int64_t>((segs + 7) / 8, 148 * 8));
   if (blocks < 1) blocks = 1;
   const RouterArgs router{logits, num_logical, replica_count, replica_slots, max_copies};
-  return launch_chained(m <= kFewTokens ? stage_kernel<true> : stage_kernel<false>, dim3(blocks), dim3(256), 0, s, static_cast<const uint4*>(hidden),
+  return launch_chained(stage_kernel, dim3(blocks), dim3(256), 0, s, static_cast<const uint4*>(hidden),
       c.at<uint2>(c.lay.x), c.at<int32_t>(c.lay.x_sf), c.at<int32_t>(c.lay.shared_x_sf), c.lay.shared_sf_rows, c.geo.num_shared_experts > 0 ? shared_bm : 0, ids, ids64, w,
       pad, c.at<int64_t>(c.lay.topk_idx), c.at<float>(c.lay.topk_weights), m, h, c.geo.num_topk, router);
 }
@@ -1122,8 +1119,10 @@ __device__ __forceinline__ __nv_bfloat162 add_residual(__nv_bfloat162 o, __nv_bf
   return __floats2bfloat162_rn(__fadd_rn(a.x, b.x), __fadd_rn(a.y, b.y));
 }
 
-// Calls of at most kNarrowTokens tokens, where latency and code on its way from DRAM are all there is to wait for (see kFewTokens): two
-// outputs per thread, a quarter of the instructions.  Past that the rows are enough to be worth 16 bytes a load.
+// Calls of at most kNarrowTokens tokens, where latency and code on its way from DRAM are all there is to wait for: two outputs per
+// thread, a quarter of the instructions.  Wide and narrow: 1 token 38.1 and 38.4 us, 2 54.0 and 53.4, 4 84.3 and 84.4, 8 149.0 and 148.7, 16 of 32
+// experts 102.7 and 102.4; past the line 17 108.2 and 107.9, 48 118.1 and 117.5, 64 119.9 and 119.6, 128 130.9 and 130.5, within 0.5 us of
+// each other: little hangs on where it lies.
 constexpr int kNarrowTokens = 16;
 __global__ void __launch_bounds__(256) combine_narrow_kernel(
     const uint32_t* __restrict__ rows, const int32_t* __restrict__ route_pos, const uint32_t* __restrict__ shared_out,
