@@ -125,7 +125,7 @@ struct PlanHeader {
   int32_t routed;              // 1 once a GEMM launch that orders the routes itself has the plan complete; zero between calls
   uint32_t claims;             // CTAs of that launch that have asked to do it, modulo its grid: zero between launches
   uint32_t next_task;          // tasks of a launch of both GEMMs that have been claimed: zero between calls
-  int32_t layer1_done;         // sum of `done` below: zero between calls
+  int32_t layer1_done;         // finished parts of GEMM1 of a launch of both GEMMs, all experts (not those on CTA pairs): zero between calls
   int32_t shared_step;         // rows of the shared expert's tiles ...
   int32_t shared_pairs;        // ... and 1 if they run on CTA pairs (neither is written where the launch orders the routes itself)
 };

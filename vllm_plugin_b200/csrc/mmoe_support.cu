@@ -760,9 +760,9 @@ __device__ void write_single_rank_plan(const RouteArgs& r, const PlanView& pv, i
 // Calls of at most kSmallRoutes routes: ONE launch.  Every block ranks the routes and builds the plan for itself in shared memory
 // (2-3 us, less than a second launch behind a grid-wide hand-over), block 0 writes it out, and the others place the
 // routes, one warp per route (block 0 with its share of them came in 0.5-1 us late).  The shared expert's scales are not placed: its GEMM1 gathers them itself.
-// The ranking and the plan are a chain of barriers in code that lies in DRAM.  Walking it once on masked routes in front of the wait saved 0.6 us of
-// calls in a row (128 tokens of 32 experts 131.2 -> 130.6) and cost 2.1 where the staging had ended already, as it has in every call
-// that finds the GPU idle (141.9 -> 144.0 from event to event; 32 tokens 129.6 -> 134.2).
+// The ranking and the plan are a chain of barriers in code that lies in DRAM.  Walking it once on masked routes in front of the wait saved 0 to 1 us
+// of calls in a row (128 tokens of 32 experts 132.1 -> 131.7, 32 tokens 113.3 -> 112.8) and cost 1 to 2 where the staging had ended
+// already, as it has in every call that finds the GPU idle (142.3 -> 143.6 from event to event, 131.0 -> 132.2).
 __global__ void __launch_bounds__(kRouteThreads) route_small_kernel(const RouteArgs r) {
   chain_wait();
   chain_release();       // in this order: the GEMM1 launch starts knowing that the staging has completed

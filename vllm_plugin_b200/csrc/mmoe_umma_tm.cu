@@ -102,8 +102,9 @@ __device__ __forceinline__ uint32_t map_to_cta(uint32_t addr, uint32_t rank) {
 }
 // Arrival on the barrier that hands columns of tensor memory back, in either CTA of the pair: ordered by the tcgen05 fences on
 // either side, and no memory access rides on it (the queue of tasks has arrivals of its own).  So the default release, of CTA scope, is enough: one of cluster scope first waits for
-// this warp's outstanding stores to global memory, which stood between every two tasks of the issuer (3840 tokens of 48 experts 970 ->
-// 942 us, 2560 of 16 387 -> 381; GEMM2, whose epilogue stores most, 294 -> 275).
+// this warp's outstanding stores to global memory, which stood between every two tasks of the issuer.  Cluster scope -> CTA scope, one card: 3840
+// tokens of 48 experts 930 -> 908 us repeated for seconds (at the power limit), 819 -> 800 in bursts of 30 calls; 2560 of 16 376 -> 369 and
+// 333 -> 326, 3001 of 96 skewed 884 -> 870 and 778 -> 765, 1021 of 384 skewed 456 -> 451 and 410 -> 405.
 __device__ __forceinline__ void mbar_arrive_pair(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
@@ -190,8 +191,10 @@ struct PairPort {
 // the shared expert this way.
 // Either dealt out beforehand, or (both layers of a single-GPU call) claimed from a counter by the leader's scheduler: SMs come free
 // one by one, over 25 us behind the placement and 50 behind GEMM1, and a pair that starts late takes fewer tasks.  GEMM2 then starts
-// where GEMM1 has ended and waits expert by expert for its counted parts, not for its last CTA.  3840 tokens of 48 experts, 30 calls in
-// a row: GEMM1's CTAs end over 52 -> 18 us, the call 966 -> 920; at the power limit 965 -> 959, 2560 of 16 381 -> 379.
+// where GEMM1 has ended and waits expert by expert for its counted parts, not for its last CTA.  Dealt out with GEMM2 behind all of GEMM1 ->
+// claimed so -> GEMM2 behind counted parts as well, the same card and conditions: 3840 tokens of 48 experts 917 -> 914 -> 908 us repeated, 804 -> 803
+// -> 800 in bursts; 2560 of 16 371 -> 372 -> 369 and 327 -> 328 -> 326; 1021 skewed 455 -> 456 -> 451 and 409 -> 410 -> 405; 3001 skewed 868 -> 867 -> 870 and 766 ->
+// 767 -> 764.  So claiming alone gives nothing, both together up to 1 %; other sizes lie within 0.4 % on either side.
 struct PairWalk {
   const TmParams& p;
   TmControl* ctl;
